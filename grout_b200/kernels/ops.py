@@ -2650,3 +2650,20 @@ def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor,
         logits.data_ptr(), n, logits.shape[1], temperature.data_ptr(), top_k.data_ptr(),
         top_p.data_ptr(), u.data_ptr(), out.data_ptr(), _stream()), "sample")
     return out
+
+
+@_profiled("sample", lambda out, logits, *a: (_nbytes(logits), 0))
+def sample_host(logits: torch.Tensor, temperature, top_k, top_p, u) -> torch.Tensor:
+    """``sample`` with what the rows ask for as NumPy arrays (float32, int32, float32, float32):
+    they travel with the launch, so nothing is copied to the device and nothing waits."""
+    _need(logits, "logits", torch.float32, 2)
+    n = logits.shape[0]
+    for t, nm, dt in ((temperature, "temperature", "float32"), (top_k, "top_k", "int32"),
+                      (top_p, "top_p", "float32"), (u, "u", "float32")):
+        if t.shape != (n,) or t.dtype != dt or not t.flags.c_contiguous:
+            raise KernelError(f"{nm} must be {n} contiguous {dt} values, found {t.dtype} {t.shape}")
+    out = torch.empty((n,), dtype=torch.int32, device=logits.device)
+    _check(_fn("sample", "gb_sample_host_f32", "piipppppp")(
+        logits.data_ptr(), n, logits.shape[1], temperature.ctypes.data, top_k.ctypes.data, top_p.ctypes.data,
+        u.ctypes.data, out.data_ptr(), _stream()), "sample")
+    return out

@@ -28,11 +28,9 @@ class DeviceSampler:
             raise ValueError("one SamplingParams and one draw per row of logits are needed")
         if all(p.greedy for p in params):
             return ops.argmax(logits)
-        host = np.zeros((4, n), dtype=np.float32)
-        for i, p in enumerate(params):
-            host[0, i] = 0.0 if p.greedy else p.temperature
-            host[1, i] = np.int32(p.top_k).view(np.float32)
-            host[2, i] = p.top_p
-            host[3, i] = draws[i]
-        dev = torch.from_numpy(host).to(self.device)
-        return ops.sample(logits, dev[0], dev[1].view(torch.int32), dev[2], dev[3])
+        # what the rows ask for travels with the launch: a copy to the device would wait for
+        # everything queued in front of it
+        return ops.sample_host(
+            logits, np.array([0.0 if p.greedy else p.temperature for p in params], dtype=np.float32),
+            np.array([p.top_k for p in params], dtype=np.int32),
+            np.array([p.top_p for p in params], dtype=np.float32), np.array(draws, dtype=np.float32))

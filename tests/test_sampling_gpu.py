@@ -84,3 +84,62 @@ def test_host_sampler_agrees_with_plain():
         want = plain_sampling.sample_next(row.tolist(), t, k, p, u)
         got = choose_one(row.numpy(), SamplingParams(True, t, k, p).normalised(), u)
         assert got == want, (t, k, p)
+
+
+def _rows_for_thresholds(V, g):
+    """Rows on which a threshold falls in every way: among distinct scores, among more equal
+    scores than are ranked directly, in a range stretched by far outliers, beside masked
+    scores, and with a NaN that top-k leaves out."""
+    normal = torch.randn(V, generator=g) * 2.0
+    rows = {"normal": normal, "equal": torch.full((V,), 0.75), "two values": (normal > 0).float(),
+            "outliers": normal.clone(), "masked": torch.where(normal > 1.0, normal, torch.tensor(float("-inf"))),
+            "flat": 1.0 + 1e-3 * torch.rand(V, generator=g)}
+    rows["outliers"][0], rows["outliers"][V // 2] = -3.0e4, 60.0
+    rows["masked"][V - 1] = 0.5                    # at least one score is there
+    return rows
+
+
+# around the cluster kernel's shares of a row (eight blocks of sixteen warps), a whole
+# vocabulary, and the first length that takes the one-block kernel
+@pytest.mark.parametrize("V", [1, 7, 8, 9, 127, 129, 4095, 33000, 400001])
+def test_sample_thresholds_of_every_kind(V):
+    rng = random.Random(V)
+    g = torch.Generator().manual_seed(V)
+    asked = [(1.0, 0, 1.0), (0.7, 20, 0.9), (0.8, 0, 0.95), (1.0, 1500, 1.0), (1.0, V - 1, 0.5), (50.0, 3, 0.7)]
+    if V > 40000:
+        asked = asked[1:3]
+    rows, prm = [], []
+    for name, row in _rows_for_thresholds(V, g).items():
+        for t, k, p in asked:
+            rows.append(row)
+            prm.append((t, max(k, 0), p, rng.random()))
+    logits = torch.stack(rows).to(DEV)
+    t, k, p, u = zip(*prm)
+    args = [torch.tensor(x, dtype=d) for x, d in ((t, torch.float32), (k, torch.int32), (p, torch.float32), (u, torch.float32))]
+    got = _ops().sample(logits, *(a.to(DEV) for a in args)).cpu().tolist()
+    assert got == _ops().sample_host(logits, *(a.numpy() for a in args)).cpu().tolist()
+    for i, row in enumerate(rows):
+        # scaled as the kernel scales, in 32 bits: two scores that this makes equal are a tie
+        scaled = (row * (1.0 / args[0][i])).tolist()
+        u = args[3][i].item()
+        # masses are 32-bit exponentials (2^-22 off) against 64-bit ones here: a draw that close
+        # to an element's edge may fall on either side of it
+        near = {plain_sampling.sample_next(scaled, 1.0, *prm[i][1:3], min(max(u + d, 0.0), 1.0 - 2.0 ** -24))
+                for d in (-2.0 ** -21, 0.0, 2.0 ** -21)}
+        assert got[i] in near, (i, prm[i], got[i], near)
+
+
+def test_sample_with_nan_and_without_a_finite_maximum():
+    nan, inf = float("nan"), float("inf")
+    rows = torch.randn(5, 300, generator=torch.Generator().manual_seed(8))
+    rows[0, 7] = nan                               # left out by top-k
+    rows[1, 7] = nan                               # in the kept set: the sum is void, the maximum is taken
+    rows[2, 250] = inf
+    rows[3] = -inf
+    rows[4] = nan
+    k = torch.tensor([5, 0, 0, 0, 0], dtype=torch.int32)
+    got = _ops().sample(rows.to(DEV), torch.ones(5, device=DEV), k.to(DEV), torch.ones(5, device=DEV),
+                        torch.full((5,), 0.5, device=DEV)).cpu().tolist()
+    finite = [v if v == v else -inf for v in rows[0].tolist()]
+    assert got[0] in sorted(range(300), key=lambda i: -finite[i])[:5]
+    assert got[1:] == [plain_sampling.argmax_first([v if v == v else -inf for v in rows[1].tolist()]), 250, 0, 0]
