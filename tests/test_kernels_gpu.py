@@ -279,6 +279,36 @@ def test_gemm_f32(M, N, K):
     assert torch.allclose(got.double(), want, atol=1e-5 * math.sqrt(K), rtol=1e-5)
 
 
+def _gemm_f32_in_order(a, w):
+    """The documented order of sums, exactly: multiply-adds (one rounding each, here through 64 bits, in which a
+    product of two 32-bit numbers is exact) over 32 k, 32 such sums in turn, those in turn."""
+    K = a.shape[1]
+    total = torch.zeros(a.shape[0], w.shape[0])
+    for c in range(0, K, 1024):
+        mid = torch.zeros_like(total)
+        for s in range(c, min(K, c + 1024), 32):
+            acc = torch.zeros_like(total)
+            for k in range(s, min(K, s + 32)):
+                acc = (acc.double() + torch.outer(a[:, k].double(), w[:, k].double())).float()
+            mid = mid + acc
+        total = total + mid
+    return total
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2, 3, 4])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (1, 9, 1024), (2, 17, 1028), (3, 33, 2050), (8, 40, 3104), (9, 65, 33),
+                                   (33, 66, 1056), (65, 130, 2052), (5, 129, 9001)])
+def test_gemm_f32_sums_in_one_order(M, N, K, kind):
+    """Every kernel adds in the documented order, whatever the tile, the split and the alignment of the rows.  (The
+    check rounds a multiply-add twice, to 64 and then to 32 bits; the few outputs where that differs are off by one
+    rounding of one of K / 32 sums.)"""
+    a, w = _rand((M, K), torch.float32, 26), _rand((N, K), torch.float32, 27)
+    got = _ops().gemm_f32(a.to(DEV), w.to(DEV), kind=kind).cpu()
+    want = _gemm_f32_in_order(a, w)
+    assert (got != want).float().mean() < 1e-4 * K / 32 + 1e-9
+    assert torch.allclose(got, want, atol=2e-6 * math.sqrt(K), rtol=1e-6)
+
+
 def test_gemm_f32_row_independent():
     """A row's result does not depend on the rows beside it (bitwise)."""
     a, w = _rand((70, 96), torch.float32, 22), _rand((50, 96), torch.float32, 23)
