@@ -782,6 +782,66 @@ def attn_generic(q, k_pages, v_pages, block_table, *, token_seq, token_pos, slot
     return out
 
 
+class _AttnF32Args(ctypes.Structure):
+    _fields_ = [("q", _P), ("k_pages", _P), ("v_pages", _P), ("block_table", _P), ("cu_q", _P), ("slots", _P),
+                ("kv_len", _P), ("out", _P), ("parts", _P), ("sinks", _P), ("n_seqs", _I), ("nq", _I), ("nkv", _I),
+                ("D", _I), ("page", _I), ("max_pages", _I), ("window", _I), ("chunk", _I), ("heads", _I),
+                ("n_qblocks", _I), ("n_parts", _I), ("page_shift", _I), ("scale", _F), ("softcap", _F)]
+
+
+ATTN_F32_TILE = 64       # keys of a tile of attn_f32
+ATTN_F32_ROWS = 32       # query rows (tokens x heads) of a prompt's block
+
+
+def attn_f32_heads(nq: int, nkv: int) -> int:
+    """Query heads of a block of ``attn_f32``: the largest divisor, up to 8, of those that share a kv head."""
+    return max(h for h in range(1, 9) if (nq // nkv) % h == 0)
+
+
+def attn_f32_takes(q, nkv: int, step) -> bool:
+    """Head sizes that are multiples of 4 up to 128, on 16-byte boundaries, and steps whose blocks fit a grid;
+    everything else is the plain kernel's."""
+    T, nq, D = q.shape
+    if D % 4 or D > 128 or q.data_ptr() % 16:
+        return False
+    if step.decode:
+        return step.n_seqs * -(-step.max_kv_len // ATTN_F32_TILE) <= 65535 and nq <= 65535
+    return step.q_blocks(ATTN_F32_ROWS // attn_f32_heads(nq, nkv)) <= 65535
+
+
+@_profiled("attn_generic", lambda out, q, *a, **k: (_nbytes(q, out), 0))
+def attn_f32(q, k_pages, v_pages, block_table, *, step, page: int, scale: float, window: Optional[int] = None,
+             softcap: Optional[float] = None, sinks: Optional[torch.Tensor] = None, chunk: int = 0) -> torch.Tensor:
+    """The 32-bit attention of a step's queries (``attention`` says what the options mean)."""
+    T, nq, nkv, D = _attn_common(q, k_pages, v_pages, block_table, step.token_seq, step.token_pos, step.slots, page)
+    _need(q, "q", torch.float32, 3)
+    _check_sinks(sinks, nq)
+    for t, nm in ((step.cu_q, "cu_q"), (step.kv_len, "kv_len")):
+        _need(t, nm, torch.int32, 1)
+    n_seqs = step.slots.shape[0]
+    if step.cu_q.shape[0] != n_seqs + 1 or step.kv_len.shape[0] != n_seqs:
+        raise KernelError("cu_q, slots and kv_len do not describe one list of sequences")
+    out = torch.empty_like(q)
+    a = _AttnF32Args()
+    a.q, a.k_pages, a.v_pages, a.block_table = q.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), block_table.data_ptr()
+    a.cu_q, a.slots, a.kv_len, a.out, a.sinks = (step.cu_q.data_ptr(), step.slots.data_ptr(), step.kv_len.data_ptr(),
+                                                 out.data_ptr(), _ptr(sinks))
+    a.n_seqs, a.nq, a.nkv, a.D, a.page, a.max_pages = n_seqs, nq, nkv, D, page, block_table.shape[1]
+    a.window, a.chunk, a.heads = int(window or 0), _chunk_arg(chunk, 0), attn_f32_heads(nq, nkv)
+    a.page_shift = page.bit_length() - 1 if page & (page - 1) == 0 else -1
+    a.scale, a.softcap = float(scale), float(softcap or 0.0)
+    a.n_qblocks = 0 if step.decode else step.q_blocks(ATTN_F32_ROWS // a.heads)
+    a.n_parts, parts = 1, None
+    if step.decode:
+        a.n_parts = -(-step.max_kv_len // ATTN_F32_TILE)
+        parts = torch.empty((n_seqs, nq, a.n_parts, D + 2), dtype=torch.float32, device=q.device)
+        a.parts = parts.data_ptr()
+    with torch.cuda.device(q.device):
+        _check(_fn("attn_f32", "gb_attn_f32", "pip")(ctypes.addressof(a), int(step.decode), _stream()), "attn_f32",
+               1 + bool(step.decode))
+    return out
+
+
 # ---------------------------------------------------------------- matrix products
 def _result(shape, dtype, device, into: Optional[torch.Tensor]) -> torch.Tensor:
     """A new tensor, or the caller's (contiguous, of that shape and type)."""
@@ -1639,8 +1699,8 @@ def attention(q, k_pages, v_pages, block_table, *, step, page: int, scale: float
               sinks: Optional[torch.Tensor] = None, keep_first: int = 0,
                     chunk: int = 0) -> torch.Tensor:
     """Attention of the step's queries over their sequences' cached keys.
-    32-bit tensors take the plain 32-bit kernel; bfloat16 takes the tensor-core
-    kernels where they accept the shape and the plain kernel elsewhere.
+    32-bit tensors take the 32-bit kernel (``attn_f32``), bfloat16 the tensor-core
+    kernels, where they accept the shape, and the plain kernel elsewhere.
     ``softcap`` c: scores become c * tanh(score / c); ``sinks`` [nq] float32: one
     more term exp(sinks[h]) in the denominator of query head h; ``keep_first`` F: with a
     window, key j < F stays visible to every later query (at its own position); ``chunk`` C: a
@@ -1671,6 +1731,9 @@ def attention(q, k_pages, v_pages, block_table, *, step, page: int, scale: float
         return attn_prefill_bf16(q, k_pages, v_pages, block_table, cu_q=step.cu_q,
                                  slots=step.slots, kv_len=step.kv_len, q_lens=step.q_lens,
                                  page=page, scale=scale, window=window, **extra)
+    if q.dtype == torch.float32 and not keep_first and attn_f32_takes(q, k_pages.shape[1], step):
+        return attn_f32(q, k_pages, v_pages, block_table, step=step, page=page, scale=scale, window=window,
+                        softcap=softcap, sinks=sinks, chunk=chunk)
     return attn_generic(q, k_pages, v_pages, block_table, token_seq=step.token_seq,
                         token_pos=step.token_pos, slots=step.slots, page=page, scale=scale,
                         window=window, **extra)

@@ -229,6 +229,8 @@ class GQAAttention(Mixer):
             mods += ("elementwise",)
         if self.ctx.dtype == torch.bfloat16:
             mods += ops.fast_attention_modules(self.Ds, self.nq, self.nkv)
+        else:
+            mods += ("attn_f32",)
         return mods
 
     def cache_spec(self):
@@ -409,6 +411,8 @@ class DifferentialAttention(Mixer):
         mods = ("qk_prepare", "attn_generic", "diff_heads") + self.qkv.kernel_modules() + self.o.kernel_modules()
         if self.ctx.dtype == torch.bfloat16:
             mods += ops.fast_attention_modules(self.Ds, 2 * self.H, self.G)
+        else:
+            mods += ("attn_f32",)
         return mods
 
     def cache_spec(self):
@@ -621,6 +625,8 @@ class LatentAttention(Mixer):
         mods += self.uq.kernel_modules() if self.uq else ()
         if self.ctx.dtype == torch.bfloat16:
             mods += ops.fast_attention_modules(self.Ds, min(self.H, self.GROUP), 1)
+        else:
+            mods += ("attn_f32",)
         return mods
 
     def cache_spec(self):

@@ -271,6 +271,76 @@ def test_qk_prepare_skips_padding_rows():
     assert torch.equal(kp.view(torch.int16), before)
 
 
+def _f32_step(lens, starts, pc, decode, bound=None):
+    """What attn_f32 reads of a step in which sequence i brings its rows starts[i] .. lens[i]."""
+    from types import SimpleNamespace
+    q_lens = [n - s for n, s in zip(lens, starts)]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    rows = [(i, p) for i, (n, s) in enumerate(zip(lens, starts)) for p in range(s, n)]
+    return SimpleNamespace(
+        cu_q=i32([0] + torch.tensor(q_lens).cumsum(0).tolist()), kv_len=i32(lens), n_seqs=len(lens), decode=decode,
+        slots=i32([pc.slot_of[i] for i in range(len(lens))]), token_seq=i32([r[0] for r in rows]),
+        token_pos=i32([r[1] for r in rows]), max_kv_len=bound or max(lens),
+        q_blocks=lambda n: sum((x + n - 1) // n for x in q_lens) + (0 if decode else 2))
+
+
+@pytest.mark.parametrize("nq,nkv,D,page,window,chunk,cap,with_sinks", [
+    (4, 2, 128, 64, None, 0, None, False), (3, 3, 4, 64, None, 0, 20.0, True), (12, 1, 64, 16, 70, 0, None, True),
+    (16, 1, 100, 48, None, 0, None, False), (10, 2, 60, 32, 600, 0, 30.0, False), (6, 2, 128, 64, None, 130, None, True)])
+def test_attn_f32(nq, nkv, D, page, window, chunk, cap, with_sinks):
+    """Against 64 bits, and the same bits for a prompt in one step, in pieces and as decode steps: lengths around the
+    edges of a tile (64) and a block's tokens; what lies in the pages behind a sequence is NaN."""
+    lens = [1, 63, 130, 513, 1100]
+    pc = Paged(lens, nkv, D, torch.float32, 17, page=page)
+    g = torch.Generator().manual_seed(18)
+    qs = [torch.randn((n, nq, D), generator=g) for n in lens]
+    sinks = torch.randn((nq,), generator=g) if with_sinks else None
+    scale = D ** -0.5
+    kw = dict(page=page, scale=scale, window=window, softcap=cap, chunk=chunk,
+              sinks=sinks.to(DEV) if with_sinks else None)
+    pages = pc.k_pages.to(DEV), pc.v_pages.to(DEV), pc.table.to(DEV)
+
+    def run(ends, starts, decode, bound=None):
+        step = _f32_step(ends, starts, pc, decode, bound)
+        q = torch.cat([x[s:n] for x, s, n in zip(qs, starts, ends)]).to(DEV)
+        assert _ops().attn_f32_takes(q, nkv, step)
+        return torch.split(_ops().attn_f32(q, *pages, step=step, **kw).cpu(), [n - s for n, s in zip(ends, starts)])
+
+    whole = run(lens, [0] * len(lens), False)
+    for x, q, k, v in zip(whole, qs, pc.k, pc.v):
+        for pos in sorted({0, len(q) // 2, len(q) - 1, min(len(q) - 1, 64), min(len(q) - 1, 512)}):
+            lo = max(0, pos - window + 1) if window else pos - pos % chunk if chunk else 0
+            kh, vh = (t[lo:pos + 1].double().repeat_interleave(nq // nkv, 1) for t in (k, v))
+            s = torch.einsum("hd,thd->ht", q[pos].double(), kh) * scale
+            s = cap * torch.tanh(s / cap) if cap else s
+            s = torch.cat([s, sinks.double()[:, None]], 1) if with_sinks else s
+            want = torch.einsum("ht,thd->hd", torch.softmax(s, 1)[:, :pos + 1 - lo], vh)
+            # 32-bit rounding of scores of order one (and of the sums): a few 1e-7 of values of order one
+            assert (x[pos].double() - want).abs().max() < 4e-6
+    cut = [n * 2 // 3 for n in lens]
+    for a, b, c in zip(whole, cut, run(lens, cut, False)):
+        assert torch.equal(a[b:], c)
+    for bound in (None, 512 * 5):
+        last = run(lens, [n - 1 for n in lens], True, bound)
+        for a, c in zip(whole, last):
+            assert torch.equal(a[-1:], c)
+
+
+def test_attn_f32_unseen_values_do_not_count():
+    """A later key of the same tile whose value is infinite leaves the rows in front of it alone; a padding sequence
+    gives zeros."""
+    nq, nkv, D, n = 2, 1, 32, 40
+    pc = Paged([n], nkv, D, torch.float32, 19)
+    pc.store(0, 30, torch.full((nkv, D), 1.0), torch.full((nkv, D), float("inf")))
+    q = torch.randn((n, nq, D), generator=torch.Generator().manual_seed(20)).to(DEV)
+    step = _f32_step([n], [0], pc, False)
+    pages = pc.k_pages.to(DEV), pc.v_pages.to(DEV), pc.table.to(DEV)
+    got = _ops().attn_f32(q, *pages, step=step, page=64, scale=0.2).cpu()
+    assert torch.isfinite(got[:30]).all() and not torch.isfinite(got[30:]).any()
+    step.slots[0] = -1
+    assert not _ops().attn_f32(q, *pages, step=step, page=64, scale=0.2).any()
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 130, 100), (70, 65, 17), (129, 200, 333)])
 def test_gemm_f32(M, N, K):
     a, w = _rand((M, K), torch.float32, 20), _rand((N, K), torch.float32, 21)
