@@ -27,7 +27,7 @@ from ..weights import DictSource, FolderSource, load_params, random_tensor
 from ..sampling import DeviceSampler, HostSampler, SamplingParams
 from .batch import make_context
 from .generate import GenerationLoop, GenerationOutput, Request
-from .graphs import StepGraphs
+from .graphs import PROMPT_TOKENS_F32, PROMPT_TOKENS_MOST, StepGraphs
 from .model import Model
 from .profile import StepProfile
 
@@ -67,8 +67,9 @@ class Engine:
         self.cache = SequenceCache(model.cache_layout(), max_tokens=max_tokens,
                                    max_slots=max_batch, max_seq_len=self.max_seq_len,
                                    dtype=dtype, device=device)
-        self.use_graphs = (dtype == torch.bfloat16) if use_graphs is None else bool(use_graphs)
-        self.graphs = StepGraphs(model, self.cache, device)
+        self.use_graphs = True if use_graphs is None else bool(use_graphs)
+        self.graphs = StepGraphs(model, self.cache, device,
+                                 prompt_tokens=PROMPT_TOKENS_MOST if dtype == torch.bfloat16 else PROMPT_TOKENS_F32)
         self.vocab_size = plan.vocab_size
         self.max_batch = self.cache.max_slots
         self.profile: Optional[StepProfile] = None

@@ -32,6 +32,9 @@ import torch
 from .batch import context_from, layout_sizes, pack_step_padded
 
 PROMPT_TOKENS_MOST = 1024       # longer prompt steps are bound by the device, not by launches
+# In 32-bit the products are bound by their multiply-adds from some 64 rows on, and filling a step up to a power of two
+# costs what its rows cost: 128 rows take 4 ms on the device (1B sizes), a step's launches 2 ms of the host.
+PROMPT_TOKENS_F32 = 128
 PROMPT_SEQS_MOST = 64
 PROMPT_TOKENS_LEAST = 16
 PROMPT_GRAPHS_MOST = 48         # captured prompt shapes kept; further shapes run launch by launch
@@ -55,11 +58,12 @@ def length_bucket(n: int, most: int, least: int = LENGTH_LEAST) -> int:
     return min(b, most)
 
 
-def prompt_bucket(n_tokens: int, n_seqs: int, n_want: int) -> Optional[Tuple[int, int, int]]:
+def prompt_bucket(n_tokens: int, n_seqs: int, n_want: int,
+                  most: int = PROMPT_TOKENS_MOST) -> Optional[Tuple[int, int, int]]:
     """(tokens, sequences, wanted rows) of the graph a prompt step runs in, or None
     when it is too large for one.  A step whose rows do not fill the bucket needs
     one sequence more, for the padding rows."""
-    tb = bucket_for(n_tokens, PROMPT_TOKENS_MOST)
+    tb = bucket_for(n_tokens, most)
     if not tb:
         return None
     tb = max(tb, PROMPT_TOKENS_LEAST)
@@ -220,8 +224,9 @@ class StepGraphs:
     memory pool: they run one after the other on one stream and keep nothing
     between replays but their logits, which stay allocated."""
 
-    def __init__(self, model, cache, device, largest: int = 256):
+    def __init__(self, model, cache, device, largest: int = 256, prompt_tokens: int = PROMPT_TOKENS_MOST):
         self.model, self.cache, self.device, self.largest = model, cache, device, largest
+        self.prompt_tokens = prompt_tokens
         self.decode_graphs: Dict[Tuple[int, int], DecodeGraph] = {}
         self.prompt_graphs: Dict[Tuple[int, int, int], PromptGraph] = {}
         self._prompt_logits_bytes = 0
@@ -252,7 +257,7 @@ class StepGraphs:
         have been captured already."""
         if self._prompts_ok is None:
             self._prompts_ok = bool(self.model.captures_prompts())
-        key = prompt_bucket(n_tokens, n_seqs, n_want) if self._prompts_ok else None
+        key = prompt_bucket(n_tokens, n_seqs, n_want, self.prompt_tokens) if self._prompts_ok else None
         if key is None:
             return None
         g = self.prompt_graphs.get(key)
