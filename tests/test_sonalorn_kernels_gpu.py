@@ -67,6 +67,19 @@ def test_stream_sum_through_norm_and_scale(dtype, N):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N,S", [(4, 1), (1001, 2), (4096, 5), (4100, 9), (8196, 3), (16384, 4), (16388, 2)])
+def test_stream_sum_at_the_widths_where_its_kernel_changes(N, S, dtype):
+    from grout_b200.kernels import ops
+    res, parts = rnd(3, N, seed=1), rnd(S, 3, N, seed=2)
+    pw, w = 1 + rnd(N, seed=3, scale=0.2), 1 + rnd(N, seed=4, scale=0.2)
+    want = res.double() + plain.rms_norm(parts.double().sum(0), pw, 1e-5)
+    r, y = ops.add_postnorm(res.to(DEV), parts.to(DEV), dtype=dtype, post_weight=pw.to(DEV), post_eps=1e-5,
+                            weight=w.to(DEV), eps=1e-6)
+    close(r, want, torch.float32, "stream")
+    close(y, plain.rms_norm(want, w, 1e-6), dtype, "its norm")
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_embedding_with_positions(dtype):
     from grout_b200.kernels import ops
     V, P, H = 37, 50, 72
