@@ -93,15 +93,11 @@ attn_f32_prompt_kernel(AttnF32Args a) {
   pdl_wait();
 
   // the block's sequence and its tokens
-  int seq, b = a.n_qblocks - 1 - blockIdx.y;    // heavy blocks first
-  const int per = ROWS / a.heads;
-  for (seq = 0; seq < a.n_seqs; ++seq) {
-    const int n = (a.cu_q[seq + 1] - a.cu_q[seq] + per - 1) / per;
-    if (b < n) break;
-    b -= n;
-  }
-  if (seq == a.n_seqs) return;
-  const int q0 = b * per;
+  const int per = ROWS / a.heads, b = a.n_qblocks - 1 - blockIdx.y;    // heavy blocks first
+  int first_block;
+  const int seq = find_query_block(a.cu_q, a.n_seqs, per, b, first_block);
+  if (seq >= a.n_seqs) return;
+  const int q0 = (b - first_block) * per;
   const int tok0 = a.cu_q[seq] + q0, q_len = a.cu_q[seq + 1] - a.cu_q[seq];
   const int tokens = min(per, q_len - q0), rows = tokens * a.heads;
   const int slot = a.slots[seq];

@@ -149,6 +149,32 @@ __device__ __forceinline__ int first_key(int pos, int window, int chunk) {
   return lo;
 }
 
+// Which sequence's query block is block b, when every sequence starts a block of its own and a block takes `per`
+// tokens: the sequence (n_seqs: none) and its first block.  For whole warps (all lanes get the answer): thirty-two
+// sequences at a time, where one after the other cost each block of 64 sequences a few microseconds.
+__device__ __forceinline__ int find_query_block(const int* cu_q, int n_seqs, int per, int b, int& first) {
+  const int lane = threadIdx.x & 31;
+  first = 0;
+  for (int base = 0; base < n_seqs; base += 32) {
+    const int seq = base + lane;
+    const int n = seq < n_seqs ? (cu_q[seq + 1] - cu_q[seq] + per - 1) / per : 0;
+    int sum = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int below = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += below;
+    }
+    const uint32_t beyond = __ballot_sync(0xffffffffu, b < first + sum);
+    if (beyond) {
+      const int at = __ffs(beyond) - 1;
+      first += __shfl_sync(0xffffffffu, sum - n, at);
+      return base + at;
+    }
+    first += __shfl_sync(0xffffffffu, sum, 31);
+  }
+  return n_seqs;
+}
+
 // Address of row `pos` of kv head `h` of a sequence in a paged cache laid out
 // [n_pages, n_kv_heads, page, D]; `table` is the sequence's row of the block table.
 __device__ __forceinline__ size_t paged_row(const int* table, int pos, int h, int nkv, int page,

@@ -1442,20 +1442,39 @@ class _AttnTcArgs(ctypes.Structure):
     _fields_ = [("block_table", _P), ("cu_q", _P), ("slots", _P), ("kv_len", _P), ("out", _P),
                 ("error", _P), ("n_seqs", _I), ("nq", _I), ("nkv", _I), ("max_pages", _I),
                 ("window", _I), ("n_qblocks", _I), ("scale_log2", _F), ("sinks", _P),
-                ("cap_log2", _F), ("cap_inv", _F), ("keep_first", _I), ("chunk", _I)]
+                ("cap_log2", _F), ("cap_inv", _F), ("keep_first", _I), ("chunk", _I), ("pack", _I)]
 
 
 PREFILL_TC_ROWS = 0        # query rows per block of the tcgen05 prefill kernel: 128, 256 or 0 = by size
 
 
-def prefill_tc_rows(blocks_of_256: int, nq: int, device) -> int:
-    """256 rows a block (two query blocks that share their key tiles, one block
-    an SM) unless that leaves most SMs without a block; then 128 (half-size
-    blocks, two an SM).  Measured on 32 heads of 128: 512 tokens 21.8 us with 128
-    rows against 25.7 us with 256; from 1,024 tokens on 256 rows are faster."""
+PREFILL_TC_PACK = 64       # the most query heads whose rows share a block
+
+
+def prefill_tc_pack(nq: int, nkv: int) -> int:
+    """Query heads whose rows can share a block: the largest power of two, up to 64, that divides those sharing a kv head."""
+    g = nq // nkv
+    return min(PREFILL_TC_PACK, g & -g)
+
+
+def prefill_tc_plan(blocks, nq: int, nkv: int, sms: int):
+    """(heads of a block, its query rows).  ``blocks(tokens)``: how many blocks of that many tokens the step makes.
+
+    Blocks of 256 rows are two query blocks that share their key tiles, one block an SM; of 128 rows, half-size ones,
+    two an SM.  Heads are packed into a block where one head a block would make more blocks of 256 than the GPU holds
+    at once, and 256 rows then want an SM's worth of blocks that mostly have a second half.  A step that fits at once
+    ends with its longest block, which packing would only lengthen.  Measured (us; packed 128 / 256 rows, one head 128 /
+    256), 32 heads of 128 on 8: 64 sequences of 17 to 700 tokens 141 / 141, 170 / 189; of 60 tokens 31.6 / 34.4, 46.5 /
+    78.7; 2,048 tokens 54.4 / 46.4, 57.5 / 47.1; 384 tokens 11.0 / 13.8, 11.2 / 10.7.  16 heads on 8, 384 tokens behind
+    768 beside five single ones 27.4 / 24.6, 27.2 / 22.4; 16 prompts of 128 tokens 10.1 / 10.0, 10.4 / 15.2."""
+    whole = blocks(256) * nq
+    pack = prefill_tc_pack(nq, nkv) if 4 * whole > 5 * sms else 1
     if PREFILL_TC_ROWS:
-        return PREFILL_TC_ROWS
-    return 256 if 5 * blocks_of_256 * nq >= 3 * _sm_count(device) else 128
+        return pack, PREFILL_TC_ROWS
+    if pack == 1:
+        return 1, 256 if 5 * whole >= 3 * sms else 128
+    of_256, of_128 = blocks(256 // pack), blocks(128 // pack)
+    return pack, 256 if of_256 * (nq // pack) >= sms and 4 * of_128 > 5 * of_256 else 128
 
 
 def attn_prefill_tc_takes(D: int, nq: int, nkv: int, page: int) -> bool:
@@ -1468,12 +1487,13 @@ def attn_prefill_tc(q, k_pages, v_pages, block_table, *, cu_q, slots, kv_len, q_
                     rows_per_block: int = 0, n_qblocks: Optional[int] = None,
                     softcap: Optional[float] = None,
                     sinks: Optional[torch.Tensor] = None, keep_first: int = 0,
-                    chunk: int = 0) -> torch.Tensor:
+                    chunk: int = 0, pack: int = 0) -> torch.Tensor:
     """Causal attention of whole prompts (or their continuation) with both
     products on the tcgen05 tensor cores.  Pages must hold finite values in the
     rows beyond a sequence's length (the cache zero-fills its pages).  The grid is
     sized from ``q_lens`` (the host's copy of the row counts) or, without them,
-    from ``n_qblocks``, an upper bound of the blocks of ``rows_per_block`` rows."""
+    from ``n_qblocks``, an upper bound of the blocks of ``rows_per_block`` rows (query rows
+    of ``pack`` heads; with ``rows_per_block`` given, as many as can share a block by default)."""
     _need(q, "q", torch.bfloat16, 3)
     T, nq, D = q.shape
     _need(k_pages, "k pages", torch.bfloat16, 4)
@@ -1493,9 +1513,13 @@ def attn_prefill_tc(q, k_pages, v_pages, block_table, *, cu_q, slots, kv_len, q_
     a.out, a.error = out.data_ptr(), _tc_error_flag(q.device).data_ptr()
     a.n_seqs, a.nq, a.nkv, a.max_pages = n_seqs, nq, nkv, block_table.shape[1]
     a.window = int(window or 0)
-    rows = int(rows_per_block) if rows_per_block else \
-        prefill_tc_rows(_q_blocks(q_lens, None, 256, T, n_seqs), nq, q.device)
-    a.n_qblocks = _q_blocks(q_lens, n_qblocks, rows, T, n_seqs)
+    a.pack, rows = prefill_tc_plan(lambda n: _q_blocks(q_lens, None, n, T, n_seqs), nq, nkv, _sm_count(q.device))
+    if rows_per_block:
+        a.pack, rows = int(pack or prefill_tc_pack(nq, nkv)), int(rows_per_block)
+    a.n_qblocks = _q_blocks(q_lens, n_qblocks, rows // a.pack, T, n_seqs)
+    while a.n_qblocks > 65535 and a.pack > 1:      # more than a grid has: fewer heads, more tokens a block
+        a.pack //= 2
+        a.n_qblocks = _q_blocks(q_lens, n_qblocks, rows // a.pack, T, n_seqs)
     a.scale_log2 = float(scale) * _LOG2E
     a.keep_first, a.chunk = int(keep_first or 0), _chunk_arg(chunk, keep_first)
     _set_cap_and_sinks(a, scale, softcap, sinks, nq)

@@ -720,6 +720,52 @@ def test_attn_prefill_tc(nq, nkv, D, window, rows_per_block):
         assert torch.allclose(got[cu[4] + 299, 0].double(), pc.v[4][3, 0].double(), atol=1e-2, rtol=1e-2)
 
 
+@pytest.mark.parametrize("rows_per_block", [128, 256])
+@pytest.mark.parametrize("nq,nkv,D,window", [(6, 1, 64, None), (16, 1, 128, None), (12, 3, 64, 40), (64, 1, 64, 70)])
+def test_attn_prefill_tc_heads_of_a_block(nq, nkv, D, window, rows_per_block):
+    """The rows of 2, 16, 4 and 64 query heads in one block: sequences of one token, around a block's tokens (128 or
+    256 rows over the heads) and of a few blocks, first ones and continued ones, a padding sequence between them."""
+    ops = _ops()
+    dt = torch.bfloat16
+    per = rows_per_block // ops.prefill_tc_pack(nq, nkv)
+    assert ops.prefill_tc_pack(nq, nkv) == {6: 2, 16: 16, 12: 4, 64: 64}[nq]
+    plan = [(0, 1), (0, per), (70, per + 1), (0, 2), (3, max(1, per - 1)), (60, 2 * per + 3)]
+    lens, q_lens = [s + n for s, n in plan], [n for _s, n in plan]
+    pc = Paged(lens, nkv, D, dt, 48, fill=300.0)
+    q = _rand((sum(q_lens), nq, D), dt, 49)
+    cu = torch.tensor([0] + q_lens).cumsum(0).tolist()
+    slots = [-1 if s == 3 else pc.slot_of[s] for s in range(len(plan))]
+    scale = 1.0 / math.sqrt(D)
+    got = ops.attn_prefill_tc(
+        q.to(DEV), pc.k_pages.to(DEV), pc.v_pages.to(DEV), pc.table.to(DEV),
+        cu_q=torch.tensor(cu, dtype=torch.int32, device=DEV), slots=torch.tensor(slots, dtype=torch.int32, device=DEV),
+        kv_len=torch.tensor(lens, dtype=torch.int32, device=DEV), q_lens=tuple(q_lens), page=64, scale=scale,
+        window=window, rows_per_block=rows_per_block).cpu()
+    ops.check_kernel_errors()
+    assert not got[cu[3]:cu[4]].any()
+    for s, (start, n) in enumerate(plan):
+        for i in sorted({0, n // 2, n - 1, min(n - 1, per // 2), min(n - 1, per)} if s != 3 else ()):
+            want = _attn_oracle(q[cu[s] + i], pc.k[s], pc.v[s], start + i, scale, window)
+            assert torch.allclose(got[cu[s] + i].double(), want, **FAST_TOL), (s, i)
+
+
+@pytest.mark.parametrize("nq,nkv", [(32, 8), (16, 8), (16, 1), (3, 3), (10, 2)])
+def test_attn_prefill_tc_takes_the_same_rows_however_they_are_blocked(nq, nkv):
+    """The plan's blocks (whatever it chooses for few and for many rows) against one head a block: the same keys in the
+    same order, so the same bits."""
+    ops = _ops()
+    for lens in ([5], [200, 1, 64], [70] * 30):
+        pc = Paged(lens, nkv, 64, torch.bfloat16, 50, fill=300.0)
+        q = _rand((sum(lens), nq, 64), torch.bfloat16, 51).to(DEV)
+        i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+        run = lambda **kw: ops.attn_prefill_tc(  # noqa: E731
+            q, pc.k_pages.to(DEV), pc.v_pages.to(DEV), pc.table.to(DEV), cu_q=i32([0] + torch.tensor(lens).cumsum(0).tolist()),
+            slots=i32(pc.slot_of), kv_len=i32(lens), page=64, scale=0.125, **kw)
+        want = run(rows_per_block=128, pack=1, q_lens=tuple(lens))
+        assert torch.equal(run(q_lens=tuple(lens)), want) and torch.equal(run(), want)
+    ops.check_kernel_errors()
+
+
 def _plant_window_edge(q, row, pc, seq, pos, window):
     """Makes query ``row`` (at position ``pos`` of sequence ``seq``) look along one
     axis only, and gives two keys a component there: the key just outside its
