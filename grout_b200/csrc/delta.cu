@@ -11,7 +11,7 @@
 //
 // Everything here is 32-bit whatever the activation type: the one projection
 // that feeds it arrives as 32-bit sums, and only y, the o projection's input, is
-// rounded.  Four kernels:
+// rounded.  Four kernels (and, further down, the forms of a decode step and of long prompts):
 //
 //   prepare  one block per token and kv head (its q and k) or run of value
 //            channels: convolution (from the rows of this step and, for the first
@@ -66,7 +66,22 @@ struct DeltaArgs {
   int prep_stride;         // floats between rows of prep: round4(Cc + 2 H) + 48 H
   int few_rows;            // 1: no sequence brings more than DELTA_B rows, 2: none more than one (a decode
                            //   step): the scan works out its one group's scalars itself, `gram` is not launched
+  int max_rows;            // the most rows any sequence brings (0: unknown)
+  float* chunks;           // [n_tokens / 32 + n_seqs, H, record] scratch of a step that goes chunk by chunk, or null
 };
+
+__device__ __forceinline__ void delta_keep_tail(const DeltaArgs& a, int seq, int first, int step);
+__device__ __forceinline__ int cc_channels(const DeltaArgs& a) { return 2 * a.G * a.dk + a.H * a.dv; }
+__device__ __forceinline__ const float* cc_gate(const DeltaArgs& a, size_t t, int h) {
+  const int Cc = cc_channels(a);
+  return a.proj + t * (Cc + a.H * a.dv + 2 * a.H) + Cc + (size_t)h * a.dv;
+}
+__device__ __forceinline__ float cc_gate_of(const DeltaArgs&, float x) { return silu_f(x); }
+// (every reader of the old tail, the prepare kernel, has finished)
+__device__ __forceinline__ void cc_out_done(const DeltaArgs& a, int seq, int h) {
+  delta_keep_tail(a, seq, h * blockDim.x + threadIdx.x, a.H * blockDim.x);
+}
+#include "delta_chunk.cuh"
 
 // One block per (token, unit): unit g < G is kv head g's q and k together, the units after that are runs of
 // DELTA_PREP_V value channels; the block of unit 0 also takes beta and the decay.
@@ -121,14 +136,13 @@ __global__ void __launch_bounds__(256) delta_prepare_kernel(const DeltaArgs a) {
   pdl_launch_dependents_if_large();
 }
 
-// The new tail of a sequence; the blocks of the row (blockIdx.y) share the channels.
-__device__ __forceinline__ void delta_keep_tail(const DeltaArgs& a, int seq) {
+// The new tail of a sequence; the caller's threads share the channels: first, first + step, ...
+__device__ __forceinline__ void delta_keep_tail(const DeltaArgs& a, int seq, int first, int step) {
   const int slot = a.slots[seq];
   const int row0 = a.cu_q[seq], n = a.cu_q[seq + 1] - row0;
   if (slot < 0 || n <= 0) return;
   const int Cc = 2 * a.G * a.dk + a.H * a.dv, C_all = Cc + a.H * a.dv + 2 * a.H;
-  short_conv_keep_tail(a.proj, C_all, a.taps, a.state + (size_t)slot * a.state_stride, Cc, row0, n,
-                       blockIdx.y * blockDim.x + threadIdx.x, gridDim.y * blockDim.x);
+  short_conv_keep_tail(a.proj, C_all, a.taps, a.state + (size_t)slot * a.state_stride, Cc, row0, n, first, step);
 }
 
 #define DELTA_LANES 8       // lanes that share a column of S
@@ -444,9 +458,301 @@ __global__ void delta_finish_kernel(const DeltaArgs a) {
   // of the old one, the prepare kernel, has finished)
   if (a.taps > 1) {
     const int seq = a.token_seq[t];
-    if (t == a.cu_q[seq]) delta_keep_tail(a, seq);
+    if (t == a.cu_q[seq]) delta_keep_tail(a, seq, blockIdx.y * blockDim.x + threadIdx.x, gridDim.y * blockDim.x);
   }
   pdl_launch_dependents_if_large();
+}
+
+// ---- a decode step in one kernel ---------------------------------------------
+// Every sequence brings one row: a block per head and sequence does all of the mixer for it.  Bound by latency (a
+// head's state is 64 KB; three kernels of few blocks were 20 us of a step of one sequence and 16 heads of 128, each its
+// own hand-over; this is 4.7), so the state, the kept inputs and the weights, which no kernel of this step writes, are
+// requested before the wait.  A column of the state is in eight lanes' registers, four columns a thread.  The heads
+// that share q and k are a cluster: all of them read the kept inputs of q and k, and the first replaces them when all
+// have.
+#define DS_COLS 128       // columns of a head: 4 passes of 32
+#define DS_TAPS 8
+template <typename T>
+__global__ void __launch_bounds__(256) delta_step_kernel(const DeltaArgs a) {
+  __shared__ float q_s[128], k_s[128], v_s[DS_COLS], o_s[DS_COLS], sums[2][8];
+  pdl_launch_dependents_if_small();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int h = blockIdx.x, seq = blockIdx.y, H = a.H, G = a.G, dk = a.dk, dv = a.dv, taps = a.taps;
+  const int kvh = h / (H / G), Cc = 2 * G * dk + H * dv, C_all = Cc + H * dv + 2 * H;
+  const int slot = a.slots[seq], t = a.cu_q[seq];
+  if (a.cu_q[seq + 1] <= t) return;              // (the same for the whole cluster)
+  float* st = slot >= 0 ? a.state + (size_t)slot * a.state_stride : nullptr;
+  float* sp = st ? st + (size_t)(taps - 1) * Cc + (size_t)h * dv * dk : nullptr;
+  const int l = tid & 7, c0 = tid >> 3;
+  float4 S[4][4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int c = p * 32 + c0, e = (i * 8 + l) * 4;
+      S[p][i] = sp && c < dv && e < dk ? *reinterpret_cast<const float4*>(sp + (size_t)c * dk + e)
+                                       : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  // this thread's channel of q or k, and of v
+  const bool is_q = tid < dk, is_qk = tid < 2 * dk, is_v = tid < dv;
+  const int cq = is_q ? kvh * dk + tid : (G + kvh) * dk + (tid - dk), cv = 2 * G * dk + h * dv + tid;
+  float kept_q[DS_TAPS], kept_v[DS_TAPS], w_q[DS_TAPS], w_v[DS_TAPS];      // [j]: the input j rows back
+#pragma unroll
+  for (int j = 0; j < DS_TAPS; ++j) {
+    kept_q[j] = kept_v[j] = w_q[j] = w_v[j] = 0.f;
+    if (j < taps) {
+      if (is_qk) w_q[j] = a.conv_w[(size_t)cq * taps + taps - 1 - j];
+      if (is_v) w_v[j] = a.conv_w[(size_t)cv * taps + taps - 1 - j];
+      if (st && j > 0) {
+        if (is_qk) kept_q[j] = st[(size_t)(taps - 1 - j) * Cc + cq];
+        if (is_v) kept_v[j] = st[(size_t)(taps - 1 - j) * Cc + cv];
+      }
+    }
+  }
+  const float rate = expf(a.a_log[h]), dt = a.dt_bias[h], nw = is_v ? a.norm_w[tid] : 0.f;
+  pdl_wait();
+  const float* row = a.proj + (size_t)t * C_all;
+  if (is_qk) kept_q[0] = row[cq];
+  float gate = 0.f;
+  if (is_v) kept_v[0] = row[cv], gate = row[Cc + h * dv + tid];
+  const float b = row[Cc + H * dv + h], al = row[Cc + H * dv + H + h];
+  float x = 0.f, v = 0.f;
+#pragma unroll
+  for (int j = 0; j < DS_TAPS; ++j) x = fmaf(w_q[j], kept_q[j], x), v = fmaf(w_v[j], kept_v[j], v);
+  // (the kept inputs have been used, so they have been read)
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  x = silu_f(x);
+  if (is_v) v_s[tid] = silu_f(v);
+  const float sq = warp_sum(is_q ? x * x : 0.f), sk = warp_sum(is_qk && !is_q ? x * x : 0.f);
+  if (lane == 0) sums[0][warp] = sq, sums[1][warp] = sk;
+  __syncthreads();
+  if (is_qk) {
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ss += sums[is_q ? 0 : 1][i];
+    const float inv = 1.0f / sqrtf(ss + a.unit_eps);
+    if (is_q) q_s[tid] = x * inv * (1.0f / sqrtf((float)dk));
+    else k_s[tid - dk] = x * inv;
+  }
+  __syncthreads();
+  const float beta = 1.0f / (1.0f + expf(-b)), g = expf(-rate * softplus_f(al + dt));
+  float4 q[4], k[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int e = (i * 8 + l) * 4;
+    q[i] = e < dk ? *reinterpret_cast<const float4*>(q_s + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+    k[i] = e < dk ? *reinterpret_cast<const float4*>(k_s + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  float kq = 0.f, dq[4], dks[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    kq = fmaf(k[i].x, q[i].x, kq), kq = fmaf(k[i].y, q[i].y, kq);
+    kq = fmaf(k[i].z, q[i].z, kq), kq = fmaf(k[i].w, q[i].w, kq);
+  }
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    float d1 = 0.f, d2 = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float4 s = S[p][i];
+      d1 = fmaf(s.x, k[i].x, d1), d1 = fmaf(s.y, k[i].y, d1), d1 = fmaf(s.z, k[i].z, d1), d1 = fmaf(s.w, k[i].w, d1);
+      d2 = fmaf(s.x, q[i].x, d2), d2 = fmaf(s.y, q[i].y, d2), d2 = fmaf(s.z, q[i].z, d2), d2 = fmaf(s.w, q[i].w, d2);
+    }
+    dks[p] = d1, dq[p] = d2;
+  }
+#pragma unroll
+  for (int m = 1; m < 8; m <<= 1) {
+    kq += __shfl_xor_sync(0xffffffffu, kq, m);
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      dks[p] += __shfl_xor_sync(0xffffffffu, dks[p], m);
+      dq[p] += __shfl_xor_sync(0xffffffffu, dq[p], m);
+    }
+  }
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const int c = p * 32 + c0;
+    const float u = c < dv ? beta * (v_s[c] - g * dks[p]) : 0.f;
+    if (l == 0 && c < dv) o_s[c] = fmaf(u, kq, g * dq[p]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float4 s = S[p][i];
+      s.x = fmaf(k[i].x, u, g * s.x), s.y = fmaf(k[i].y, u, g * s.y);
+      s.z = fmaf(k[i].z, u, g * s.z), s.w = fmaf(k[i].w, u, g * s.w);
+      const int e = (i * 8 + l) * 4;
+      if (sp && c < dv && e < dk) *reinterpret_cast<float4*>(sp + (size_t)c * dk + e) = s;
+    }
+  }
+  __syncthreads();
+  float ss = 0.f;
+  for (int j = lane; j < dv; j += 32) ss += o_s[j] * o_s[j];
+  const float inv = 1.0f / sqrtf(warp_sum(ss) / (float)dv + a.norm_eps);
+  if (is_v) ((T*)a.y)[((size_t)t * H + h) * dv + tid] = from_f32<T>(o_s[tid] * inv * nw * silu_f(gate));
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (st) {
+#pragma unroll
+    for (int j = 0; j < DS_TAPS; ++j)
+      if (j < taps - 1) {
+        if (is_v) st[(size_t)(taps - 2 - j) * Cc + cv] = kept_v[j];
+        if (is_qk && h % (H / G) == 0) st[(size_t)(taps - 2 - j) * Cc + cq] = kept_q[j];
+      }
+  }
+  pdl_launch_dependents_if_large();
+}
+
+// Heads of up to 128 by 128 in whole pieces of four on 16-byte boundaries, up to eight taps and clusters of eight.
+static bool delta_step_takes(const DeltaArgs& a) {
+  const int Cc = 2 * a.G * a.dk + a.H * a.dv;
+  return a.few_rows == 2 && a.dk <= 128 && a.dk % 4 == 0 && a.dv <= DS_COLS && a.taps <= DS_TAPS && a.H / a.G <= 8 &&
+         a.n_seqs <= 65535 && a.state_stride % 4 == 0 && ((long long)(a.taps - 1) * Cc) % 4 == 0 &&
+         (((uintptr_t)a.state) & 15) == 0;
+}
+
+// ---- many rows: chunk by chunk (delta_chunk.cuh) -------------------------------
+// With c_t = g_1 .. g_t inside a chunk, what that file calls e^L is one number a row:
+//   A_ti = (c_t / c_i) (k_t . k_i),  B_ti = (c_t / c_i) (q_t . k_i),  u_t = beta_t (v_t - S_0^T c_t k_t - sum_{i<t} A_ti u_i)
+// (quotients are products of the g between).  This kernel takes every chunk of every head at the same time, solves
+// the triangular system for the right-hand sides beta v and beta c k, and leaves the record.  The scan below
+// walks 2,048 rows (16 heads of 128) in 512 turns of a microsecond, 502 us and 36 for their products; this kernel takes
+// 56 us, the two behind it 140 and 64 (with the norm and the gate, which took 40 more behind the scan).
+#define DC_MIN 64         // a step goes chunk by chunk when a sequence may bring this many rows
+__global__ void __launch_bounds__(256, 2) delta_local_kernel(const DeltaArgs a) {
+  constexpr int LD = CC_MAX_DK + 4;
+  extern __shared__ __align__(16) float sm[];
+  float *Ks = sm, *Qs = Ks + CC_ROWS * LD, *As = Qs + CC_ROWS * LD, *Bs = As + CC_ROWS * CC_ROWS;
+  float *quot = Bs + CC_ROWS * CC_ROWS, *beta = quot + CC_ROWS * (CC_ROWS + 1), *cum = beta + CC_ROWS;
+  pdl_launch_dependents_if_small();
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int h = blockIdx.y, seq = blockIdx.z, z = blockIdx.x;
+  const int H = a.H, G = a.G, dk = a.dk, dv = a.dv, kvh = h / (H / G), Cc = cc_channels(a), P = a.prep_stride;
+  pdl_wait();
+  const int first = a.cu_q[seq], n_seq = a.cu_q[seq + 1] - first;
+  const int n = min(CC_ROWS, n_seq - z * CC_ROWS), row0 = first + z * CC_ROWS;
+  if (n <= 0) return;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int i = 0; i < CC_ROWS * (CC_MAX_DK / 4) / 256; ++i) {
+    const int at = i * 256 + tid, t = at / (CC_MAX_DK / 4), d = at % (CC_MAX_DK / 4) * 4;
+    const float* p = a.prep + (size_t)(row0 + t) * P;
+    const bool in = t < n && d < dk;
+    *reinterpret_cast<float4*>(Qs + t * LD + d) = in ? *reinterpret_cast<const float4*>(p + kvh * dk + d) : zero;
+    *reinterpret_cast<float4*>(Ks + t * LD + d) = in ? *reinterpret_cast<const float4*>(p + (G + kvh) * dk + d) : zero;
+  }
+  if (tid < 32) {          // a warp: lane i has the quotients c_t / c_i of row i, and c_t in front of all of them
+    const float* p = a.prep + (size_t)(row0 + lane) * P + Cc + h;
+    beta[lane] = lane < n ? p[0] : 0.f;
+    const float g = lane < n ? p[H] : 1.f;
+    float run = 0.f, all = 1.f;
+#pragma unroll
+    for (int t = 0; t < CC_ROWS; ++t) {
+      const float gt = __shfl_sync(0xffffffffu, g, t);
+      run = t == lane ? 1.f : run * gt;
+      all *= gt;
+      quot[t * (CC_ROWS + 1) + lane] = run;      // (zero for t < i)
+      if (lane == 0) cum[t] = all;
+    }
+  }
+  __syncthreads();
+  const size_t entry = (cc_entry(first, z, seq) * H + h) * cc_record(dk, dv);
+  float* wq = a.chunks + entry;
+  float* kd = wq + (size_t)dk * CC_ROWS;
+  float* gc = kd + (size_t)CC_ROWS * dk;
+  float* qb = wq + cc_at_qb(dk);
+  float* u0 = wq + cc_at_su(dk) + (size_t)dk * dv;
+  {                        // two rows by two of both products a thread
+    const int t0 = tid / 16, i0 = tid % 16;
+    float kk[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, qk[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll 4
+    for (int d = 0; d < dk; d += 4) {
+      float4 ki[2], kt[2], qt[2];
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        ki[x] = *reinterpret_cast<const float4*>(Ks + (i0 + 16 * x) * LD + d);
+        kt[x] = *reinterpret_cast<const float4*>(Ks + (t0 + 16 * x) * LD + d);
+        qt[x] = *reinterpret_cast<const float4*>(Qs + (t0 + 16 * x) * LD + d);
+      }
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+          kk[x][y] = fmaf(kt[x].x, ki[y].x, kk[x][y]), qk[x][y] = fmaf(qt[x].x, ki[y].x, qk[x][y]);
+          kk[x][y] = fmaf(kt[x].y, ki[y].y, kk[x][y]), qk[x][y] = fmaf(qt[x].y, ki[y].y, qk[x][y]);
+          kk[x][y] = fmaf(kt[x].z, ki[y].z, kk[x][y]), qk[x][y] = fmaf(qt[x].z, ki[y].z, qk[x][y]);
+          kk[x][y] = fmaf(kt[x].w, ki[y].w, kk[x][y]), qk[x][y] = fmaf(qt[x].w, ki[y].w, qk[x][y]);
+        }
+    }
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+      for (int y = 0; y < 2; ++y) {
+        const int t = t0 + 16 * x, i = i0 + 16 * y;
+        const float w = quot[t * (CC_ROWS + 1) + i];
+        As[t * CC_ROWS + i] = i < t ? w * kk[x][y] : 0.f;
+        Bs[t * CC_ROWS + i] = i <= t ? w * qk[x][y] : 0.f;
+      }
+  }
+  __syncthreads();
+  // the substitution: a thread takes one right-hand side (dv of values, then dk of c k)
+  for (int c = tid; c < dv + dk; c += 256) {
+    float x[CC_ROWS];
+    const int d = c - dv;
+#pragma unroll
+    for (int t = 0; t < CC_ROWS; ++t) {
+      if (d < 0) x[t] = t < n ? a.prep[(size_t)(row0 + t) * P + 2 * G * dk + h * dv + c] : 0.f;
+      else x[t] = Ks[t * LD + d] * cum[t];
+    }
+#pragma unroll
+    for (int t = 0; t < CC_ROWS; ++t) {
+      float s = x[t];
+#pragma unroll
+      for (int i0 = 0; i0 < t; i0 += 4) {        // (entries of A from the diagonal on are zero, x there still finite)
+        const float4 w = *reinterpret_cast<const float4*>(As + t * CC_ROWS + i0);
+        s = fmaf(-w.x, x[i0], s);
+        if (i0 + 1 < t) s = fmaf(-w.y, x[i0 + 1], s);
+        if (i0 + 2 < t) s = fmaf(-w.z, x[i0 + 2], s);
+        if (i0 + 3 < t) s = fmaf(-w.w, x[i0 + 3], s);
+      }
+      x[t] = beta[t] * s;
+    }
+    if (d < 0) {
+#pragma unroll
+      for (int t = 0; t < CC_ROWS; ++t) u0[(size_t)t * dv + c] = x[t];
+    } else {
+      float4* out = reinterpret_cast<float4*>(wq + (size_t)d * CC_ROWS);
+#pragma unroll
+      for (int t = 0; t < CC_ROWS; t += 4) out[t / 4] = make_float4(x[t], x[t + 1], x[t + 2], x[t + 3]);
+    }
+  }
+  pdl_launch_dependents_if_large();
+  for (int i = tid; i < 8 * dk; i += 256) {      // c q, four rows of a channel a thread
+    const int d = i / 8, t = (i % 8) * 4;
+    *reinterpret_cast<float4*>(qb + (size_t)d * CC_ROWS + t) =
+        make_float4(Qs[t * LD + d] * cum[t], Qs[(t + 1) * LD + d] * cum[t + 1], Qs[(t + 2) * LD + d] * cum[t + 2],
+                    Qs[(t + 3) * LD + d] * cum[t + 3]);
+  }
+  for (int i = tid; i < CC_ROWS * CC_ROWS; i += 256)     // B by columns
+    qb[(size_t)dk * CC_ROWS + i] = Bs[(i % CC_ROWS) * CC_ROWS + i / CC_ROWS];
+  for (int i = tid; i < CC_ROWS * dk; i += 256) {        // what is left of a row's key at the chunk's end
+    const int t = i / dk, d = i % dk;
+    kd[i] = Ks[t * LD + d] * quot[(CC_ROWS - 1) * (CC_ROWS + 1) + t];
+  }
+  for (int d = tid; d < dk; d += 256) gc[d] = cum[CC_ROWS - 1];
+}
+
+static bool delta_chunks_take(const DeltaArgs& a) {
+  return a.chunks && !a.few_rows && a.max_rows >= DC_MIN && a.dk <= CC_MAX_DK && a.dk % 4 == 0 && a.dv % 4 == 0 &&
+         a.dv <= CC_MAX_DV && a.H <= 65535 && a.n_seqs <= 65535 && (((uintptr_t)a.chunks) & 15) == 0;
+}
+
+template <typename T>
+static int delta_by_chunks(const DeltaArgs& a, cudaStream_t s) {
+  const size_t smem = (2 * CC_ROWS * (CC_MAX_DK + 4) + 2 * CC_ROWS * CC_ROWS + CC_ROWS * (CC_ROWS + 1) + 2 * CC_ROWS) *
+                      sizeof(float);
+  cudaError_t ce = cudaFuncSetAttribute(delta_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (ce != cudaSuccess) return (int)ce;
+  const int e = gb_launch(delta_local_kernel, dim3((a.max_rows + CC_ROWS - 1) / CC_ROWS, a.H, a.n_seqs), dim3(256), smem,
+                          s, a);
+  return e ? e : delta_chain_and_out<T>(a, a.max_rows, s);
 }
 
 template <int R, int B>
@@ -485,10 +791,13 @@ static int delta_forward(const DeltaArgs& a, cudaStream_t s) {
   int e = delta_check(a);
   if (e) return e;
   if (a.n_tokens == 0) return 0;
+  if (delta_step_takes(a))
+    return gb_launch_cluster(delta_step_kernel<T>, dim3(a.H, a.n_seqs), dim3(256), 0, s, a.H / a.G, a);
   const int units = a.G + (a.H * a.dv + DELTA_PREP_V - 1) / DELTA_PREP_V;
   e = gb_launch(delta_prepare_kernel, dim3(a.n_tokens, units), dim3(256),
                 (size_t)2 * a.dk * sizeof(float), s, a);
   if (e) return e;
+  if (delta_chunks_take(a)) return delta_by_chunks<T>(a, s);
   if (!a.few_rows) {
     e = gb_launch(delta_gram_kernel, dim3(a.n_tokens, a.H), dim3(128), 0, s, a);
     if (e) return e;
@@ -509,6 +818,7 @@ static int delta_forward(const DeltaArgs& a, cudaStream_t s) {
   return gb_launch(delta_finish_kernel<T>, dim3(a.n_tokens, rows_y), dim3(warps * 32), 0, s, a);
 }
 
-// Four launches: prepare, gram (not for a step of few rows a sequence), scan, finish.
+// One launch for a decode step; prepare, local, chain and out by chunks; else prepare, gram (not for a step of few rows a
+// sequence), scan and finish.
 GB_EXPORT int gb_delta_forward_f32(const DeltaArgs* a, cudaStream_t s) { return delta_forward<float>(*a, s); }
 GB_EXPORT int gb_delta_forward_bf16(const DeltaArgs* a, cudaStream_t s) { return delta_forward<bf16>(*a, s); }

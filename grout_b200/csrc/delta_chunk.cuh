@@ -1,0 +1,311 @@
+// The delta rule chunk by chunk: what the chunked forms of delta.cu (one decay per head) and channel_delta.cu (one per
+// channel) share.  Both write the same record for every chunk of every head; with S_0 the state in front of a chunk,
+//
+//   U = U0 - W S_0;   S_n = diag(gC) S_0 + Kd^T U;   O = [e^L q | B] [S_0 ; U]
+//
+//   chain   walks a sequence's chunks in order, a block per head and COLS columns of S with the state in shared
+//           memory: U and the next state, tiled 32-bit products; it leaves U and the state in front of every chunk
+//           in the record
+//   out     takes every chunk of every head at the same time: the read-outs, and their norm and gate
+//
+// The including file's arguments have cu_q, slots, state, state_stride, taps, H, dk, dv, n_seqs, norm_eps, norm_w, y and
+// chunks, and for them cc_channels(a) (the convolved channels), cc_gate(a, t, h) (the gate's logits of a row and head),
+// cc_gate_of(a, x) and cc_out_done(a, seq, h) (called by a sequence's first block of every head).
+#pragma once
+
+#define CC_ROWS 32       // rows of a chunk
+#define CC_MAX_DK 128
+#define CC_MAX_DV 1024
+
+// A chunk's record for one head: W [dk][32] (per channel the 32 rows) | Kd [32][dk] (e^{L_n - L} k) |
+// gC [dk] (e^{L_n}) | QB [dk + 32][32] (per channel the rows of e^L q, then per row i the column of
+// B) | SU [dk + 32][dv] (S_0, then U0, which becomes U)
+__host__ __device__ __forceinline__ size_t cc_record(int dk, int dv) {
+  return (size_t)2 * dk * CC_ROWS + dk + (size_t)(dk + CC_ROWS) * (CC_ROWS + dv);
+}
+__host__ __device__ __forceinline__ int cc_at_qb(int dk) { return 2 * dk * CC_ROWS + dk; }
+__host__ __device__ __forceinline__ int cc_at_su(int dk) { return cc_at_qb(dk) + (dk + CC_ROWS) * CC_ROWS; }
+// Chunk z of a sequence whose rows start at `first` has an entry that no other chunk has.
+__host__ __device__ __forceinline__ size_t cc_entry(int first, int z, int seq) {
+  return (size_t)(first / CC_ROWS + z + seq);
+}
+
+__device__ __forceinline__ void cc_copy16(float* smem, const float* gmem) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem));
+}
+
+typedef unsigned long long cc_pair;      // two 32-bit numbers
+__device__ __forceinline__ cc_pair cc_both(float a) {
+  cc_pair r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
+  return r;
+}
+__device__ __forceinline__ void cc_fma2(cc_pair& d, cc_pair a, cc_pair b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ void cc_unpack(cc_pair v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+
+// floats of a chain block's stage: W | Kd | gC | U0's columns
+__host__ __device__ __forceinline__ int cc_stage(int dk, int cols) { return 2 * dk * CC_ROWS + dk + CC_ROWS * cols; }
+__host__ __device__ __forceinline__ size_t cc_chain_smem(int dk, int cols) {   // two stages, S, partial sums, U
+  return (size_t)(2 * cc_stage(dk, cols) + dk * cols + (128 / cols + 1) * CC_ROWS * cols) * sizeof(float);
+}
+
+// Bound by a chunk's chain of three steps with a barrier behind each, so what counts is how few instructions a thread has
+// between them: packed multiply-adds over pairs of rows, and, where a step has few sequences and heads, 16 columns a
+// block: 64 chunks of one sequence and 16 heads of 128 in 140 us, 2.2 a chunk.
+template <typename Args, int COLS>
+__global__ void __launch_bounds__(256) delta_chain_kernel(const Args a) {
+  static_assert(COLS == 16 || COLS == 32, "columns of a block");
+  extern __shared__ __align__(16) float sm[];
+  constexpr int CT = COLS / 4;                   // threads along the columns of W S, four columns each
+  constexpr int SPLITS = 256 / (8 * CT);         // parts of the channels' sum: 4 or 8
+  constexpr int SC = COLS / 8;                   // columns of the state a thread updates
+  pdl_launch_dependents_if_small();
+  const int tid = threadIdx.x;
+  const int h = blockIdx.y, seq = blockIdx.z, col0 = blockIdx.x * COLS;
+  const int H = a.H, dk = a.dk, dv = a.dv, Cc = cc_channels(a);
+  const int stage = cc_stage(dk, COLS);
+  float* S = sm + 2 * stage;                     // [dk][COLS]
+  float* P = S + dk * COLS;                      // [SPLITS][CC_ROWS][COLS]: a part of the channels' share of W S each
+  float* U = P + SPLITS * CC_ROWS * COLS;        // [CC_ROWS][COLS]
+  pdl_wait();
+  const int first = a.cu_q[seq], n_seq = a.cu_q[seq + 1] - first;
+  if (n_seq <= 0) return;
+  const int slot = a.slots[seq];
+  float* sp = slot >= 0 ? a.state + (size_t)slot * a.state_stride + (size_t)(a.taps - 1) * Cc + (size_t)h * dv * dk
+                        : nullptr;
+  const int chunks = (n_seq + CC_ROWS - 1) / CC_ROWS;
+  auto record = [&](int z) { return a.chunks + (cc_entry(first, z, seq) * H + h) * cc_record(dk, dv); };
+  const int whole = 2 * dk * CC_ROWS + dk;                 // (dk is a multiple of four)
+  auto stage_in = [&](int z) {
+    float* dst = sm + (z & 1) * stage;
+    const float* src = record(z);
+    for (int i = tid * 4; i < whole; i += 1024) cc_copy16(dst + i, src + i);
+    const int t = tid / CT, c = (tid % CT) * 4;
+    if (t < CC_ROWS && col0 + c < dv)
+      cc_copy16(dst + whole + t * COLS + c, src + cc_at_su(dk) + (size_t)(dk + t) * dv + col0 + c);
+    cp_async_commit();
+  };
+  for (int s = 0; s < 2 && col0 + COLS > dv; ++s)          // columns no copy brings
+    for (int i = tid; i < CC_ROWS * COLS; i += 256)
+      if (col0 + i % COLS >= dv) sm[s * stage + whole + i] = 0.f;
+  stage_in(0);
+  // the state: element (k, c) of the head's matrix lies at c dk + k
+  for (int i = tid; i < dk * COLS; i += 256) {
+    const int c = i / dk, k = i % dk;
+    S[k * COLS + c] = sp && col0 + c < dv ? sp[(size_t)(col0 + c) * dk + k] : 0.f;
+  }
+  // tiles: 4 rows by 4 columns of W S a thread, a part of the channels each; 4 rows by SC columns of the state
+  const int part = tid / (8 * CT), tr = tid % (8 * CT) / CT * 4, tc = tid % CT * 4;
+  const int per = (dk + SPLITS - 1) / SPLITS, k_lo = part * per, k_hi = min(dk, k_lo + per);
+  const int sk = tid / 8 * 4, sc = tid % 8 * SC;
+  const bool col_in = col0 + sc < dv;                      // (dv is a multiple of four)
+  for (int z = 0; z < chunks; ++z) {
+    if (z + 1 < chunks) { stage_in(z + 1); cp_async_wait<1>(); } else { cp_async_wait<0>(); }
+    __syncthreads();
+    const float* w = sm + (z & 1) * stage;
+    const float* kd = w + dk * CC_ROWS;
+    const float* gc = kd + CC_ROWS * dk;
+    const float* u0 = gc + dk;
+    float* su = record(z) + cc_at_su(dk) + col0;
+    cc_pair acc[2][4];                           // [pair of rows][column]
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+#pragma unroll 8
+    for (int k = k_lo; k < k_hi; ++k) {
+      const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(w + k * CC_ROWS + tr);
+      const float4 y = *reinterpret_cast<const float4*>(S + k * COLS + tc);
+      const float yv[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const cc_pair yy = cc_both(yv[j]);
+        cc_fma2(acc[0][j], x.x, yy);
+        cc_fma2(acc[1][j], x.y, yy);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      float lo[4], hi[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) cc_unpack(acc[i][j], lo[j], hi[j]);
+      float* p = P + (part * CC_ROWS + tr + 2 * i) * COLS + tc;
+      *reinterpret_cast<float4*>(p) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+      *reinterpret_cast<float4*>(p + COLS) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+    }
+    __syncthreads();
+    for (int i = tid * 4; i < CC_ROWS * COLS; i += 1024) {  // U = U0 - W S, four columns of a row a thread
+      float4 u = *reinterpret_cast<const float4*>(u0 + i);
+#pragma unroll
+      for (int q = 0; q < SPLITS; ++q) {
+        const float4 x = *reinterpret_cast<const float4*>(P + q * CC_ROWS * COLS + i);
+        u.x -= x.x, u.y -= x.y, u.z -= x.z, u.w -= x.w;
+      }
+      *reinterpret_cast<float4*>(U + i) = u;
+      if (col0 + i % COLS < dv) *reinterpret_cast<float4*>(su + (size_t)(dk + i / COLS) * dv + i % COLS) = u;
+    }
+    __syncthreads();
+    if (sk < dk) {                               // S <- diag(gC) S + Kd^T U
+      cc_pair s[2][SC];                          // [pair of rows][column]
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        float lo[SC], hi[SC];
+#pragma unroll
+        for (int j = 0; j < SC; ++j) lo[j] = S[(sk + 2 * i) * COLS + sc + j], hi[j] = S[(sk + 2 * i + 1) * COLS + sc + j];
+        if (col_in) {
+          float* to = su + (size_t)(sk + 2 * i) * dv + sc;
+          if constexpr (SC == 4) {
+            *reinterpret_cast<float4*>(to) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+            *reinterpret_cast<float4*>(to + dv) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+          } else {
+            *reinterpret_cast<float2*>(to) = make_float2(lo[0], lo[1]);
+            *reinterpret_cast<float2*>(to + dv) = make_float2(hi[0], hi[1]);
+          }
+        }
+        const float g0 = gc[sk + 2 * i], g1 = gc[sk + 2 * i + 1];
+#pragma unroll
+        for (int j = 0; j < SC; ++j) {
+          const float x = g0 * lo[j], y = g1 * hi[j];
+          asm("mov.b64 %0, {%1, %2};" : "=l"(s[i][j]) : "f"(x), "f"(y));
+        }
+      }
+#pragma unroll 8
+      for (int t = 0; t < CC_ROWS; ++t) {
+        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(kd + t * dk + sk);
+#pragma unroll
+        for (int j = 0; j < SC; ++j) {
+          const cc_pair yy = cc_both(U[t * COLS + sc + j]);
+          cc_fma2(s[0][j], x.x, yy);
+          cc_fma2(s[1][j], x.y, yy);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < SC; ++j) cc_unpack(s[i][j], S[(sk + 2 * i) * COLS + sc + j], S[(sk + 2 * i + 1) * COLS + sc + j]);
+    }
+    __syncthreads();                             // S is whole, the stage and P may be overwritten
+  }
+  pdl_launch_dependents_if_large();
+  if (sp)
+    for (int i = tid; i < dk * COLS; i += 256) {
+      const int c = i / dk, k = i % dk;
+      if (col0 + c < dv) sp[(size_t)(col0 + c) * dk + k] = S[k * COLS + c];
+    }
+}
+
+// The read-outs of a chunk: [32 x (dk + 32)] times [(dk + 32) x dv], 128 columns at a time, a thread 4 rows
+// (its warp's) by 4 columns, 32 elements of the sum staged together (two stages); then the norm
+// over a row's dv numbers, the weight and the gate.
+#define CO_COLS 128
+#define CO_STAGE (CC_ROWS * (CC_ROWS + CO_COLS))
+template <typename T, typename Args>
+__global__ void __launch_bounds__(256) delta_out_kernel(const Args a) {
+  extern __shared__ __align__(16) float sm[];    // two stages [A: 32 x 32 | B: 32 x CO_COLS] | the read-outs [32][dv]
+  pdl_launch_dependents_if_small();
+  const int tid = threadIdx.x, lane = tid & 31, row = tid / 32 * 4;
+  const int h = blockIdx.y, seq = blockIdx.z, z = blockIdx.x;
+  const int H = a.H, dk = a.dk, dv = a.dv, K = dk + CC_ROWS;
+  float* os = sm + 2 * CO_STAGE;
+  pdl_wait();
+  const int first = a.cu_q[seq], n = min(CC_ROWS, a.cu_q[seq + 1] - first - z * CC_ROWS);
+  if (n <= 0) return;
+  if (z == 0) cc_out_done(a, seq, h);
+  const float* rec = a.chunks + (cc_entry(first, z, seq) * H + h) * cc_record(dk, dv);
+  const float* qb = rec + cc_at_qb(dk);
+  const float* su = rec + cc_at_su(dk);
+  const int tiles = (K + CC_ROWS - 1) / CC_ROWS, col_tiles = (dv + CO_COLS - 1) / CO_COLS;
+  auto stage_in = [&](int s) {                   // stage s: column tile s / tiles, rows (s % tiles) 32 ..
+    float* as = sm + (s & 1) * CO_STAGE;
+    float* bs = as + CC_ROWS * CC_ROWS;
+    const int k0 = s % tiles * CC_ROWS, c0 = s / tiles * CO_COLS;
+    {
+      const int k = tid / 8, r = (tid % 8) * 4;
+      if (k0 + k < K) cc_copy16(as + k * CC_ROWS + r, qb + (size_t)(k0 + k) * CC_ROWS + r);
+    }
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+      const int k = tid / 32 + 8 * it, c = lane * 4;
+      if (k0 + k < K && c0 + c < dv) cc_copy16(bs + k * CO_COLS + c, su + (size_t)(k0 + k) * dv + c0 + c);
+    }
+    cp_async_commit();
+  };
+  float acc[4][4];
+  stage_in(0);
+  const int stages = tiles * col_tiles;
+  for (int s = 0; s < stages; ++s) {
+    if (s + 1 < stages) { stage_in(s + 1); cp_async_wait<1>(); } else { cp_async_wait<0>(); }
+    __syncthreads();
+    const float* as = sm + (s & 1) * CO_STAGE;
+    const float* bs = as + CC_ROWS * CC_ROWS;
+    if (s % tiles == 0) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    }
+    const int nk = min(CC_ROWS, K - s % tiles * CC_ROWS);
+#pragma unroll 8
+    for (int k = 0; k < nk; ++k) {               // (columns beyond dv hold what no one reads)
+      const float4 x = *reinterpret_cast<const float4*>(as + k * CC_ROWS + row);
+      const float4 y = *reinterpret_cast<const float4*>(bs + k * CO_COLS + lane * 4);
+      const float xv[4] = {x.x, x.y, x.z, x.w}, yv[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(xv[i], yv[j], acc[i][j]);
+    }
+    const int c = s / tiles * CO_COLS + lane * 4;
+    if (s % tiles == tiles - 1 && c < dv) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        *reinterpret_cast<float4*>(os + (row + i) * dv + c) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    }
+    __syncthreads();
+  }
+  pdl_launch_dependents_if_large();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {                  // (a warp finishes the rows it has made)
+    const int r = row + i;
+    if (r >= n) break;
+    const size_t t = (size_t)first + z * CC_ROWS + r;
+    float ss = 0.f;
+    for (int j = lane; j < dv; j += 32) ss = fmaf(os[r * dv + j], os[r * dv + j], ss);
+    const float inv = 1.0f / sqrtf(warp_sum(ss) / (float)dv + a.norm_eps);
+    const float* gate = cc_gate(a, t, h);
+    T* y = (T*)a.y + (t * H + h) * dv;
+    for (int j = lane; j < dv; j += 32) y[j] = from_f32<T>(os[r * dv + j] * inv * a.norm_w[j] * cc_gate_of(a, gate[j]));
+  }
+}
+
+template <typename Args, int COLS>
+static int delta_chain(const Args& a, cudaStream_t s) {
+  size_t smem = cc_chain_smem(a.dk, COLS);
+  const dim3 grid((a.dv + COLS - 1) / COLS, a.H, a.n_seqs);
+  // a grid that has an SM for every block: one block an SM, wherever it finds room first (two would
+  // halve each other's pace while other SMs stand idle)
+  if ((long long)grid.x * grid.y * grid.z <= 148 && smem < 120 * 1024) smem = 120 * 1024;
+  const cudaError_t e = cudaFuncSetAttribute(delta_chain_kernel<Args, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  return gb_launch(delta_chain_kernel<Args, COLS>, grid, dim3(256), smem, s, a);
+}
+
+// The two kernels behind the records of a step whose sequences bring at most max_rows rows.
+template <typename T, typename Args>
+static int delta_chain_and_out(const Args& a, int max_rows, cudaStream_t s) {
+  // 16 columns a block while that gives an SM at most one block
+  const long long narrow = (long long)((a.dv + 15) / 16) * a.H * a.n_seqs;
+  int e = narrow <= 148 ? delta_chain<Args, 16>(a, s) : delta_chain<Args, 32>(a, s);
+  if (e) return e;
+  const size_t smem = (2 * CO_STAGE + CC_ROWS * a.dv) * sizeof(float);
+  const cudaError_t ce = cudaFuncSetAttribute(delta_out_kernel<T, Args>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)smem);
+  if (ce != cudaSuccess) return (int)ce;
+  return gb_launch(delta_out_kernel<T, Args>, dim3((max_rows + CC_ROWS - 1) / CC_ROWS, a.H, a.n_seqs), dim3(256), smem, s, a);
+}

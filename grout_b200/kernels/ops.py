@@ -1793,7 +1793,12 @@ class _DeltaArgs(ctypes.Structure):
                 ("token_seq", _P), ("cu_q", _P), ("slots", _P), ("state", _P), ("state_stride", _L),
                 ("prep", _P), ("o", _P), ("y", _P), ("n_tokens", _I), ("n_seqs", _I), ("H", _I),
                 ("G", _I), ("dk", _I), ("dv", _I), ("taps", _I), ("unit_eps", _F), ("norm_eps", _F),
-                ("prep_stride", _I), ("few_rows", _I)]
+                ("prep_stride", _I), ("few_rows", _I), ("max_rows", _I), ("chunks", _P)]
+
+
+DELTA_CHUNK = 32                  # rows of a chunk of the kernels' chunked form (CC_ROWS)
+DELTA_CHUNK_MIN = 64              # a sequence of this many rows in a step: the step goes chunk by chunk (DC_MIN)
+DELTA_CHUNK_BYTES = 4 << 30       # scratch that a step's chunks may take; larger steps walk their rows
 
 
 def delta_state_floats(H: int, G: int, dk: int, dv: int, taps: int) -> int:
@@ -1819,7 +1824,8 @@ def delta_forward(proj: torch.Tensor, state: torch.Tensor, conv_w: torch.Tensor,
     sequences whose slot is not negative; ``conv_w`` [2 G dk + H dv, taps].  Returns
     y [T, H dv] in ``dtype``: every head's read-out, normalised over dv, times ``norm_w``
     and silu(gate).  ``max_rows``: the most rows any sequence of the step brings, when the
-    host knows it (a decode step: 1); steps of at most four rows a sequence take one launch less."""
+    host knows it (a decode step: 1); steps of at most four rows a sequence take one launch less, a
+    decode step takes one, and from ``DELTA_CHUNK_MIN`` rows on a step goes chunk by chunk."""
     _need(proj, "projection", torch.float32, 2)
     _need(state, "state", torch.float32, 2)
     Cc = 2 * G * dk + H * dv
@@ -1854,8 +1860,18 @@ def delta_forward(proj: torch.Tensor, state: torch.Tensor, conv_w: torch.Tensor,
     a.n_tokens, a.n_seqs, a.H, a.G, a.dk, a.dv, a.taps = T, n_seqs, H, G, dk, dv, taps
     a.unit_eps, a.norm_eps, a.prep_stride = float(unit_eps), float(norm_eps), prep_stride
     a.few_rows = 0 if max_rows is None or not 0 < max_rows <= 4 else (2 if max_rows == 1 else 1)
+    # (delta_step_takes of the kernels, for the count of launches)
+    one_kernel = (a.few_rows == 2 and dk <= 128 and dk % 4 == 0 and dv <= 128 and taps <= 8 and H // G <= 8 and
+                  n_seqs <= 65535 and state.stride(0) % 4 == 0 and (taps - 1) * Cc % 4 == 0 and state.data_ptr() % 16 == 0)
+    a.max_rows = int(max_rows or 0)
+    if a.max_rows >= DELTA_CHUNK_MIN and dk <= 128 and dk % 4 == 0 and dv % 4 == 0:
+        C = DELTA_CHUNK
+        n = (T // C + n_seqs) * H * (2 * dk * C + dk + (dk + C) * (C + dv))
+        if 4 * n <= DELTA_CHUNK_BYTES:
+            chunks = torch.empty(n, dtype=torch.float32, device=proj.device)
+            a.chunks = chunks.data_ptr()
     _check(_fn("delta", f"gb_delta_forward_{_suffix(dtype)}", "pp")(ctypes.addressof(a), _stream()),
-           "delta_forward", 3 if a.few_rows else 4)
+           "delta_forward", 1 if one_kernel else 3 if a.few_rows else 4)
     return y
 
 

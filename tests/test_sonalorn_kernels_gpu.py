@@ -185,6 +185,59 @@ def test_delta_rule_whole_in_portions_and_token_by_token(m):
     close(half, want, torch.bfloat16, "bfloat16 output")
 
 
+@pytest.mark.parametrize("m", [dict(heads=2, kv_heads=2, dim=128, vdim=128, conv=4), DELTA_SHAPES[0], DELTA_SHAPES[1],
+                               dict(heads=8, kv_heads=1, dim=64, vdim=48, conv=8), DELTA_SHAPES[3],
+                               dict(heads=16, kv_heads=4, dim=12, vdim=128, conv=3),
+                               dict(heads=2, kv_heads=1, dim=128, vdim=144, conv=2)])
+def test_delta_rule_chunk_by_chunk_and_step_by_step(m):
+    """When the host knows how many rows a sequence brings at most, prompts go chunk by chunk (32 rows) and decode
+    steps through one kernel: sequences of 1, 31, 32, 33, 64 and 100 rows in one step, a padding sequence and one
+    without rows between them, go on with 3 decode steps.  Against the plain rule, and against the kernels that
+    take any rows; strong and weak decays side by side; 32-bit sums of values of order one, a bar of 1e-5."""
+    from grout_b200.kernels import ops
+    H, G, dk, dv, taps = m["heads"], m["kv_heads"], m["dim"], m["vdim"], m["conv"]
+    W, lens, more = 24, [1, 31, 32, 33, 64, 100], 3
+    w = _delta_weights(H, G, dk, dv, taps, W, seed=13)
+    xs = [rnd(n + more, W, seed=14 + i) for i, n in enumerate(lens)]
+    g = lambda t: t.float().to(DEV).contiguous()  # noqa: E731
+    wp = torch.cat([w[k] for k in ("q", "k", "v", "g", "b", "a")], 0).double()
+    conv = g(torch.cat([w["q.conv"], w["k.conv"], w["v.conv"]], 0))
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+
+    def play(known):
+        state = torch.zeros(len(lens) + 1, ops.delta_state_floats(H, G, dk, dv, taps), device=DEV)
+        outs = [[] for _ in lens]
+
+        def step(parts, max_rows):            # parts: (sequence or -1, rows [n, W])
+            ns = [len(x) for _i, x in parts]
+            y = ops.delta_forward(
+                g(torch.cat([x for _i, x in parts]).double() @ wp.T), state, conv, g(w["A_log"]), g(w["dt_bias"]),
+                g(w["norm"]), H=H, G=G, dk=dk, dv=dv, taps=taps, unit_eps=1e-6, norm_eps=1e-5, dtype=torch.float32,
+                token_seq=i32([k for k, n in enumerate(ns) for _ in range(n)]),
+                cu_q=i32([0] + torch.tensor(ns).cumsum(0).tolist()), slots=i32([i for i, _x in parts]),
+                max_rows=max_rows if known else None).cpu()
+            for (i, _x), rows in zip(parts, torch.split(y, ns)):
+                if 0 <= i < len(lens):
+                    outs[i].append(rows)
+
+        firsts = [(i, x[:n]) for i, (n, x) in enumerate(zip(lens, xs))]
+        step(firsts[:3] + [(-1, rnd(40, W, seed=1)), (6, xs[0][:0])] + firsts[3:], max(lens))
+        for k in range(more):
+            order = [5, 0, 3, 1, 4, 2]
+            step([(i, xs[i][lens[i] + k:lens[i] + k + 1]) for i in order] + [(-1, xs[0][:1])], 1)
+        assert float(state[6].abs().max()) == 0.0
+        return [torch.cat(o) for o in outs], state
+
+    got, state = play(True)
+    old, old_state = play(False)
+    for i, x in enumerate(xs):
+        close(got[i], _delta_plain(w, m, x), torch.float32, str(lens[i]))
+        # (a read-out is normalised and gated, which scales its rounding, some 1e-7 of its largest terms, up with it: the
+        # bar goes with the largest value, which is beyond one)
+        assert float((got[i] - old[i]).abs().max()) < 1e-5 * max(1.0, float(old[i].abs().max())), lens[i]
+    assert float((state - old_state).abs().max()) < 1e-5 * max(1.0, float(old_state.abs().max()))
+
+
 def test_delta_rule_batches_slots_used_again_and_padding():
     from grout_b200.kernels import ops
     m = DELTA_SHAPES[0]
