@@ -13,7 +13,7 @@
 // are still on their way), the block's two consumer warps take 32 keys of every
 // tile each, with their own (max, sum, accumulator), and merge them at the end.
 //
-// With one split the block writes the output.  Otherwise it writes a 32-bit
+// With one split, or a sequence of a few tiles, the block writes the output.  Otherwise it writes a 32-bit
 // partial (accumulator relative to its max, max, sum) to scratch and counts
 // itself in at the (sequence, kv head)'s counter; the block that finds all
 // others counted combines the splits in split order,
@@ -32,6 +32,9 @@
 #include "tc_common.cuh"
 
 #define DA_BN 64                    // keys per tile: one page
+// Sequences of up to this many tiles are not split (a step of seven sequences, 36 layers, us: 54 keys 2,346 whole, 2,445 in
+// two; 250 keys 2,432 whole, 2,446 in two, 2,444 in three; 480 keys 2,561 whole, 2,476 in four).
+#define DA_WHOLE 4
 #define DA_WARPS 2                  // consumer warps; warp DA_WARPS holds the producer lane
 #define DA_CONSUMERS (DA_WARPS * 32)
 #define DA_THREADS (DA_CONSUMERS + 32)
@@ -114,8 +117,6 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k,
   // (both loads at once: the length does not wait for the slot)
   const int slot = a.slots[seq], len_seq = a.kv_len[seq];
   const int kv_len = slot < 0 ? 0 : len_seq;
-  const bool single = a.n_splits == 1;
-
   // key tiles of this split
   const int pos = kv_len - 1;
   const int key_lo = first_key(pos, a.window, a.chunk);
@@ -125,7 +126,10 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k,
   const int keep = a.window > 0 ? a.keep_first : 0;
   const int n_kept = min((min(keep, key_lo) + DA_BN - 1) / DA_BN, tile_lo);
   const int n_tiles = kv_len > 0 ? n_kept + pos / DA_BN - tile_lo + 1 : 0;
-  const int per_split = (n_tiles + a.n_splits - 1) / a.n_splits;
+  // a short sequence is one block's, whatever the step's longest is split into
+  const bool single = a.n_splits == 1 || n_tiles <= DA_WHOLE;
+  if (single && split > 0) return;
+  const int per_split = single ? n_tiles : (n_tiles + a.n_splits - 1) / a.n_splits;
   const int t_begin = split * per_split;
   const int t_end = min(n_tiles, t_begin + per_split);
   const int my_tiles = max(0, t_end - t_begin);

@@ -1537,13 +1537,17 @@ def decode_splits(n_seqs: int, nkv: int, max_kv_len: int, device) -> int:
     three per SM; with S splits a block streams 1/S of a sequence's 32-key tiles
     plus a fixed cost of about three tiles (query load, merge, partial store), so
     the step costs waves(S) * (tiles / S + 3).  The smallest S within 3 % of the
-    cheapest is taken, with at least 256 keys a split."""
+    cheapest is taken, with at least 128 keys a split, or 256 up to 512 keys, where the bound holds for sequences of any
+    length below it (40 keys: 2,330 us in two splits, 2,360 in four).  A decode step of one sequence of the 4B sizes, us: at 900 keys
+    2,440 in four, 2,352 in eight; 1,800 keys 2,447 in
+    eight, 2,414 in sixteen (four sequences: 2,689 in eight, 2,587 in twelve)."""
     if DECODE_SPLITS_OVERRIDE:
         return DECODE_SPLITS_OVERRIDE
     slots = 3 * _sm_count(device)
     pairs = max(1, n_seqs * nkv)
     tiles = max(1, (max_kv_len + 31) // 32)
-    most = max(1, min(64, (max_kv_len + 255) // 256))
+    least = 128 if max_kv_len > 512 else 256
+    most = max(1, min(64, (max_kv_len + least - 1) // least))
     cost = {s: ((pairs * s + slots - 1) // slots) * (tiles / s + 3.0) for s in range(1, most + 1)}
     best = min(cost.values())
     return min(s for s, c in cost.items() if c <= 1.03 * best)
@@ -1651,7 +1655,8 @@ def decode_tma_splits(n_seqs: int, nkv: int, max_kv_len: int, device, per_sm: in
     sequence's 64-key tiles plus a fixed cost of about six tiles (descriptor and
     block-table loads before the first copy, the partial store and the combining
     at the end), so the step costs waves(S) * (tiles / S + 6).  The smallest S
-    within 3 % of the cheapest is taken, with at least 256 keys a split.
+    within 3 % of the cheapest is taken, with at least 128 keys a split (seven sequences of 480 keys: a step of the 4B
+    sizes takes 2,476 us with four splits, 2,542 with two).
     Measured (us, 32 query and 8 kv heads of 128): 8 sequences of 2,049 keys 16.8
     with the 4 splits this picks (19.8 with 2, 21.7 with 8); 64 sequences 86.3 with
     1 (99.4 with 2); one sequence 9.1 with 8 or 9 (17.7 with 2)."""
@@ -1660,7 +1665,7 @@ def decode_tma_splits(n_seqs: int, nkv: int, max_kv_len: int, device, per_sm: in
     places = per_sm * _sm_count(device)
     pairs = max(1, n_seqs * nkv)
     tiles = max(1, (max_kv_len + 63) // 64)
-    most = max(1, min(64, (max_kv_len + 255) // 256))
+    most = max(1, min(64, (max_kv_len + 127) // 128))
     cost = {s: ((pairs * s + places - 1) // places) * (-(-tiles // s) + 6.0) for s in range(1, most + 1)}
     best = min(cost.values())
     return min(s for s, c in cost.items() if c <= 1.03 * best)
