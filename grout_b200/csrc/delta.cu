@@ -136,6 +136,80 @@ __global__ void __launch_bounds__(256) delta_prepare_kernel(const DeltaArgs a) {
   pdl_launch_dependents_if_large();
 }
 
+// The same for steps of many rows: a block takes a run of DP_RUN rows, a thread a channel of them (q and k of one kv
+// head, or 256 value channels), so an input is read once instead of once for each tap, all of a run's are on
+// their way together, and the sums of squares of all rows meet behind one barrier.  Bound by memory; 2,048 rows of 4,096
+// channels 32 us (80 with a block a row).
+#define DP_RUN 16
+#define DP_TAPS 8
+__global__ void __launch_bounds__(256) delta_prepare_rows_kernel(const DeltaArgs a) {
+  __shared__ float sums[DP_RUN][8];
+  pdl_launch_dependents_if_small();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, unit = blockIdx.y;
+  const int H = a.H, G = a.G, dk = a.dk, dv = a.dv, taps = a.taps;
+  const int Cc = 2 * G * dk + H * dv, C_all = Cc + H * dv + 2 * H, P = a.prep_stride;
+  const bool qk = unit < G, is_q = tid < dk;
+  const int c = !qk ? 2 * G * dk + (unit - G) * 256 + tid : is_q ? unit * dk + tid : (G + unit) * dk + (tid - dk);
+  const bool mine = qk ? tid < 2 * dk : c < Cc;
+  float w[DP_TAPS];                    // [j] meets the input j rows back
+#pragma unroll
+  for (int j = 0; j < DP_TAPS; ++j) w[j] = mine && j < taps ? a.conv_w[(size_t)c * taps + taps - 1 - j] : 0.f;
+  int seq, run;
+  run_of_block(a.cu_q, a.n_seqs, DP_RUN, false, blockIdx.x, seq, run);
+  const int first = a.cu_q[seq], n = min(DP_RUN, a.cu_q[seq + 1] - first - run * DP_RUN), row0 = first + run * DP_RUN;
+  if (n <= 0) return;
+  const int slot = a.slots[seq];
+  pdl_wait();
+  float x[DP_RUN + DP_TAPS - 1];       // the DP_TAPS - 1 inputs in front of the run, then the run's
+#pragma unroll
+  for (int i = 0; i < DP_TAPS - 1; ++i) {
+    const int back = DP_TAPS - 1 - i;  // so many rows in front of the run's first
+    x[i] = 0.f;
+    if (!mine || back >= taps) continue;
+    if (run > 0) x[i] = a.proj[(size_t)(row0 - back) * C_all + c];
+    else if (slot >= 0) x[i] = a.state[(size_t)slot * a.state_stride + (size_t)(taps - 1 - back) * Cc + c];
+  }
+#pragma unroll
+  for (int i = 0; i < DP_RUN; ++i) x[DP_TAPS - 1 + i] = mine && i < n ? a.proj[(size_t)(row0 + i) * C_all + c] : 0.f;
+  float y[DP_RUN];
+#pragma unroll
+  for (int i = 0; i < DP_RUN; ++i) {
+    float acc = 0.f;
+#pragma unroll
+    for (int j = 0; j < DP_TAPS; ++j) acc = fmaf(w[j], x[DP_TAPS - 1 + i - j], acc);
+    y[i] = silu_f(acc);
+  }
+  float* out = a.prep + (size_t)row0 * P + c;
+  if (!qk) {
+#pragma unroll
+    for (int i = 0; i < DP_RUN; ++i)
+      if (mine && i < n) out[(size_t)i * P] = y[i];
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < DP_RUN; ++i) {   // (a warp is all q, all k or idle)
+    const float ss = warp_sum(mine ? y[i] * y[i] : 0.f);
+    if (lane == 0) sums[i][warp] = ss;
+  }
+  __syncthreads();
+  const int w0 = is_q ? 0 : dk / 32;
+  const float scale = is_q ? 1.0f / sqrtf((float)dk) : 1.0f;
+#pragma unroll
+  for (int i = 0; i < DP_RUN; ++i) {
+    float ss = 0.f;
+    for (int u = 0; u < dk / 32; ++u) ss += sums[i][min(7, w0 + u)];
+    if (mine && i < n) out[(size_t)i * P] = y[i] * (1.0f / sqrtf(ss + a.unit_eps) * scale);
+  }
+  if (unit == 0)
+    for (int i = tid; i < n * H; i += 256) {
+      const int t = row0 + i / H, h = i % H;
+      const float* row = a.proj + (size_t)t * C_all + Cc + H * dv;
+      a.prep[(size_t)t * P + Cc + h] = 1.0f / (1.0f + expf(-row[h]));
+      a.prep[(size_t)t * P + Cc + H + h] = expf(-expf(a.a_log[h]) * softplus_f(row[H + h] + a.dt_bias[h]));
+    }
+  pdl_launch_dependents_if_large();
+}
+
 // The new tail of a sequence; the caller's threads share the channels: first, first + step, ...
 __device__ __forceinline__ void delta_keep_tail(const DeltaArgs& a, int seq, int first, int step) {
   const int slot = a.slots[seq];
@@ -794,8 +868,12 @@ static int delta_forward(const DeltaArgs& a, cudaStream_t s) {
   if (delta_step_takes(a))
     return gb_launch_cluster(delta_step_kernel<T>, dim3(a.H, a.n_seqs), dim3(256), 0, s, a.H / a.G, a);
   const int units = a.G + (a.H * a.dv + DELTA_PREP_V - 1) / DELTA_PREP_V;
-  e = gb_launch(delta_prepare_kernel, dim3(a.n_tokens, units), dim3(256),
-                (size_t)2 * a.dk * sizeof(float), s, a);
+  if (!a.few_rows && a.n_tokens >= 4 * DP_RUN && a.dk % 32 == 0 && a.dk <= 128 && a.taps <= DP_TAPS) {
+    const int runs = a.n_tokens / DP_RUN + a.n_seqs;         // (run_of_block)
+    e = gb_launch(delta_prepare_rows_kernel, dim3(runs, a.G + (a.H * a.dv + 255) / 256), dim3(256), 0, s, a);
+  } else {
+    e = gb_launch(delta_prepare_kernel, dim3(a.n_tokens, units), dim3(256), (size_t)2 * a.dk * sizeof(float), s, a);
+  }
   if (e) return e;
   if (delta_chunks_take(a)) return delta_by_chunks<T>(a, s);
   if (!a.few_rows) {
