@@ -688,7 +688,7 @@ static bool delta_step_takes(const DeltaArgs& a) {
 // (quotients are products of the g between).  This kernel takes every chunk of every head at the same time, solves
 // the triangular system for the right-hand sides beta v and beta c k, and leaves the record.  The scan below
 // walks 2,048 rows (16 heads of 128) in 512 turns of a microsecond, 502 us and 36 for their products; this kernel takes
-// 56 us, the two behind it 140 and 64 (with the norm and the gate, which took 40 more behind the scan).
+// 56 us, the two behind it 135 and 64 (with the norm and the gate, which took 40 more behind the scan).
 #define DC_MIN 64         // a step goes chunk by chunk when a sequence may bring this many rows
 __global__ void __launch_bounds__(256, 2) delta_local_kernel(const DeltaArgs a) {
   constexpr int LD = CC_MAX_DK + 4;

@@ -35,28 +35,16 @@ __device__ __forceinline__ void cc_copy16(float* smem, const float* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem));
 }
 
-typedef unsigned long long cc_pair;      // two 32-bit numbers
-__device__ __forceinline__ cc_pair cc_both(float a) {
-  cc_pair r;
-  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
-  return r;
-}
-__device__ __forceinline__ void cc_fma2(cc_pair& d, cc_pair a, cc_pair b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
-}
-__device__ __forceinline__ void cc_unpack(cc_pair v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-
 // floats of a chain block's stage: W | Kd | gC | U0's columns
 __host__ __device__ __forceinline__ int cc_stage(int dk, int cols) { return 2 * dk * CC_ROWS + dk + CC_ROWS * cols; }
 __host__ __device__ __forceinline__ size_t cc_chain_smem(int dk, int cols) {   // two stages, S, partial sums, U
   return (size_t)(2 * cc_stage(dk, cols) + dk * cols + (128 / cols + 1) * CC_ROWS * cols) * sizeof(float);
 }
 
-// Bound by a chunk's chain of three steps with a barrier behind each, so what counts is how few instructions a thread has
-// between them: packed multiply-adds over pairs of rows, and, where a step has few sequences and heads, 16 columns a
-// block: 64 chunks of one sequence and 16 heads of 128 in 140 us, 2.2 a chunk.
+// Bound by a chunk's chain of three steps with a barrier behind each and, in a block of 32 columns, by their
+// multiply-adds; so where a step has few sequences and heads a block has 16 columns: 64 chunks of one sequence and 16
+// heads of 128 in 135 us, 2.1 a chunk.  (Multiply-adds packed two by two were no faster, 140 us: every pair of equal
+// factors has to be made first.)
 template <typename Args, int COLS>
 __global__ void __launch_bounds__(256) delta_chain_kernel(const Args a) {
   static_assert(COLS == 16 || COLS == 32, "columns of a block");
@@ -112,32 +100,26 @@ __global__ void __launch_bounds__(256) delta_chain_kernel(const Args a) {
     const float* gc = kd + CC_ROWS * dk;
     const float* u0 = gc + dk;
     float* su = record(z) + cc_at_su(dk) + col0;
-    cc_pair acc[2][4];                           // [pair of rows][column]
+    float acc[4][4];
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
 #pragma unroll 8
     for (int k = k_lo; k < k_hi; ++k) {
-      const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(w + k * CC_ROWS + tr);
+      const float4 x = *reinterpret_cast<const float4*>(w + k * CC_ROWS + tr);
+      const float xv[4] = {x.x, x.y, x.z, x.w};
       const float4 y = *reinterpret_cast<const float4*>(S + k * COLS + tc);
       const float yv[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const cc_pair yy = cc_both(yv[j]);
-        cc_fma2(acc[0][j], x.x, yy);
-        cc_fma2(acc[1][j], x.y, yy);
-      }
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(xv[i], yv[j], acc[i][j]);
     }
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      float lo[4], hi[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) cc_unpack(acc[i][j], lo[j], hi[j]);
-      float* p = P + (part * CC_ROWS + tr + 2 * i) * COLS + tc;
-      *reinterpret_cast<float4*>(p) = make_float4(lo[0], lo[1], lo[2], lo[3]);
-      *reinterpret_cast<float4*>(p + COLS) = make_float4(hi[0], hi[1], hi[2], hi[3]);
-    }
+    for (int i = 0; i < 4; ++i)
+      *reinterpret_cast<float4*>(P + (part * CC_ROWS + tr + i) * COLS + tc) =
+          make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
     __syncthreads();
     for (int i = tid * 4; i < CC_ROWS * COLS; i += 1024) {  // U = U0 - W S, four columns of a row a thread
       float4 u = *reinterpret_cast<const float4*>(u0 + i);
@@ -151,43 +133,39 @@ __global__ void __launch_bounds__(256) delta_chain_kernel(const Args a) {
     }
     __syncthreads();
     if (sk < dk) {                               // S <- diag(gC) S + Kd^T U
-      cc_pair s[2][SC];                          // [pair of rows][column]
+      float s[4][SC];
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        float lo[SC], hi[SC];
-#pragma unroll
-        for (int j = 0; j < SC; ++j) lo[j] = S[(sk + 2 * i) * COLS + sc + j], hi[j] = S[(sk + 2 * i + 1) * COLS + sc + j];
+      for (int i = 0; i < 4; ++i) {
+        const float g = gc[sk + i];
+        float x[SC];
+        if constexpr (SC == 4) *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(S + (sk + i) * COLS + sc);
+        else *reinterpret_cast<float2*>(x) = *reinterpret_cast<const float2*>(S + (sk + i) * COLS + sc);
         if (col_in) {
-          float* to = su + (size_t)(sk + 2 * i) * dv + sc;
-          if constexpr (SC == 4) {
-            *reinterpret_cast<float4*>(to) = make_float4(lo[0], lo[1], lo[2], lo[3]);
-            *reinterpret_cast<float4*>(to + dv) = make_float4(hi[0], hi[1], hi[2], hi[3]);
-          } else {
-            *reinterpret_cast<float2*>(to) = make_float2(lo[0], lo[1]);
-            *reinterpret_cast<float2*>(to + dv) = make_float2(hi[0], hi[1]);
-          }
+          float* to = su + (size_t)(sk + i) * dv + sc;
+          if constexpr (SC == 4) *reinterpret_cast<float4*>(to) = *reinterpret_cast<const float4*>(x);
+          else *reinterpret_cast<float2*>(to) = *reinterpret_cast<const float2*>(x);
         }
-        const float g0 = gc[sk + 2 * i], g1 = gc[sk + 2 * i + 1];
 #pragma unroll
-        for (int j = 0; j < SC; ++j) {
-          const float x = g0 * lo[j], y = g1 * hi[j];
-          asm("mov.b64 %0, {%1, %2};" : "=l"(s[i][j]) : "f"(x), "f"(y));
-        }
+        for (int j = 0; j < SC; ++j) s[i][j] = g * x[j];
       }
 #pragma unroll 8
       for (int t = 0; t < CC_ROWS; ++t) {
-        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(kd + t * dk + sk);
+        const float4 x = *reinterpret_cast<const float4*>(kd + t * dk + sk);
+        const float xv[4] = {x.x, x.y, x.z, x.w};
+        float y[SC];
+        if constexpr (SC == 4) *reinterpret_cast<float4*>(y) = *reinterpret_cast<const float4*>(U + t * COLS + sc);
+        else *reinterpret_cast<float2*>(y) = *reinterpret_cast<const float2*>(U + t * COLS + sc);
 #pragma unroll
-        for (int j = 0; j < SC; ++j) {
-          const cc_pair yy = cc_both(U[t * COLS + sc + j]);
-          cc_fma2(s[0][j], x.x, yy);
-          cc_fma2(s[1][j], x.y, yy);
-        }
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < SC; ++j) s[i][j] = fmaf(xv[i], y[j], s[i][j]);
       }
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < SC; ++j) cc_unpack(s[i][j], S[(sk + 2 * i) * COLS + sc + j], S[(sk + 2 * i + 1) * COLS + sc + j]);
+      for (int i = 0; i < 4; ++i) {
+        float* to = S + (sk + i) * COLS + sc;
+        if constexpr (SC == 4) *reinterpret_cast<float4*>(to) = make_float4(s[i][0], s[i][1], s[i][2], s[i][3]);
+        else *reinterpret_cast<float2*>(to) = make_float2(s[i][0], s[i][1]);
+      }
     }
     __syncthreads();                             // S is whole, the stage and P may be overwritten
   }
