@@ -338,8 +338,7 @@ __global__ void __launch_bounds__(256) channel_delta_step_kernel(const ChannelDe
                           : nullptr;
   const bool wide = (dk & 3) == 0 && (((uintptr_t)head) & 15) == 0;
   if (head)                                       // on its way to L2 while the kernel before drains
-    for (int i = tid * 32; i < dk * dv; i += 256 * 32)
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(head + i));
+    for (int i = tid * 32; i < dk * dv; i += 256 * 32) prefetch_l2(head + i);
   pdl_wait();
   if (a.cu_q[seq + 1] - t <= 0) return;
   const float* p = a.prep + (size_t)t * a.prep_stride;

@@ -85,6 +85,10 @@ __device__ __forceinline__ void pdl_launch_dependents() {
 #endif
 }
 
+// A line on its way to L2.  It carries no data into the kernel, so it may be asked for before pdl_wait() even where
+// another kernel still writes it.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // A kernel whose whole grid is resident at once (a handful of blocks) loses
 // nothing by letting its successor in on entry, and the successor (typically a
 // matrix product) can then stream its weights while this kernel runs.

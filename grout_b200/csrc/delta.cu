@@ -540,10 +540,11 @@ __global__ void delta_finish_kernel(const DeltaArgs a) {
 // ---- a decode step in one kernel ---------------------------------------------
 // Every sequence brings one row: a block per head and sequence does all of the mixer for it.  Bound by latency (a
 // head's state is 64 KB; three kernels of few blocks were 20 us of a step of one sequence and 16 heads of 128, each its
-// own hand-over; this is 4.7), so the state, the kept inputs and the weights, which no kernel of this step writes, are
-// requested before the wait.  A column of the state is in eight lanes' registers, four columns a thread.  The heads
-// that share q and k are a cluster: all of them read the kept inputs of q and k, and the first replaces them when all
-// have.
+// own hand-over; this is 4.7), so the weights, which no kernel writes, are requested before the wait, and the state and
+// the kept inputs are on their way to L2 by then.  They are read behind it: the kernel in front may be another step of
+// the same sequences, which writes both at its end.  A column of the state is in eight lanes' registers, four columns a
+// thread.  The heads that share q and k are a cluster: all of them read the kept inputs of q and k, and the first
+// replaces them when all have.
 #define DS_COLS 128       // columns of a head: 4 passes of 32
 #define DS_TAPS 8
 template <typename T>
@@ -558,6 +559,32 @@ __global__ void __launch_bounds__(256) delta_step_kernel(const DeltaArgs a) {
   float* st = slot >= 0 ? a.state + (size_t)slot * a.state_stride : nullptr;
   float* sp = st ? st + (size_t)(taps - 1) * Cc + (size_t)h * dv * dk : nullptr;
   const int l = tid & 7, c0 = tid >> 3;
+  // this thread's channel of q or k, and of v
+  const bool is_q = tid < dk, is_qk = tid < 2 * dk, is_v = tid < dv;
+  const int cq = is_q ? kvh * dk + tid : (G + kvh) * dk + (tid - dk), cv = 2 * G * dk + h * dv + tid;
+  if (st) {                                      // (32 bytes a request of the kept inputs, whose rows start anywhere)
+    for (int i = tid * 32; i < dk * dv; i += 256 * 32) prefetch_l2(sp + i);
+    if (lane % 8 == 0)
+      for (int j = 1; j < taps; ++j) {
+        if (is_qk) prefetch_l2(st + (size_t)(taps - 1 - j) * Cc + cq);
+        if (is_v) prefetch_l2(st + (size_t)(taps - 1 - j) * Cc + cv);
+      }
+  }
+  float w_q[DS_TAPS], w_v[DS_TAPS];              // [j]: of the input j rows back
+#pragma unroll
+  for (int j = 0; j < DS_TAPS; ++j) {
+    w_q[j] = j < taps && is_qk ? a.conv_w[(size_t)cq * taps + taps - 1 - j] : 0.f;
+    w_v[j] = j < taps && is_v ? a.conv_w[(size_t)cv * taps + taps - 1 - j] : 0.f;
+  }
+  const float rate = expf(a.a_log[h]), dt = a.dt_bias[h], nw = is_v ? a.norm_w[tid] : 0.f;
+  pdl_wait();
+  float kept_q[DS_TAPS], kept_v[DS_TAPS];
+#pragma unroll
+  for (int j = 1; j < DS_TAPS; ++j) {
+    kept_q[j] = st && j < taps && is_qk ? st[(size_t)(taps - 1 - j) * Cc + cq] : 0.f;
+    kept_v[j] = st && j < taps && is_v ? st[(size_t)(taps - 1 - j) * Cc + cv] : 0.f;
+  }
+  kept_q[0] = kept_v[0] = 0.f;
   float4 S[4][4];
 #pragma unroll
   for (int p = 0; p < 4; ++p)
@@ -567,24 +594,6 @@ __global__ void __launch_bounds__(256) delta_step_kernel(const DeltaArgs a) {
       S[p][i] = sp && c < dv && e < dk ? *reinterpret_cast<const float4*>(sp + (size_t)c * dk + e)
                                        : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-  // this thread's channel of q or k, and of v
-  const bool is_q = tid < dk, is_qk = tid < 2 * dk, is_v = tid < dv;
-  const int cq = is_q ? kvh * dk + tid : (G + kvh) * dk + (tid - dk), cv = 2 * G * dk + h * dv + tid;
-  float kept_q[DS_TAPS], kept_v[DS_TAPS], w_q[DS_TAPS], w_v[DS_TAPS];      // [j]: the input j rows back
-#pragma unroll
-  for (int j = 0; j < DS_TAPS; ++j) {
-    kept_q[j] = kept_v[j] = w_q[j] = w_v[j] = 0.f;
-    if (j < taps) {
-      if (is_qk) w_q[j] = a.conv_w[(size_t)cq * taps + taps - 1 - j];
-      if (is_v) w_v[j] = a.conv_w[(size_t)cv * taps + taps - 1 - j];
-      if (st && j > 0) {
-        if (is_qk) kept_q[j] = st[(size_t)(taps - 1 - j) * Cc + cq];
-        if (is_v) kept_v[j] = st[(size_t)(taps - 1 - j) * Cc + cv];
-      }
-    }
-  }
-  const float rate = expf(a.a_log[h]), dt = a.dt_bias[h], nw = is_v ? a.norm_w[tid] : 0.f;
-  pdl_wait();
   const float* row = a.proj + (size_t)t * C_all;
   if (is_qk) kept_q[0] = row[cq];
   float gate = 0.f;

@@ -238,6 +238,47 @@ def test_delta_rule_chunk_by_chunk_and_step_by_step(m):
     assert float((state - old_state).abs().max()) < 1e-5 * max(1.0, float(old_state.abs().max()))
 
 
+@pytest.mark.parametrize("n_seqs,m", [(1, dict(heads=16, kv_heads=16, dim=128, vdim=128, conv=4)),
+                                      (3, dict(heads=8, kv_heads=2, dim=64, vdim=96, conv=3))])
+def test_delta_decode_steps_queued_behind_one_another(n_seqs, m):
+    """Decode steps of one state with nothing between them (all arguments made beforehand, then captured in one graph)
+    give the bits of steps that are waited for one by one: a step sees the state and the kept inputs that the step in
+    front of it left."""
+    from grout_b200.kernels import ops
+    H, G, dk, dv, taps = m["heads"], m["kv_heads"], m["dim"], m["vdim"], m["conv"]
+    W, steps = 24, 12
+    w = _delta_weights(H, G, dk, dv, taps, W, seed=23)
+    g = lambda t: t.float().to(DEV).contiguous()  # noqa: E731
+    wp = torch.cat([w[k] for k in ("q", "k", "v", "g", "b", "a")], 0).double()
+    projs = [g(rnd(n_seqs, W, seed=30 + i).double() @ wp.T) for i in range(steps)]
+    args = (g(torch.cat([w["q.conv"], w["k.conv"], w["v.conv"]], 0)), g(w["A_log"]), g(w["dt_bias"]), g(w["norm"]))
+    i32 = lambda n: torch.arange(n, dtype=torch.int32, device=DEV)  # noqa: E731
+    kw = dict(H=H, G=G, dk=dk, dv=dv, taps=taps, unit_eps=1e-6, norm_eps=1e-5, dtype=torch.float32, max_rows=1,
+              token_seq=i32(n_seqs), cu_q=i32(n_seqs + 1), slots=i32(n_seqs))
+    state = torch.zeros(n_seqs, ops.delta_state_floats(H, G, dk, dv, taps), device=DEV)
+
+    def play(wait):
+        out = []
+        for p in projs:
+            out.append(ops.delta_forward(p, state, *args, **kw))
+            if wait:
+                torch.cuda.synchronize()
+        return out
+
+    want, last = play(True), state.clone()
+    assert float((want[1] - want[0]).abs().max()) > 0.01
+    state.zero_()
+    torch.cuda.synchronize()
+    got = play(False)
+    assert all(torch.equal(a, b) for a, b in zip(got, want)) and torch.equal(state, last)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = play(False)
+    state.zero_()
+    graph.replay()
+    assert all(torch.equal(a, b) for a, b in zip(got, want)) and torch.equal(state, last)
+
+
 def test_delta_rule_batches_slots_used_again_and_padding():
     from grout_b200.kernels import ops
     m = DELTA_SHAPES[0]
