@@ -545,10 +545,14 @@ __global__ void delta_finish_kernel(const DeltaArgs a) {
 // the same sequences, which writes both at its end.  A column of the state is in eight lanes' registers, four columns a
 // thread.  The heads that share q and k are a cluster: all of them read the kept inputs of q and k, and the first
 // replaces them when all have.
+// From some ten sequences on it is bound by the states' way through memory, and two blocks an SM (128 registers a thread)
+// keep it busy while one of them waits.  Projection, rule and output product of a layer of 16 heads on 8 at 1, 4, 8, 16,
+// 32 and 64 sequences, us: 20.7, 23.2, 23.2, 25.3, 39.5 and 67.4; with one block an SM 21.1, 22.9, 23.0, 29.8, 47.0 and
+// 80.5; prepare, scan and finish 28.6, 31.0, 30.8, 35.3, 48.5 and 74.9.
 #define DS_COLS 128       // columns of a head: 4 passes of 32
 #define DS_TAPS 8
 template <typename T>
-__global__ void __launch_bounds__(256) delta_step_kernel(const DeltaArgs a) {
+__global__ void __launch_bounds__(256, 2) delta_step_kernel(const DeltaArgs a) {
   __shared__ float q_s[128], k_s[128], v_s[DS_COLS], o_s[DS_COLS], sums[2][8];
   pdl_launch_dependents_if_small();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;

@@ -239,7 +239,8 @@ def test_delta_rule_chunk_by_chunk_and_step_by_step(m):
 
 
 @pytest.mark.parametrize("n_seqs,m", [(1, dict(heads=16, kv_heads=16, dim=128, vdim=128, conv=4)),
-                                      (3, dict(heads=8, kv_heads=2, dim=64, vdim=96, conv=3))])
+                                      (3, dict(heads=8, kv_heads=2, dim=64, vdim=96, conv=3)),
+                                      (40, dict(heads=16, kv_heads=4, dim=64, vdim=64, conv=4))])
 def test_delta_decode_steps_queued_behind_one_another(n_seqs, m):
     """Decode steps of one state with nothing between them (all arguments made beforehand, then captured in one graph)
     give the bits of steps that are waited for one by one: a step sees the state and the kept inputs that the step in
