@@ -1537,18 +1537,23 @@ def decode_splits(n_seqs: int, nkv: int, max_kv_len: int, device) -> int:
     three per SM; with S splits a block streams 1/S of a sequence's 32-key tiles
     plus a fixed cost of about three tiles (query load, merge, partial store), so
     the step costs waves(S) * (tiles / S + 3).  The smallest S within 3 % of the
-    cheapest is taken, with at least 128 keys a split, or 256 up to 512 keys, where the bound holds for sequences of any
-    length below it (40 keys: 2,330 us in two splits, 2,360 in four).  A decode step of one sequence of the 4B sizes, us: at 900 keys
-    2,440 in four, 2,352 in eight; 1,800 keys 2,447 in
-    eight, 2,414 in sixteen (four sequences: 2,689 in eight, 2,587 in twelve)."""
+    cheapest is taken, with at least 256 keys a split, or, for bounds of 513 to 2,048 keys,
+    128 keys and up to eight splits, or sixteen.  A decode step of the 4B sizes, us, with
+    128 and with 256 keys a split: one sequence of 800 keys 2,384 / 2,442, 970 2,384 / 2,440, 1,100
+    2,419 / 2,400 (the bound is 2,048 then), 1,500 2,436 / 2,427, 1,950 2,411 / 2,467; four
+    of 970 2,502 / 2,542, of 1,900 2,643 (twelve splits; thirteen 2,665) / 2,634.  Beyond 2,048
+    keys the merge of so many parts costs more than shorter splits give: one sequence of 4,000 keys 2,595 (31
+    splits) / 2,505, of 5,000 2,760 / 2,598, two of 4,000 2,735 / 2,615.  Up to 512 the bound holds for sequences
+    of any length below it: 40 keys 2,330 in two splits, 2,360 in four."""
     if DECODE_SPLITS_OVERRIDE:
         return DECODE_SPLITS_OVERRIDE
     slots = 3 * _sm_count(device)
     pairs = max(1, n_seqs * nkv)
     tiles = max(1, (max_kv_len + 31) // 32)
-    least = 128 if max_kv_len > 512 else 256
-    most = max(1, min(64, (max_kv_len + least - 1) // least))
-    cost = {s: ((pairs * s + slots - 1) // slots) * (tiles / s + 3.0) for s in range(1, most + 1)}
+    fine = 512 < max_kv_len <= 2048
+    most = max(1, min(64, -(-max_kv_len // (128 if fine else 256))))
+    cost = {s: ((pairs * s + slots - 1) // slots) * (tiles / s + 3.0) for s in range(1, most + 1)
+            if not fine or s <= 8 or s == 16}
     best = min(cost.values())
     return min(s for s, c in cost.items() if c <= 1.03 * best)
 

@@ -146,3 +146,19 @@ def test_the_blocks_a_kernel_sizes_its_grid_with():
     assert ctx.q_blocks(64) == 2 + 1 + 1 and ctx.q_blocks(128) == 3
     ctx.q_lens = ()                          # a captured step: the most the rows can make
     assert ctx.q_blocks(64) == 137 // 64 + 3 >= 4
+
+
+def test_the_splits_of_decode_attention(monkeypatch):
+    """At least 256 keys a split, as beyond 2,048 keys no finer split was faster; 128 from 513 to 2,048, in counts of up
+    to eight, or sixteen."""
+    from grout_b200.kernels import ops
+    monkeypatch.setattr(ops, "_sm_count", lambda device: 148)
+    splits = lambda n, bound: ops.decode_splits(n, 8, bound, "cuda")  # noqa: E731
+    assert [splits(1, b) for b in (512, 1024, 2048, 4096, 8192)] == [2, 8, 16, 16, 31]
+    assert [splits(4, b) for b in (512, 1024, 2048, 4096)] == [2, 8, 8, 13]
+    for n in range(1, 8):
+        for bound in range(1, 20000, 37):
+            s = splits(n, bound)
+            fine = 512 < bound <= 2048
+            assert 1 <= s <= max(1, -(-bound // (128 if fine else 256)))
+            assert not fine or s <= 8 or s == 16
