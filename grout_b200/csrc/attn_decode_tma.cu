@@ -57,6 +57,7 @@ struct DecodeTmaArgs {
   ScoreCap cap;            // the score cap (off when cap_log2 == 0)
   int keep_first;          // with a window: a sequence's first keep_first keys stay visible behind it
   int chunk;               // > 0: a query sees the keys of its own chunk of positions only
+  int ordered;             // 1: blocks take the sequences by length (2 to DA_ORDERED of them)
 };
 
 #define DA_STAMP(slot)                                                                          \
@@ -69,26 +70,44 @@ __device__ __forceinline__ void consumer_sync() {
   asm volatile("bar.sync 1, %0;" ::"n"(DA_CONSUMERS) : "memory");
 }
 
-// The sequence whose keys are the r-th most (ties by index), for whole warps.  Blocks start in the order of their
-// index, so the longest sequences' go first and the short ones fill the gaps at the end: 64 sequences of 25 to 708 keys
-// in an order without a trend 18.0 us instead of 23.5.  Up to 64 sequences; more are taken as they
-// come, which many waves of blocks even out.
+// The sequence a block takes, its slot and its length: the r-th longest one (ties by index).  Blocks start in the order
+// of their index, so with more blocks than the GPU holds at once the longest sequences' go first and the short ones fill
+// the gaps at the end.  32 query heads on 8, us, in an order without a trend, ordered / as they come: 64 sequences of 25
+// to 708 keys 15.9 / 22.0; 64 equal ones of 60 keys 10.1 / 9.3 (the finding, which a step does before its wait), of 900
+// 48.1 / 48.1.  Lengths and slots come together,
+// a thread a sequence, so that finding the sequence costs no second trip to memory.  A step that fits at once is taken as it
+// comes (32 sequences of 25 to 708 keys 14.2; ordered 14.6), and so are more than 64 sequences, which
+// would gain up to 192 of them (65: 21.6, and 15.4 where the caller has the longest first; 96: 26.7 and 22.2; 128: 35.0
+// and 31.9; 192: 47.2 and 46.8).
 #define DA_ORDERED 64
-__device__ __forceinline__ int seq_of_rank(const int* kv_len, int n_seqs, int r) {
-  if (n_seqs > DA_ORDERED || n_seqs < 2) return r;
-  const int lane = threadIdx.x & 31;
-  const int a = lane < n_seqs ? kv_len[lane] : -1, b = lane + 32 < n_seqs ? kv_len[lane + 32] : -1;
-  int above_a = 0, above_b = 0;                  // sequences in front of this lane's two
-#pragma unroll 8
-  for (int i = 0; i < 32; ++i) {
-    const int x = __shfl_sync(0xffffffffu, a, i), y = __shfl_sync(0xffffffffu, b, i);
-    above_a += (x > a || (x == a && i < lane)) + (y > a);
-    above_b += (x >= b) + (y > b || (y == b && i < lane));
+__device__ __forceinline__ void sequence_of_block(const DecodeTmaArgs& a, int r, int& seq, int& slot, int& len) {
+  if (!a.ordered) {
+    seq = r, slot = a.slots[r], len = a.kv_len[r];
+    return;
   }
-  const uint32_t in_a = __ballot_sync(0xffffffffu, lane < n_seqs && above_a == r);
-  const uint32_t in_b = __ballot_sync(0xffffffffu, lane + 32 < n_seqs && above_b == r);
-  return in_a ? __ffs(in_a) - 1 : 31 + __ffs(in_b);
+  __shared__ __align__(16) uint32_t keys[DA_ORDERED];      // longer ones are larger, and no two are equal
+  __shared__ int found[3];
+  const int i = threadIdx.x;
+  int my_len = 0, my_slot = -1;
+  if (i < DA_ORDERED) {
+    if (i < a.n_seqs) my_len = a.kv_len[i], my_slot = a.slots[i];
+    keys[i] = i < a.n_seqs ? (uint32_t)min(my_len, 1 << 25) * DA_ORDERED + (DA_ORDERED - i) : 0u;
+  }
+  __syncthreads();
+  if (i < a.n_seqs) {
+    const uint32_t mine = keys[i];
+    int above = 0;
+#pragma unroll
+    for (int j = 0; j < DA_ORDERED; j += 4) {
+      const uint4 k = *reinterpret_cast<const uint4*>(keys + j);
+      above += (k.x > mine) + (k.y > mine) + (k.z > mine) + (k.w > mine);
+    }
+    if (above == r) found[0] = i, found[1] = my_slot, found[2] = my_len;
+  }
+  __syncthreads();
+  seq = found[0], slot = found[1], len = found[2];
 }
+static_assert(DA_ORDERED <= DA_THREADS, "a thread a sequence");
 
 template <int DS, int STAGES>   // D = 64 * DS
 __global__ void __launch_bounds__(DA_THREADS)
@@ -111,11 +130,11 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k,
   volatile int* issued = &issued_s;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int split = blockIdx.x, kvh = blockIdx.y, seq = seq_of_rank(a.kv_len, a.n_seqs, blockIdx.z);
+  const int split = blockIdx.x, kvh = blockIdx.y;
   const int G = a.nq / a.nkv;
   const int h0 = kvh * G;
-  // (both loads at once: the length does not wait for the slot)
-  const int slot = a.slots[seq], len_seq = a.kv_len[seq];
+  int seq, slot, len_seq;
+  sequence_of_block(a, blockIdx.z, seq, slot, len_seq);
   const int kv_len = slot < 0 ? 0 : len_seq;
   // key tiles of this split
   const int pos = kv_len - 1;
@@ -462,6 +481,7 @@ GB_EXPORT int gb_attn_decode_tma(const void* k_pages, const void* v_pages, long 
   if ((D != 64 && D != 128) || a->nq / a->nkv > 16 || page != DA_BN) return GB_ERR_UNSUPPORTED;
   if (a->n_seqs > 65535 || a->nkv > 65535) return GB_ERR_UNSUPPORTED;
   if (a->n_seqs == 0) return 0;
+  if (a->ordered && (a->n_seqs < 2 || a->n_seqs > DA_ORDERED)) return GB_ERR_BAD_ARG;
   const uint64_t rows = (uint64_t)n_pages * a->nkv * page;
   if (rows > 0x7fffffffull) return GB_ERR_UNSUPPORTED;       // TMA coordinates are 32-bit
   CUtensorMap mk, mv;

@@ -1626,9 +1626,10 @@ class _DecodeTmaArgs(ctypes.Structure):
                 ("part_o", _P), ("part_ml", _P), ("counters", _P), ("error", _P), ("n_seqs", _I),
                 ("nq", _I), ("nkv", _I), ("max_pages", _I), ("window", _I), ("n_splits", _I),
                 ("scale_log2", _F), ("stamps", _P), ("sinks", _P), ("cap_log2", _F),
-                ("cap_inv", _F), ("keep_first", _I), ("chunk", _I)]
+                ("cap_inv", _F), ("keep_first", _I), ("chunk", _I), ("ordered", _I)]
 
 
+DECODE_TMA_ORDERED = 64       # the most sequences that are taken by length (DA_ORDERED of the kernel)
 DECODE_TMA_STAMPS: Optional[torch.Tensor] = None      # int64 [blocks, 12] for tuning, or None
 _TC_ERROR_NAMES[131] = "a role of the decode attention kernel waited 2 s on a barrier"
 # Which decode attention runs: "auto" takes the TMA kernel where the shape allows and the
@@ -1718,6 +1719,8 @@ def attn_decode_tma(q, k_pages, v_pages, block_table, *, slots, kv_len, page: in
     a.n_seqs, a.nq, a.nkv, a.max_pages = B, nq, nkv, block_table.shape[1]
     a.window, a.n_splits, a.scale_log2 = int(window or 0), ns, float(scale) * _LOG2E
     a.stamps = _ptr(DECODE_TMA_STAMPS)
+    # (blocks that all fit on the GPU at once gain nothing by an order)
+    a.ordered = int(1 < B <= DECODE_TMA_ORDERED and B * nkv * ns > per_sm * _sm_count(q.device))
     a.keep_first, a.chunk = int(keep_first or 0), _chunk_arg(chunk, keep_first)
     _set_cap_and_sinks(a, scale, softcap, sinks, nq)
     with torch.cuda.device(q.device):

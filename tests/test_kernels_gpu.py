@@ -768,7 +768,7 @@ def test_attn_prefill_tc_takes_the_same_rows_however_they_are_blocked(nq, nkv):
 
 @pytest.mark.parametrize("n_splits", [1, 3])
 @pytest.mark.parametrize("n", [1, 2, 31, 33, 64, 65])
-def test_attn_decode_tma_takes_every_sequence_once(n, n_splits):
+def test_attn_decode_tma_takes_every_sequence_once(n, n_splits, monkeypatch):
     """Blocks take the sequences by length (up to 64 of them): equal lengths, one page, and a few pages among them,
     against the kernel that takes them as they come."""
     ops = _ops()
@@ -778,10 +778,15 @@ def test_attn_decode_tma_takes_every_sequence_once(n, n_splits):
     q = _rand((n, nq, D), torch.bfloat16, 53).to(DEV)
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
     args = (q, pc.k_pages.to(DEV), pc.v_pages.to(DEV), pc.table.to(DEV))
-    kw = dict(slots=i32(pc.slot_of), kv_len=i32(lens), page=64, scale=0.125, max_kv_len=512)
-    got, want = ops.attn_decode_tma(*args, n_splits=n_splits, **kw), ops.attn_decode_bf16(*args, n_splits=1, **kw)
+    slots = [-1 if n > 2 and i == n // 2 else x for i, x in enumerate(pc.slot_of)]       # a padding row among them
+    kw = dict(slots=i32(slots), kv_len=i32(lens), page=64, scale=0.125, max_kv_len=512)
+    want = ops.attn_decode_bf16(*args, n_splits=1, **kw)
+    got = ops.attn_decode_tma(*args, n_splits=n_splits, **kw)
+    monkeypatch.setattr(ops, "_sm_count", lambda device: 0)      # more blocks than such a GPU holds: taken by length
+    ordered = ops.attn_decode_tma(*args, n_splits=n_splits, **kw)
     ops.check_kernel_errors()
     assert torch.allclose(got.float(), want.float(), atol=2e-2, rtol=2e-2)
+    assert torch.equal(got, ordered)
 
 
 def _plant_window_edge(q, row, pc, seq, pos, window):
