@@ -701,7 +701,8 @@ static bool delta_step_takes(const DeltaArgs& a) {
 // (quotients are products of the g between).  This kernel takes every chunk of every head at the same time, solves
 // the triangular system for the right-hand sides beta v and beta c k, and leaves the record.  The scan below
 // walks 2,048 rows (16 heads of 128) in 512 turns of a microsecond, 502 us and 36 for their products; this kernel takes
-// 56 us, the two behind it 135 and 64 (with the norm and the gate, which took 40 more behind the scan).
+// 58 us, the two behind it 149 and 67 (with the norm and the gate, which took 40 more behind the scan).  Decays are
+// multiplied up with the rounding of each product carried along, and the products of two rows are sums of chains of eight.
 #define DC_MIN 64         // a step goes chunk by chunk when a sequence may bring this many rows
 __global__ void __launch_bounds__(256, 2) delta_local_kernel(const DeltaArgs a) {
   constexpr int LD = CC_MAX_DK + 4;
@@ -729,14 +730,17 @@ __global__ void __launch_bounds__(256, 2) delta_local_kernel(const DeltaArgs a) 
     const float* p = a.prep + (size_t)(row0 + lane) * P + Cc + h;
     beta[lane] = lane < n ? p[0] : 0.f;
     const float g = lane < n ? p[H] : 1.f;
-    float run = 0.f, all = 1.f;
+    float run = 0.f, run_lost = 0.f, all = 1.f, all_lost = 0.f;      // (lost: what the products' roundings left out)
 #pragma unroll
     for (int t = 0; t < CC_ROWS; ++t) {
       const float gt = __shfl_sync(0xffffffffu, g, t);
-      run = t == lane ? 1.f : run * gt;
-      all *= gt;
-      quot[t * (CC_ROWS + 1) + lane] = run;      // (zero for t < i)
-      if (lane == 0) cum[t] = all;
+      const float r = __fmul_rn(run, gt), p = __fmul_rn(all, gt);
+      run_lost = t == lane ? 0.f : fmaf(run_lost, gt, fmaf(run, gt, -r));
+      run = t == lane ? 1.f : r;
+      all_lost = fmaf(all_lost, gt, fmaf(all, gt, -p));
+      all = p;
+      quot[t * (CC_ROWS + 1) + lane] = run + run_lost;               // (zero for t < i)
+      if (lane == 0) cum[t] = all + all_lost;
     }
   }
   __syncthreads();
@@ -748,25 +752,47 @@ __global__ void __launch_bounds__(256, 2) delta_local_kernel(const DeltaArgs a) 
   float* u0 = wq + cc_at_su(dk) + (size_t)dk * dv;
   {                        // two rows by two of both products a thread
     const int t0 = tid / 16, i0 = tid % 16;
-    float kk[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, qk[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-#pragma unroll 4
-    for (int d = 0; d < dk; d += 4) {
-      float4 ki[2], kt[2], qt[2];
+    float kk[2][2][4], qk[2][2][4];              // a sum for every fourth channel, of chains of eight
 #pragma unroll
-      for (int x = 0; x < 2; ++x) {
-        ki[x] = *reinterpret_cast<const float4*>(Ks + (i0 + 16 * x) * LD + d);
-        kt[x] = *reinterpret_cast<const float4*>(Ks + (t0 + 16 * x) * LD + d);
-        qt[x] = *reinterpret_cast<const float4*>(Qs + (t0 + 16 * x) * LD + d);
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+      for (int y = 0; y < 2; ++y)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) kk[x][y][j] = qk[x][y][j] = 0.f;
+#pragma unroll 1
+    for (int d0 = 0; d0 < dk; d0 += 32) {        // (channels beyond dk are zero)
+      float ck[2][2][4], cq[2][2][4];
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int y = 0; y < 2; ++y)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) ck[x][y][j] = cq[x][y][j] = 0.f;
+#pragma unroll 2
+      for (int d = d0; d < d0 + 32; d += 4) {
+        float4 ki[2], kt[2], qt[2];
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          ki[x] = *reinterpret_cast<const float4*>(Ks + (i0 + 16 * x) * LD + d);
+          kt[x] = *reinterpret_cast<const float4*>(Ks + (t0 + 16 * x) * LD + d);
+          qt[x] = *reinterpret_cast<const float4*>(Qs + (t0 + 16 * x) * LD + d);
+        }
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+          for (int y = 0; y < 2; ++y) {
+            ck[x][y][0] = fmaf(kt[x].x, ki[y].x, ck[x][y][0]), cq[x][y][0] = fmaf(qt[x].x, ki[y].x, cq[x][y][0]);
+            ck[x][y][1] = fmaf(kt[x].y, ki[y].y, ck[x][y][1]), cq[x][y][1] = fmaf(qt[x].y, ki[y].y, cq[x][y][1]);
+            ck[x][y][2] = fmaf(kt[x].z, ki[y].z, ck[x][y][2]), cq[x][y][2] = fmaf(qt[x].z, ki[y].z, cq[x][y][2]);
+            ck[x][y][3] = fmaf(kt[x].w, ki[y].w, ck[x][y][3]), cq[x][y][3] = fmaf(qt[x].w, ki[y].w, cq[x][y][3]);
+          }
       }
 #pragma unroll
       for (int x = 0; x < 2; ++x)
 #pragma unroll
-        for (int y = 0; y < 2; ++y) {
-          kk[x][y] = fmaf(kt[x].x, ki[y].x, kk[x][y]), qk[x][y] = fmaf(qt[x].x, ki[y].x, qk[x][y]);
-          kk[x][y] = fmaf(kt[x].y, ki[y].y, kk[x][y]), qk[x][y] = fmaf(qt[x].y, ki[y].y, qk[x][y]);
-          kk[x][y] = fmaf(kt[x].z, ki[y].z, kk[x][y]), qk[x][y] = fmaf(qt[x].z, ki[y].z, qk[x][y]);
-          kk[x][y] = fmaf(kt[x].w, ki[y].w, kk[x][y]), qk[x][y] = fmaf(qt[x].w, ki[y].w, qk[x][y]);
-        }
+        for (int y = 0; y < 2; ++y)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) kk[x][y][j] += ck[x][y][j], qk[x][y][j] += cq[x][y][j];
     }
 #pragma unroll
     for (int x = 0; x < 2; ++x)
@@ -774,8 +800,9 @@ __global__ void __launch_bounds__(256, 2) delta_local_kernel(const DeltaArgs a) 
       for (int y = 0; y < 2; ++y) {
         const int t = t0 + 16 * x, i = i0 + 16 * y;
         const float w = quot[t * (CC_ROWS + 1) + i];
-        As[t * CC_ROWS + i] = i < t ? w * kk[x][y] : 0.f;
-        Bs[t * CC_ROWS + i] = i <= t ? w * qk[x][y] : 0.f;
+        const float *u = kk[x][y], *v = qk[x][y];
+        As[t * CC_ROWS + i] = i < t ? w * ((u[0] + u[1]) + (u[2] + u[3])) : 0.f;
+        Bs[t * CC_ROWS + i] = i <= t ? w * ((v[0] + v[1]) + (v[2] + v[3])) : 0.f;
       }
   }
   __syncthreads();
@@ -790,16 +817,16 @@ __global__ void __launch_bounds__(256, 2) delta_local_kernel(const DeltaArgs a) 
     }
 #pragma unroll
     for (int t = 0; t < CC_ROWS; ++t) {
-      float s = x[t];
+      float s = 0.f;
 #pragma unroll
       for (int i0 = 0; i0 < t; i0 += 4) {        // (entries of A from the diagonal on are zero, x there still finite)
         const float4 w = *reinterpret_cast<const float4*>(As + t * CC_ROWS + i0);
-        s = fmaf(-w.x, x[i0], s);
-        if (i0 + 1 < t) s = fmaf(-w.y, x[i0 + 1], s);
-        if (i0 + 2 < t) s = fmaf(-w.z, x[i0 + 2], s);
-        if (i0 + 3 < t) s = fmaf(-w.w, x[i0 + 3], s);
+        s = fmaf(w.x, x[i0], s);
+        if (i0 + 1 < t) s = fmaf(w.y, x[i0 + 1], s);
+        if (i0 + 2 < t) s = fmaf(w.z, x[i0 + 2], s);
+        if (i0 + 3 < t) s = fmaf(w.w, x[i0 + 3], s);
       }
-      x[t] = beta[t] * s;
+      x[t] = beta[t] * (x[t] - s);
     }
     if (d < 0) {
 #pragma unroll

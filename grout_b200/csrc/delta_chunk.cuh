@@ -43,8 +43,12 @@ __host__ __device__ __forceinline__ size_t cc_chain_smem(int dk, int cols) {   /
 
 // Bound by a chunk's chain of three steps with a barrier behind each and, in a block of 32 columns, by their
 // multiply-adds; so where a step has few sequences and heads a block has 16 columns: 64 chunks of one sequence and 16
-// heads of 128 in 135 us, 2.1 a chunk.  (Multiply-adds packed two by two were no faster, 140 us: every pair of equal
-// factors has to be made first.)
+// heads of 128 in 149 us, 2.3 a chunk.  (Multiply-adds packed two by two were no faster, 140 us where one by one took 135:
+// every pair of equal factors has to be made first.)
+// The sums are taken so that no error grows beyond the row-by-row form's: W S in parts that are added up before they are
+// subtracted, a chunk's share of the state before the state is added to it, the read-outs by 32 terms (135 us and 64
+// for the read-outs otherwise, and with the products of the preparation in one chain the read-outs of 2,048 rows are
+// 1.4e-7 off where row by row they are 1.04e-7, with slow decays 2.5e-7 where they are 1.55e-7; so 1.05e-7 and 1.53e-7).
 template <typename Args, int COLS>
 __global__ void __launch_bounds__(256) delta_chain_kernel(const Args a) {
   static_assert(COLS == 16 || COLS == 32, "columns of a block");
@@ -123,21 +127,23 @@ __global__ void __launch_bounds__(256) delta_chain_kernel(const Args a) {
     __syncthreads();
     for (int i = tid * 4; i < CC_ROWS * COLS; i += 1024) {  // U = U0 - W S, four columns of a row a thread
       float4 u = *reinterpret_cast<const float4*>(u0 + i);
+      float4 x[SPLITS];
 #pragma unroll
-      for (int q = 0; q < SPLITS; ++q) {
-        const float4 x = *reinterpret_cast<const float4*>(P + q * CC_ROWS * COLS + i);
-        u.x -= x.x, u.y -= x.y, u.z -= x.z, u.w -= x.w;
-      }
+      for (int q = 0; q < SPLITS; ++q) x[q] = *reinterpret_cast<const float4*>(P + q * CC_ROWS * COLS + i);
+#pragma unroll
+      for (int n = SPLITS / 2; n > 0; n /= 2)
+#pragma unroll
+        for (int q = 0; q < n; ++q) x[q].x += x[q + n].x, x[q].y += x[q + n].y, x[q].z += x[q + n].z, x[q].w += x[q + n].w;
+      u.x -= x[0].x, u.y -= x[0].y, u.z -= x[0].z, u.w -= x[0].w;
       *reinterpret_cast<float4*>(U + i) = u;
       if (col0 + i % COLS < dv) *reinterpret_cast<float4*>(su + (size_t)(dk + i / COLS) * dv + i % COLS) = u;
     }
     __syncthreads();
     if (sk < dk) {                               // S <- diag(gC) S + Kd^T U
-      float s[4][SC];
+      float s[4][SC], was[4][SC];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float g = gc[sk + i];
-        float x[SC];
+        float* x = was[i];
         if constexpr (SC == 4) *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(S + (sk + i) * COLS + sc);
         else *reinterpret_cast<float2*>(x) = *reinterpret_cast<const float2*>(S + (sk + i) * COLS + sc);
         if (col_in) {
@@ -146,7 +152,7 @@ __global__ void __launch_bounds__(256) delta_chain_kernel(const Args a) {
           else *reinterpret_cast<float2*>(to) = *reinterpret_cast<const float2*>(x);
         }
 #pragma unroll
-        for (int j = 0; j < SC; ++j) s[i][j] = g * x[j];
+        for (int j = 0; j < SC; ++j) s[i][j] = 0.f;
       }
 #pragma unroll 8
       for (int t = 0; t < CC_ROWS; ++t) {
@@ -163,6 +169,9 @@ __global__ void __launch_bounds__(256) delta_chain_kernel(const Args a) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         float* to = S + (sk + i) * COLS + sc;
+        const float g = gc[sk + i];
+#pragma unroll
+        for (int j = 0; j < SC; ++j) s[i][j] = fmaf(g, was[i][j], s[i][j]);
         if constexpr (SC == 4) *reinterpret_cast<float4*>(to) = make_float4(s[i][0], s[i][1], s[i][2], s[i][3]);
         else *reinterpret_cast<float2*>(to) = make_float2(s[i][0], s[i][1]);
       }
@@ -213,7 +222,7 @@ __global__ void __launch_bounds__(256) delta_out_kernel(const Args a) {
     }
     cp_async_commit();
   };
-  float acc[4][4];
+  float acc[4][4];                               // the sum over the stages' sums
   stage_in(0);
   const int stages = tiles * col_tiles;
   for (int s = 0; s < stages; ++s) {
@@ -228,6 +237,11 @@ __global__ void __launch_bounds__(256) delta_out_kernel(const Args a) {
         for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
     }
     const int nk = min(CC_ROWS, K - s % tiles * CC_ROWS);
+    float part[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) part[i][j] = 0.f;
 #pragma unroll 8
     for (int k = 0; k < nk; ++k) {               // (columns beyond dv hold what no one reads)
       const float4 x = *reinterpret_cast<const float4*>(as + k * CC_ROWS + row);
@@ -236,8 +250,12 @@ __global__ void __launch_bounds__(256) delta_out_kernel(const Args a) {
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(xv[i], yv[j], acc[i][j]);
+        for (int j = 0; j < 4; ++j) part[i][j] = fmaf(xv[i], yv[j], part[i][j]);
     }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] += part[i][j];
     const int c = s / tiles * CO_COLS + lane * 4;
     if (s % tiles == tiles - 1 && c < dv) {
 #pragma unroll

@@ -238,6 +238,54 @@ def test_delta_rule_chunk_by_chunk_and_step_by_step(m):
     assert float((state - old_state).abs().max()) < 1e-5 * max(1.0, float(old_state.abs().max()))
 
 
+def _delta_in_64_bits(proj, lens, conv, a_log, dt_bias, norm, H, G, dk, dv, taps):
+    """The rule on the projection's 32-bit sums, all in 64 bits: (read-outs, states [sequence, head, value, key])."""
+    conv, a_log, dt_bias, norm = (t.double() for t in (conv, a_log, dt_bias, norm))
+    Cc, outs, states = 2 * G * dk + H * dv, [], []
+    unit = lambda t: t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6)  # noqa: E731
+    for x in torch.split(proj.double(), lens):
+        n = len(x)
+        c = sum(conv[:, j] * torch.cat([torch.zeros(taps - 1 - j, Cc).double(), x[:, :Cc]])[:n] for j in range(taps))
+        q, k, v = torch.split(c * torch.sigmoid(c), [G * dk, G * dk, H * dv], 1)
+        q, k = (unit(t.view(n, G, dk)).repeat_interleave(H // G, 1) for t in (q, k))
+        v, gate, b, a = v.view(n, H, dv), x[:, Cc:Cc + H * dv].view(n, H, dv), x[:, -2 * H:-H], x[:, -H:]
+        g = torch.exp(-torch.exp(a_log) * torch.nn.functional.softplus(a + dt_bias))
+        S, o = torch.zeros(H, dv, dk).double(), torch.empty(n, H, dv).double()
+        for t in range(n):
+            S = S * g[t][:, None, None]
+            u = torch.sigmoid(b[t])[:, None] * (v[t] - torch.einsum("hvk,hk->hv", S, k[t]))
+            S = S + u[:, :, None] * k[t][:, None]
+            o[t] = torch.einsum("hvk,hk->hv", S, q[t]) * dk ** -0.5
+        y = o / torch.sqrt((o * o).mean(-1, keepdim=True) + 1e-5) * norm * gate * torch.sigmoid(gate)
+        outs.append(y.reshape(n, -1)), states.append(S)
+    return torch.cat(outs), torch.stack(states)
+
+
+@pytest.mark.parametrize("decay", [0.0, -4.0])
+def test_delta_rule_by_chunks_is_as_exact_as_row_by_row(decay):
+    """The relative error against 64 bits of read-outs and states, chunk by chunk and row by row: both are 32-bit sums in
+    short chains, so neither is more than a tenth above the other (sums over a whole head in one chain, and products of
+    decays that lose each rounding, were a third to two thirds above)."""
+    from grout_b200.kernels import ops
+    H, G, dk, dv, taps, lens = 4, 2, 128, 128, 4, [300, 90]
+    Cc = 2 * G * dk + H * dv
+    proj, conv = rnd(sum(lens), Cc + H * dv + 2 * H, seed=41), 1 + rnd(Cc, taps, seed=42, scale=0.1)
+    a_log, dt, norm = decay + rnd(H, seed=43, scale=0.1), rnd(H, seed=44, scale=0.1), 1 + rnd(dv, seed=45, scale=0.1)
+    want, want_state = _delta_in_64_bits(proj, lens, conv, a_log, dt, norm, H, G, dk, dv, taps)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    off = lambda x, y: float((x.double() - y).norm() / y.norm())  # noqa: E731
+    errors = []
+    for max_rows in (max(lens), None):
+        state = torch.zeros(2, ops.delta_state_floats(H, G, dk, dv, taps), device=DEV)
+        y = ops.delta_forward(proj.to(DEV), state, *(t.to(DEV).contiguous() for t in (conv, a_log, dt, norm)),
+                              H=H, G=G, dk=dk, dv=dv, taps=taps, unit_eps=1e-6, norm_eps=1e-5, dtype=torch.float32,
+                              token_seq=i32([0] * lens[0] + [1] * lens[1]), cu_q=i32([0, lens[0], sum(lens)]),
+                              slots=i32([0, 1]), max_rows=max_rows)
+        errors.append((off(y.cpu(), want), off(state[:, (taps - 1) * Cc:].cpu().view(2, H, dv, dk), want_state)))
+    (chunks, chunk_state), (rows, row_state) = errors
+    assert chunks < 1.1 * rows and chunk_state < 1.1 * row_state, errors
+
+
 @pytest.mark.parametrize("n_seqs,m", [(1, dict(heads=16, kv_heads=16, dim=128, vdim=128, conv=4)),
                                       (3, dict(heads=8, kv_heads=2, dim=64, vdim=96, conv=3)),
                                       (40, dict(heads=16, kv_heads=4, dim=64, vdim=64, conv=4))])
