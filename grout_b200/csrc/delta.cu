@@ -139,7 +139,9 @@ __global__ void __launch_bounds__(256) delta_prepare_kernel(const DeltaArgs a) {
 // The same for steps of many rows: a block takes a run of DP_RUN rows, a thread a channel of them (q and k of one kv
 // head, or 256 value channels), so an input is read once instead of once for each tap, all of a run's are on
 // their way together, and the sums of squares of all rows meet behind one barrier.  Bound by memory; 2,048 rows of 4,096
-// channels 32 us (80 with a block a row).
+// channels 32 us (80 with a block a row).  From 256 rows on, eight a sequence: a whole rule of 100 rows takes 47 us with
+// runs and 43 without (16 heads of 128), 64 sequences of one and two rows 106 and 92, 316 rows in 61 sequences 200 and
+// 190, 256 rows 86 and 88, 63 sequences of 16 rows 203 and 220.
 #define DP_RUN 16
 #define DP_TAPS 8
 __global__ void __launch_bounds__(256) delta_prepare_rows_kernel(const DeltaArgs a) {
@@ -703,7 +705,6 @@ static bool delta_step_takes(const DeltaArgs& a) {
 // walks 2,048 rows (16 heads of 128) in 512 turns of a microsecond, 502 us and 36 for their products; this kernel takes
 // 58 us, the two behind it 149 and 67 (with the norm and the gate, which took 40 more behind the scan).  Decays are
 // multiplied up with the rounding of each product carried along, and the products of two rows are sums of chains of eight.
-#define DC_MIN 64         // a step goes chunk by chunk when a sequence may bring this many rows
 __global__ void __launch_bounds__(256, 2) delta_local_kernel(const DeltaArgs a) {
   constexpr int LD = CC_MAX_DK + 4;
   extern __shared__ __align__(16) float sm[];
@@ -854,7 +855,7 @@ __global__ void __launch_bounds__(256, 2) delta_local_kernel(const DeltaArgs a) 
 }
 
 static bool delta_chunks_take(const DeltaArgs& a) {
-  return a.chunks && !a.few_rows && a.max_rows >= DC_MIN && a.dk <= CC_MAX_DK && a.dk % 4 == 0 && a.dv % 4 == 0 &&
+  return a.chunks && !a.few_rows && a.max_rows > 0 && a.dk <= CC_MAX_DK && a.dk % 4 == 0 && a.dv % 4 == 0 &&
          a.dv <= CC_MAX_DV && a.H <= 65535 && a.n_seqs <= 65535 && (((uintptr_t)a.chunks) & 15) == 0;
 }
 
@@ -908,7 +909,7 @@ static int delta_forward(const DeltaArgs& a, cudaStream_t s) {
   if (delta_step_takes(a))
     return gb_launch_cluster(delta_step_kernel<T>, dim3(a.H, a.n_seqs), dim3(256), 0, s, a.H / a.G, a);
   const int units = a.G + (a.H * a.dv + DELTA_PREP_V - 1) / DELTA_PREP_V;
-  if (!a.few_rows && a.n_tokens >= 4 * DP_RUN && a.dk % 32 == 0 && a.dk <= 128 && a.taps <= DP_TAPS) {
+  if (!a.few_rows && a.n_tokens >= 256 && a.n_tokens / 8 >= a.n_seqs && a.dk % 32 == 0 && a.dk <= 128 && a.taps <= DP_TAPS) {
     const int runs = a.n_tokens / DP_RUN + a.n_seqs;         // (run_of_block)
     e = gb_launch(delta_prepare_rows_kernel, dim3(runs, a.G + (a.H * a.dv + 255) / 256), dim3(256), 0, s, a);
   } else {

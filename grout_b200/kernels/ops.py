@@ -1810,8 +1810,19 @@ class _DeltaArgs(ctypes.Structure):
 
 
 DELTA_CHUNK = 32                  # rows of a chunk of the kernels' chunked form (CC_ROWS)
-DELTA_CHUNK_MIN = 64              # a sequence of this many rows in a step: the step goes chunk by chunk (DC_MIN)
 DELTA_CHUNK_BYTES = 4 << 30       # scratch that a step's chunks may take; larger steps walk their rows
+
+
+def delta_chunks_pay(T: int, n_seqs: int, max_rows: int) -> bool:
+    """Whether a step of T rows in ``n_seqs`` sequences, the longest of at most ``max_rows`` rows, goes chunk by chunk.
+    Row by row a step takes as long as its longest sequence, or as its rows where they fill the GPU; chunk by chunk
+    some 50 us for the first chunk, and every sequence costs its last chunk of 32 rows whole.  A captured
+    step knows its bucket only: the row count is its bound, and its sequences may be short ones.  Measured (us, chunk by
+    chunk / row by row, 16 heads of 128, then 32): 100 rows 65 / 43, 74 / 55; 130 in a step captured for 256 84 / 68, 101 /
+    132; 300 88 / 97, 117 / 133; 300 captured for 512 105 / 123, 150 / 206; seven of 70 captured for 512 133 / 114,
+    216 / 183; eight of 120 captured for 1,024 166 / 199, 294 / 340; 64 of one and two rows 353 / 92, 661 / 156; 16 of 128
+    277 / 361, 485 / 673; 64 of 64 583 / 694, 1,080 / 1,296; 2,048 304 / 588, 482 / 831."""
+    return T >= 48 * n_seqs if T >= 2048 else max_rows > 256 and T >= 72 * n_seqs
 
 
 def delta_state_floats(H: int, G: int, dk: int, dv: int, taps: int) -> int:
@@ -1838,7 +1849,7 @@ def delta_forward(proj: torch.Tensor, state: torch.Tensor, conv_w: torch.Tensor,
     y [T, H dv] in ``dtype``: every head's read-out, normalised over dv, times ``norm_w``
     and silu(gate).  ``max_rows``: the most rows any sequence of the step brings, when the
     host knows it (a decode step: 1); steps of at most four rows a sequence take one launch less, a
-    decode step takes one, and from ``DELTA_CHUNK_MIN`` rows on a step goes chunk by chunk."""
+    decode step takes one, and steps of long sequences (``delta_chunks_pay``) go chunk by chunk."""
     _need(proj, "projection", torch.float32, 2)
     _need(state, "state", torch.float32, 2)
     Cc = 2 * G * dk + H * dv
@@ -1877,7 +1888,7 @@ def delta_forward(proj: torch.Tensor, state: torch.Tensor, conv_w: torch.Tensor,
     one_kernel = (a.few_rows == 2 and dk <= 128 and dk % 4 == 0 and dv <= 128 and taps <= 8 and H // G <= 8 and
                   n_seqs <= 65535 and state.stride(0) % 4 == 0 and (taps - 1) * Cc % 4 == 0 and state.data_ptr() % 16 == 0)
     a.max_rows = int(max_rows or 0)
-    if a.max_rows >= DELTA_CHUNK_MIN and dk <= 128 and dk % 4 == 0 and dv % 4 == 0:
+    if not a.few_rows and dk <= 128 and dk % 4 == 0 and dv % 4 == 0 and delta_chunks_pay(T, n_seqs, a.max_rows):
         C = DELTA_CHUNK
         n = (T // C + n_seqs) * H * (2 * dk * C + dk + (dk + C) * (C + dv))
         if 4 * n <= DELTA_CHUNK_BYTES:

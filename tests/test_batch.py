@@ -162,3 +162,12 @@ def test_the_splits_of_decode_attention(monkeypatch):
             fine = 512 < bound <= 2048
             assert 1 <= s <= max(1, -(-bound // (128 if fine else 256)))
             assert not fine or s <= 8 or s == 16
+
+
+def test_the_steps_whose_delta_rule_goes_by_chunks():
+    """Steps of long sequences do; many short ones, and captured steps whose sequences may be short, do not."""
+    from grout_b200.kernels.ops import delta_chunks_pay
+    by_chunks = [(2048, 1, 2048), (300, 1, 300), (512, 2, 512), (1024, 8, 1024), (4096, 64, 64), (2048, 16, 128)]
+    by_rows = [(128, 64, 128), (1024, 64, 1024), (1024, 32, 1024), (256, 2, 256), (100, 1, 100), (512, 8, 512),
+               (124, 61, 64), (316, 61, 256), (3000, 1500, 1400), (1, 1, 0)]
+    assert all(delta_chunks_pay(*c) for c in by_chunks) and not any(delta_chunks_pay(*c) for c in by_rows)

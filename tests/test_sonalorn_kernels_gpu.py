@@ -189,12 +189,13 @@ def test_delta_rule_whole_in_portions_and_token_by_token(m):
                                dict(heads=8, kv_heads=1, dim=64, vdim=48, conv=8), DELTA_SHAPES[3],
                                dict(heads=16, kv_heads=4, dim=12, vdim=128, conv=3),
                                dict(heads=2, kv_heads=1, dim=128, vdim=144, conv=2)])
-def test_delta_rule_chunk_by_chunk_and_step_by_step(m):
+def test_delta_rule_chunk_by_chunk_and_step_by_step(m, monkeypatch):
     """When the host knows how many rows a sequence brings at most, prompts go chunk by chunk (32 rows) and decode
     steps through one kernel: sequences of 1, 31, 32, 33, 64 and 100 rows in one step, a padding sequence and one
     without rows between them, go on with 3 decode steps.  Against the plain rule, and against the kernels that
     take any rows; strong and weak decays side by side; 32-bit sums of values of order one, a bar of 1e-5."""
     from grout_b200.kernels import ops
+    monkeypatch.setattr(ops, "delta_chunks_pay", lambda T, n_seqs, max_rows: max_rows >= 64)
     H, G, dk, dv, taps = m["heads"], m["kv_heads"], m["dim"], m["vdim"], m["conv"]
     W, lens, more = 24, [1, 31, 32, 33, 64, 100], 3
     w = _delta_weights(H, G, dk, dv, taps, W, seed=13)
@@ -268,6 +269,7 @@ def test_delta_rule_by_chunks_is_as_exact_as_row_by_row(decay):
     decays that lose each rounding, were a third to two thirds above)."""
     from grout_b200.kernels import ops
     H, G, dk, dv, taps, lens = 4, 2, 128, 128, 4, [300, 90]
+    assert ops.delta_chunks_pay(sum(lens), 2, max(lens))
     Cc = 2 * G * dk + H * dv
     proj, conv = rnd(sum(lens), Cc + H * dv + 2 * H, seed=41), 1 + rnd(Cc, taps, seed=42, scale=0.1)
     a_log, dt, norm = decay + rnd(H, seed=43, scale=0.1), rnd(H, seed=44, scale=0.1), 1 + rnd(dv, seed=45, scale=0.1)
