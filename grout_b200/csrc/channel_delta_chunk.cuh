@@ -25,6 +25,9 @@ __device__ __forceinline__ const float* cc_gate(const ChannelDeltaArgs& a, size_
 __device__ __forceinline__ float cc_gate_of(const ChannelDeltaArgs&, float x) { return cd_sigmoid(x); }
 __device__ __forceinline__ void cc_out_done(const ChannelDeltaArgs&, int, int) {}
 #include "delta_chunk.cuh"
+__device__ __forceinline__ int cc_from(const ChannelDeltaArgs&) { return 0; }
+__device__ __forceinline__ int cc_to(const ChannelDeltaArgs&, int chunks) { return chunks; }
+__device__ __forceinline__ size_t cc_place(const ChannelDeltaArgs&, int first, int z, int seq) { return cc_entry(first, z, seq); }
 
 #define CC_HALF 16
 #define CC_MIN 64        // a step goes chunk by chunk when a sequence brings this many rows
@@ -239,5 +242,5 @@ static int cc_run(const ChannelDeltaArgs& a, cudaStream_t s) {
   const int chunks = (a.max_rows + CC_ROWS - 1) / CC_ROWS;
   int e = a.dk <= 32 ? cc_local<1>(a, chunks, s) : a.dk <= 64 ? cc_local<2>(a, chunks, s) : cc_local<4>(a, chunks, s);
   if (e) return e;
-  return delta_chain_and_out<T>(a, a.max_rows, s);
+  return delta_chain_and_out<T>(a, chunks, s);
 }

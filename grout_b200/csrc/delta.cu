@@ -67,7 +67,10 @@ struct DeltaArgs {
   int few_rows;            // 1: no sequence brings more than DELTA_B rows, 2: none more than one (a decode
                            //   step): the scan works out its one group's scalars itself, `gram` is not launched
   int max_rows;            // the most rows any sequence brings (0: unknown)
-  float* chunks;           // [n_tokens / 32 + n_seqs, H, record] scratch of a step that goes chunk by chunk, or null
+  float* chunks;           // scratch of a step that goes chunk by chunk, or null: [n_tokens / 32 + n_seqs, H, record], or
+                           //   with `window` [group, window, H, record]
+  int group, window;       // window > 0: the step goes by `group` sequences and `window` of their chunks at a time
+  int z0;                  // the first chunk of the launch's window
 };
 
 __device__ __forceinline__ void delta_keep_tail(const DeltaArgs& a, int seq, int first, int step);
@@ -82,6 +85,13 @@ __device__ __forceinline__ void cc_out_done(const DeltaArgs& a, int seq, int h) 
   delta_keep_tail(a, seq, h * blockDim.x + threadIdx.x, a.H * blockDim.x);
 }
 #include "delta_chunk.cuh"
+__device__ __forceinline__ int cc_from(const DeltaArgs& a) { return a.z0; }
+__device__ __forceinline__ int cc_to(const DeltaArgs& a, int chunks) {
+  return a.window ? min(chunks, a.z0 + a.window) : chunks;
+}
+__device__ __forceinline__ size_t cc_place(const DeltaArgs& a, int first, int z, int seq) {
+  return a.window ? (size_t)seq * a.window + (z - a.z0) : cc_entry(first, z, seq);
+}
 
 // One block per (token, unit): unit g < G is kv head g's q and k together, the units after that are runs of
 // DELTA_PREP_V value channels; the block of unit 0 also takes beta and the decay.
@@ -712,7 +722,7 @@ __global__ void __launch_bounds__(256, 2) delta_local_kernel(const DeltaArgs a) 
   float *quot = Bs + CC_ROWS * CC_ROWS, *beta = quot + CC_ROWS * (CC_ROWS + 1), *cum = beta + CC_ROWS;
   pdl_launch_dependents_if_small();
   const int tid = threadIdx.x, lane = tid & 31;
-  const int h = blockIdx.y, seq = blockIdx.z, z = blockIdx.x;
+  const int h = blockIdx.y, seq = blockIdx.z, z = cc_from(a) + blockIdx.x;
   const int H = a.H, G = a.G, dk = a.dk, dv = a.dv, kvh = h / (H / G), Cc = cc_channels(a), P = a.prep_stride;
   pdl_wait();
   const int first = a.cu_q[seq], n_seq = a.cu_q[seq + 1] - first;
@@ -745,7 +755,7 @@ __global__ void __launch_bounds__(256, 2) delta_local_kernel(const DeltaArgs a) 
     }
   }
   __syncthreads();
-  const size_t entry = (cc_entry(first, z, seq) * H + h) * cc_record(dk, dv);
+  const size_t entry = (cc_place(a, first, z, seq) * H + h) * cc_record(dk, dv);
   float* wq = a.chunks + entry;
   float* kd = wq + (size_t)dk * CC_ROWS;
   float* gc = kd + (size_t)CC_ROWS * dk;
@@ -856,18 +866,31 @@ __global__ void __launch_bounds__(256, 2) delta_local_kernel(const DeltaArgs a) 
 
 static bool delta_chunks_take(const DeltaArgs& a) {
   return a.chunks && !a.few_rows && a.max_rows > 0 && a.dk <= CC_MAX_DK && a.dk % 4 == 0 && a.dv % 4 == 0 &&
-         a.dv <= CC_MAX_DV && a.H <= 65535 && a.n_seqs <= 65535 && (((uintptr_t)a.chunks) & 15) == 0;
+         a.dv <= CC_MAX_DV && a.H <= 65535 && (a.window ? a.group : a.n_seqs) <= 65535 &&
+         (((uintptr_t)a.chunks) & 15) == 0;
 }
 
+// All at once, or, where the scratch would be too large, by groups of sequences and windows of their chunks: the state
+// goes from one window to the next through its place in the cache, in the same 32 bits.  (A padding sequence has no
+// place: its read-outs, which nobody reads, start anew with every window.)
 template <typename T>
-static int delta_by_chunks(const DeltaArgs& a, cudaStream_t s) {
+static int delta_by_chunks(DeltaArgs a, cudaStream_t s) {
   const size_t smem = (2 * CC_ROWS * (CC_MAX_DK + 4) + 2 * CC_ROWS * CC_ROWS + CC_ROWS * (CC_ROWS + 1) + 2 * CC_ROWS) *
                       sizeof(float);
   cudaError_t ce = cudaFuncSetAttribute(delta_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (ce != cudaSuccess) return (int)ce;
-  const int e = gb_launch(delta_local_kernel, dim3((a.max_rows + CC_ROWS - 1) / CC_ROWS, a.H, a.n_seqs), dim3(256), smem,
-                          s, a);
-  return e ? e : delta_chain_and_out<T>(a, a.max_rows, s);
+  const int all = (a.max_rows + CC_ROWS - 1) / CC_ROWS, n_seqs = a.n_seqs, *cu_q = a.cu_q, *slots = a.slots;
+  const int window = a.window ? a.window : all, group = a.window ? a.group : n_seqs;
+  for (int q = 0; q < n_seqs; q += group) {
+    a.cu_q = cu_q + q, a.slots = slots + q, a.n_seqs = n_seqs - q < group ? n_seqs - q : group;
+    for (a.z0 = 0; a.z0 < all; a.z0 += window) {
+      const int chunks = all - a.z0 < window ? all - a.z0 : window;
+      int e = gb_launch(delta_local_kernel, dim3(chunks, a.H, a.n_seqs), dim3(256), smem, s, a);
+      if (!e) e = delta_chain_and_out<T>(a, chunks, s);
+      if (e) return e;
+    }
+  }
+  return 0;
 }
 
 template <int R, int B>
@@ -891,7 +914,7 @@ static int scan_launch(const DeltaArgs& a, cudaStream_t s) {
 
 static int delta_check(const DeltaArgs& a) {
   if (a.n_tokens < 0 || a.n_seqs <= 0 || a.H <= 0 || a.G <= 0 || a.H % a.G || a.dk <= 0 ||
-      a.dv <= 0 || a.taps <= 0 || !a.proj || !a.state || !a.prep || !a.o || !a.y)
+      a.dv <= 0 || a.taps <= 0 || !a.proj || !a.state || !a.prep || (!a.o && !a.chunks) || !a.y)
     return GB_ERR_BAD_ARG;
   if (a.dk > 32 * DELTA_LANES) return GB_ERR_UNSUPPORTED;
   const int Cc = 2 * a.G * a.dk + a.H * a.dv;
@@ -916,7 +939,9 @@ static int delta_forward(const DeltaArgs& a, cudaStream_t s) {
     e = gb_launch(delta_prepare_kernel, dim3(a.n_tokens, units), dim3(256), (size_t)2 * a.dk * sizeof(float), s, a);
   }
   if (e) return e;
+  if (a.window && (a.window < 0 || a.group < 1)) return GB_ERR_BAD_ARG;
   if (delta_chunks_take(a)) return delta_by_chunks<T>(a, s);
+  if (!a.o) return GB_ERR_BAD_ARG;
   if (!a.few_rows) {
     e = gb_launch(delta_gram_kernel, dim3(a.n_tokens, a.H), dim3(128), 0, s, a);
     if (e) return e;

@@ -10,7 +10,9 @@
 //
 // The including file's arguments have cu_q, slots, state, state_stride, taps, H, dk, dv, n_seqs, norm_eps, norm_w, y and
 // chunks, and for them cc_channels(a) (the convolved channels), cc_gate(a, t, h) (the gate's logits of a row and head),
-// cc_gate_of(a, x) and cc_out_done(a, seq, h) (called by a sequence's first block of every head).
+// cc_gate_of(a, x), cc_out_done(a, seq, h) (called by a sequence's first block of every head), and, where a launch takes a
+// part of the chunks only, the first of them cc_from(a), the end of them cc_to(a, chunks) and the place of a record
+// cc_place(a, first, z, seq) (else 0, chunks and cc_entry).
 #pragma once
 
 #define CC_ROWS 32       // rows of a chunk
@@ -70,8 +72,9 @@ __global__ void __launch_bounds__(256) delta_chain_kernel(const Args a) {
   const int slot = a.slots[seq];
   float* sp = slot >= 0 ? a.state + (size_t)slot * a.state_stride + (size_t)(a.taps - 1) * Cc + (size_t)h * dv * dk
                         : nullptr;
-  const int chunks = (n_seq + CC_ROWS - 1) / CC_ROWS;
-  auto record = [&](int z) { return a.chunks + (cc_entry(first, z, seq) * H + h) * cc_record(dk, dv); };
+  const int z_lo = cc_from(a), z_hi = cc_to(a, (n_seq + CC_ROWS - 1) / CC_ROWS);
+  if (z_lo >= z_hi) return;
+  auto record = [&](int z) { return a.chunks + (cc_place(a, first, z, seq) * H + h) * cc_record(dk, dv); };
   const int whole = 2 * dk * CC_ROWS + dk;                 // (dk is a multiple of four)
   auto stage_in = [&](int z) {
     float* dst = sm + (z & 1) * stage;
@@ -85,7 +88,7 @@ __global__ void __launch_bounds__(256) delta_chain_kernel(const Args a) {
   for (int s = 0; s < 2 && col0 + COLS > dv; ++s)          // columns no copy brings
     for (int i = tid; i < CC_ROWS * COLS; i += 256)
       if (col0 + i % COLS >= dv) sm[s * stage + whole + i] = 0.f;
-  stage_in(0);
+  stage_in(z_lo);
   // the state: element (k, c) of the head's matrix lies at c dk + k
   for (int i = tid; i < dk * COLS; i += 256) {
     const int c = i / dk, k = i % dk;
@@ -96,8 +99,8 @@ __global__ void __launch_bounds__(256) delta_chain_kernel(const Args a) {
   const int per = (dk + SPLITS - 1) / SPLITS, k_lo = part * per, k_hi = min(dk, k_lo + per);
   const int sk = tid / 8 * 4, sc = tid % 8 * SC;
   const bool col_in = col0 + sc < dv;                      // (dv is a multiple of four)
-  for (int z = 0; z < chunks; ++z) {
-    if (z + 1 < chunks) { stage_in(z + 1); cp_async_wait<1>(); } else { cp_async_wait<0>(); }
+  for (int z = z_lo; z < z_hi; ++z) {
+    if (z + 1 < z_hi) { stage_in(z + 1); cp_async_wait<1>(); } else { cp_async_wait<0>(); }
     __syncthreads();
     const float* w = sm + (z & 1) * stage;
     const float* kd = w + dk * CC_ROWS;
@@ -196,14 +199,14 @@ __global__ void __launch_bounds__(256) delta_out_kernel(const Args a) {
   extern __shared__ __align__(16) float sm[];    // two stages [A: 32 x 32 | B: 32 x CO_COLS] | the read-outs [32][dv]
   pdl_launch_dependents_if_small();
   const int tid = threadIdx.x, lane = tid & 31, row = tid / 32 * 4;
-  const int h = blockIdx.y, seq = blockIdx.z, z = blockIdx.x;
+  const int h = blockIdx.y, seq = blockIdx.z, z = cc_from(a) + blockIdx.x;
   const int H = a.H, dk = a.dk, dv = a.dv, K = dk + CC_ROWS;
   float* os = sm + 2 * CO_STAGE;
   pdl_wait();
   const int first = a.cu_q[seq], n = min(CC_ROWS, a.cu_q[seq + 1] - first - z * CC_ROWS);
   if (n <= 0) return;
   if (z == 0) cc_out_done(a, seq, h);
-  const float* rec = a.chunks + (cc_entry(first, z, seq) * H + h) * cc_record(dk, dv);
+  const float* rec = a.chunks + (cc_place(a, first, z, seq) * H + h) * cc_record(dk, dv);
   const float* qb = rec + cc_at_qb(dk);
   const float* su = rec + cc_at_su(dk);
   const int tiles = (K + CC_ROWS - 1) / CC_ROWS, col_tiles = (dv + CO_COLS - 1) / CO_COLS;
@@ -292,9 +295,9 @@ static int delta_chain(const Args& a, cudaStream_t s) {
   return gb_launch(delta_chain_kernel<Args, COLS>, grid, dim3(256), smem, s, a);
 }
 
-// The two kernels behind the records of a step whose sequences bring at most max_rows rows.
+// The two kernels behind the records of a launch that takes at most `chunks` chunks of every sequence.
 template <typename T, typename Args>
-static int delta_chain_and_out(const Args& a, int max_rows, cudaStream_t s) {
+static int delta_chain_and_out(const Args& a, int chunks, cudaStream_t s) {
   // 16 columns a block while that gives an SM at most one block
   const long long narrow = (long long)((a.dv + 15) / 16) * a.H * a.n_seqs;
   int e = narrow <= 148 ? delta_chain<Args, 16>(a, s) : delta_chain<Args, 32>(a, s);
@@ -303,5 +306,5 @@ static int delta_chain_and_out(const Args& a, int max_rows, cudaStream_t s) {
   const cudaError_t ce = cudaFuncSetAttribute(delta_out_kernel<T, Args>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               (int)smem);
   if (ce != cudaSuccess) return (int)ce;
-  return gb_launch(delta_out_kernel<T, Args>, dim3((max_rows + CC_ROWS - 1) / CC_ROWS, a.H, a.n_seqs), dim3(256), smem, s, a);
+  return gb_launch(delta_out_kernel<T, Args>, dim3(chunks, a.H, a.n_seqs), dim3(256), smem, s, a);
 }

@@ -1806,11 +1806,12 @@ class _DeltaArgs(ctypes.Structure):
                 ("token_seq", _P), ("cu_q", _P), ("slots", _P), ("state", _P), ("state_stride", _L),
                 ("prep", _P), ("o", _P), ("y", _P), ("n_tokens", _I), ("n_seqs", _I), ("H", _I),
                 ("G", _I), ("dk", _I), ("dv", _I), ("taps", _I), ("unit_eps", _F), ("norm_eps", _F),
-                ("prep_stride", _I), ("few_rows", _I), ("max_rows", _I), ("chunks", _P)]
+                ("prep_stride", _I), ("few_rows", _I), ("max_rows", _I), ("chunks", _P), ("group", _I), ("window", _I),
+                ("z0", _I)]
 
 
 DELTA_CHUNK = 32                  # rows of a chunk of the kernels' chunked form (CC_ROWS)
-DELTA_CHUNK_BYTES = 4 << 30       # scratch that a step's chunks may take; larger steps walk their rows
+DELTA_CHUNK_BYTES = 1280 << 20    # scratch that a step's chunks may take; larger steps go by groups and windows of them
 
 
 def delta_chunks_pay(T: int, n_seqs: int, max_rows: int) -> bool:
@@ -1823,6 +1824,24 @@ def delta_chunks_pay(T: int, n_seqs: int, max_rows: int) -> bool:
     216 / 183; eight of 120 captured for 1,024 166 / 199, 294 / 340; 64 of one and two rows 353 / 92, 661 / 156; 16 of 128
     277 / 361, 485 / 673; 64 of 64 583 / 694, 1,080 / 1,296; 2,048 304 / 588, 482 / 831."""
     return T >= 48 * n_seqs if T >= 2048 else max_rows > 256 and T >= 72 * n_seqs
+
+
+def delta_record(dk: int, dv: int) -> int:
+    """Floats of a chunk's record for one head (cc_record of the kernels)."""
+    return 2 * dk * DELTA_CHUNK + dk + (dk + DELTA_CHUNK) * (DELTA_CHUNK + dv)
+
+
+def delta_chunk_plan(T: int, n_seqs: int, max_rows: int, H: int, dk: int, dv: int):
+    """(records that a step's chunks need for every head, sequences of a group, chunks of a window): all at once
+    (0, 0) where ``DELTA_CHUNK_BYTES`` hold them.  Eight sequences of 2,048 rows (32 heads of 128) would take 2.3 GB and
+    3,160 us at once; in windows of 38 chunks 3,300 us, of 15 chunks 3,525 (row by row 5,265)."""
+    fit = max(1, DELTA_CHUNK_BYTES // (4 * H * delta_record(dk, dv)))
+    at_once = T // DELTA_CHUNK + n_seqs
+    if at_once <= fit:
+        return at_once, 0, 0
+    window = min(-(-max_rows // DELTA_CHUNK), max(8, fit // n_seqs), fit)
+    group = min(n_seqs, fit // window)
+    return group * window, group, window
 
 
 def delta_state_floats(H: int, G: int, dk: int, dv: int, taps: int) -> int:
@@ -1873,14 +1892,13 @@ def delta_forward(proj: torch.Tensor, state: torch.Tensor, conv_w: torch.Tensor,
     # group of four rows that it opens
     prep_stride = (Cc + 2 * H + 3) // 4 * 4 + 48 * H
     prep = torch.empty((T, prep_stride), dtype=torch.float32, device=proj.device)
-    o = torch.empty((T, H, dv), dtype=torch.float32, device=proj.device)
     y = torch.empty((T, H * dv), dtype=dtype, device=proj.device)
     a = _DeltaArgs()
     a.proj, a.conv_w, a.a_log, a.dt_bias, a.norm_w = (proj.data_ptr(), conv_w.data_ptr(),
                                                       a_log.data_ptr(), dt_bias.data_ptr(), norm_w.data_ptr())
     a.token_seq, a.cu_q, a.slots = token_seq.data_ptr(), cu_q.data_ptr(), slots.data_ptr()
     a.state, a.state_stride = state.data_ptr(), state.stride(0)
-    a.prep, a.o, a.y = prep.data_ptr(), o.data_ptr(), y.data_ptr()
+    a.prep, a.y = prep.data_ptr(), y.data_ptr()
     a.n_tokens, a.n_seqs, a.H, a.G, a.dk, a.dv, a.taps = T, n_seqs, H, G, dk, dv, taps
     a.unit_eps, a.norm_eps, a.prep_stride = float(unit_eps), float(norm_eps), prep_stride
     a.few_rows = 0 if max_rows is None or not 0 < max_rows <= 4 else (2 if max_rows == 1 else 1)
@@ -1888,14 +1906,24 @@ def delta_forward(proj: torch.Tensor, state: torch.Tensor, conv_w: torch.Tensor,
     one_kernel = (a.few_rows == 2 and dk <= 128 and dk % 4 == 0 and dv <= 128 and taps <= 8 and H // G <= 8 and
                   n_seqs <= 65535 and state.stride(0) % 4 == 0 and (taps - 1) * Cc % 4 == 0 and state.data_ptr() % 16 == 0)
     a.max_rows = int(max_rows or 0)
-    if not a.few_rows and dk <= 128 and dk % 4 == 0 and dv % 4 == 0 and delta_chunks_pay(T, n_seqs, a.max_rows):
-        C = DELTA_CHUNK
-        n = (T // C + n_seqs) * H * (2 * dk * C + dk + (dk + C) * (C + dv))
-        if 4 * n <= DELTA_CHUNK_BYTES:
-            chunks = torch.empty(n, dtype=torch.float32, device=proj.device)
-            a.chunks = chunks.data_ptr()
+    launches = 1 if one_kernel else 3 if a.few_rows else 4
+    o = chunks = None
+    if (not a.few_rows and dk <= 128 and dk % 4 == 0 and dv % 4 == 0 and dv <= 1024 and H <= 65535 and
+            n_seqs <= 65535 and delta_chunks_pay(T, n_seqs, a.max_rows)):
+        records, a.group, a.window = delta_chunk_plan(T, n_seqs, a.max_rows, H, dk, dv)
+        try:
+            chunks = torch.empty(records * H * delta_record(dk, dv), dtype=torch.float32, device=proj.device)
+        except torch.OutOfMemoryError:       # a step that has room row by row goes row by row
+            a.group = a.window = 0
+    if chunks is not None:
+        a.chunks = chunks.data_ptr()
+        if a.window:
+            launches = 1 + 3 * -(-n_seqs // a.group) * -(-a.max_rows // (DELTA_CHUNK * a.window))
+    else:
+        o = torch.empty((T, H, dv), dtype=torch.float32, device=proj.device)
+        a.o = o.data_ptr()
     _check(_fn("delta", f"gb_delta_forward_{_suffix(dtype)}", "pp")(ctypes.addressof(a), _stream()),
-           "delta_forward", 1 if one_kernel else 3 if a.few_rows else 4)
+           "delta_forward", launches)
     return y
 
 

@@ -171,3 +171,14 @@ def test_the_steps_whose_delta_rule_goes_by_chunks():
     by_rows = [(128, 64, 128), (1024, 64, 1024), (1024, 32, 1024), (256, 2, 256), (100, 1, 100), (512, 8, 512),
                (124, 61, 64), (316, 61, 256), (3000, 1500, 1400), (1, 1, 0)]
     assert all(delta_chunks_pay(*c) for c in by_chunks) and not any(delta_chunks_pay(*c) for c in by_rows)
+
+
+def test_the_scratch_of_the_delta_rule_by_chunks():
+    """The records of a step's chunks never take more than their bound, and the groups and windows cover the step."""
+    from grout_b200.kernels import ops
+    for H, dk, dv in ((16, 128, 128), (32, 128, 128), (64, 128, 256), (4, 64, 64)):
+        record = 4 * H * ops.delta_record(dk, dv)
+        for n, rows in ((1, 300), (1, 2048), (1, 40960), (8, 2048), (64, 250), (300, 100), (2000, 64)):
+            records, group, window = ops.delta_chunk_plan(n * rows, n, rows, H, dk, dv)
+            assert records * record <= ops.DELTA_CHUNK_BYTES
+            assert records == (group * window if window else n * rows // 32 + n) and (not window or 1 <= group <= n)

@@ -262,6 +262,36 @@ def _delta_in_64_bits(proj, lens, conv, a_log, dt_bias, norm, H, G, dk, dv, taps
     return torch.cat(outs), torch.stack(states)
 
 
+@pytest.mark.parametrize("fit,parts", [(1000, 0), (12, 2), (8, 3), (3, 2)])
+def test_delta_rule_by_groups_and_windows_of_chunks(fit, parts, monkeypatch):
+    """However many records the scratch holds: groups of sequences and windows of chunks give the bits of all at once,
+    read-outs and states; without room for any scratch a step goes row by row."""
+    from grout_b200.kernels import ops
+    H, G, dk, dv, taps, lens = 4, 2, 32, 64, 3, [300, 65, 1, 130, 32]
+    monkeypatch.setattr(ops, "delta_chunks_pay", lambda T, n_seqs, max_rows: max_rows > 4)
+    Cc, i32 = 2 * G * dk + H * dv, lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    proj = rnd(sum(lens), Cc + H * dv + 2 * H, seed=51).to(DEV)
+    w = [t.to(DEV) for t in (rnd(Cc, taps, seed=52), rnd(H, seed=53), rnd(H, seed=54), rnd(dv, seed=55))]
+
+    def run(max_rows=max(lens)):
+        state = rnd(6, ops.delta_state_floats(H, G, dk, dv, taps), seed=56, scale=0.1).to(DEV)
+        y = ops.delta_forward(proj, state, *w, H=H, G=G, dk=dk, dv=dv, taps=taps, unit_eps=1e-6, norm_eps=1e-5,
+                              dtype=torch.float32, token_seq=i32([k for k, n in enumerate(lens) for _ in range(n)]),
+                              cu_q=i32([0] + torch.tensor(lens).cumsum(0).tolist()), slots=i32([4, 0, 2, 5, 1]),
+                              max_rows=max_rows)
+        return y, state
+
+    want = run()
+    monkeypatch.setattr(ops, "DELTA_CHUNK_BYTES", fit * 4 * H * ops.delta_record(dk, dv))
+    records, group, window = ops.delta_chunk_plan(sum(lens), len(lens), max(lens), H, dk, dv)
+    assert records <= fit and (-(-10 // window) * -(-5 // group) >= parts if parts else not window)
+    got = run()
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    monkeypatch.setattr(ops, "delta_chunk_plan", lambda *a: ((1 << 42) // (4 * H * ops.delta_record(dk, dv)), 0, 0))
+    got, want = run(), run(None)                  # (four terabytes)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
 @pytest.mark.parametrize("decay", [0.0, -4.0])
 def test_delta_rule_by_chunks_is_as_exact_as_row_by_row(decay):
     """The relative error against 64 bits of read-outs and states, chunk by chunk and row by row: both are 32-bit sums in
