@@ -1457,8 +1457,9 @@ def prefill_tc_pack(nq: int, nkv: int) -> int:
     return min(PREFILL_TC_PACK, g & -g)
 
 
-def prefill_tc_plan(blocks, nq: int, nkv: int, sms: int):
-    """(heads of a block, its query rows).  ``blocks(tokens)``: how many blocks of that many tokens the step makes.
+def prefill_tc_plan(blocks, nq: int, nkv: int, sms: int, one_head: bool = False):
+    """(heads of a block, its query rows).  ``blocks(tokens)``: how many blocks of that many tokens the step makes;
+    ``one_head``: no heads are packed.
 
     Blocks of 256 rows are two query blocks that share their key tiles, one block an SM; of 128 rows, half-size ones,
     two an SM.  Heads are packed into a block where one head a block would make more blocks of 256 than the GPU holds
@@ -1468,7 +1469,7 @@ def prefill_tc_plan(blocks, nq: int, nkv: int, sms: int):
     78.7; 2,048 tokens 54.4 / 46.4, 57.5 / 47.1; 384 tokens 11.0 / 13.8, 11.2 / 10.7.  16 heads on 8, 384 tokens behind
     768 beside five single ones 27.4 / 24.6, 27.2 / 22.4; 16 prompts of 128 tokens 10.1 / 10.0, 10.4 / 15.2."""
     whole = blocks(256) * nq
-    pack = prefill_tc_pack(nq, nkv) if 4 * whole > 5 * sms else 1
+    pack = prefill_tc_pack(nq, nkv) if 4 * whole > 5 * sms and not one_head else 1
     if PREFILL_TC_ROWS:
         return pack, PREFILL_TC_ROWS
     if pack == 1:
@@ -1492,8 +1493,9 @@ def attn_prefill_tc(q, k_pages, v_pages, block_table, *, cu_q, slots, kv_len, q_
     products on the tcgen05 tensor cores.  Pages must hold finite values in the
     rows beyond a sequence's length (the cache zero-fills its pages).  The grid is
     sized from ``q_lens`` (the host's copy of the row counts) or, without them,
-    from ``n_qblocks``, an upper bound of the blocks of ``rows_per_block`` rows (query rows
-    of ``pack`` heads; with ``rows_per_block`` given, as many as can share a block by default)."""
+    from ``n_qblocks``, an upper bound of the blocks of ``rows_per_block`` query rows.  A block has the rows of
+    ``pack`` heads: with ``rows_per_block`` given, as many as can share a block by default, or one where
+    the caller brings the bound."""
     _need(q, "q", torch.bfloat16, 3)
     T, nq, D = q.shape
     _need(k_pages, "k pages", torch.bfloat16, 4)
@@ -1513,13 +1515,15 @@ def attn_prefill_tc(q, k_pages, v_pages, block_table, *, cu_q, slots, kv_len, q_
     a.out, a.error = out.data_ptr(), _tc_error_flag(q.device).data_ptr()
     a.n_seqs, a.nq, a.nkv, a.max_pages = n_seqs, nq, nkv, block_table.shape[1]
     a.window = int(window or 0)
-    a.pack, rows = prefill_tc_plan(lambda n: _q_blocks(q_lens, None, n, T, n_seqs), nq, nkv, _sm_count(q.device))
+    a.pack, rows = prefill_tc_plan(lambda n: _q_blocks(q_lens, None, n, T, n_seqs), nq, nkv, _sm_count(q.device),
+                                   one_head=n_qblocks is not None)
     if rows_per_block:
-        a.pack, rows = int(pack or prefill_tc_pack(nq, nkv)), int(rows_per_block)
+        rows = int(rows_per_block)
+        a.pack = int(pack or (prefill_tc_pack(nq, nkv) if n_qblocks is None else 1))
     a.n_qblocks = _q_blocks(q_lens, n_qblocks, rows // a.pack, T, n_seqs)
-    while a.n_qblocks > 65535 and a.pack > 1:      # more than a grid has: fewer heads, more tokens a block
+    while n_qblocks is None and a.n_qblocks > 65535 and a.pack > 1:  # more than a grid has: fewer heads, more tokens a block
         a.pack //= 2
-        a.n_qblocks = _q_blocks(q_lens, n_qblocks, rows // a.pack, T, n_seqs)
+        a.n_qblocks = _q_blocks(q_lens, None, rows // a.pack, T, n_seqs)
     a.scale_log2 = float(scale) * _LOG2E
     a.keep_first, a.chunk = int(keep_first or 0), _chunk_arg(chunk, keep_first)
     _set_cap_and_sinks(a, scale, softcap, sinks, nq)

@@ -766,6 +766,24 @@ def test_attn_prefill_tc_takes_the_same_rows_however_they_are_blocked(nq, nkv):
     ops.check_kernel_errors()
 
 
+@pytest.mark.parametrize("rows_per_block", [0, 128, 256])
+def test_attn_prefill_tc_with_the_callers_bound_of_blocks(rows_per_block):
+    """A bound that counts blocks of query rows of one head covers all rows."""
+    ops = _ops()
+    nq, nkv, D, lens = 16, 2, 64, [1100, 300]
+    pc = Paged(lens, nkv, D, torch.bfloat16, 54, fill=300.0)
+    q = _rand((sum(lens), nq, D), torch.bfloat16, 55).to(DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    run = lambda **kw: ops.attn_prefill_tc(  # noqa: E731
+        q, pc.k_pages.to(DEV), pc.v_pages.to(DEV), pc.table.to(DEV), cu_q=i32([0, 1100, 1400]), slots=i32(pc.slot_of),
+        kv_len=i32(lens), page=64, scale=0.125, **kw)
+    want = run(rows_per_block=128, pack=1, q_lens=tuple(lens))
+    bound = sum(-(-n // (rows_per_block or 128)) for n in lens)
+    torch.full_like(q, float("nan"))               # (what the next allocation is likely to hold)
+    assert torch.equal(run(rows_per_block=rows_per_block, n_qblocks=bound), want)
+    ops.check_kernel_errors()
+
+
 @pytest.mark.parametrize("n_splits", [1, 3])
 @pytest.mark.parametrize("n", [1, 2, 31, 33, 64, 65])
 def test_attn_decode_tma_takes_every_sequence_once(n, n_splits, monkeypatch):
