@@ -1772,7 +1772,8 @@ def attention(q, k_pages, v_pages, block_table, *, step, page: int, scale: float
         return attn_prefill_bf16(q, k_pages, v_pages, block_table, cu_q=step.cu_q,
                                  slots=step.slots, kv_len=step.kv_len, q_lens=step.q_lens,
                                  page=page, scale=scale, window=window, **extra)
-    if q.dtype == torch.float32 and not keep_first and attn_f32_takes(q, k_pages.shape[1], step):
+    if (q.dtype == torch.float32 and not keep_first and (k_pages.data_ptr() | v_pages.data_ptr()) % 16 == 0
+            and attn_f32_takes(q, k_pages.shape[1], step)):
         return attn_f32(q, k_pages, v_pages, block_table, step=step, page=page, scale=scale, window=window,
                         softcap=softcap, sinks=sinks, chunk=chunk)
     return attn_generic(q, k_pages, v_pages, block_table, token_seq=step.token_seq,

@@ -326,6 +326,27 @@ def test_attn_f32(nq, nkv, D, page, window, chunk, cap, with_sinks):
             assert torch.equal(a[-1:], c)
 
 
+@pytest.mark.parametrize("off", ["q", "k", "v"])
+def test_32_bit_attention_of_unaligned_tensors(off):
+    """Queries or pages that do not start on 16 bytes are the plain kernel's."""
+    nq, nkv, D, lens = 4, 2, 32, [70, 5]
+    pc = Paged(lens, nkv, D, torch.float32, 56)
+    q = torch.randn((2, nq, D), generator=torch.Generator().manual_seed(57)).to(DEV)
+    step = _f32_step(lens, [n - 1 for n in lens], pc, True)
+    step.q_lens = (1, 1)
+
+    def shifted(t):
+        flat = torch.empty(t.numel() + 1, device=DEV)[1:].view(t.shape)
+        assert flat.data_ptr() % 16
+        return flat.copy_(t)
+
+    k, v, table = pc.k_pages.to(DEV), pc.v_pages.to(DEV), pc.table.to(DEV)
+    kw = dict(step=step, page=64, scale=0.2)
+    want = _ops().attention(q, k, v, table, **kw)
+    got = _ops().attention(*(shifted(t) if n == off else t for n, t in (("q", q), ("k", k), ("v", v))), table, **kw)
+    assert float((got - want).abs().max()) < 4e-6     # (two orders of the same 32-bit sums)
+
+
 def test_attn_f32_unseen_values_do_not_count():
     """A later key of the same tile whose value is infinite leaves the rows in front of it alone; a padding sequence
     gives zeros."""
