@@ -28,7 +28,7 @@ struct AttnF32Args {
   const int* slots;          // [n_seqs]
   const int* kv_len;         // [n_seqs]
   float* out;                // [n_tokens, nq, D]
-  float* parts;              // [n_seqs, nq, n_parts, D + 2], decode steps
+  float* parts;              // [n_seqs of a launch, nq, n_parts, D + 2], decode steps
   const float* sinks;        // [nq] or null
   int n_seqs, nq, nkv, D, page, max_pages, window, chunk, heads, n_qblocks, n_parts, page_shift;   // page_shift: log2(page), or -1
   float scale, softcap;
@@ -89,11 +89,11 @@ attn_f32_prompt_kernel(AttnF32Args a) {
   constexpr int LP = AF_BN + 4;
   const int tid = threadIdx.x, tx = tid % AF_LANES, ty = tid / AF_LANES;
   const int group = a.nq / a.nkv, subs = group / a.heads;
-  const int kvh = blockIdx.x / subs, head0 = kvh * group + blockIdx.x % subs * a.heads;
+  const int hx = blockIdx.x % (a.nkv * subs), kvh = hx / subs, head0 = kvh * group + hx % subs * a.heads;
   pdl_wait();
 
   // the block's sequence and its tokens
-  const int per = ROWS / a.heads, b = a.n_qblocks - 1 - blockIdx.y;    // heavy blocks first
+  const int per = ROWS / a.heads, b = a.n_qblocks - 1 - (int)(blockIdx.x / (a.nkv * subs));    // heavy blocks first
   int first_block;
   const int seq = find_query_block(a.cu_q, a.n_seqs, per, b, first_block);
   if (seq >= a.n_seqs) return;
@@ -247,9 +247,9 @@ attn_f32_prompt_kernel(AttnF32Args a) {
   }
 }
 
-// One tile of keys of a decode step's sequence for `heads` query heads: block (x, y) has kv head and heads x, sequence
-// and tile y.  A score is one thread's, a column's sum over the keys is one thread's; the sums of exponentials are added
-// by sixteen threads a row as in the kernel above.
+// One tile of keys of a decode step's sequence for `heads` query heads; the tiles of a sequence count from the one that
+// holds its first visible key.  A score is one thread's, a column's sum over the keys is one thread's; the sums of
+// exponentials are added by sixteen threads a row as in the kernel above.
 #define AD_THREADS 256
 __global__ void __launch_bounds__(AD_THREADS)
 attn_f32_decode_kernel(AttnF32Args a) {
@@ -261,18 +261,18 @@ attn_f32_decode_kernel(AttnF32Args a) {
   float* p_s = q_s + a.heads * D;                // [heads][64]
   const int tid = threadIdx.x;
   const int group = a.nq / a.nkv, subs = group / a.heads;
-  const int kvh = blockIdx.x / subs, head0 = kvh * group + blockIdx.x % subs * a.heads;
+  const int hx = blockIdx.x % (a.nkv * subs), kvh = hx / subs, head0 = kvh * group + hx % subs * a.heads;
   pdl_wait();
-  const int seq = blockIdx.y / a.n_parts, tile = blockIdx.y % a.n_parts;
+  const int at = blockIdx.x / (a.nkv * subs), seq = at / a.n_parts, part = at % a.n_parts;
   const int slot = a.slots[seq];
   const size_t row0 = (size_t)a.cu_q[seq] * a.nq + head0;
   if (slot < 0) {
-    if (tile == 0)
+    if (part == 0)
       for (int i = tid; i < a.heads * D; i += AD_THREADS) a.out[row0 * D + i] = 0.f;
     return;
   }
-  const int pos = a.kv_len[seq] - 1, lo = first_key(pos, a.window, a.chunk), key0 = tile * AF_BN;
-  if (key0 > pos || key0 + AF_BN <= lo) return;  // (the merge does not look at this tile either)
+  const int pos = a.kv_len[seq] - 1, lo = first_key(pos, a.window, a.chunk), key0 = (lo / AF_BN + part) * AF_BN;
+  if (key0 > pos) return;                        // (the merge does not look at this part either)
   const int* table = a.block_table + (size_t)slot * a.max_pages;
   auto load = [&](float* dst, const float* pages, int ld) {
 #pragma unroll 4
@@ -311,7 +311,7 @@ attn_f32_decode_kernel(AttnF32Args a) {
     p_s[i] = key <= pos && key >= lo ? v : -INFINITY;
   }
   __syncthreads();
-  float* parts = a.parts + (((size_t)seq * a.nq + head0) * a.n_parts + tile) * (D + 2);
+  float* parts = a.parts + (((size_t)seq * a.nq + head0) * a.n_parts + part) * (D + 2);
   const size_t part_ld = (size_t)a.n_parts * (D + 2);
   if (tid < 8 * AF_LANES) {                      // whole warps, whatever the number of heads
     const int r = tid / AF_LANES, tx = tid % AF_LANES;
@@ -356,12 +356,12 @@ __global__ void attn_f32_merge_kernel(AttnF32Args a) {
   const int seq = blockIdx.x, h = blockIdx.y, D = a.D;
   if (a.slots[seq] < 0) return;
   const int pos = a.kv_len[seq] - 1;
-  const int p_lo = first_key(pos, a.window, a.chunk) / AF_BN, p_hi = pos / AF_BN;
+  const int parts = pos / AF_BN - first_key(pos, a.window, a.chunk) / AF_BN + 1;
   const float* p = a.parts + ((size_t)seq * a.nq + h) * a.n_parts * (D + 2);
   const int d = threadIdx.x;
   float m = -INFINITY, l = 0.f, o = 0.f;
 #pragma unroll 8
-  for (int i = p_lo; i <= p_hi; ++i) {
+  for (int i = 0; i < parts; ++i) {
     const float pm = p[(size_t)i * (D + 2) + D], pl = p[(size_t)i * (D + 2) + D + 1], po = p[(size_t)i * (D + 2) + d];
     const float m_new = fmaxf(m, pm), was = af_scale(m, m_new), now = af_scale(pm, m_new);
     l = fmaf(l, was, pl * now);
@@ -379,32 +379,40 @@ __global__ void attn_f32_merge_kernel(AttnF32Args a) {
 }
 
 // heads: query heads of a block's rows, a divisor of those that share a kv head, at most 8.  decode: every sequence
-// brings one token; n_parts = ceil(longest / 64) tiles a sequence.
-GB_EXPORT int gb_attn_f32(const AttnF32Args* a, int decode, cudaStream_t stream) {
-  if (a->n_seqs <= 0 || a->nq <= 0 || a->nkv <= 0 || a->nq % a->nkv || a->max_pages <= 0 || a->page <= 0 ||
-      a->n_qblocks < 0 || a->chunk < 0 || a->n_parts < 1 || a->heads < 1 || a->heads > 8 ||
-      (a->nq / a->nkv) % a->heads)
+// brings one token; n_parts: the most tiles that a sequence's visible keys lie in; `group` sequences go at a time, whose
+// parts the scratch holds.  Blocks are numbered along one axis, heads first, so that no number of sequences, tiles or
+// tokens that a step can have is beyond a grid.
+GB_EXPORT int gb_attn_f32(const AttnF32Args* args, int decode, int group, cudaStream_t stream) {
+  AttnF32Args a = *args;
+  if (a.n_seqs <= 0 || a.nq <= 0 || a.nkv <= 0 || a.nq % a.nkv || a.max_pages <= 0 || a.page <= 0 || a.n_qblocks < 0 ||
+      a.chunk < 0 || a.n_parts < 1 || a.heads < 1 || a.heads > 8 || (a.nq / a.nkv) % a.heads)
     return GB_ERR_BAD_ARG;
-  if (a->D % 4 || a->D < 4 || a->D > 128 || ((size_t)a->q & 15) || ((size_t)a->out & 15) || ((size_t)a->k_pages & 15) ||
-      ((size_t)a->v_pages & 15))
+  if (a.D % 4 || a.D < 4 || a.D > 128 || a.nq > 65535 || ((size_t)a.q & 15) || ((size_t)a.out & 15) ||
+      ((size_t)a.k_pages & 15) || ((size_t)a.v_pages & 15))
     return GB_ERR_UNSUPPORTED;
+  const long long heads = a.nq / a.heads;
   if (!decode) {
     constexpr int RT = 4, TY = 8;
-    if (a->n_qblocks > 65535) return GB_ERR_UNSUPPORTED;
-    if (!a->n_qblocks) return 0;
-    const size_t smem = ((size_t)(RT * TY + AF_BN) * (a->D + 4) + AF_BN * a->D + RT * TY * (AF_BN + 4)) * sizeof(float);
+    if (heads * a.n_qblocks > 0x7fffffffll) return GB_ERR_UNSUPPORTED;
+    if (!a.n_qblocks) return 0;
+    const size_t smem = ((size_t)(RT * TY + AF_BN) * (a.D + 4) + AF_BN * a.D + RT * TY * (AF_BN + 4)) * sizeof(float);
     auto* kernel = attn_f32_prompt_kernel<RT, TY>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    return gb_launch(kernel, dim3(a->nq / a->heads, a->n_qblocks), dim3(TY * AF_LANES), smem, stream, *a);
+    return gb_launch(kernel, dim3((unsigned)(heads * a.n_qblocks)), dim3(TY * AF_LANES), smem, stream, a);
   }
-  if ((long long)a->n_seqs * a->n_parts > 65535 || a->nq > 65535) return GB_ERR_UNSUPPORTED;
-  if (!a->parts) return GB_ERR_BAD_ARG;
-  const size_t smem = ((size_t)AF_BN * (a->D + 4) + AF_BN * a->D + a->heads * (a->D + AF_BN)) * sizeof(float);
+  if (!a.parts || group < 1) return GB_ERR_BAD_ARG;
+  if (heads * a.n_parts * (group < a.n_seqs ? group : a.n_seqs) > 0x7fffffffll) return GB_ERR_UNSUPPORTED;
+  const size_t smem = ((size_t)AF_BN * (a.D + 4) + AF_BN * a.D + a.heads * (a.D + AF_BN)) * sizeof(float);
   cudaError_t e = cudaFuncSetAttribute(attn_f32_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024);
   if (e != cudaSuccess) return (int)e;
-  int rc = gb_launch(attn_f32_decode_kernel, dim3(a->nq / a->heads, a->n_seqs * a->n_parts), dim3(AD_THREADS), smem,
-                     stream, *a);
-  if (rc) return rc;
-  return gb_launch(attn_f32_merge_kernel, dim3(a->n_seqs, a->nq), dim3(a->D), 0, stream, *a);
+  for (int s = 0; s < args->n_seqs; s += group) {
+    a.cu_q = args->cu_q + s, a.slots = args->slots + s, a.kv_len = args->kv_len + s;
+    a.n_seqs = args->n_seqs - s < group ? args->n_seqs - s : group;
+    int rc = gb_launch(attn_f32_decode_kernel, dim3((unsigned)(heads * a.n_seqs * a.n_parts)), dim3(AD_THREADS), smem, stream,
+                       a);
+    if (!rc) rc = gb_launch(attn_f32_merge_kernel, dim3(a.n_seqs, a.nq), dim3(a.D), 0, stream, a);
+    if (rc) return rc;
+  }
+  return 0;
 }

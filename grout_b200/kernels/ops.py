@@ -791,6 +791,7 @@ class _AttnF32Args(ctypes.Structure):
 
 ATTN_F32_TILE = 64       # keys of a tile of attn_f32
 ATTN_F32_ROWS = 32       # query rows (tokens x heads) of a prompt's block
+ATTN_F32_BYTES = 256 << 20     # scratch of a decode step's parts; more sequences than it holds go one group after another
 
 
 def attn_f32_heads(nq: int, nkv: int) -> int:
@@ -799,14 +800,17 @@ def attn_f32_heads(nq: int, nkv: int) -> int:
 
 
 def attn_f32_takes(q, nkv: int, step) -> bool:
-    """Head sizes that are multiples of 4 up to 128, on 16-byte boundaries, and steps whose blocks fit a grid;
-    everything else is the plain kernel's."""
-    T, nq, D = q.shape
-    if D % 4 or D > 128 or q.data_ptr() % 16:
-        return False
-    if step.decode:
-        return step.n_seqs * -(-step.max_kv_len // ATTN_F32_TILE) <= 65535 and nq <= 65535
-    return step.q_blocks(ATTN_F32_ROWS // attn_f32_heads(nq, nkv)) <= 65535
+    """Head sizes that are multiples of 4 up to 128, on 16-byte boundaries; everything else is the plain kernel's.
+    Nothing of the step counts, so that a row's kernel, and with it the order of its sums, does not depend on the
+    step it is in."""
+    _T, nq, D = q.shape
+    return D % 4 == 0 and D <= 128 and nq <= 65535 and q.data_ptr() % 16 == 0
+
+
+def attn_f32_parts(max_kv_len: int, window: Optional[int], chunk: int) -> int:
+    """The most tiles that the keys which a decode row sees lie in."""
+    seen = min(window or max_kv_len, chunk or max_kv_len)
+    return min(-(-max_kv_len // ATTN_F32_TILE), (seen + ATTN_F32_TILE - 2) // ATTN_F32_TILE + 1)
 
 
 @_profiled("attn_generic", lambda out, q, *a, **k: (_nbytes(q, out), 0))
@@ -831,14 +835,15 @@ def attn_f32(q, k_pages, v_pages, block_table, *, step, page: int, scale: float,
     a.page_shift = page.bit_length() - 1 if page & (page - 1) == 0 else -1
     a.scale, a.softcap = float(scale), float(softcap or 0.0)
     a.n_qblocks = 0 if step.decode else step.q_blocks(ATTN_F32_ROWS // a.heads)
-    a.n_parts, parts = 1, None
+    a.n_parts, group, parts = 1, 1, None
     if step.decode:
-        a.n_parts = -(-step.max_kv_len // ATTN_F32_TILE)
-        parts = torch.empty((n_seqs, nq, a.n_parts, D + 2), dtype=torch.float32, device=q.device)
+        a.n_parts = attn_f32_parts(step.max_kv_len, a.window, a.chunk)
+        group = min(n_seqs, max(1, ATTN_F32_BYTES // (4 * nq * a.n_parts * (D + 2))))
+        parts = torch.empty((group, nq, a.n_parts, D + 2), dtype=torch.float32, device=q.device)
         a.parts = parts.data_ptr()
     with torch.cuda.device(q.device):
-        _check(_fn("attn_f32", "gb_attn_f32", "pip")(ctypes.addressof(a), int(step.decode), _stream()), "attn_f32",
-               1 + bool(step.decode))
+        _check(_fn("attn_f32", "gb_attn_f32", "piip")(ctypes.addressof(a), int(step.decode), group, _stream()), "attn_f32",
+               2 * -(-n_seqs // group) if step.decode else 1)
     return out
 
 

@@ -182,3 +182,15 @@ def test_the_scratch_of_the_delta_rule_by_chunks():
             records, group, window = ops.delta_chunk_plan(n * rows, n, rows, H, dk, dv)
             assert records * record <= ops.DELTA_CHUNK_BYTES
             assert records == (group * window if window else n * rows // 32 + n) and (not window or 1 <= group <= n)
+
+
+def test_the_tiles_a_32_bit_decode_row_may_touch():
+    """Never fewer than a row's visible keys lie in, whatever its position, and no more than any row's."""
+    from grout_b200.kernels.ops import attn_f32_parts
+    for bound in (1, 64, 65, 300):
+        for window, chunk in ((None, 0), (1, 0), (2, 0), (64, 0), (65, 0), (66, 0), (500, 0), (0, 1), (0, 64), (0, 100)):
+            most = 0
+            for pos in range(bound):
+                lo = max(0, pos - window + 1) if window else pos - pos % chunk if chunk else 0
+                most = max(most, pos // 64 - lo // 64 + 1)
+            assert most <= attn_f32_parts(bound, window, chunk) <= most + 1

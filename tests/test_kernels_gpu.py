@@ -326,6 +326,33 @@ def test_attn_f32(nq, nkv, D, page, window, chunk, cap, with_sinks):
             assert torch.equal(a[-1:], c)
 
 
+@pytest.mark.parametrize("window,chunk", [(None, 0), (65, 0), (1, 0), (64, 0), (None, 64), (None, 100)])
+def test_attn_f32_decode_steps_of_any_bound(window, chunk, monkeypatch):
+    """More sequences times tiles of the bound than a grid is high, and a scratch that holds a few sequences at a time:
+    the same kernel, and the same bits as with the bound that the lengths need."""
+    ops = _ops()
+    nq, nkv, D = 4, 2, 8
+    lens = [(1, 63, 64, 65, 130, 200)[i % 6] for i in range(180)]
+    pc = Paged(lens, nkv, D, torch.float32, 58)
+    q = torch.randn((len(lens), nq, D), generator=torch.Generator().manual_seed(59)).to(DEV)
+    pages = pc.k_pages.to(DEV), pc.v_pages.to(DEV), pc.table.to(DEV)
+
+    def run(bound):
+        step = _f32_step(lens, [n - 1 for n in lens], pc, True, bound)
+        step.q_lens = (1,) * len(lens)
+        return ops.attention(q, *pages, step=step, page=64, scale=0.3, window=window, chunk=chunk)
+
+    want = run(None)
+    step = _f32_step(lens, [n - 1 for n in lens], pc, True, None)
+    plain = ops.attn_generic(q, *pages, token_seq=step.token_seq, token_pos=step.token_pos, slots=step.slots, page=64,
+                             scale=0.3, window=window, chunk=chunk)
+    assert float((want - plain).abs().max()) < 4e-6
+    assert torch.equal(run(64 * 400), want)
+    parts = ops.attn_f32_parts(200, window, chunk)
+    monkeypatch.setattr(ops, "ATTN_F32_BYTES", 7 * 4 * nq * parts * (D + 2))
+    assert torch.equal(run(None), want)
+
+
 @pytest.mark.parametrize("off", ["q", "k", "v"])
 def test_32_bit_attention_of_unaligned_tensors(off):
     """Queries or pages that do not start on 16 bytes are the plain kernel's."""
