@@ -813,7 +813,9 @@ def attn_f32_parts(max_kv_len: int, window: Optional[int], chunk: int) -> int:
     return min(-(-max_kv_len // ATTN_F32_TILE), (seen + ATTN_F32_TILE - 2) // ATTN_F32_TILE + 1)
 
 
-@_profiled("attn_generic", lambda out, q, *a, **k: (_nbytes(q, out), 0))
+# (a report has one row for the attention of the 32-bit path, whichever of its kernels ran)
+@_profiled("attn_generic", lambda out, q, k_pages, *a, step, **k: _cost_attention(
+    out, q, k_pages, kv_len=step.kv_len, slots=step.slots, cu_q=step.cu_q, window=k.get("window"), chunk=k.get("chunk")))
 def attn_f32(q, k_pages, v_pages, block_table, *, step, page: int, scale: float, window: Optional[int] = None,
              softcap: Optional[float] = None, sinks: Optional[torch.Tensor] = None, chunk: int = 0) -> torch.Tensor:
     """The 32-bit attention of a step's queries (``attention`` says what the options mean)."""

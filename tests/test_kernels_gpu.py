@@ -374,6 +374,23 @@ def test_32_bit_attention_of_unaligned_tensors(off):
     assert float((got - want).abs().max()) < 4e-6     # (two orders of the same 32-bit sums)
 
 
+def test_attn_f32_is_profiled_with_its_keys_and_products():
+    ops = _ops()
+    nq, nkv, D, lens = 4, 2, 32, [70, 5]
+    pc = Paged(lens, nkv, D, torch.float32, 60)
+    q = torch.randn((sum(lens), nq, D), generator=torch.Generator().manual_seed(61)).to(DEV)
+    step = _f32_step(lens, [0, 0], pc, False)
+    ops.set_profile(ops.OpProfile())
+    try:
+        ops.attn_f32(q, pc.k_pages.to(DEV), pc.v_pages.to(DEV), pc.table.to(DEV), step=step, page=64, scale=0.2)
+        prof = ops._PROFILE
+    finally:
+        ops.set_profile(None)
+    calls, _ms, nbytes, flops = prof.totals()["attn_generic"]
+    pairs = sum(n * (n + 1) // 2 for n in lens)
+    assert calls == 1 and nbytes == 4 * (2 * q.numel() + 2 * sum(lens) * nkv * D) and flops == 4 * pairs * nq * D
+
+
 def test_attn_f32_unseen_values_do_not_count():
     """A later key of the same tile whose value is infinite leaves the rows in front of it alone; a padding sequence
     gives zeros."""
