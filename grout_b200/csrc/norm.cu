@@ -410,7 +410,9 @@ __global__ void add_postnorm_kernel(const PostNormArgs a) {
 // 16,384 on 16-byte boundaries.  A decode step's row is a chain of latencies (the partial sums, two block-wide sums), so
 // everything that no kernel of the step writes, the weights, is asked for before the wait, and all of the row at once
 // behind it; a prompt's rows are bound by memory, and small blocks keep many of them in flight.  Rows of 2,048,
-// inside a step of one row: 4.3 us exposed (7.9 with the row in shared memory, a value at a time).
+// inside a step of one row: 4.3 us exposed (7.9 with the row in shared memory, a value at a time).  One row of eight partial
+// sums and 1,024 rows of one, back to back, us, with the row in shared memory behind the stroke: 2,048 wide 2.7, 7.9 / 5.3,
+// 13.8; 8,192 4.6, 23 / 14.9, 46; 8,196 6.9, 35 / 15.3, 45; 10,240 7.2, 44 / 17.9, 66; 16,384 9.0, 64 / 27, 144.
 template <typename T> __device__ __forceinline__ float4 pn_load4(const T* p);
 template <> __device__ __forceinline__ float4 pn_load4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
 template <> __device__ __forceinline__ float4 pn_load4<bf16>(const bf16* p) {
@@ -426,20 +428,24 @@ __device__ __forceinline__ void pn_store4(bf16* p, float4 v) {
   *reinterpret_cast<uint2*>(p) = u;
 }
 
-template <typename T, int V>
-__global__ void __launch_bounds__(512) add_postnorm_vec_kernel(const PostNormArgs a) {
+// EARLY: the weights are asked for in front of the wait; the threads of wide rows, of which there are up to 1,024, have no
+// registers to hold them (64, and 64 bytes of spills in bfloat16), and read them where they are used.
+template <typename T, int V, int THREADS, bool EARLY>
+__global__ void __launch_bounds__(THREADS) add_postnorm_vec_kernel(const PostNormArgs a) {
   __shared__ float scratch[32];
   pdl_launch_dependents_if_small();
   const int N = a.N, r = blockIdx.x, tid = threadIdx.x, step = blockDim.x;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), one = make_float4(1.f, 1.f, 1.f, 1.f);
   float4 wp[V], ws[V], wy[V];      // what multiplies the delta, the same again, and the row
+  const auto weight = [&](const float* w, int at) { return at < N && w ? *reinterpret_cast<const float4*>(w + at) : one; };
+  if constexpr (EARLY) {
 #pragma unroll
-  for (int i = 0; i < V; ++i) {
-    const int at = (tid + i * step) * 4;
-    const bool in = at < N;
-    wp[i] = in && a.post_w ? *reinterpret_cast<const float4*>(a.post_w + at) : one;
-    ws[i] = in && a.scale ? *reinterpret_cast<const float4*>(a.scale + at) : one;
-    wy[i] = in && a.w ? *reinterpret_cast<const float4*>(a.w + at) : one;
+    for (int i = 0; i < V; ++i) {
+      const int at = (tid + i * step) * 4;
+      wp[i] = weight(a.post_w, at);
+      ws[i] = weight(a.scale, at);
+      wy[i] = weight(a.w, at);
+    }
   }
   pdl_wait();
   const size_t s = a.rows ? (size_t)a.rows[r] : (size_t)r;
@@ -454,7 +460,7 @@ __global__ void __launch_bounds__(512) add_postnorm_vec_kernel(const PostNormArg
   }
   if (a.parts) {
     const float* pin = a.parts + s * N;
-    constexpr int U = V <= 2 ? 4 : V == 4 ? 2 : 1;
+    constexpr int U = V <= 2 ? 4 : EARLY ? 2 : 1;
     int k = 0;
     for (; k + U <= a.n_parts; k += U) {       // asked for U at a time, added in their order
       float4 p[U][V];
@@ -488,6 +494,7 @@ __global__ void __launch_bounds__(512) add_postnorm_vec_kernel(const PostNormArg
     }
 #pragma unroll
     for (int i = 0; i < V; ++i) {
+      if constexpr (!EARLY) wp[i] = weight(a.post_w, (tid + i * step) * 4), ws[i] = weight(a.scale, (tid + i * step) * 4);
       v[i].x += d[i].x * inv_d * wp[i].x * ws[i].x, v[i].y += d[i].y * inv_d * wp[i].y * ws[i].y;
       v[i].z += d[i].z * inv_d * wp[i].z * ws[i].z, v[i].w += d[i].w * inv_d * wp[i].w * ws[i].w;
     }
@@ -508,6 +515,7 @@ __global__ void __launch_bounds__(512) add_postnorm_vec_kernel(const PostNormArg
 #pragma unroll
   for (int i = 0; i < V; ++i) {
     const int at = (tid + i * step) * 4;
+    if constexpr (!EARLY) wy[i] = weight(a.w, at);
     if (at < N)
       pn_store4((T*)a.y + (size_t)r * N + at, make_float4(v[i].x * inv * wy[i].x, v[i].y * inv * wy[i].y,
                                                           v[i].z * inv * wy[i].z, v[i].w * inv * wy[i].w));
@@ -515,10 +523,10 @@ __global__ void __launch_bounds__(512) add_postnorm_vec_kernel(const PostNormArg
   pdl_launch_dependents_if_large();
 }
 
-template <typename T, int V>
+template <typename T, int V, int THREADS, bool EARLY>
 static int add_postnorm_vec_launch(const PostNormArgs& a, cudaStream_t stream) {
   const int threads = ((a.N / 4 + V - 1) / V + 31) / 32 * 32;    // by N only
-  return gb_launch(add_postnorm_vec_kernel<T, V>, dim3(a.n_rows), dim3(threads), 0, stream, a);
+  return gb_launch(add_postnorm_vec_kernel<T, V, THREADS, EARLY>, dim3(a.n_rows), dim3(threads), 0, stream, a);
 }
 
 template <typename T>
@@ -531,9 +539,9 @@ static int add_postnorm_launch(const PostNormArgs& a, cudaStream_t stream) {
   if (a.N % 4 == 0 && a.N <= 16384 && !(vectors & 15) && !(((uintptr_t)a.delta | (uintptr_t)a.y) & (4 * sizeof(T) - 1)) &&
       !(a.parts && a.part_stride % 4)) {
     // (by N only, so that a row's sums do not depend on the step; the alignment is the same for every step's buffers)
-    if (a.N <= 4096) return add_postnorm_vec_launch<T, 2>(a, stream);
-    if (a.N <= 8192) return add_postnorm_vec_launch<T, 4>(a, stream);
-    return add_postnorm_vec_launch<T, 8>(a, stream);
+    if (a.N <= 4096) return add_postnorm_vec_launch<T, 2, 512, true>(a, stream);
+    if (a.N <= 8192) return add_postnorm_vec_launch<T, 4, 512, true>(a, stream);
+    return add_postnorm_vec_launch<T, 4, 1024, false>(a, stream);
   }
   const size_t smem = (size_t)a.N * sizeof(float);
   if (smem > 200 * 1024) return GB_ERR_UNSUPPORTED;

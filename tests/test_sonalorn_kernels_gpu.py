@@ -67,7 +67,7 @@ def test_stream_sum_through_norm_and_scale(dtype, N):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("N,S", [(4, 1), (1001, 2), (4096, 5), (4100, 9), (8196, 3), (16384, 4), (16388, 2)])
+@pytest.mark.parametrize("N,S", [(4, 1), (1001, 2), (4096, 5), (4100, 9), (8196, 3), (12288, 5), (16384, 4), (16388, 2)])
 def test_stream_sum_at_the_widths_where_its_kernel_changes(N, S, dtype):
     from grout_b200.kernels import ops
     res, parts = rnd(3, N, seed=1), rnd(S, 3, N, seed=2)
