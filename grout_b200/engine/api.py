@@ -67,7 +67,9 @@ class Engine:
         self.cache = SequenceCache(model.cache_layout(), max_tokens=max_tokens,
                                    max_slots=max_batch, max_seq_len=self.max_seq_len,
                                    dtype=dtype, device=device)
-        self.use_graphs = True if use_graphs is None else bool(use_graphs)
+        # 32-bit steps run from graphs when all parts are this library's: a caller's own part may read the device or keep
+        # count of its steps, which a replay does not do, and in 32-bit it has always been called for every step
+        self.use_graphs = (dtype == torch.bfloat16 or model.own_parts()) if use_graphs is None else bool(use_graphs)
         self.graphs = StepGraphs(model, self.cache, device,
                                  prompt_tokens=PROMPT_TOKENS_MOST if dtype == torch.bfloat16 else PROMPT_TOKENS_F32)
         self.vocab_size = plan.vocab_size

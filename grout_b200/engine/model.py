@@ -103,6 +103,13 @@ class Model:
                    for top in [self.embedding, *self.blocks, self.final_norm, self.head]
                    for p in _walk(top))
 
+    def own_parts(self) -> bool:
+        """Whether every part is one of this library's, none a caller's own."""
+        package = __name__.partition(".")[0]
+        return all(type(p).__module__.partition(".")[0] == package
+                   for top in [self.embedding, *self.blocks, self.final_norm, self.head]
+                   for p in _walk(top))
+
     # -- forward -----------------------------------------------------------
     def forward(self, step: StepContext, cache: SequenceCache) -> Optional[torch.Tensor]:
         """Runs the step's tokens through every scheduled layer; returns 32-bit

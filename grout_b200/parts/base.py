@@ -111,7 +111,8 @@ class Part:
         the host copies ``q_lens``, ``starts`` and ``slot_list``, which a captured
         step leaves empty.  Rows of slot -1 and sequences without rows are
         padding.  The default is False: the step then runs launch by launch.
-        (Decode steps are always captured; their contract is the mixer's.)"""
+        (Decode steps are captured whatever the parts say, in 32-bit unless the model has a part of the
+        caller's own; their contract is the mixer's.)"""
         return False
 
 

@@ -206,3 +206,24 @@ def test_toy_model_steps_in_every_cut(toy, dtype, graphs):
         for g, x in zip(got, want):
             assert_close(g, x, dtype, "toy batch")
     eng.cache.check()
+
+
+def test_a_part_of_ones_own_is_called_for_every_32_bit_step(toy, monkeypatch):
+    """A part that reads the device in its forward runs in 32-bit decode steps: by default they are captured only when
+    all parts are the library's."""
+    from grout_b200.engine import Engine
+    from grout_b200.parts.base import _REGISTRY
+    d, w = toy
+    part, calls = _REGISTRY["mixer", "toy_decay_state"], []
+    forward = part.forward
+
+    def reading(self, x, step, cache):
+        calls.append(int(step.slots.max()))              # waits for the device
+        return forward(self, x, step, cache)
+
+    monkeypatch.setattr(part, "forward", reading)
+    eng = Engine.load(d, dtype="float32", max_tokens=2048, max_batch=4)
+    assert not eng.use_graphs
+    tokens = random_tokens(20, TOY["vocab"], 950)
+    assert_close(run_tail_decoded(eng, tokens, tail=5), _toy_oracle(w, TOY, tokens), "float32", "toy")
+    assert len(calls) == 2 * 6 and min(calls) >= 0       # its layer runs twice in each of six steps
