@@ -71,7 +71,7 @@ __device__ __forceinline__ void stage_rows(float* dst, const float* src, int row
 template <int MT, int ROWS_N, int ROWS_STAGES, bool VEC>
 __global__ void __launch_bounds__(ROWS_N * 16)
 f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N,
-                int K, int lda, int ldw, int ldc, int tiles, int m_tiles) {
+                int K, int lda, int ldw, int ldc, int tiles, int m_tiles, int settled) {
   constexpr int ROWS_THREADS = ROWS_N * 16;
   extern __shared__ float4 sm4[];
   float* sm = (float*)sm4;
@@ -88,7 +88,8 @@ f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
     const int tile = blockIdx.x + (u / chunks) * gridDim.x;
     n0 = tile / m_tiles * ROWS_N, m0 = tile % m_tiles * MT, k0 = u % chunks * CHUNK;
   };
-  // the first weights, which no kernel writes, are asked for before the wait
+  // the first weights are asked for before the wait where no kernel still writes them
+  if (!settled) pdl_wait();
 #pragma unroll
   for (int s = 0; s < ROWS_STAGES; ++s) {
     if (s < total_units) {
@@ -214,7 +215,7 @@ constexpr size_t tile_smem(int slots) {     // tiles, ring, and the chunks' sums
 template <int BM, int BN, int TM, int TN, bool VEC>
 __global__ void __launch_bounds__(TILE_THREADS)
 f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, float* C, int M, int N, int K, int lda,
-                int ldw, int ldc, int split, int per_rank) {
+                int ldw, int ldc, int split, int per_rank, int settled) {
   static_assert((BM / TM) * (BN / TN) == TILE_THREADS, "threads");
   static_assert((TM == 4 || TM == 8) && (TN == 4 || TN == 8), "outputs of a thread");
   static_assert(tile_smem<BM, BN>(1) >= BM * BN * sizeof(float), "one slot of sums fits where the tiles were");
@@ -301,6 +302,7 @@ f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
 #pragma unroll
     for (int j = 0; j < TN / 2; ++j) acc[i][j] = mid[i][j] = 0ull;
 
+  if (!settled) pdl_wait();
   for (int s = 0; s < TILE_STAGES; ++s)
     if (s < steps) copy_w(s);
   pdl_wait();
@@ -389,7 +391,7 @@ static int sm_count() {
 
 template <int MT, int ROWS_N, int ROWS_STAGES, bool VEC>
 static int launch_rows(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc,
-                       int sms, cudaStream_t stream) {
+                       int sms, int settled, cudaStream_t stream) {
   constexpr size_t smem = (ROWS_STAGES * (ROWS_N + MT) * CHUNK + 32 * (ROWS_N * MT + 1)) * sizeof(float);
   auto* kernel = f32_rows_kernel<MT, ROWS_N, ROWS_STAGES, VEC>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -401,12 +403,12 @@ static int launch_rows(const float* A, const float* W, float* C, int M, int N, i
   const int each = (int)((tiles + fit - 1) / fit);           // whole tiles a block, as even as they come
   const int blocks = (int)((tiles + each - 1) / each);
   return gb_launch(kernel, dim3(blocks), dim3(ROWS_N * 16), smem, stream, A, W, C, M, N, K, lda, ldw, ldc,
-                   (int)tiles, m_tiles);
+                   (int)tiles, m_tiles, settled);
 }
 
 template <int BM, int BN, int TM, int TN, bool VEC>
 static int launch_tile(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc,
-                       cudaStream_t stream) {
+                       int settled, cudaStream_t stream) {
   const int chunks = (K + CHUNK - 1) / CHUNK;
   // one block for each chunk of a tile, or for a few where the cluster of eight would not do; sums of several chunks
   // take shared memory that two blocks of the large tile would not have
@@ -420,12 +422,12 @@ static int launch_tile(const float* A, const float* W, float* C, int M, int N, i
   dim3 grid((M + BM - 1) / BM * split, (N + BN - 1) / BN);
   if (grid.y > 65535) return GB_ERR_UNSUPPORTED;
   return gb_launch_cluster(kernel, grid, dim3(TILE_THREADS), smem, stream, split, A, W, C, M, N, K, lda, ldw, ldc,
-                           split, per_rank);
+                           split, per_rank, settled);
 }
 
 template <bool VEC>
 static int launch(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, int kind,
-                  cudaStream_t stream) {
+                  int settled, cudaStream_t stream) {
   const int sms = sm_count();
   if (kind == 0) {
     // Measured on 2,048-wide layers (us; rows / small / medium / large): 16 rows x 12,288 62 / 70 / 98 / 121; 24 rows
@@ -441,25 +443,26 @@ static int launch(const float* A, const float* W, float* C, int M, int N, int K,
   switch (kind) {
     case 1:
       // two blocks an SM up to four rows (three stages for one), a larger block from there
-      if (M <= 1) return launch_rows<1, 8, 3, VEC>(A, W, C, M, N, K, lda, ldw, ldc, sms, stream);
-      if (M <= 2) return launch_rows<2, 8, 2, VEC>(A, W, C, M, N, K, lda, ldw, ldc, sms, stream);
-      if (M <= 4) return launch_rows<4, 8, 2, VEC>(A, W, C, M, N, K, lda, ldw, ldc, sms, stream);
-      return launch_rows<8, 16, 2, VEC>(A, W, C, M, N, K, lda, ldw, ldc, sms, stream);
-    case 2: return launch_tile<32, 64, 4, 4, VEC>(A, W, C, M, N, K, lda, ldw, ldc, stream);
-    case 3: return launch_tile<64, 64, 8, 4, VEC>(A, W, C, M, N, K, lda, ldw, ldc, stream);
-    case 4: return launch_tile<64, 128, 8, 8, VEC>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+      if (M <= 1) return launch_rows<1, 8, 3, VEC>(A, W, C, M, N, K, lda, ldw, ldc, sms, settled, stream);
+      if (M <= 2) return launch_rows<2, 8, 2, VEC>(A, W, C, M, N, K, lda, ldw, ldc, sms, settled, stream);
+      if (M <= 4) return launch_rows<4, 8, 2, VEC>(A, W, C, M, N, K, lda, ldw, ldc, sms, settled, stream);
+      return launch_rows<8, 16, 2, VEC>(A, W, C, M, N, K, lda, ldw, ldc, sms, settled, stream);
+    case 2: return launch_tile<32, 64, 4, 4, VEC>(A, W, C, M, N, K, lda, ldw, ldc, settled, stream);
+    case 3: return launch_tile<64, 64, 8, 4, VEC>(A, W, C, M, N, K, lda, ldw, ldc, settled, stream);
+    case 4: return launch_tile<64, 128, 8, 8, VEC>(A, W, C, M, N, K, lda, ldw, ldc, settled, stream);
   }
   return GB_ERR_BAD_ARG;
 }
 
 // kind: 0 chooses; 1 the stream of weights, 2, 3 and 4 the small, the medium and the large tile.  All give the same
-// bits.
+// bits.  settled: no kernel that may still run writes W (a model's weights), so that its first tiles may be read before
+// the kernel in front has finished.
 GB_EXPORT int gb_gemm_nt_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc,
-                             int kind, cudaStream_t stream) {
+                             int kind, int settled, cudaStream_t stream) {
   if (M < 0 || N <= 0 || K <= 0 || lda < K || ldw < K || ldc < N) return GB_ERR_BAD_ARG;
   if (M == 0) return 0;
   // 16-byte loads want every row to start on 16 bytes and to end on a whole piece
   const bool vec = !(K % 4 || lda % 4 || ldw % 4 || ((size_t)A & 15) || ((size_t)W & 15));
-  return vec ? launch<true>(A, W, C, M, N, K, lda, ldw, ldc, kind, stream)
-             : launch<false>(A, W, C, M, N, K, lda, ldw, ldc, kind, stream);
+  return vec ? launch<true>(A, W, C, M, N, K, lda, ldw, ldc, kind, settled, stream)
+             : launch<false>(A, W, C, M, N, K, lda, ldw, ldc, kind, settled, stream);
 }

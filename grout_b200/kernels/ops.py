@@ -861,10 +861,12 @@ def _result(shape, dtype, device, into: Optional[torch.Tensor]) -> torch.Tensor:
 
 
 @_profiled("gemm_f32", _cost_gemm)
-def gemm_f32(a: torch.Tensor, w: torch.Tensor, into: Optional[torch.Tensor] = None, kind: int = 0) -> torch.Tensor:
+def gemm_f32(a: torch.Tensor, w: torch.Tensor, into: Optional[torch.Tensor] = None, kind: int = 0,
+             settled: bool = False) -> torch.Tensor:
     """a [M, K] . w [N, K]^T in true 32-bit on the CUDA cores (written into ``into`` when given).
     ``kind``: 0 chooses the kernel; 1 the stream of weights, 2, 3 and 4 the small, the medium and the
-    large tile.  All give the same bits."""
+    large tile.  All give the same bits.  ``settled``: w is not the result of a kernel of this library that
+    may still run (a model's weights), so it may be read while the kernel in front finishes."""
     _need(a, "activations", torch.float32, 2)
     _need(w, "weight", torch.float32, 2)
     M, K = a.shape
@@ -872,8 +874,8 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, into: Optional[torch.Tensor] = No
     if w.shape[1] != K:
         raise KernelError(f"weight is {tuple(w.shape)} for activations of width {K}")
     c = _result((M, N), torch.float32, a.device, into)
-    _check(_fn("gemm_f32", "gb_gemm_nt_f32", "pppiiiiiiip")(
-        a.data_ptr(), w.data_ptr(), c.data_ptr(), M, N, K, K, K, N, int(kind), _stream()), "gemm_f32")
+    _check(_fn("gemm_f32", "gb_gemm_nt_f32", "pppiiiiiiiip")(
+        a.data_ptr(), w.data_ptr(), c.data_ptr(), M, N, K, K, K, N, int(kind), int(settled), _stream()), "gemm_f32")
     return c
 
 

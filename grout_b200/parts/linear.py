@@ -68,8 +68,8 @@ class Linear:
         w = self.weight
         if w.dtype == torch.float32:
             if into is not None:
-                return ops.gemm_f32(ops.cast(x, torch.float32), w, into=into)
-            y = ops.gemm_f32(ops.cast(x, torch.float32), w)
+                return ops.gemm_f32(ops.cast(x, torch.float32), w, into=into, settled=True)
+            y = ops.gemm_f32(ops.cast(x, torch.float32), w, settled=True)
             return ops.cast(y, out_dtype)
         if x.dtype != torch.bfloat16:
             raise ops.KernelError("a bfloat16 weight takes bfloat16 activations")

@@ -444,6 +444,31 @@ def test_gemm_f32_sums_in_one_order(M, N, K, kind):
     assert torch.allclose(got, want, atol=2e-6 * math.sqrt(K), rtol=1e-6)
 
 
+@pytest.mark.parametrize("kind", [1, 2, 3, 4])
+def test_gemm_f32_of_a_weight_that_was_just_computed(kind):
+    """The second operand is the result of the kernel in front, which lets its successor in on entry: the product reads it
+    when it is there."""
+    ops = _ops()
+    M, N, K = 3, 64, 2048
+    a, w0 = _rand((M, K), torch.float32, 62).to(DEV), _rand((N, K), torch.float32, 63).to(DEV)
+    w, want = w0.clone(), []
+    for i in range(8):
+        ops.scale_softcap_(w, 0.5 + 0.25 * i, None)
+        torch.cuda.synchronize()
+        want.append(ops.gemm_f32(a, w, kind=kind))
+    w.copy_(w0)
+    torch.cuda.synchronize()
+    graph, got = torch.cuda.CUDAGraph(), []
+    with torch.cuda.graph(graph):
+        for i in range(8):
+            ops.scale_softcap_(w, 0.5 + 0.25 * i, None)
+            got.append(ops.gemm_f32(a, w, kind=kind))
+    w.copy_(w0)
+    graph.replay()
+    for x, y in zip(got, want):
+        assert torch.equal(x, y)
+
+
 def test_gemm_f32_row_independent():
     """A row's result does not depend on the rows beside it (bitwise)."""
     a, w = _rand((70, 96), torch.float32, 22), _rand((50, 96), torch.float32, 23)
