@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(256) delta_chain_kernel(const Args a) {
 #define CO_COLS 128
 #define CO_STAGE (CC_ROWS * (CC_ROWS + CO_COLS))
 template <typename T, typename Args>
-__global__ void __launch_bounds__(256) delta_out_kernel(const Args a) {
+__global__ void __launch_bounds__(256, 4) delta_out_kernel(const Args a) {
   extern __shared__ __align__(16) float sm[];    // two stages [A: 32 x 32 | B: 32 x CO_COLS] | the read-outs [32][dv]
   pdl_launch_dependents_if_small();
   const int tid = threadIdx.x, lane = tid & 31, row = tid / 32 * 4;
@@ -239,21 +239,35 @@ __global__ void __launch_bounds__(256) delta_out_kernel(const Args a) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
     }
-    const int nk = min(CC_ROWS, K - s % tiles * CC_ROWS);
+    // The terms of U go up to a row's own: those of later rows, whose factors are zero, may not be finite.  (All bounds
+    // are multiples of four: `below` terms are all four rows', the next four one row's less each.)
+    const int k0 = s % tiles * CC_ROWS, nk = min(CC_ROWS, K - k0), own = dk + row - k0, below = max(0, min(nk, own));
     float part[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) part[i][j] = 0.f;
-#pragma unroll 8
-    for (int k = 0; k < nk; ++k) {               // (columns beyond dv hold what no one reads)
+    const auto term = [&](int k, int from) {     // (columns beyond dv hold what no one reads)
       const float4 x = *reinterpret_cast<const float4*>(as + k * CC_ROWS + row);
       const float4 y = *reinterpret_cast<const float4*>(bs + k * CO_COLS + lane * 4);
       const float xv[4] = {x.x, x.y, x.z, x.w}, yv[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) part[i][j] = fmaf(xv[i], yv[j], part[i][j]);
+        for (int j = 0; j < 4; ++j)
+          if (i >= from) part[i][j] = fmaf(xv[i], yv[j], part[i][j]);
+    };
+    if (below == nk) {
+#pragma unroll 8
+      for (int k = 0; k < nk; ++k) term(k, 0);
+    } else {
+#pragma unroll 1
+      for (int k = 0; k < below; k += 4)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) term(k + u, 0);
+      if (own >= 0)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) term(own + u, u);
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i)

@@ -292,6 +292,31 @@ def test_delta_rule_by_groups_and_windows_of_chunks(fit, parts, monkeypatch):
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
 
 
+@pytest.mark.parametrize("dk", [64, 44])
+@pytest.mark.parametrize("at", [0, 63, 149, 282])
+def test_delta_rule_by_chunks_rows_in_front_of_one_that_is_not_finite(at, dk):
+    """A row of infinities (its products are NaN) leaves the rows in front of it as they are, to the bit, and the other
+    sequence too."""
+    from grout_b200.kernels import ops
+    H, G, dv, taps, lens = 4, 2, 48, 3, [300, 120]
+    assert ops.delta_chunks_pay(sum(lens), 2, max(lens))
+    Cc, i32 = 2 * G * dk + H * dv, lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    proj = rnd(sum(lens), Cc + H * dv + 2 * H, seed=61)
+    w = [t.to(DEV) for t in (rnd(Cc, taps, seed=62), rnd(H, seed=63), rnd(H, seed=64), rnd(dv, seed=65))]
+
+    def run(x):
+        state = torch.zeros(2, ops.delta_state_floats(H, G, dk, dv, taps), device=DEV)
+        return ops.delta_forward(x.to(DEV), state, *w, H=H, G=G, dk=dk, dv=dv, taps=taps, unit_eps=1e-6, norm_eps=1e-5,
+                                 dtype=torch.float32, token_seq=i32([0] * 300 + [1] * 120), cu_q=i32([0, 300, 420]),
+                                 slots=i32([0, 1]), max_rows=300).cpu()
+
+    want = run(proj)
+    proj[at] = float("inf")
+    got = run(proj)
+    assert torch.equal(got[:at], want[:at]) and torch.equal(got[300:], want[300:])
+    assert not torch.isfinite(got[at:300]).all(1).any()
+
+
 @pytest.mark.parametrize("decay", [0.0, -4.0])
 def test_delta_rule_by_chunks_is_as_exact_as_row_by_row(decay):
     """The relative error against 64 bits of read-outs and states, chunk by chunk and row by row: both are 32-bit sums in
