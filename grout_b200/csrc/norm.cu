@@ -408,9 +408,9 @@ __global__ void add_postnorm_kernel(const PostNormArgs a) {
 
 // The same with the row in registers, V pieces of four values a thread: for widths that are multiples of four up to
 // 16,384 on 16-byte boundaries.  A decode step's row is a chain of latencies (the partial sums, two block-wide sums), so
-// everything that no kernel of the step writes, the weights, is asked for before the wait, and all of the row at once
-// behind it; a prompt's rows are bound by memory, and small blocks keep many of them in flight.  Rows of 2,048,
-// inside a step of one row: 4.3 us exposed (7.9 with the row in shared memory, a value at a time).  One row of eight partial
+// the weights are on their way to L2 before the wait (a kernel in front may have made them, so they are read behind it),
+// and all of the row is asked for at once behind it; a prompt's rows are bound by memory, and small blocks keep many of
+// them in flight.  Rows of 2,048, inside a step of one row: 4.3 us exposed (7.9 with the row in shared memory, a value at a time).  One row of eight partial
 // sums and 1,024 rows of one, back to back, us, with the row in shared memory behind the stroke: 2,048 wide 2.7, 7.9 / 5.3,
 // 13.8; 8,192 4.6, 23 / 14.9, 46; 8,196 6.9, 35 / 15.3, 45; 10,240 7.2, 44 / 17.9, 66; 16,384 9.0, 64 / 27, 144.
 template <typename T> __device__ __forceinline__ float4 pn_load4(const T* p);
@@ -428,7 +428,7 @@ __device__ __forceinline__ void pn_store4(bf16* p, float4 v) {
   *reinterpret_cast<uint2*>(p) = u;
 }
 
-// EARLY: the weights are asked for in front of the wait; the threads of wide rows, of which there are up to 1,024, have no
+// EARLY: the weights are asked for with the row; the threads of wide rows, of which there are up to 1,024, have no
 // registers to hold them (64, and 64 bytes of spills in bfloat16), and read them where they are used.
 template <typename T, int V, int THREADS, bool EARLY>
 __global__ void __launch_bounds__(THREADS) add_postnorm_vec_kernel(const PostNormArgs a) {
@@ -439,6 +439,16 @@ __global__ void __launch_bounds__(THREADS) add_postnorm_vec_kernel(const PostNor
   float4 wp[V], ws[V], wy[V];      // what multiplies the delta, the same again, and the row
   const auto weight = [&](const float* w, int at) { return at < N && w ? *reinterpret_cast<const float4*>(w + at) : one; };
   if constexpr (EARLY) {
+    const auto fetch = [&](const float* w, int at) { if (at < N && w) prefetch_l2(w + at); };
+    if (tid % 8 == 0)              // (eight threads' pieces are a line)
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        const int at = (tid + i * step) * 4;
+        fetch(a.post_w, at), fetch(a.scale, at), fetch(a.w, at);
+      }
+  }
+  pdl_wait();
+  if constexpr (EARLY) {
 #pragma unroll
     for (int i = 0; i < V; ++i) {
       const int at = (tid + i * step) * 4;
@@ -447,7 +457,6 @@ __global__ void __launch_bounds__(THREADS) add_postnorm_vec_kernel(const PostNor
       wy[i] = weight(a.w, at);
     }
   }
-  pdl_wait();
   const size_t s = a.rows ? (size_t)a.rows[r] : (size_t)r;
   float4 v[V], d[V];
   float ss = 0.f;

@@ -79,6 +79,43 @@ def test_stream_sum_at_the_widths_where_its_kernel_changes(N, S, dtype):
     close(y, plain.rms_norm(want, w, 1e-6), dtype, "its norm")
 
 
+def _just_computed(vectors, call):
+    """``call()`` eight times, each right behind the kernels that write ``vectors`` and let their successor in on entry:
+    waited for one by one, then in one graph, with the same bits."""
+    from grout_b200.kernels import ops
+    first = [v.clone() for v in vectors]
+
+    def play(wait):
+        out = []
+        for i in range(8):
+            for v in vectors:
+                ops.scale_softcap_(v, 0.5 + 0.25 * i, None)
+            if wait:
+                torch.cuda.synchronize()
+            out += call()
+        return out
+
+    want, graph = play(True), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        got = play(False)
+    for v, f in zip(vectors, first):
+        v.copy_(f)
+    graph.replay()
+    assert len(got) == len(want) and all(torch.equal(x, y) for x, y in zip(got, want))
+
+
+@pytest.mark.parametrize("N", [1001, 2048, 8192, 10240])
+def test_stream_sum_with_vectors_that_were_just_computed(N):
+    from grout_b200.kernels import ops
+    res, d = rnd(3, N, seed=1).to(DEV), rnd(3, N, seed=2).to(DEV)
+    vectors = [(1 + rnd(N, seed=3 + i, scale=0.2)).to(DEV) for i in range(3)]
+    rows = torch.arange(3, dtype=torch.int32, device=DEV)
+    for on in ([vectors[0]], [vectors[1]], [vectors[2]], vectors):
+        _just_computed(on, lambda: ops.add_postnorm(res, d, dtype=torch.float32, rows=rows, post_weight=vectors[0],
+                                                    post_eps=1e-5, scale=vectors[1], weight=vectors[2], eps=1e-6))
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_embedding_with_positions(dtype):
     from grout_b200.kernels import ops
