@@ -163,15 +163,16 @@ __global__ void __launch_bounds__(256) delta_prepare_rows_kernel(const DeltaArgs
   const bool qk = unit < G, is_q = tid < dk;
   const int c = !qk ? 2 * G * dk + (unit - G) * 256 + tid : is_q ? unit * dk + tid : (G + unit) * dk + (tid - dk);
   const bool mine = qk ? tid < 2 * dk : c < Cc;
-  float w[DP_TAPS];                    // [j] meets the input j rows back
-#pragma unroll
-  for (int j = 0; j < DP_TAPS; ++j) w[j] = mine && j < taps ? a.conv_w[(size_t)c * taps + taps - 1 - j] : 0.f;
+  if (mine) prefetch_l2(a.conv_w + (size_t)c * taps);
   int seq, run;
   run_of_block(a.cu_q, a.n_seqs, DP_RUN, false, blockIdx.x, seq, run);
   const int first = a.cu_q[seq], n = min(DP_RUN, a.cu_q[seq + 1] - first - run * DP_RUN), row0 = first + run * DP_RUN;
   if (n <= 0) return;
   const int slot = a.slots[seq];
   pdl_wait();
+  float w[DP_TAPS];                    // [j] meets the input j rows back
+#pragma unroll
+  for (int j = 0; j < DP_TAPS; ++j) w[j] = mine && j < taps ? a.conv_w[(size_t)c * taps + taps - 1 - j] : 0.f;
   float x[DP_RUN + DP_TAPS - 1];       // the DP_TAPS - 1 inputs in front of the run, then the run's
 #pragma unroll
   for (int i = 0; i < DP_TAPS - 1; ++i) {
@@ -586,6 +587,12 @@ __global__ void __launch_bounds__(256, 2) delta_step_kernel(const DeltaArgs a) {
         if (is_v) prefetch_l2(st + (size_t)(taps - 1 - j) * Cc + cv);
       }
   }
+  // (the weights as well: a kernel in front may have made them)
+  if (is_qk) prefetch_l2(a.conv_w + (size_t)cq * taps);
+  if (is_v) prefetch_l2(a.conv_w + (size_t)cv * taps);
+  if (is_v && lane == 0) prefetch_l2(a.norm_w + tid);
+  if (tid == 0) prefetch_l2(a.a_log + h), prefetch_l2(a.dt_bias + h);
+  pdl_wait();
   float w_q[DS_TAPS], w_v[DS_TAPS];              // [j]: of the input j rows back
 #pragma unroll
   for (int j = 0; j < DS_TAPS; ++j) {
@@ -593,7 +600,6 @@ __global__ void __launch_bounds__(256, 2) delta_step_kernel(const DeltaArgs a) {
     w_v[j] = j < taps && is_v ? a.conv_w[(size_t)cv * taps + taps - 1 - j] : 0.f;
   }
   const float rate = expf(a.a_log[h]), dt = a.dt_bias[h], nw = is_v ? a.norm_w[tid] : 0.f;
-  pdl_wait();
   float kept_q[DS_TAPS], kept_v[DS_TAPS];
 #pragma unroll
   for (int j = 1; j < DS_TAPS; ++j) {

@@ -422,6 +422,30 @@ def test_delta_decode_steps_queued_behind_one_another(n_seqs, m):
     assert all(torch.equal(a, b) for a, b in zip(got, want)) and torch.equal(state, last)
 
 
+@pytest.mark.parametrize("rows", [1, 3, 300])
+def test_delta_rule_with_weights_that_were_just_computed(rows):
+    from grout_b200.kernels import ops
+    m = dict(heads=16, kv_heads=8, dim=64, vdim=64, conv=4)
+    H, G, dk, dv, taps = m["heads"], m["kv_heads"], m["dim"], m["vdim"], m["conv"]
+    w = _delta_weights(H, G, dk, dv, taps, 24, seed=24)
+    g = lambda t: t.float().to(DEV).contiguous()  # noqa: E731
+    wp = torch.cat([w[k] for k in ("q", "k", "v", "g", "b", "a")], 0).double()
+    proj = g(rnd(rows, 24, seed=29).double() @ wp.T)
+    args = (g(torch.cat([w["q.conv"], w["k.conv"], w["v.conv"]], 0)), g(w["A_log"]), g(w["dt_bias"]), g(w["norm"]))
+    i32 = lambda *x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    kw = dict(H=H, G=G, dk=dk, dv=dv, taps=taps, unit_eps=1e-6, norm_eps=1e-5, dtype=torch.float32, max_rows=rows,
+              token_seq=torch.zeros(rows, dtype=torch.int32, device=DEV), cu_q=i32(0, rows), slots=i32(0))
+    # a state for each call, made beforehand, so that nothing stands between the weights' kernel and the rule's
+    states = [torch.zeros(1, ops.delta_state_floats(H, G, dk, dv, taps), device=DEV) for _ in range(32)]
+
+    def call():
+        s = states.pop()
+        return [ops.delta_forward(proj, s, *args, **kw), s]
+
+    for on in ([args[0]], [args[3]]):
+        _just_computed(on, call)
+
+
 def test_delta_rule_batches_slots_used_again_and_padding():
     from grout_b200.kernels import ops
     m = DELTA_SHAPES[0]
