@@ -977,8 +977,9 @@ sample_cluster_kernel(const float* __restrict__ logits, int V, int per_block, co
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
-    if (__any_sync(0xffffffffu, any)) at = c;
-    reached = at == c && seen + p >= threshold;
+    any = __any_sync(0xffffffffu, any);
+    if (any) at = c;
+    reached = any && seen + p >= threshold;     // (a draw of zero is reached by the first member, not in front of it)
     if (!reached) seen += p;
   }
   for (int k = 0; k < SC_STRIDE; ++k) {

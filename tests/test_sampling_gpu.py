@@ -1,4 +1,5 @@
 """Argmax and sampling kernels against the plain sampler, fed the same draws."""
+import itertools
 import random
 
 import pytest
@@ -99,20 +100,14 @@ def _rows_for_thresholds(V, g):
     return rows
 
 
-# around the cluster kernel's shares of a row (eight blocks of sixteen warps), a whole
-# vocabulary, and the first length that takes the one-block kernel
-@pytest.mark.parametrize("V", [1, 7, 8, 9, 127, 129, 4095, 33000, 400001])
-def test_sample_thresholds_of_every_kind(V):
-    rng = random.Random(V)
+def _check_thresholds(V, asked, draw):
+    """Every row of _rows_for_thresholds with everything asked, against the plain sampler."""
     g = torch.Generator().manual_seed(V)
-    asked = [(1.0, 0, 1.0), (0.7, 20, 0.9), (0.8, 0, 0.95), (1.0, 1500, 1.0), (1.0, V - 1, 0.5), (50.0, 3, 0.7)]
-    if V > 40000:
-        asked = asked[1:3]
     rows, prm = [], []
     for name, row in _rows_for_thresholds(V, g).items():
         for t, k, p in asked:
             rows.append(row)
-            prm.append((t, max(k, 0), p, rng.random()))
+            prm.append((t, max(k, 0), p, draw()))
     logits = torch.stack(rows).to(DEV)
     t, k, p, u = zip(*prm)
     args = [torch.tensor(x, dtype=d) for x, d in ((t, torch.float32), (k, torch.int32), (p, torch.float32), (u, torch.float32))]
@@ -127,6 +122,22 @@ def test_sample_thresholds_of_every_kind(V):
         near = {plain_sampling.sample_next(scaled, 1.0, *prm[i][1:3], min(max(u + d, 0.0), 1.0 - 2.0 ** -24))
                 for d in (-2.0 ** -21, 0.0, 2.0 ** -21)}
         assert got[i] in near, (i, prm[i], got[i], near)
+
+
+# around the cluster kernel's shares of a row (eight blocks of sixteen warps), and the first
+# length that takes the one-block kernel
+@pytest.mark.parametrize("V", [1, 7, 8, 9, 127, 129, 4095, 33000, 400001])
+def test_sample_thresholds_of_every_kind(V):
+    asked = [(1.0, 0, 1.0), (0.7, 20, 0.9), (0.8, 0, 0.95), (1.0, 1500, 1.0), (1.0, V - 1, 0.5), (50.0, 3, 0.7)]
+    _check_thresholds(V, asked[1:3] if V > 40000 else asked, random.Random(V).random)
+
+
+# a block's share takes more than one turn of its loads: a vocabulary, one whose rows do not start
+# on 16 bytes, and the longest row of the cluster kernel (all of a block's shared memory)
+@pytest.mark.parametrize("V", [151936, 151939, 400000])
+def test_sample_whole_vocabularies(V):
+    draws = itertools.cycle([random.Random(V).random(), 0.0, 1.0 - 2.0 ** -24])
+    _check_thresholds(V, [(0.7, 20, 0.9), (1.0, 1500, 1.0)], lambda: next(draws))
 
 
 def test_sample_with_nan_and_without_a_finite_maximum():
