@@ -840,13 +840,14 @@ def test_attn_prefill_tc_heads_of_a_block(nq, nkv, D, window, rows_per_block):
 
 
 @pytest.mark.parametrize("nq,nkv", [(32, 8), (16, 8), (16, 1), (3, 3), (10, 2)])
-def test_attn_prefill_tc_takes_the_same_rows_however_they_are_blocked(nq, nkv):
+@pytest.mark.parametrize("D", [64, 128])
+def test_attn_prefill_tc_takes_the_same_rows_however_they_are_blocked(nq, nkv, D):
     """The plan's blocks (whatever it chooses for few and for many rows) against one head a block: the same keys in the
     same order, so the same bits."""
     ops = _ops()
     for lens in ([5], [200, 1, 64], [70] * 30):
-        pc = Paged(lens, nkv, 64, torch.bfloat16, 50, fill=300.0)
-        q = _rand((sum(lens), nq, 64), torch.bfloat16, 51).to(DEV)
+        pc = Paged(lens, nkv, D, torch.bfloat16, 50, fill=300.0)
+        q = _rand((sum(lens), nq, D), torch.bfloat16, 51).to(DEV)
         i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
         run = lambda **kw: ops.attn_prefill_tc(  # noqa: E731
             q, pc.k_pages.to(DEV), pc.v_pages.to(DEV), pc.table.to(DEV), cu_q=i32([0] + torch.tensor(lens).cumsum(0).tolist()),

@@ -140,6 +140,19 @@ def test_sample_whole_vocabularies(V):
     _check_thresholds(V, [(0.7, 20, 0.9), (1.0, 1500, 1.0)], lambda: next(draws))
 
 
+@pytest.mark.parametrize("n", [63, 64, 65, 130])
+def test_sample_host_rows_beyond_one_launch(n):
+    """What a launch carries is for 64 rows: more go in several launches, each row with its own."""
+    rng = random.Random(n)
+    logits = torch.randn(n, 1003, generator=torch.Generator().manual_seed(n)).to(DEV)
+    args = [torch.tensor([rng.choice(c) for _ in range(n)], dtype=d) for c, d in
+            (((0.5, 0.9, 1.3), torch.float32), ((0, 1, 40), torch.int32), ((0.6, 1.0), torch.float32))]
+    args.append(torch.tensor([rng.random() for _ in range(n)]))
+    got = _ops().sample_host(logits, *(a.numpy() for a in args)).cpu().tolist()
+    assert got == _ops().sample(logits, *(a.to(DEV) for a in args)).cpu().tolist()
+    assert got == [_ops().sample(logits[i:i + 1], *(a[i:i + 1].to(DEV) for a in args)).item() for i in range(n)]
+
+
 def test_sample_with_nan_and_without_a_finite_maximum():
     nan, inf = float("nan"), float("inf")
     rows = torch.randn(5, 300, generator=torch.Generator().manual_seed(8))
