@@ -189,9 +189,12 @@ f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
 // tiles of 16 k in shared memory (two buffers; the next tile waits in registers).  Two neighbouring columns are one
 // packed multiply-add (fma.rn.f32x2: two independent roundings).  A chain's and a chunk's sums are in registers, the
 // chunks' in C.  The k-major rows are stored at column ^ (8 (k / 4)), so that the
-// transposing stores touch all banks once.  Where the tiles are too few for the GPU, a cluster of blocks shares a
-// tile, each with its own chunks, and adds them in turn through distributed shared memory.  (Activations stored twice,
-// so that no register pair has to be made, were slower: 1.60 ms, shared memory then being the bound.)
+// transposing stores touch all banks once.  A cluster of blocks shares a tile, each
+// with its own chunks, and adds them in turn through distributed shared memory, wherever K has more than one chunk and
+// their sums leave room for a second block on the SM: by K alone, not by how many tiles there are.  With the kernel that the
+// rule takes, shared / whole tiles, us: 128 rows x 2,048 of 2,048 55 / 94, 600 rows 168 / 197, 1,200 rows 285 / 313 (of
+// 6,144 782 / 920), x 12,288 1,401 / 1,407; only 2,048 rows x 12,288 would gain (2,338 / 2,258).  (Activations stored
+// twice, so that no register pair has to be made, were slower: 1.60 ms, shared memory then being the bound.)
 #define TILE_K 16
 #define TILE_THREADS 128
 #define TILE_STAGES 3
