@@ -70,15 +70,21 @@ __device__ __forceinline__ unsigned long long now_ns() {
 }
 // Waits for the phase with the given parity; false when the time limit expired
 // or (where a flag is given) another role of the block has already given up.
+// The loop is one copy of the poll (left to itself the compiler unrolls it, a few KB of
+// instructions at each of a kernel's dozen waits, and a role that waits then runs through
+// instructions that are in no cache: one user's request at the 4B sizes, 36 steps, 84.0 ms
+// with the polls written out, 80.5 with one; a prompt of 2,048 tokens 15.9 and 15.5).
 __device__ __forceinline__ bool mbar_wait(void* bar, uint32_t parity, volatile int* abort_flag,
                                           unsigned long long limit_ns = TC_WAIT_LIMIT_NS) {
   if (mbar_try(bar, parity)) return true;
   const unsigned long long t0 = now_ns();
-  for (;;) {
-    for (int i = 0; i < 64; ++i)
-      if (mbar_try(bar, parity)) return true;
-    if (abort_flag && *abort_flag) return mbar_try(bar, parity);
-    if (now_ns() - t0 > limit_ns) return false;
+#pragma unroll 1
+  for (int i = 1;; ++i) {
+    if (mbar_try(bar, parity)) return true;
+    if ((i & 63) == 0) {
+      if (abort_flag && *abort_flag) return mbar_try(bar, parity);
+      if (now_ns() - t0 > limit_ns) return false;
+    }
   }
 }
 // The same for a whole converged warp: every lane polls and the lanes agree on
@@ -89,11 +95,13 @@ __device__ __forceinline__ bool mbar_wait_warp(void* bar, uint32_t parity, volat
                                                unsigned long long limit_ns = TC_WAIT_LIMIT_NS) {
   if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
   const unsigned long long t0 = now_ns();
-  for (;;) {
-    for (int i = 0; i < 64; ++i)
-      if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
-    const bool stop = (abort_flag && *abort_flag) || now_ns() - t0 > limit_ns;
-    if (__any_sync(0xffffffffu, stop)) return __all_sync(0xffffffffu, mbar_try(bar, parity));
+#pragma unroll 1
+  for (int i = 1;; ++i) {
+    if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
+    if ((i & 63) == 0) {
+      const bool stop = (abort_flag && *abort_flag) || now_ns() - t0 > limit_ns;
+      if (__any_sync(0xffffffffu, stop)) return __all_sync(0xffffffffu, mbar_try(bar, parity));
+    }
   }
 }
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
