@@ -14,6 +14,7 @@ from ..parts.base import BuildContext, ParamSpec, Part, build_part
 from ..parts.norm import Averaged, HyperConnected, with_offset
 from ..parts.plan import ModelPlan
 from .batch import StepContext
+from .stack import StackOf, stack_layers
 
 
 def _walk(part: Part):
@@ -33,6 +34,7 @@ class Model:
         self._layout: Optional[CacheLayout] = None
         self.stream_vectors: Dict[str, torch.Tensor] = {}    # 32-bit [rows, hidden] each
         self.averages: Dict[int, torch.Tensor] = {}          # schedule index -> 32-bit weights of its depth average
+        self._stack = StackOf()                              # the layers of a decode step as one kernel
 
     # -- tensors -----------------------------------------------------------
     def _named_parts(self) -> List[Tuple[str, Part]]:
@@ -95,6 +97,8 @@ class Model:
         for top in [self.embedding, *self.blocks, self.final_norm, self.head]:
             for p in _walk(top):
                 mods.extend(p.kernel_modules())
+        if stack_layers(self) is not None:
+            mods.append("decode_stack")
         return tuple(dict.fromkeys(mods))
 
     def captures_prompts(self) -> bool:
@@ -131,7 +135,11 @@ class Model:
         res = None
         if self.embedding.starts_stream:      # the embedding is the 32-bit stream already
             res, pending = pending, None
-        for i, e in enumerate(self.plan.schedule):
+        stack = self._stack.get(self, cache) if step.decode else None
+        entries = self.plan.schedule
+        if stack is not None and stack.takes(step):
+            res, pending, entries = stack.forward(res, pending, step), None, ()
+        for i, e in enumerate(entries):
             owner = i if e.cache_of is None else e.cache_of
             view = cache.view(owner) if owner in layout.where else None
             if e.add is not None:

@@ -1,0 +1,139 @@
+"""A decode step's layers as one kernel (``csrc/decode_stack.cu``), for models whose layers it knows.
+
+The kernel runs a plain pre-norm decoder layer: RMS norms, grouped-query attention over the whole
+paged cache with 128-wide heads (with or without the heads' norms, the whole head rotated), a
+gated SiLU feed-forward, bfloat16 weights.  ``stack_layers`` says whether a model is that, layer
+by layer and attribute by attribute; anything else (a window, a cap, a bias, a part of the
+caller's own, 32-bit weights, another product kernel asked for) goes layer by layer as before."""
+from __future__ import annotations
+
+import weakref
+from typing import List, Optional
+
+import torch
+
+from ..kernels import ops
+from ..parts.block import PreNormBlock
+from ..parts.feedforward import SwiGLU
+from ..parts.linear import Linear
+from ..parts.mixer import GQAAttention
+from ..parts.norm import RMSNorm
+from ..parts.position import RotaryHalfSplit
+
+HEAD = 128
+
+
+def _plain_linear(lin, out_features: int, in_features: int) -> bool:
+    return (type(lin) is Linear and lin.weight.dtype == torch.bfloat16 and lin.decode_kernel == "tc"
+            and lin.weight.is_contiguous() and tuple(lin.weight.shape) == (out_features, in_features)
+            and lin.weight.data_ptr() % 16 == 0)
+
+
+def _plain_norm(norm, width: int) -> bool:
+    return type(norm) is RMSNorm and norm.weight is not None and tuple(norm.weight.shape) == (width,)
+
+
+def _plain_attention(m) -> bool:
+    rot = m.position.rotary() if type(m) is GQAAttention else None
+    return (type(m) is GQAAttention and m.D == m.Dv == m.Ds == HEAD and type(m.position) is RotaryHalfSplit
+            and rot is not None and rot.rot_dim == HEAD and not rot.interleaved and rot.amplitude == 1.0
+            and m.window is None and not m.chunk and not m.keep_first and m.softcap is None and m.sink is None
+            and not m.head_gate and not m.beside and not m.shares_kv and not m.values_are_keys
+            and not m.conv_path and m.q_temp is None
+            and _plain_linear(m.qkv, (m.nq + 2 * m.nkv) * HEAD, m.hidden) and _plain_linear(m.o, m.hidden, m.nq * HEAD))
+
+
+def _plain_layer(block) -> bool:
+    if type(block) is not PreNormBlock or type(block.feedforward) is not SwiGLU or not _plain_attention(block.mixer):
+        return False
+    m, f = block.mixer, block.feedforward
+    return (f.interleave == 8 and f.hidden == m.hidden and _plain_linear(f.gate_up, 2 * f.intermediate, f.hidden)
+            and _plain_linear(f.down, f.hidden, f.intermediate)
+            and _plain_norm(block.norm1, m.hidden) and _plain_norm(block.norm2, m.hidden))
+
+
+def _sizes(block):
+    m = block.mixer
+    return (m.hidden, block.feedforward.intermediate, m.nq, m.nkv, m.scale, m.qk_norm_eps, block.norm1.eps,
+            block.norm2.eps)
+
+
+def stack_layers(model) -> Optional[List]:
+    """The model's blocks in the order they run when the kernel can run all of them, else None."""
+    plan = model.plan
+    if model.ctx.dtype != torch.bfloat16 or not plan.schedule:
+        return None
+    if any(e.cache_of is not None or e.add is not None or e.average is not None for e in plan.schedule):
+        return None
+    blocks = [model.blocks[e.layer] for e in plan.schedule]
+    if not all(_plain_layer(b) for b in blocks) or len({_sizes(b) for b in blocks}) != 1:
+        return None
+    first = blocks[0]
+    if first.norm1.eps != first.norm2.eps:
+        return None
+    freq = first.mixer.position.rotary().inv_freq
+    if not all(torch.equal(b.mixer.position.rotary().inv_freq, freq) for b in blocks[1:]):
+        return None
+    return blocks
+
+
+class DecodeStack:
+    """The kernel's view of one model and one cache: every layer's tensor maps and vectors on the
+    device, and the scratch of its launches, which are ordered on one stream as the steps of an
+    engine are."""
+
+    def __init__(self, blocks, views, max_rows: int = ops.DECODE_STACK_ROWS):
+        hidden, ff, nq, nkv, scale, qk_eps, eps, _eps = _sizes(blocks[0])
+        device = blocks[0].mixer.qkv.weight.device
+        self.hidden, self.max_rows = hidden, max_rows
+        vector = lambda t: None if t is None else t.float().contiguous()
+        self._layers = []                 # (the tensors that the device's table points at)
+        for b, view in zip(blocks, views):
+            m, f = b.mixer, b.feedforward
+            self._layers.append(dict(
+                qkv=m.qkv.weight, o=m.o.weight, gate_up=f.gate_up.weight, down=f.down.weight, k_pages=view.k_pages,
+                v_pages=view.v_pages, norm1=vector(b.norm1.weight), norm2=vector(b.norm2.weight),
+                q_norm=vector(m.q_norm_w), k_norm=vector(m.k_norm_w)))
+        self.block_table = views[0].block_table
+        self.state = ops.decode_stack_state(self._layers, hidden, ff, nq, nkv, max_rows, device)
+        self.args = dict(eps=eps, qk_eps=qk_eps or 0.0, scale=scale,
+                         inv_freq=blocks[0].mixer.position.rotary().inv_freq.contiguous())
+
+    @classmethod
+    def of(cls, model, cache) -> Optional["DecodeStack"]:
+        """None when the model is not one that the kernel runs, or its sizes have no plan."""
+        blocks = stack_layers(model)
+        if blocks is None:
+            return None
+        views = [cache.view(i) for i in range(len(blocks))]
+        table = views[0].block_table
+        for b, v in zip(blocks, views):
+            if (v.page != 64 or v.k_pages.dtype != torch.bfloat16 or v.block_table.data_ptr() != table.data_ptr()
+                    or tuple(v.k_pages.shape[1:]) != (b.mixer.nkv, 64, HEAD) or v.v_pages.shape != v.k_pages.shape
+                    or v.k_pages.data_ptr() == v.v_pages.data_ptr()):
+                return None
+        hidden, ff, nq, nkv = _sizes(blocks[0])[:4]
+        if not ops.decode_stack_takes(hidden, ff, nq, nkv, table.device):
+            return None
+        return cls(blocks, views)
+
+    def takes(self, step) -> bool:
+        return step.decode and 0 < step.n_tokens <= self.max_rows and step.n_seqs == step.n_tokens
+
+    def forward(self, res, pending, step) -> torch.Tensor:
+        """The 32-bit stream behind the last layer, [T, hidden]."""
+        return ops.decode_stack(self.state, res, pending, slots=step.slots, kv_len=step.kv_len,
+                                block_table=self.block_table, **self.args)
+
+
+class StackOf:
+    """A model's ``DecodeStack``, made for the cache that its steps use (and made anew for another)."""
+
+    def __init__(self):
+        self._cache, self._stack = None, None
+
+    def get(self, model, cache) -> Optional[DecodeStack]:
+        if self._cache is None or self._cache() is not cache:
+            self._stack = DecodeStack.of(model, cache)
+            self._cache = weakref.ref(cache)
+        return self._stack

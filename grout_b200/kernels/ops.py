@@ -1126,7 +1126,10 @@ _TC_ERROR_NAMES = {111: "a role of the tcgen05 attention kernel waited 2 s on a 
                    121: "the pair product's MMA lane waited 2 s for a stage that never arrived",
                    122: "the pair product's producer waited 2 s for a stage that was never released",
                    123: "the pair product's epilogue waited 2 s for an accumulator that was never finished",
-                   124: "the pair product's MMA lane waited 2 s for an accumulator that was never drained"}
+                   124: "the pair product's MMA lane waited 2 s for an accumulator that was never drained",
+                   151: "a warp of the layers' kernel waited 2 s for a stage that never arrived",
+                   152: "the stream of the layers' kernel waited 2 s for a stage that was never released",
+                   153: "a block of the layers' kernel waited 2 s for the others"}
 
 
 def _tc_error_flag(device) -> torch.Tensor:
@@ -1811,6 +1814,111 @@ def diff_heads(x: torch.Tensor, v_dim: int, lam: float, eps: float, mult: float)
     a.lam, a.eps, a.mult = float(lam), float(eps), float(mult)
     _check(_fn("diff_heads", f"gb_diff_heads_{_suffix(x.dtype)}", "pp")(ctypes.addressof(a), _stream()),
            "diff_heads")
+    return out
+
+
+# ---------------------------------------------------------------- a decode step's layers
+class _StackArgs(ctypes.Structure):
+    _fields_ = [("layers", _P), ("n_layers", _I), ("T", _I), ("hidden", _I), ("ff", _I), ("nq", _I), ("nkv", _I),
+                ("slot_bytes", _I), ("n_slots", _I), ("act_at", _I), ("kb_qkv", _I), ("kb_o", _I), ("kb_down", _I),
+                ("eps", _F), ("qk_eps", _F), ("scale_log2", _F), ("x_in", _P), ("res_in", _P), ("x_out", _P),
+                ("inv_freq", _P), ("slots", _P), ("kv_len", _P), ("block_table", _P), ("max_pages", _I),
+                ("xb", _P), ("ab", _P), ("hb", _P), ("ss", _P), ("qkv", _P), ("part_o", _P), ("part_ml", _P),
+                ("sync", _P), ("error", _P), ("stamps", _P)]
+
+
+DECODE_STACK_ROWS = 8          # DS_ROWS
+DECODE_STACK_STAMPS = None     # int64 [blocks, 16]: times of the phases of a layer (tuning)
+
+
+def decode_stack_takes(hidden: int, ff: int, nq: int, nkv: int, device) -> bool:
+    """Whether the kernel has a plan for layers of these sizes on this GPU."""
+    return _fn("decode_stack", "gb_decode_stack_layer_bytes", "iiiii")(hidden, ff, nq, nkv, _sm_count(device)) > 0
+
+
+def decode_stack_state(layers, hidden: int, ff: int, nq: int, nkv: int, max_rows: int, device) -> dict:
+    """What launches over these layers share: their table on the device and scratch for ``max_rows`` rows.
+    ``layers``: dicts of the weights (bf16: qkv, o, gate_up, down), pages and 32-bit norm weights of each.  The tensors
+    must outlive the state; launches that use it must be ordered on one stream."""
+    P = _sm_count(device)
+    size = _fn("decode_stack", "gb_decode_stack_layer_bytes", "iiiii")(hidden, ff, nq, nkv, P)
+    if size <= 0:
+        raise KernelError(f"no plan for layers of {hidden} / {ff} with {nq} / {nkv} heads")
+    host = torch.zeros(size * len(layers) + 64, dtype=torch.uint8)
+    skip = -host.data_ptr() % 64                 # tensor maps lie on 64 bytes
+    encode = _fn("decode_stack", "gb_decode_stack_encode", "piiiiippppppl" + "pppp")
+    for i, t in enumerate(layers):
+        for n, shape in (("qkv", ((nq + 2 * nkv) * 128, hidden)), ("o", (hidden, nq * 128)),
+                         ("gate_up", (2 * ff, hidden)), ("down", (hidden, ff))):
+            _need(t[n], n, torch.bfloat16, 2)
+            if tuple(t[n].shape) != shape:
+                raise KernelError(f"{n} is {tuple(t[n].shape)}, expected {shape}")
+        for n in ("k_pages", "v_pages"):
+            _need(t[n], n, torch.bfloat16, 4)
+            if tuple(t[n].shape[1:]) != (nkv, 64, 128) or t[n].shape != t["k_pages"].shape:
+                raise KernelError(f"{n} are {tuple(t[n].shape)}, expected [*, {nkv}, 64, 128]")
+        for n, width in (("norm1", hidden), ("norm2", hidden), ("q_norm", 128), ("k_norm", 128)):
+            if t[n] is not None or n in ("norm1", "norm2"):
+                _need(t[n], n, torch.float32, 1)
+                if t[n].shape[0] != width:
+                    raise KernelError(f"{n} has {t[n].shape[0]} elements, expected {width}")
+        _check(encode(host.data_ptr() + skip + i * size, hidden, ff, nq, nkv, P, t["qkv"].data_ptr(), t["o"].data_ptr(),
+                      t["gate_up"].data_ptr(), t["down"].data_ptr(), t["k_pages"].data_ptr(), t["v_pages"].data_ptr(),
+                      t["k_pages"].shape[0], _ptr(t["norm1"]), _ptr(t["norm2"]), _ptr(t["q_norm"]), _ptr(t["k_norm"])),
+               "decode_stack_encode", 0)
+    f32 = lambda n: torch.zeros(n, dtype=torch.float32, device=device)
+    b16 = lambda n: torch.zeros(n, dtype=torch.bfloat16, device=device)
+    T, splits = max_rows, 32
+    return dict(sizes=(len(layers), hidden, ff, nq, nkv), rows=T, blocks=P,
+                layers=host[skip:skip + size * len(layers)].to(device),
+                xb=b16(T * hidden), ab=b16(T * nq * 128), hb=b16(T * ff), ss=f32(T * P), qkv=f32(T * (nq + 2 * nkv) * 128),
+                part_o=f32(T * nq * splits * 128), part_ml=f32(T * nq * splits * 2),
+                sync=torch.zeros(2, dtype=torch.int32, device=device))
+
+
+def _cost_decode_stack(out, state, res, pending, *, kv_len, slots, **kw):
+    n, hidden, ff, nq, nkv = state["sizes"]
+    weights = n * 2 * (hidden * (2 * nq + 2 * nkv) * 128 + 3 * hidden * ff)
+    T = out.shape[0]
+    keys = torch.where(slots >= 0, kv_len, torch.zeros_like(kv_len)).double().sum()
+    return (lambda: weights + float(keys.item()) * n * nkv * 512), \
+        (lambda: float(T) * weights + float(keys.item()) * n * nq * 512)
+
+
+@_profiled("decode_stack", _cost_decode_stack)
+def decode_stack(state: dict, res: Optional[torch.Tensor], pending: Optional[torch.Tensor], *, slots, kv_len, block_table,
+                 inv_freq: Optional[torch.Tensor], eps: float, qk_eps: float, scale: float) -> torch.Tensor:
+    """Every layer of ``state`` over T rows, one new token of a sequence each: the stream in front of them (``pending``
+    [T, hidden] bf16, or ``res`` in 32-bit) -> the 32-bit stream behind them.  Keys and values of the rows whose slot is not
+    negative are stored."""
+    n, hidden, ff, nq, nkv = state["sizes"]
+    if (res is None) == (pending is None):
+        raise KernelError("decode_stack takes the stream either in 32-bit or as bfloat16 rows")
+    src = res if res is not None else pending
+    _need(src, "stream", torch.float32 if res is not None else torch.bfloat16, 2)
+    T = src.shape[0]
+    if src.shape[1] != hidden or not 0 < T <= state["rows"]:
+        raise KernelError(f"the stream is {tuple(src.shape)}, expected [1 .. {state['rows']}, {hidden}]")
+    for t, nm, nd in ((slots, "slots", 1), (kv_len, "kv_len", 1), (block_table, "block table", 2)):
+        _need(t, nm, torch.int32, nd)
+    if slots.shape[0] != T or kv_len.shape[0] != T:
+        raise KernelError("one slot and one length per row are needed")
+    if inv_freq is not None:
+        _need(inv_freq, "inv_freq", torch.float32, 1)
+        if inv_freq.shape[0] != 64:
+            raise KernelError("the kernel rotates whole heads of 128")
+    out = torch.empty((T, hidden), dtype=torch.float32, device=src.device)
+    a = _StackArgs()
+    a.layers, a.n_layers, a.T, a.hidden, a.ff, a.nq, a.nkv = state["layers"].data_ptr(), n, T, hidden, ff, nq, nkv
+    a.eps, a.qk_eps, a.scale_log2 = float(eps), float(qk_eps), float(scale) * _LOG2E
+    a.x_in, a.res_in, a.x_out, a.inv_freq = _ptr(pending), _ptr(res), out.data_ptr(), _ptr(inv_freq)
+    a.slots, a.kv_len, a.block_table, a.max_pages = slots.data_ptr(), kv_len.data_ptr(), block_table.data_ptr(), block_table.shape[1]
+    for name in ("xb", "ab", "hb", "ss", "qkv", "part_o", "part_ml", "sync"):
+        setattr(a, name, state[name].data_ptr())
+    a.error, a.stamps = _tc_error_flag(src.device).data_ptr(), _ptr(DECODE_STACK_STAMPS)
+    with torch.cuda.device(src.device):
+        _check(_fn("decode_stack", "gb_decode_stack", "pip")(
+            ctypes.addressof(a), state["blocks"], _stream()), "decode_stack")
     return out
 
 

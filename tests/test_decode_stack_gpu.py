@@ -1,0 +1,102 @@
+"""Decode steps whose layers run as one kernel, against the plain implementation and the kernels of each layer."""
+import pytest
+import torch
+
+from helpers import assert_close
+from plain import qwen3 as plain
+
+pytestmark = pytest.mark.gpu
+
+
+def config(hidden, ff, nq, nkv, layers=2):
+    return dict(architectures=["Qwen3ForCausalLM"], model_type="qwen3", vocab_size=512, hidden_size=hidden,
+                intermediate_size=ff, num_hidden_layers=layers, num_attention_heads=nq, num_key_value_heads=nkv,
+                head_dim=128, rope_theta=1000000.0, rms_norm_eps=1e-6, max_position_embeddings=2048,
+                tie_word_embeddings=False, use_sliding_window=False, eos_token_id=511)
+
+
+# groups of 1, 2, 4, 8 query heads; odd and even shares of every product; gate|up of one and of several tiles of rows
+MODELS = {"group2": config(256, 1216, 4, 2), "group1": config(320, 2432, 2, 2, 3), "group8": config(576, 1472, 8, 1),
+          "group4": config(2560, 9728, 32, 8)}
+
+
+@pytest.fixture(scope="module")
+def engines(tmp_path_factory):
+    from grout_b200.engine import Engine
+    from grout_b200.weights import write_random_model
+    made = {}
+
+    def get(name):
+        if name not in made:
+            d = str(tmp_path_factory.mktemp(name))
+            write_random_model(MODELS[name], 3, d)
+            made[name] = (d, Engine.load(d, dtype="bfloat16", max_tokens=8192, max_batch=9, max_seq_len=2048))
+        return made[name]
+    return get
+
+
+def played(eng, lens, steps, seed):
+    """Prompts of ``lens`` tokens, then ``steps`` decode steps: the tokens, and the decode steps' logits per sequence."""
+    g = torch.Generator().manual_seed(seed)
+    toks = [torch.randint(0, 511, (n + steps,), generator=g).tolist() for n in lens]
+    slots = [eng.open_sequence() for _ in lens]
+    for s, t, n in zip(slots, toks, lens):
+        eng.step([(s, t[:n])], [[]])
+    out = [eng.step([(s, [t[n + i]]) for s, t, n in zip(slots, toks, lens)], [[0]] * len(slots)) for i in range(steps)]
+    eng.check()
+    for s in slots:
+        eng.close_sequence(s)
+    return toks, torch.stack(out, dim=1)
+
+
+@pytest.mark.parametrize("lens", [[1], [63], [64, 5], [127, 128, 700], [1, 62, 190, 191, 192, 333, 1500, 64]], ids=str)
+@pytest.mark.parametrize("name", ["group1", "group2", "group8"])
+def test_logits_against_the_plain_implementation(engines, name, lens):
+    from safetensors import safe_open
+    d, eng = engines(name)
+    assert eng.model._stack.get(eng.model, eng.cache) is not None
+    with safe_open(f"{d}/model.safetensors", "pt") as f:
+        w = {k: f.get_tensor(k) for k in f.keys()}
+    toks, got = played(eng, lens, 3, 11)
+    for i, n in enumerate(lens):
+        rows = list(range(n, n + 3))
+        assert_close(got[i], plain.logits(w, MODELS[name], toks[i], rows=rows), "bfloat16", f"{name} {lens} sequence {i}")
+
+
+@pytest.mark.parametrize("lens", [[40], [2000], [100, 900, 3], [300] * 8], ids=str)
+def test_as_close_as_layer_by_layer(engines, monkeypatch, lens):
+    """The kernel and the kernels of each layer round the same activations to 16 bits and differ in the order of their
+    32-bit sums, so their logits differ as two runs of 16-bit activations do: by no more than either's own error, which
+    at these sizes is about 1 % of the logits."""
+    from grout_b200.engine import stack
+    _d, eng = engines("group4")
+    _t, got = played(eng, lens, 3, 5)
+    monkeypatch.setattr(stack.DecodeStack, "takes", lambda self, step: False)
+    eng.graphs.decode_graphs.clear()
+    _t, ref = played(eng, lens, 3, 5)
+    eng.graphs.decode_graphs.clear()
+    err = float((got.double() - ref.double()).norm() / ref.double().norm())
+    assert err < 0.02, err
+
+
+def test_same_bits_every_time(engines):
+    _d, eng = engines("group2")
+    _t, a = played(eng, [70, 200, 900], 3, 21)
+    _t, b = played(eng, [70, 200, 900], 3, 21)
+    assert torch.equal(a, b)
+
+
+def test_more_rows_than_the_kernel_takes_go_layer_by_layer(engines):
+    from grout_b200.engine.batch import make_context
+    _d, eng = engines("group2")
+    st = eng.model._stack.get(eng.model, eng.cache)
+    for n, takes in ((1, True), (8, True), (9, False)):
+        assert st.takes(make_context([(0, 0, [1])] * n, None, "cuda")) is takes
+    assert not st.takes(make_context([(0, 0, [1, 2])], None, "cuda"))
+
+
+@pytest.mark.parametrize("change", [dict(head_dim=64), dict(use_sliding_window=True, sliding_window=128, max_window_layers=0)])
+def test_other_layers_go_layer_by_layer(change):
+    from grout_b200.engine import Engine
+    eng = Engine.random(dict(config(256, 1216, 4, 2), **change), 0, max_tokens=512, max_batch=2, max_seq_len=256)
+    assert eng.model._stack.get(eng.model, eng.cache) is None
