@@ -28,8 +28,8 @@
 // Products: mma.sync m16n8k16 with 16 weight rows as A (ldmatrix from the ring's 128-byte
 // swizzled tiles) and up to eight activation rows as B.  tcgen05 has no tile this narrow in use:
 // an SM gets 23 bytes of weights a clock, one such instruction every 22 clocks.  The activations
-// lie in global memory in the order of B's fragments (stack_fragment); warps of their own bring
-// them into the ring's slots beside the weights as soon as the barrier in front of them is passed.
+// lie in global memory in the order of B's fragments (stack_fragment); a lane of its own has
+// them copied into the ring's slots beside the weights as soon as the barrier in front of them is passed.
 // The warps divide a stage's columns or rows, and their sums meet in shared memory in a fixed
 // order.  Sums are 32-bit throughout.
 //
@@ -43,8 +43,8 @@
 #define DS_FOURS 3                          // fours of consumer warps, which take turns at the ring's stages
 #define DS_WARPS (4 * DS_FOURS)             // consumer warps; warp DS_WARPS feeds the ring (128 registers a thread)
 #define DS_CONSUMERS (DS_WARPS * 32)
-#define DS_FEEDERS 3                        // the warps behind it bring the activations, taking turns at the stages
-#define DS_THREADS (DS_CONSUMERS + 32 + 32 * DS_FEEDERS)
+#define DS_THREADS (DS_CONSUMERS + 64)      // warp DS_WARPS + 1 brings the activations
+#define DS_BLOCKS_MOST 160
 #define DS_ROWS 8                           // most activation rows
 #define DS_FEW 4                            // up to so many, o and down have longer stages
 #define DS_TILES 3                          // most 16-row tiles a warp holds sums of
@@ -168,8 +168,20 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, i
 __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(addr)
-               : "memory");
+               : "r"(addr));
+}
+__device__ __forceinline__ void lds4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
+}
+// Writes to global memory that other blocks' bulk copies will read.
+__device__ __forceinline__ void ds_fence_async() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, int bytes, void* bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
+      "r"(bytes), "r"(smem_u32(bar))
+      : "memory");
 }
 __device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -212,6 +224,7 @@ struct StackShared {
   uint64_t full[DS_SLOTS_MOST], empty[DS_SLOTS_MOST];
   float2 turn[DS_UNITS_MOST][64];        // cosine and sine of a unit's new position
   float rstd[DS_ROWS];
+  float ss[DS_ROWS * DS_BLOCKS_MOST];    // the blocks' sums of squares, on their way while a product runs
   float red_m[DS_WARPS * 8], red_l[DS_WARPS * 8];
   StackUnit units[DS_UNITS_MOST];
   int n_units, split_any;
@@ -289,7 +302,6 @@ struct StackConsumer {
     }
     arrived += P;
     if (tid == 0) {
-      __threadfence();
       ds_add_release(a.sync, 1);
       const unsigned long long t0 = now_ns();
 #pragma unroll 1
@@ -316,11 +328,21 @@ struct StackConsumer {
     }
   }
 
-  // 1 / rms of the rows, from the blocks' sums of squares: a warp a row.
+  // 1 / rms of the rows, from the blocks' sums of squares: a warp a row, asked for in front of the product and summed up
+  // behind it (waiting for them in front cost the first four a trip to L2 before its first stage).
+  __device__ __forceinline__ void ask_factors() {
+    if (warp < a.T)
+      for (int i = lane; i < P; i += 32)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(sh.ss + warp * DS_BLOCKS_MOST + i)),
+                     "l"(a.ss + warp * P + i)
+                     : "memory");
+  }
   __device__ __forceinline__ void row_factors() {
     if (warp < a.T) {
+      cp_async_commit();
+      cp_async_wait<0>();
       float s = 0.f;
-      for (int i = lane; i < P; i += 32) s += a.ss[warp * P + i];
+      for (int i = lane; i < P; i += 32) s += sh.ss[warp * DS_BLOCKS_MOST + i];      // (what this lane asked for)
       s = warp_sum(s);
       if (lane == 0) sh.rstd[warp] = rsqrtf(s / (float)a.hidden + a.eps);
     }
@@ -330,22 +352,26 @@ struct StackConsumer {
   // in `red` as [part][activation row][pitch], summed up by whoever reads them over the `parts` it returns.
   //
   // Four warps take a stage, the fours taking turns, so that a four has the time of several stages for its waits and
-  // instructions; among them they divide the stage's steps of 32 columns or, from three tiles of 16 rows on, the tiles.
+  // instructions; among them they divide the stage's steps of 32 columns, or its 16-row tiles where there are more than
+  // three, or both two by two where twelve partial sums of three tiles have no room.  A warp asks for the operands of
+  // two steps before it multiplies: one step after the other a stage of six steps took it 0.85 us.
   __device__ __forceinline__ int product(int K, int rows, int kb, int& pitch) {
     const int steps = 2 * kb, K32 = K >> 5, tiles = (rows + 15) >> 4;
     const int stages = (K / 64 + kb - 1) / kb;
-    const bool by_tiles = tiles >= 3;
-    const int j = warp & 3, quad = warp >> 2;
-    const int s_off = by_tiles ? 0 : j, s_inc = by_tiles ? 1 : 4, t_off = by_tiles ? j : 0, t_inc = by_tiles ? 4 : 1;
-    const int part = by_tiles ? quad : warp, parts = by_tiles ? DS_FOURS : DS_WARPS;
     pitch = ((rows + 11) & ~15) + 4;
+    const int j = warp & 3, quad = warp >> 2;
+    // log2 of the ways in which the tiles are divided; the steps are divided in 4 >> ways
+    const int ways = tiles > 3 ? 2 : (DS_WARPS * a.T * pitch * 4 > DS_RED_BYTES ? 1 : 0);
+    const int t_off = j & ((1 << ways) - 1), s_off = j >> ways, s_inc = 4 >> ways;
+    const int part = quad * s_inc + s_off, parts = DS_FOURS * s_inc;
+    const int n_tiles = (tiles - t_off + (1 << ways) - 1) >> ways;
     const int g = lane >> 2, c = lane & 3;
     float acc[DS_TILES][4];
 #pragma unroll
     for (int i = 0; i < DS_TILES; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
     // (columns beyond the rows get some other row's values: nobody reads what becomes of them)
     const uint32_t act = a.act_at + min(g, a.T - 1) * 64 + c * 16, act_pitch = a.T * 64;
-    const uint32_t ring32 = smem_u32(ring);
+    const uint32_t ring32 = smem_u32(ring), tile_pitch = 2048u << ways;
     const uint32_t half = lane >> 4, lane_row = (lane & 15) + t_off * 16;
     int s = quad;
     StackRing r = at;
@@ -355,23 +381,37 @@ struct StackConsumer {
       wait_full(r);
       const uint32_t base = ring32 + (uint32_t)r.slot * a.slot_bytes;
       const int end = min(steps, K32 - s * steps);
-#pragma unroll 2
-      for (int step = s_off; step < end; step += s_inc) {
-        const uint32_t row0 = (step >> 1) * rows + lane_row, ch = (step & 1) * 4 + half;
-        uint32_t f[4];
-        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                     : "=r"(f[0]), "=r"(f[1]), "=r"(f[2]), "=r"(f[3])
-                     : "r"(base + act + step * act_pitch)
-                     : "memory");
 #pragma unroll
-        for (int t = 0; t < DS_TILES; ++t) {
-          if (t_off + t * t_inc < tiles) {
-            const uint32_t row = row0 + t * t_inc * 16;
-            uint32_t w[4], v[4];
-            ldsm4(w, base + row * 128 + ((ch ^ (row & 7)) << 4));
-            ldsm4(v, base + row * 128 + (((ch + 2) ^ (row & 7)) << 4));
-            mma_16816(acc[t], w, f[0], f[1]);
-            mma_16816(acc[t], v, f[2], f[3]);
+      for (int i = 0; i < 4; i += 2) {
+        const int step0 = s_off + i * s_inc;
+        if (step0 < end) {
+          const bool two = step0 + s_inc < end;
+          const int step1 = two ? step0 + s_inc : step0;
+          const uint32_t row0 = (step0 >> 1) * rows + lane_row, row1 = (step1 >> 1) * rows + lane_row;
+          // (a step is four 16-byte chunks of a 64-column block; the second pair of them is two chunks on)
+          const uint32_t w0 = base + row0 * 128 + ((((step0 & 1) * 4 + half) ^ (row0 & 7)) << 4);
+          const uint32_t w1 = base + row1 * 128 + ((((step1 & 1) * 4 + half) ^ (row1 & 7)) << 4);
+          uint32_t f0[4], f1[4], w[2][4][4];       // (a tile's operands while the one before it is multiplied)
+          lds4(f0, base + act + step0 * act_pitch);
+          lds4(f1, base + act + step1 * act_pitch);
+          auto tile = [&](int t, uint32_t (&v)[4][4]) {
+            ldsm4(v[0], w0 + t * tile_pitch);
+            ldsm4(v[1], (w0 ^ 32u) + t * tile_pitch);
+            ldsm4(v[2], w1 + t * tile_pitch);
+            ldsm4(v[3], (w1 ^ 32u) + t * tile_pitch);
+          };
+          if (n_tiles > 0) tile(0, w[0]);
+#pragma unroll
+          for (int t = 0; t < DS_TILES; ++t) {
+            if (t < n_tiles) {
+              if (t + 1 < DS_TILES && t + 1 < n_tiles) tile(t + 1, w[(t + 1) & 1]);
+              mma_16816(acc[t], w[t & 1][0], f0[0], f0[1]);
+              mma_16816(acc[t], w[t & 1][1], f0[2], f0[3]);
+              if (two) {
+                mma_16816(acc[t], w[t & 1][2], f1[0], f1[1]);
+                mma_16816(acc[t], w[t & 1][3], f1[2], f1[3]);
+              }
+            }
           }
         }
       }
@@ -382,8 +422,8 @@ struct StackConsumer {
     float* out = red + part * a.T * pitch;
 #pragma unroll
     for (int t = 0; t < DS_TILES; ++t) {
-      const int row = (t_off + t * t_inc) * 16 + g;
-      if (t_off + t * t_inc < tiles) {
+      const int row = (t_off + (t << ways)) * 16 + g;
+      if (t < n_tiles) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const int rr = row + (e >> 1) * 8, col = 2 * c + (e & 1);
@@ -637,6 +677,7 @@ struct StackConsumer {
       }
       if (ui + 1 < sh.n_units) ds_sync();                  // red is the next unit's queries
     }
+    ds_fence_async();
   }
 
   // The splits of the block's (sequence, head) rows, a warp a row.
@@ -676,6 +717,7 @@ struct StackConsumer {
       *reinterpret_cast<uint32_t*>(a.ab + stack_fragment(k, seq, a.T)) = pack2(O.x * inv, O.y * inv);
       *reinterpret_cast<uint32_t*>(a.ab + stack_fragment(k + 2, seq, a.T)) = pack2(O.z * inv, O.w * inv);
     }
+    ds_fence_async();
   }
 };
 
@@ -695,7 +737,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
 
   if (tid == 0) {
     for (int i = 0; i < a.n_slots; ++i) {
-      mbar_init(&sh.full[i], 33);        // the weights' lane and a warp of the activations'
+      mbar_init(&sh.full[i], 1);
       mbar_init(&sh.empty[i], 4);
     }
     sh.abort = 0;
@@ -754,7 +796,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
   if (warp == DS_WARPS) {
     // ------------------------------------------------------------------ the stream
     // One lane, and few instructions a stage: with a page broadcast, a vote and divisions in the loop a stage took
-    // 0.45 us to ask for, whatever its size.
+    // 0.45 us to ask for, whatever its size.  A stage's barrier expects its activations too, which come later.
     if (lane == 0) {
       StackRing at = {0, 0};
       bool ok = true;
@@ -814,10 +856,11 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
           } else if (phase == GATE_UP) {
             const int k_end = a.hidden, row0 = share.first * 16;
             const bool half = share.half >= 0;
+            const int act = 128 * a.T;
             const int half_row = (share.half & 1) * 4, half_group = share.half >> 1, whole_bytes = share.whole * 2048;
 #pragma unroll 1
             for (int k = 0; k < k_end; k += 64) {
-              uint8_t* dst = next_stage(gu_rows * 128);
+              uint8_t* dst = next_stage(gu_rows * 128 + act);
               if (!ok) break;
               tma_load_2d(dst, &L->gate_up[big_g], k, row0, &sh.full[at.slot]);
               if (half) tma_load_4d(dst + whole_bytes, &L->half, k, half_row, 0, half_group, &sh.full[at.slot]);
@@ -827,10 +870,10 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
             const CUtensorMap* map = phase == QKV ? &L->qkv[big_q] : (phase == O ? &L->o[more][big_c] : &L->down[more][big_c]);
             const int blocks = (phase == QKV ? a.hidden : (phase == O ? a.nq * 128 : a.ff)) / 64;
             const int kb = phase == QKV ? a.kb_qkv : (phase == O ? a.kb_o : a.kb_down);
-            const int row0 = phase == QKV ? q0 : c0, bytes = (phase == QKV ? q_rows : c_rows) * 128 * kb;
+            const int row0 = phase == QKV ? q0 : c0, bytes = (phase == QKV ? q_rows : c_rows) * 128 * kb, act = 128 * a.T;
 #pragma unroll 1
             for (int k = 0; k < blocks; k += kb) {
-              uint8_t* dst = next_stage(bytes);
+              uint8_t* dst = next_stage(bytes + act * min(kb, blocks - k));
               if (!ok) break;
               tma_load_3d(dst, map, 0, row0, k, &sh.full[at.slot]);
               sent();
@@ -848,13 +891,13 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
       }
     }
     __syncwarp();
-  } else if (warp > DS_WARPS) {
+  } else if (warp == DS_WARPS + 1) {
     // ------------------------------------------------------------------ the activations
-    // They go where the consumers find them beside the weights, in the same order and under the same barrier; loaded
-    // by the consumers themselves, into registers and a few stages ahead, each stage cost them a trip to L2 (0.48 us).
+    // They go where the consumers find them beside the weights, in the same order and under the same barrier, a bulk
+    // copy a stage: loaded by the consumers themselves, into registers and a few stages ahead, each stage cost them a
+    // trip to L2 (0.48 us), and 16-byte copies whose 32 lanes each arrive at the barrier took a warp 0.45 us a stage.
     StackRing at = {0, 0};
-    const int mine = warp - DS_WARPS - 1;
-    int gone = 0, turn = 0;              // turn: of the feeders, at the stage that comes next
+    int gone = 0;
     bool ok = true;
     const uint32_t ring32 = smem_u32(ring);
 #pragma unroll 1
@@ -862,37 +905,31 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
 #pragma unroll 1
       for (int phase = QKV; phase <= DOWN && ok; ++phase) {
         if (phase == MERGE) continue;
-        int stages = 0, bytes = 0, left = 0;
-        const uint8_t* src = nullptr;
+        int stages = 0;
         if (phase == ATTENTION) {
           for (int ui = 0; ui < sh.n_units; ++ui) stages += 2 * sh.units[ui].tiles;
-        } else {
-          const int K = phase == O ? a.nq * 128 : (phase == DOWN ? a.ff : a.hidden);
-          const int kb = phase == QKV ? a.kb_qkv : (phase == O ? a.kb_o : (phase == DOWN ? a.kb_down : 1));
-          stages = (K / 64 + kb - 1) / kb, bytes = kb * 128 * a.T, left = K * 2 * a.T;
-          src = reinterpret_cast<const uint8_t*>(phase == O ? a.ab : (phase == DOWN ? a.hb : a.xb));
-          if (!(ok = stack_until(&sh.go, gone++, &sh.abort))) break;
-          __threadfence_block();
+          const int to = at.slot + stages, rounds = to / a.n_slots;
+          at.round += rounds;
+          at.slot = to - rounds * a.n_slots;
+          continue;
         }
+        const int K = phase == O ? a.nq * 128 : (phase == DOWN ? a.ff : a.hidden);
+        const int kb = phase == QKV ? a.kb_qkv : (phase == O ? a.kb_o : (phase == DOWN ? a.kb_down : 1));
+        const int bytes = kb * 128 * a.T;
+        int left = K * 2 * a.T;
+        const uint8_t* src = reinterpret_cast<const uint8_t*>(phase == O ? a.ab : (phase == DOWN ? a.hb : a.xb));
+        if (!(ok = stack_until(&sh.go, gone++, &sh.abort))) break;
+        __threadfence_block();
+        ds_fence_async();
 #pragma unroll 1
-        for (int i = 0; i < stages; ++i) {
-          if (turn == mine) {
-            if (!(ok = stack_issued(sh, (int)at.round * a.n_slots + at.slot))) break;
-            const int n = min(bytes, left);
-            const uint32_t dst = ring32 + at.slot * a.slot_bytes + a.act_at;
-#pragma unroll 4
-            for (int o = lane * 16; o < n; o += 512)
-              asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + o), "l"(src + o) : "memory");
-            asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" ::"r"(smem_u32(&sh.full[at.slot])) : "memory");
-          }
-          turn = turn + 1 == DS_FEEDERS ? 0 : turn + 1;
-          src += bytes, left -= bytes;
+        for (; left > 0; left -= bytes) {
+          if (!(ok = stack_issued(sh, (int)at.round * a.n_slots + at.slot))) break;
+          if (lane == 0) bulk_load(ring32 + at.slot * a.slot_bytes + a.act_at, src, min(bytes, left), &sh.full[at.slot]);
+          src += bytes;
           at.skip(1, a.n_slots);
         }
       }
     }
-    cp_async_commit();
-    cp_async_wait<0>();
     __syncwarp();
   } else {
     // ------------------------------------------------------------------ the work
@@ -906,6 +943,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
         a.xb[stack_fragment(c0 + lane, warp, a.T)] = __float2bfloat16(x * a.layers[0].norm1[c0 + lane]);
       }
       w.publish(warp, x * x);
+      ds_fence_async();
     }
     int phase = -1, layer = 0;
     bool ok = true;
@@ -927,11 +965,12 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
         const bool normed = phase == QKV || phase == GATE_UP;
         const int rows = phase == QKV ? q_rows : (phase == GATE_UP ? gu_rows : c_rows);
         w.go();
-        if (normed) w.row_factors();
+        if (normed) w.ask_factors();
         int pitch;
         const int parts = w.product(normed ? a.hidden : (phase == O ? a.nq * 128 : a.ff), rows,
                                     phase == QKV ? a.kb_qkv : (phase == O ? a.kb_o : (phase == DOWN ? a.kb_down : 1)), pitch);
         DS_STAMP(phase * 2 + 1);
+        if (normed) w.row_factors();
         ds_sync();
         const int stride = a.T * pitch;
         if (!normed) {
@@ -945,19 +984,22 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
               if (last) a.x_out[(size_t)warp * a.hidden + c0 + lane] = x;
             }
             w.publish(warp, x * x);
+            ds_fence_async();
           }
           if (last) break;
         } else if (phase == QKV) {
 #pragma unroll 1
-          for (int i = tid; i < q_rows * a.T; i += DS_CONSUMERS) {
-            const int t = i / q_rows, r = i - t * q_rows;
-            a.qkv[(size_t)t * N + q0 + r] = w.summed(red + t * pitch + r, parts, stride) * sh.rstd[t];
-          }
+          for (int t = warp; t < a.T; t += DS_WARPS)
+#pragma unroll 1
+            for (int r = lane; r < q_rows; r += 32)
+              a.qkv[(size_t)t * N + q0 + r] = w.summed(red + t * pitch + r, parts, stride) * sh.rstd[t];
         } else {
           const int whole = share.whole * 8, n = whole + (share.half >= 0 ? 4 : 0);
+          const int chunks = (n + 31) >> 5;
 #pragma unroll 1
-          for (int i = tid; i < n * a.T; i += DS_CONSUMERS) {
-            const int t = i / n, f = i - t * n;
+          for (int i = warp; i < chunks * a.T; i += DS_WARPS) {
+            const int t = i / chunks, f = (i - t * chunks) * 32 + lane;
+            if (f >= n) continue;
             const bool in_whole = f < whole;
             const int rg = in_whole ? (f >> 3) * 16 + (f & 7) : share.whole * 16 + f - whole;
             const int ru = in_whole ? rg + 8 : rg + 4;
@@ -967,6 +1009,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
             const float up = w.summed(s + ru, parts, stride) * sh.rstd[t];
             a.hb[stack_fragment(feature, t, a.T)] = __float2bfloat16(__fdividef(gate, 1.0f + __expf(-gate)) * up);
           }
+          ds_fence_async();
         }
       }
     }
@@ -1011,25 +1054,28 @@ struct StackPlan {
 static int stack_plan(int hidden, int ff, int nq, int nkv, int P, int T, StackPlan* plan) {
   const int N = (nq + 2 * nkv) * 128, groups = ff / 8;
   if (hidden <= 0 || ff <= 0 || nq <= 0 || nkv <= 0 || P <= 0) return GB_ERR_BAD_ARG;
-  if (hidden % 64 || ff % 64 || nq % nkv || nq / nkv > 8 || N > (1 << 20) || ff > (1 << 20) || P > 2048)
+  if (hidden % 64 || ff % 64 || nq % nkv || nq / nkv > 8 || N > (1 << 20) || ff > (1 << 20))
     return GB_ERR_UNSUPPORTED;
   const int c_most = (hidden + P - 1) / P, q_most = (N + P - 1) / P, h_most = (2 * groups + P - 1) / P;
   const int h_least = 2 * groups / P;
   // every block has a share of everything, and it fits where it is kept
-  if (hidden < P || N < P || h_least < 2 || c_most > DS_OWN_MOST || q_most > 256) return GB_ERR_UNSUPPORTED;
+  if (hidden < P || N < P || h_least < 2 || c_most > DS_OWN_MOST || q_most > 256 || P > DS_BLOCKS_MOST) return GB_ERR_UNSUPPORTED;
   if (DS_ROWS * nkv > DS_UNITS_MOST * P) return GB_ERR_UNSUPPORTED;
   const int gu_rows = h_most * 8;
   int at = gu_rows * 128;
   at = (at < 2 * DS_TILE_BYTES ? 2 * DS_TILE_BYTES : at + 1023) / 1024 * 1024;
   // 64-column blocks a stage: as the slot holds, at most `most`, and none where the warps' sums do not fit
   auto blocks = [&](int rows, int most) {
-    const int tiles = (rows + 15) / 16, parts = tiles >= 3 ? DS_FOURS : DS_WARPS, pitch = (rows + 11) / 16 * 16 + 4;
+    const int tiles = (rows + 15) / 16, parts = DS_FOURS * (tiles > 3 ? 1 : 2), pitch = (rows + 11) / 16 * 16 + 4;
     if (tiles > 4 * DS_TILES || parts * DS_ROWS * pitch * 4 > DS_RED_BYTES) return 0;
     const int fits = at / (rows * 128);
+    if (tiles > 3 && most > 2) most = 2;       // (a warp takes up to four steps of a stage)
     return fits < most ? fits : most;
   };
   plan->act_at = at;
   plan->kb_qkv = blocks(q_most, 4), plan->kb_o[0] = blocks(c_most, 8), plan->kb_o[1] = blocks(c_most, 4);
+  // (o and down: two tiles at most, whose twelve partial sums always fit, so eight blocks are four steps a warp)
+  static_assert(DS_WARPS * DS_ROWS * 36 * 4 <= DS_RED_BYTES, "");
   if (plan->kb_qkv < 1 || plan->kb_o[1] < 1 || blocks(gu_rows, 1) < 1 || h_most / 2 * 16 > 256) return GB_ERR_UNSUPPORTED;
   const int kb_o = plan->kb_o[T > DS_FEW], kb = kb_o > plan->kb_qkv ? kb_o : plan->kb_qkv;
   plan->slot_bytes = (at + kb * 128 * T + 1023) / 1024 * 1024;
