@@ -36,6 +36,8 @@
 // Every wait (a stage of the ring, the grid barrier) is bounded by wall-clock time; a block that
 // gives up records a code, lets its copies in flight land and leaves.  The launch is cooperative:
 // all blocks are resident or none.
+#include <stddef.h>
+
 #include "tc_common.cuh"
 
 #include "attn_mma.cuh"
@@ -67,17 +69,19 @@ struct StackLayer {
   CUtensorMap qkv[2], o[2][2], gate_up[2], down[2][2];     // (o, down: [few, more rows of activations][..])
   CUtensorMap half;                // half a group of eight gates and their ups: 4 + 4 rows
   CUtensorMap k, v;
-  const float *norm1, *norm2, *q_norm, *k_norm;
-  bf16 *k_pages, *v_pages;
-  long long pad_[2];
 };
+// What else a layer has, as 32-bit words in one row: the two norms' weights [hidden], those of q and k [128] (ones where
+// the heads have no norms), the addresses of its pages of keys and of values [2 each].
+__host__ __device__ __forceinline__ int stack_row_words(int hidden) { return 2 * hidden + 256 + 4; }
 static_assert(sizeof(StackLayer) % 64 == 0, "tensor maps are 64-byte aligned");
 
 struct StackArgs {
   const StackLayer* layers;
+  const float* rows;                         // [n_layers][stack_row_words]
   int n_layers, T, hidden, ff, nq, nkv;      // T: activation rows = sequences, head size 128
   int slot_bytes, n_slots, act_at;           // the ring, where a slot's activations begin
   int kb_qkv, kb_o, kb_down;                 // 64-column blocks of a stage
+  int qk_norm;                               // whether the heads of q and k have norms
   float eps, qk_eps, scale_log2;
   const bf16* x_in;                          // [T, hidden]: the stream in front of the first layer
   const float* res_in;                       // or the same in 32-bit
@@ -197,7 +201,7 @@ __device__ __forceinline__ uint32_t transposed8x8(uint32_t v) {
 
 // The attention's work: a unit is one split of one (sequence, kv head) pair.
 struct StackUnit {
-  int seq, kvh, tile0, tiles, split, splits, slot, len;
+  int seq, kvh, tile0, tiles, split, splits, slot, len, page;      // page: of the new key
 };
 
 // Tiles a unit takes: the fewest, DS_FOURS or more (as many tiles are taken at once), that make no
@@ -225,6 +229,9 @@ struct StackShared {
   float2 turn[DS_UNITS_MOST][64];        // cosine and sine of a unit's new position
   float rstd[DS_ROWS];
   float ss[DS_ROWS * DS_BLOCKS_MOST];    // the blocks' sums of squares, on their way while a product runs
+  float norm[DS_ROWS * 32];              // the weights of the norm behind o or down, a copy a row
+  float qk_w[256];                       // the layer's norms of q and k ...
+  bf16* kv_pages[2];                     // ... and its pages
   float red_m[DS_WARPS * 8], red_l[DS_WARPS * 8];
   StackUnit units[DS_UNITS_MOST];
   int n_units, split_any;
@@ -232,6 +239,10 @@ struct StackShared {
   int pages[DS_PAGES];                   // of the block's tiles, as far as there is room
   int abort, issued, go;                 // issued: stages asked for; go: phases whose activations are there
 };
+
+static_assert(offsetof(StackShared, turn) % 16 == 0 && offsetof(StackShared, qk_w) % 16 == 0 &&
+                  offsetof(StackShared, kv_pages) % 16 == 0,
+              "copied or read by 16 bytes");
 
 // A place in the order of stages, which is the same for the warps that fill the ring and for
 // those that empty it: every phase's loop counts stages from the same numbers.
@@ -267,7 +278,7 @@ struct StackConsumer {
   uint8_t* ring;
   float* red;
   StackRing at;                // the first stage of the phase
-  int tid, warp, lane, p, P;
+  int tid, warp, lane, p, P, c_rows;
   bool bad;
   int gone;
   unsigned arrived;            // arrivals the grid barrier has had when all have come
@@ -328,19 +339,31 @@ struct StackConsumer {
     }
   }
 
-  // 1 / rms of the rows, from the blocks' sums of squares: a warp a row, asked for in front of the product and summed up
-  // behind it (waiting for them in front cost the first four a trip to L2 before its first stage).
-  __device__ __forceinline__ void ask_factors() {
-    if (warp < a.T)
-      for (int i = lane; i < P; i += 32)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(sh.ss + warp * DS_BLOCKS_MOST + i)),
-                     "l"(a.ss + warp * P + i)
+  // What the phase needs behind its product, asked for in front of it: read where it is used, each cost a trip to
+  // L2 or, the weights between one step and the next having been through it, to memory.
+  // In front of a product of normalised rows the blocks' sums of squares (a warp a row), of qkv the attention's vectors
+  // too; else `norm`, the weights of the next norm.
+  __device__ __forceinline__ void ask(const float* row, const float* norm, bool normed, bool qkv) {
+    if (warp < a.T) {
+      if (normed) {
+        for (int i = lane; i < P; i += 32)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(sh.ss + warp * DS_BLOCKS_MOST + i)),
+                       "l"(a.ss + warp * P + i)
+                       : "memory");
+      } else if (lane < c_rows) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(sh.norm + warp * 32 + lane)), "l"(norm + lane)
                      : "memory");
+      }
+    } else if (qkv && warp >= DS_ROWS) {
+      const int i = (warp - DS_ROWS) * 32 + lane;
+      if (i < 65)
+        cp_async16(i < 64 ? (void*)(sh.qk_w + i * 4) : (void*)sh.kv_pages, row + 2 * a.hidden + i * 4, true);
+    }
+    cp_async_commit();
   }
+  // 1 / rms of the rows
   __device__ __forceinline__ void row_factors() {
     if (warp < a.T) {
-      cp_async_commit();
-      cp_async_wait<0>();
       float s = 0.f;
       for (int i = lane; i < P; i += 32) s += sh.ss[warp * DS_BLOCKS_MOST + i];      // (what this lane asked for)
       s = warp_sum(s);
@@ -434,14 +457,13 @@ struct StackConsumer {
     return parts;
   }
 
+  // A sum over the parts, in their order, from loads that do not wait for one another.
   __device__ __forceinline__ float summed(const float* at0, int parts, int stride) {
-    float s = 0.f;
-#pragma unroll 2
-    for (int i = 0; i < parts; i += DS_FOURS) {
+    float v[DS_WARPS], s = 0.f;
 #pragma unroll
-      for (int j = 0; j < DS_FOURS; ++j) s += at0[j * stride];
-      at0 += DS_FOURS * stride;
-    }
+    for (int i = 0; i < DS_WARPS; ++i) v[i] = i < parts ? at0[i * stride] : 0.f;
+#pragma unroll
+    for (int i = 0; i < DS_WARPS; ++i) s += v[i];
     return s;
   }
 
@@ -452,7 +474,7 @@ struct StackConsumer {
   }
 
   // ---- attention -----------------------------------------------------------------------------
-  __device__ __forceinline__ void attention(const StackLayer& L) {
+  __device__ __forceinline__ void attention() {
     const int G = a.nq / a.nkv, N = (a.nq + 2 * a.nkv) * 128;
     const int g = lane >> 2, c = lane & 3;
     bf16* q_s = reinterpret_cast<bf16*>(red);              // [8][DS_QLD]
@@ -470,15 +492,14 @@ struct StackConsumer {
         const int head = warp < G ? u.kvh * G + warp : (warp == G ? a.nq + u.kvh : a.nq + a.nkv + u.kvh);
         const bool is_v = warp == G + 1;
         const float* src = a.qkv + (size_t)u.seq * N + head * 128;
-        const float* w = is_v ? nullptr : (warp < G ? L.q_norm : L.k_norm);
         const float2 lo = __ldcg(reinterpret_cast<const float2*>(src) + lane);
         const float2 hi = __ldcg(reinterpret_cast<const float2*>(src + 64) + lane);
-        float2 wl = make_float2(1.f, 1.f), wh = wl;
-        if (w) wl = __ldg(reinterpret_cast<const float2*>(w) + lane), wh = __ldg(reinterpret_cast<const float2*>(w + 64) + lane);
         float x0 = lo.x, x1 = lo.y, y0 = hi.x, y1 = hi.y;
-        if (w) {
+        if (a.qk_norm && !is_v) {
+          const float2* w = reinterpret_cast<const float2*>(sh.qk_w + (warp < G ? 0 : 128));
           const float ssq = warp_sum(x0 * x0 + x1 * x1 + y0 * y0 + y1 * y1);
           const float f = rsqrtf(ssq / 128.f + a.qk_eps);
+          const float2 wl = w[lane], wh = w[32 + lane];
           x0 = x0 * f * wl.x, x1 = x1 * f * wl.y, y0 = y0 * f * wh.x, y1 = y1 * f * wh.y;
         }
         if (a.inv_freq && !is_v) {
@@ -492,8 +513,7 @@ struct StackConsumer {
         reinterpret_cast<uint32_t*>(dst)[lane] = p0;
         reinterpret_cast<uint32_t*>(dst + 64)[lane] = p1;
         if (warp >= G) {
-          bf16* page = (is_v ? L.v_pages : L.k_pages) +
-                       paged_row(a.block_table + (size_t)u.slot * a.max_pages, pos, u.kvh, a.nkv, 64, 128);
+          bf16* page = sh.kv_pages[is_v] + (((size_t)u.page * a.nkv + u.kvh) * 64 + (pos & 63)) * 128;
           reinterpret_cast<uint32_t*>(page)[lane] = p0;
           reinterpret_cast<uint32_t*>(page + 64)[lane] = p1;
         }
@@ -763,6 +783,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
         w.tile0 = min(sh.tiles[t], w.split * per);
         w.tiles = min(sh.tiles[t], w.tile0 + per) - w.tile0;
         w.slot = a.slots[t], w.len = a.kv_len[t];
+        w.page = a.block_table[(size_t)w.slot * a.max_pages + (w.len - 1) / 64];
       }
       first += here;
     }
@@ -896,51 +917,68 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
     // They go where the consumers find them beside the weights, in the same order and under the same barrier, a bulk
     // copy a stage: loaded by the consumers themselves, into registers and a few stages ahead, each stage cost them a
     // trip to L2 (0.48 us), and 16-byte copies whose 32 lanes each arrive at the barrier took a warp 0.45 us a stage.
-    StackRing at = {0, 0};
-    int gone = 0;
-    bool ok = true;
-    const uint32_t ring32 = smem_u32(ring);
+    if (lane == 0) {
+      StackRing at = {0, 0};
+      int gone = 0, stage = 0, issued = 0;       // issued: as last looked at
+      bool ok = true;
+      const uint32_t ring32 = smem_u32(ring);
+      auto until = [&](volatile int* count, int more_than) -> int {
+        int n = *count;
+        if (n > more_than) return n;
+        const unsigned long long t0 = now_ns();
 #pragma unroll 1
-    for (int layer = 0; layer < a.n_layers && ok; ++layer) {
+        for (int i = 1; (n = *count) <= more_than; ++i)
+          if ((i & 63) == 0 && (*(volatile int*)&sh.abort || now_ns() - t0 > TC_WAIT_LIMIT_NS)) {
+            ok = false;
+            break;
+          }
+        return n;
+      };
 #pragma unroll 1
-      for (int phase = QKV; phase <= DOWN && ok; ++phase) {
-        if (phase == MERGE) continue;
-        int stages = 0;
-        if (phase == ATTENTION) {
-          for (int ui = 0; ui < sh.n_units; ++ui) stages += 2 * sh.units[ui].tiles;
-          const int to = at.slot + stages, rounds = to / a.n_slots;
-          at.round += rounds;
-          at.slot = to - rounds * a.n_slots;
-          continue;
-        }
-        const int K = phase == O ? a.nq * 128 : (phase == DOWN ? a.ff : a.hidden);
-        const int kb = phase == QKV ? a.kb_qkv : (phase == O ? a.kb_o : (phase == DOWN ? a.kb_down : 1));
-        const int bytes = kb * 128 * a.T;
-        int left = K * 2 * a.T;
-        const uint8_t* src = reinterpret_cast<const uint8_t*>(phase == O ? a.ab : (phase == DOWN ? a.hb : a.xb));
-        if (!(ok = stack_until(&sh.go, gone++, &sh.abort))) break;
-        __threadfence_block();
-        ds_fence_async();
+      for (int layer = 0; layer < a.n_layers && ok; ++layer) {
 #pragma unroll 1
-        for (; left > 0; left -= bytes) {
-          if (!(ok = stack_issued(sh, (int)at.round * a.n_slots + at.slot))) break;
-          if (lane == 0) bulk_load(ring32 + at.slot * a.slot_bytes + a.act_at, src, min(bytes, left), &sh.full[at.slot]);
-          src += bytes;
-          at.skip(1, a.n_slots);
+        for (int phase = QKV; phase <= DOWN && ok; ++phase) {
+          if (phase == MERGE) continue;
+          if (phase == ATTENTION) {
+            int stages = 0;
+            for (int ui = 0; ui < sh.n_units; ++ui) stages += 2 * sh.units[ui].tiles;
+            stage += stages;
+            const int to = at.slot + stages, rounds = to / a.n_slots;
+            at.round += rounds;
+            at.slot = to - rounds * a.n_slots;
+            continue;
+          }
+          const int K = phase == O ? a.nq * 128 : (phase == DOWN ? a.ff : a.hidden);
+          const int kb = phase == QKV ? a.kb_qkv : (phase == O ? a.kb_o : (phase == DOWN ? a.kb_down : 1));
+          const int bytes = kb * 128 * a.T;
+          int left = K * 2 * a.T;
+          const uint8_t* src = reinterpret_cast<const uint8_t*>(phase == O ? a.ab : (phase == DOWN ? a.hb : a.xb));
+          until(&sh.go, gone++);
+          __threadfence_block();
+          ds_fence_async();
+#pragma unroll 1
+          for (; left > 0 && ok; left -= bytes) {
+            if (issued <= stage) issued = until(&sh.issued, stage);
+            if (!ok) break;
+            bulk_load(ring32 + at.slot * a.slot_bytes + a.act_at, src, min(bytes, left), &sh.full[at.slot]);
+            src += bytes;
+            ++stage;
+            at.skip(1, a.n_slots);
+          }
         }
       }
     }
     __syncwarp();
   } else {
     // ------------------------------------------------------------------ the work
-    StackConsumer w = {a, sh, ring, red, {0, 0}, tid, warp, lane, p, P, false, 0, 0u};
+    StackConsumer w = {a, sh, ring, red, {0, 0}, tid, warp, lane, p, P, c_rows, false, 0, 0u};
     // the block's columns of the stream: a warp a row of the batch, a lane a column
     float x = 0.f;
     if (warp < a.T) {
       if (lane < c_rows) {
         const size_t i = (size_t)warp * a.hidden + c0 + lane;
         x = a.res_in ? a.res_in[i] : __bfloat162float(a.x_in[i]);
-        a.xb[stack_fragment(c0 + lane, warp, a.T)] = __float2bfloat16(x * a.layers[0].norm1[c0 + lane]);
+        a.xb[stack_fragment(c0 + lane, warp, a.T)] = __float2bfloat16(x * a.rows[c0 + lane]);
       }
       w.publish(warp, x * x);
       ds_fence_async();
@@ -953,10 +991,9 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
       if (phase == DOWN) ++layer;
       phase = phase == DOWN ? QKV : phase + 1;
       if (phase == MERGE && !sh.split_any) ++phase;
-      const StackLayer& L = a.layers[layer];
       DS_STAMP(phase * 2);
       if (phase == ATTENTION) {
-        w.attention(L);
+        w.attention();
         DS_STAMP(phase * 2 + 1);
       } else if (phase == MERGE) {
         w.merge(unit_tiles);
@@ -964,21 +1001,23 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
       } else {
         const bool normed = phase == QKV || phase == GATE_UP;
         const int rows = phase == QKV ? q_rows : (phase == GATE_UP ? gu_rows : c_rows);
+        const bool last = phase == DOWN && layer + 1 == a.n_layers;
+        const float* row = a.rows + (size_t)layer * stack_row_words(a.hidden);
         w.go();
-        if (normed) w.ask_factors();
+        // (behind the last layer comes no norm of the stack's: its factors are read and not used)
+        w.ask(row, (phase == O ? row + a.hidden : (last ? row : row + stack_row_words(a.hidden))) + c0, normed, phase == QKV);
         int pitch;
         const int parts = w.product(normed ? a.hidden : (phase == O ? a.nq * 128 : a.ff), rows,
                                     phase == QKV ? a.kb_qkv : (phase == O ? a.kb_o : (phase == DOWN ? a.kb_down : 1)), pitch);
         DS_STAMP(phase * 2 + 1);
+        cp_async_wait<0>();
         if (normed) w.row_factors();
         ds_sync();
         const int stride = a.T * pitch;
         if (!normed) {
-          const bool last = phase == DOWN && layer + 1 == a.n_layers;
-          const float* norm = last ? L.norm1 : (phase == O ? L.norm2 : a.layers[layer + 1].norm1);
           if (warp < a.T) {
             if (lane < c_rows) {
-              const float weight = __ldg(norm + c0 + lane);
+              const float weight = sh.norm[warp * 32 + lane];
               x += w.summed(red + warp * pitch + lane, parts, stride);
               a.xb[stack_fragment(c0 + lane, warp, a.T)] = __float2bfloat16(x * weight);
               if (last) a.x_out[(size_t)warp * a.hidden + c0 + lane] = x;
@@ -1108,16 +1147,16 @@ GB_EXPORT int gb_decode_stack_share(int hidden, int ff, int nq, int nkv, int P, 
 }
 GB_EXPORT int gb_decode_stack_fragment(int k, int t, int T) { return stack_fragment(k, t, T); }
 
-// Writes a layer's entry (tensor maps and pointers) to host memory.
+GB_EXPORT int gb_decode_stack_row_words(int hidden) { return stack_row_words(hidden); }
+
+// Writes a layer's entry (its tensor maps) to host memory.
 GB_EXPORT int gb_decode_stack_encode(void* entry, int hidden, int ff, int nq, int nkv, int P, const void* w_qkv,
                                      const void* w_o, const void* w_gate_up, const void* w_down, void* k_pages,
-                                     void* v_pages, long long n_pages, const float* norm1, const float* norm2,
-                                     const float* q_norm, const float* k_norm) {
+                                     void* v_pages, long long n_pages) {
   StackPlan plan;
   int e = stack_plan(hidden, ff, nq, nkv, P, DS_ROWS, &plan);
   if (e) return e;
-  if (!entry || ((uintptr_t)entry & 63) || !w_qkv || !w_o || !w_gate_up || !w_down || !k_pages || !v_pages || !norm1 ||
-      !norm2 || n_pages <= 0)
+  if (!entry || ((uintptr_t)entry & 63) || !w_qkv || !w_o || !w_gate_up || !w_down || !k_pages || !v_pages || n_pages <= 0)
     return GB_ERR_BAD_ARG;
   if ((unsigned long long)n_pages * nkv * 64 > 0x7fffffffull) return GB_ERR_UNSUPPORTED;
   StackLayer* L = (StackLayer*)entry;
@@ -1141,8 +1180,6 @@ GB_EXPORT int gb_decode_stack_encode(void* entry, int hidden, int ff, int nq, in
   const uint64_t rows = (uint64_t)n_pages * nkv * 64;
   if ((e = tc_make_map_2d(&L->k, k_pages, rows, 128, 256, 64, 64))) return e;
   if ((e = tc_make_map_2d(&L->v, v_pages, rows, 128, 256, 64, 64))) return e;
-  L->norm1 = norm1, L->norm2 = norm2, L->q_norm = q_norm, L->k_norm = k_norm;
-  L->k_pages = (bf16*)k_pages, L->v_pages = (bf16*)v_pages;
   return 0;
 }
 
@@ -1152,7 +1189,7 @@ GB_EXPORT int gb_decode_stack(StackArgs* a, int P, cudaStream_t s) {
   if (a->T < 1 || a->T > DS_ROWS) return GB_ERR_BAD_ARG;
   int e = stack_plan(a->hidden, a->ff, a->nq, a->nkv, P, a->T, &plan);
   if (e) return e;
-  if (a->n_layers < 1 || a->max_pages <= 0 || !a->layers || !a->x_out || (!a->x_in && !a->res_in) || !a->slots ||
+  if (a->n_layers < 1 || a->max_pages <= 0 || !a->layers || !a->rows || ((uintptr_t)a->rows & 15) || !a->x_out || (!a->x_in && !a->res_in) || !a->slots ||
       !a->kv_len || !a->block_table || !a->xb || !a->ab || !a->hb || !a->ss || !a->qkv || !a->part_o || !a->part_ml ||
       !a->sync || !a->error)
     return GB_ERR_BAD_ARG;

@@ -86,14 +86,12 @@ class DecodeStack:
         hidden, ff, nq, nkv, scale, qk_eps, eps, _eps = _sizes(blocks[0])
         device = blocks[0].mixer.qkv.weight.device
         self.hidden, self.max_rows = hidden, max_rows
-        vector = lambda t: None if t is None else t.float().contiguous()
         self._layers = []                 # (the tensors that the device's table points at)
         for b, view in zip(blocks, views):
             m, f = b.mixer, b.feedforward
             self._layers.append(dict(
                 qkv=m.qkv.weight, o=m.o.weight, gate_up=f.gate_up.weight, down=f.down.weight, k_pages=view.k_pages,
-                v_pages=view.v_pages, norm1=vector(b.norm1.weight), norm2=vector(b.norm2.weight),
-                q_norm=vector(m.q_norm_w), k_norm=vector(m.k_norm_w)))
+                v_pages=view.v_pages, norm1=b.norm1.weight, norm2=b.norm2.weight, q_norm=m.q_norm_w, k_norm=m.k_norm_w))
         self.block_table = views[0].block_table
         self.state = ops.decode_stack_state(self._layers, hidden, ff, nq, nkv, max_rows, device)
         self.args = dict(eps=eps, qk_eps=qk_eps or 0.0, scale=scale,

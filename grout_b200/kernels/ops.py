@@ -1819,9 +1819,9 @@ def diff_heads(x: torch.Tensor, v_dim: int, lam: float, eps: float, mult: float)
 
 # ---------------------------------------------------------------- a decode step's layers
 class _StackArgs(ctypes.Structure):
-    _fields_ = [("layers", _P), ("n_layers", _I), ("T", _I), ("hidden", _I), ("ff", _I), ("nq", _I), ("nkv", _I),
+    _fields_ = [("layers", _P), ("rows", _P), ("n_layers", _I), ("T", _I), ("hidden", _I), ("ff", _I), ("nq", _I), ("nkv", _I),
                 ("slot_bytes", _I), ("n_slots", _I), ("act_at", _I), ("kb_qkv", _I), ("kb_o", _I), ("kb_down", _I),
-                ("eps", _F), ("qk_eps", _F), ("scale_log2", _F), ("x_in", _P), ("res_in", _P), ("x_out", _P),
+                ("qk_norm", _I), ("eps", _F), ("qk_eps", _F), ("scale_log2", _F), ("x_in", _P), ("res_in", _P), ("x_out", _P),
                 ("inv_freq", _P), ("slots", _P), ("kv_len", _P), ("block_table", _P), ("max_pages", _I),
                 ("xb", _P), ("ab", _P), ("hb", _P), ("ss", _P), ("qkv", _P), ("part_o", _P), ("part_ml", _P),
                 ("sync", _P), ("error", _P), ("stamps", _P)]
@@ -1838,7 +1838,7 @@ def decode_stack_takes(hidden: int, ff: int, nq: int, nkv: int, device) -> bool:
 
 def decode_stack_state(layers, hidden: int, ff: int, nq: int, nkv: int, max_rows: int, device) -> dict:
     """What launches over these layers share: their table on the device and scratch for ``max_rows`` rows.
-    ``layers``: dicts of the weights (bf16: qkv, o, gate_up, down), pages and 32-bit norm weights of each.  The tensors
+    ``layers``: dicts of the weights (bf16: qkv, o, gate_up, down), pages and norm weights of each.  Weights and pages
     must outlive the state; launches that use it must be ordered on one stream."""
     P = _sm_count(device)
     size = _fn("decode_stack", "gb_decode_stack_layer_bytes", "iiiii")(hidden, ff, nq, nkv, P)
@@ -1846,7 +1846,10 @@ def decode_stack_state(layers, hidden: int, ff: int, nq: int, nkv: int, max_rows
         raise KernelError(f"no plan for layers of {hidden} / {ff} with {nq} / {nkv} heads")
     host = torch.zeros(size * len(layers) + 64, dtype=torch.uint8)
     skip = -host.data_ptr() % 64                 # tensor maps lie on 64 bytes
-    encode = _fn("decode_stack", "gb_decode_stack_encode", "piiiiippppppl" + "pppp")
+    encode = _fn("decode_stack", "gb_decode_stack_encode", "piiiiippppppl")
+    words = _fn("decode_stack", "gb_decode_stack_row_words", "i")(hidden)
+    rows = torch.ones((len(layers), words), dtype=torch.float32, device=device)   # a layer's norms, and where its pages are
+    normed = layers[0]["q_norm"] is not None
     for i, t in enumerate(layers):
         for n, shape in (("qkv", ((nq + 2 * nkv) * 128, hidden)), ("o", (hidden, nq * 128)),
                          ("gate_up", (2 * ff, hidden)), ("down", (hidden, ff))):
@@ -1858,19 +1861,25 @@ def decode_stack_state(layers, hidden: int, ff: int, nq: int, nkv: int, max_rows
             if tuple(t[n].shape[1:]) != (nkv, 64, 128) or t[n].shape != t["k_pages"].shape:
                 raise KernelError(f"{n} are {tuple(t[n].shape)}, expected [*, {nkv}, 64, 128]")
         for n, width in (("norm1", hidden), ("norm2", hidden), ("q_norm", 128), ("k_norm", 128)):
-            if t[n] is not None or n in ("norm1", "norm2"):
-                _need(t[n], n, torch.float32, 1)
+            if normed or n in ("norm1", "norm2"):
+                _need(t[n], n, ndim=1)
                 if t[n].shape[0] != width:
                     raise KernelError(f"{n} has {t[n].shape[0]} elements, expected {width}")
+                at = {"norm1": 0, "norm2": hidden, "q_norm": 2 * hidden, "k_norm": 2 * hidden + 128}[n]
+                rows[i, at:at + width] = t[n].float()
+            elif t[n] is not None:
+                raise KernelError("either all layers have norms of q and k or none has")
+        where = torch.tensor([t["k_pages"].data_ptr(), t["v_pages"].data_ptr()], dtype=torch.int64)
+        rows.view(torch.int32)[i, words - 4:] = where.view(torch.int32).to(device)
         _check(encode(host.data_ptr() + skip + i * size, hidden, ff, nq, nkv, P, t["qkv"].data_ptr(), t["o"].data_ptr(),
                       t["gate_up"].data_ptr(), t["down"].data_ptr(), t["k_pages"].data_ptr(), t["v_pages"].data_ptr(),
-                      t["k_pages"].shape[0], _ptr(t["norm1"]), _ptr(t["norm2"]), _ptr(t["q_norm"]), _ptr(t["k_norm"])),
+                      t["k_pages"].shape[0]),
                "decode_stack_encode", 0)
     f32 = lambda n: torch.zeros(n, dtype=torch.float32, device=device)
     b16 = lambda n: torch.zeros(n, dtype=torch.bfloat16, device=device)
     T, splits = max_rows, 32
     return dict(sizes=(len(layers), hidden, ff, nq, nkv), rows=T, blocks=P,
-                layers=host[skip:skip + size * len(layers)].to(device),
+                layers=host[skip:skip + size * len(layers)].to(device), table=rows, qk_norm=int(normed),
                 xb=b16(T * hidden), ab=b16(T * nq * 128), hb=b16(T * ff), ss=f32(T * P), qkv=f32(T * (nq + 2 * nkv) * 128),
                 part_o=f32(T * nq * splits * 128), part_ml=f32(T * nq * splits * 2),
                 sync=torch.zeros(2, dtype=torch.int32, device=device))
@@ -1909,6 +1918,7 @@ def decode_stack(state: dict, res: Optional[torch.Tensor], pending: Optional[tor
             raise KernelError("the kernel rotates whole heads of 128")
     out = torch.empty((T, hidden), dtype=torch.float32, device=src.device)
     a = _StackArgs()
+    a.rows, a.qk_norm = state["table"].data_ptr(), state["qk_norm"]
     a.layers, a.n_layers, a.T, a.hidden, a.ff, a.nq, a.nkv = state["layers"].data_ptr(), n, T, hidden, ff, nq, nkv
     a.eps, a.qk_eps, a.scale_log2 = float(eps), float(qk_eps), float(scale) * _LOG2E
     a.x_in, a.res_in, a.x_out, a.inv_freq = _ptr(pending), _ptr(res), out.data_ptr(), _ptr(inv_freq)
