@@ -389,9 +389,13 @@ struct StackConsumer {
     const int part = quad * s_inc + s_off, parts = DS_FOURS * s_inc;
     const int n_tiles = (tiles - t_off + (1 << ways) - 1) >> ways;
     const int g = lane >> 2, c = lane & 3;
-    float acc[DS_TILES][4];
+    // Two sums a tile, so that no product waits for the one before it: a warp issues in order, and one chain of eight
+    // took a four 0.97 us a stage.  The odd tile's are the last ones.
+    float acc[DS_TILES][2][4];
 #pragma unroll
-    for (int i = 0; i < DS_TILES; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+    for (int i = 0; i < DS_TILES; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[i][0][e] = acc[i][1][e] = 0.f;
     // (columns beyond the rows get some other row's values: nobody reads what becomes of them)
     const uint32_t act = a.act_at + min(g, a.T - 1) * 64 + c * 16, act_pitch = a.T * 64;
     const uint32_t ring32 = smem_u32(ring), tile_pitch = 2048u << ways;
@@ -414,26 +418,37 @@ struct StackConsumer {
           // (a step is four 16-byte chunks of a 64-column block; the second pair of them is two chunks on)
           const uint32_t w0 = base + row0 * 128 + ((((step0 & 1) * 4 + half) ^ (row0 & 7)) << 4);
           const uint32_t w1 = base + row1 * 128 + ((((step1 & 1) * 4 + half) ^ (row1 & 7)) << 4);
-          uint32_t f0[4], f1[4], w[2][4][4];       // (a tile's operands while the one before it is multiplied)
+          uint32_t f0[4], f1[4], w[2][4][4];
           lds4(f0, base + act + step0 * act_pitch);
           lds4(f1, base + act + step1 * act_pitch);
-          auto tile = [&](int t, uint32_t (&v)[4][4]) {
+          auto load = [&](int t, uint32_t (&v)[4][4]) {
             ldsm4(v[0], w0 + t * tile_pitch);
             ldsm4(v[1], (w0 ^ 32u) + t * tile_pitch);
             ldsm4(v[2], w1 + t * tile_pitch);
             ldsm4(v[3], (w1 ^ 32u) + t * tile_pitch);
           };
-          if (n_tiles > 0) tile(0, w[0]);
-#pragma unroll
-          for (int t = 0; t < DS_TILES; ++t) {
-            if (t < n_tiles) {
-              if (t + 1 < DS_TILES && t + 1 < n_tiles) tile(t + 1, w[(t + 1) & 1]);
-              mma_16816(acc[t], w[t & 1][0], f0[0], f0[1]);
-              mma_16816(acc[t], w[t & 1][1], f0[2], f0[3]);
-              if (two) {
-                mma_16816(acc[t], w[t & 1][2], f1[0], f1[1]);
-                mma_16816(acc[t], w[t & 1][3], f1[2], f1[3]);
-              }
+          if (n_tiles > 1) {
+            load(0, w[0]);
+            load(1, w[1]);
+            mma_16816(acc[0][0], w[0][0], f0[0], f0[1]);
+            mma_16816(acc[1][0], w[1][0], f0[0], f0[1]);
+            mma_16816(acc[0][1], w[0][1], f0[2], f0[3]);
+            mma_16816(acc[1][1], w[1][1], f0[2], f0[3]);
+            if (two) {
+              mma_16816(acc[0][0], w[0][2], f1[0], f1[1]);
+              mma_16816(acc[1][0], w[1][2], f1[0], f1[1]);
+              mma_16816(acc[0][1], w[0][3], f1[2], f1[3]);
+              mma_16816(acc[1][1], w[1][3], f1[2], f1[3]);
+            }
+          }
+          if (n_tiles & 1) {                     // (the third, or the only one)
+            float(&last)[2][4] = acc[2];
+            load(n_tiles - 1, w[0]);
+            mma_16816(last[0], w[0][0], f0[0], f0[1]);
+            mma_16816(last[1], w[0][1], f0[2], f0[3]);
+            if (two) {
+              mma_16816(last[0], w[0][2], f1[0], f1[1]);
+              mma_16816(last[1], w[0][3], f1[2], f1[3]);
             }
           }
         }
@@ -444,13 +459,13 @@ struct StackConsumer {
     pass(stages);
     float* out = red + part * a.T * pitch;
 #pragma unroll
-    for (int t = 0; t < DS_TILES; ++t) {
-      const int row = (t_off + (t << ways)) * 16 + g;
-      if (t < n_tiles) {
+    for (int i = 0; i < DS_TILES; ++i) {
+      const int t = i == 2 ? n_tiles - 1 : i;
+      if (i == 2 ? (n_tiles & 1) : n_tiles > 1) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const int rr = row + (e >> 1) * 8, col = 2 * c + (e & 1);
-          if (rr < rows && col < a.T) out[col * pitch + rr] = acc[t][e];
+          const int rr = (t_off + (t << ways)) * 16 + g + (e >> 1) * 8, col = 2 * c + (e & 1);
+          if (rr < rows && col < a.T) out[col * pitch + rr] = acc[i][0][e] + acc[i][1][e];
         }
       }
     }
@@ -818,7 +833,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
     // ------------------------------------------------------------------ the stream
     // One lane, and few instructions a stage: with a page broadcast, a vote and divisions in the loop a stage took
     // 0.45 us to ask for, whatever its size.  A stage's barrier expects its activations too, which come later.
-    if (lane == 0) {
+    if (elect_one()) {
       StackRing at = {0, 0};
       bool ok = true;
       // the next stage's place, once it is free; its barrier expects `bytes`
@@ -917,7 +932,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
     // They go where the consumers find them beside the weights, in the same order and under the same barrier, a bulk
     // copy a stage: loaded by the consumers themselves, into registers and a few stages ahead, each stage cost them a
     // trip to L2 (0.48 us), and 16-byte copies whose 32 lanes each arrive at the barrier took a warp 0.45 us a stage.
-    if (lane == 0) {
+    if (elect_one()) {
       StackRing at = {0, 0};
       int gone = 0, stage = 0, issued = 0;       // issued: as last looked at
       bool ok = true;
