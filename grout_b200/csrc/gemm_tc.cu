@@ -263,7 +263,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   // writes global memory before that wait has returned.
   if (warp == 0) {
     // ---------------------------------------------------------------- producer
-    if (lane == 0) {
+    // (elected, not picked by its number: the compiler then keeps addresses and descriptors in uniform registers, and
+    // this lane's and the MMA lane's instructions are on the path of everything.  A batch of four through a 1B model
+    // with a recurrent state, prompts and 12 decode steps: 22.5 -> 21.9 ms.)
+    if (elect_one()) {
       const long long n_units = (re0 - rb0) + (re1 - rb1);
       // The operand that no kernel writes (the weights) is requested for the first
       // ring of stages before this kernel waits for its producer; the other
@@ -353,7 +356,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issue
-    if (lane == 0) {
+    if (elect_one()) {
       int s = 0;              // stage and round by counting: every instruction of this
       uint32_t round = 0;     // lane is on the path of the products
       bool first = true;

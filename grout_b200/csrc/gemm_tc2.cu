@@ -122,7 +122,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
 
   if (warp == 0) {
     // ------------------------------------------------------------------ loads (both blocks)
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       int s = 0;            // stage and round are kept by counting: this lane's every
       uint32_t round = 0;   // instruction is on the path of the loads
