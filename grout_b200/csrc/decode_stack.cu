@@ -1211,12 +1211,9 @@ GB_EXPORT int gb_decode_stack(StackArgs* a, int P, cudaStream_t s) {
   a->slot_bytes = plan.slot_bytes, a->n_slots = plan.n_slots;
   a->act_at = plan.act_at, a->kb_qkv = plan.kb_qkv, a->kb_o = a->kb_down = plan.kb_o[a->T > DS_FEW];
   const size_t smem = 1024 + (size_t)plan.n_slots * plan.slot_bytes + DS_RED_BYTES + sizeof(StackShared);
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t r = cudaFuncSetAttribute(decode_stack_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DS_SMEM_MOST);
-    if (r != cudaSuccess) return (int)r;
-    configured = true;
-  }
+  // (each launch, which is once a capture: the attribute is a device's)
+  const cudaError_t set = cudaFuncSetAttribute(decode_stack_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DS_SMEM_MOST);
+  if (set != cudaSuccess) return (int)set;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(P);
   cfg.blockDim = dim3(DS_THREADS);

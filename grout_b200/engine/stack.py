@@ -124,14 +124,30 @@ class DecodeStack:
                                 block_table=self.block_table, **self.args)
 
 
+def _weights_of(model) -> tuple:
+    """What a ``DecodeStack`` was made from: where the weights lie and, of the norms, which it copies, which version."""
+    out = []
+    for b in model.blocks:
+        for lin in (getattr(getattr(b, "mixer", None), "qkv", None), getattr(getattr(b, "mixer", None), "o", None),
+                    getattr(getattr(b, "feedforward", None), "gate_up", None),
+                    getattr(getattr(b, "feedforward", None), "down", None)):
+            out.append(lin.weight.data_ptr() if type(lin) is Linear else id(lin))
+        for w in (getattr(getattr(b, "norm1", None), "weight", None), getattr(getattr(b, "norm2", None), "weight", None),
+                  getattr(getattr(b, "mixer", None), "q_norm_w", None), getattr(getattr(b, "mixer", None), "k_norm_w", None)):
+            out.append((w.data_ptr(), w._version) if isinstance(w, torch.Tensor) else id(w))
+    return tuple(out)
+
+
 class StackOf:
-    """A model's ``DecodeStack``, made for the cache that its steps use (and made anew for another)."""
+    """A model's ``DecodeStack``, made for the cache that its steps use, and made anew for another cache or other weights
+    (steps that are replayed from a captured graph do not come here: they read what was there at the capture)."""
 
     def __init__(self):
-        self._cache, self._stack = None, None
+        self._cache, self._made_from, self._stack = None, None, None
 
     def get(self, model, cache) -> Optional[DecodeStack]:
-        if self._cache is None or self._cache() is not cache:
+        made_from = _weights_of(model)
+        if self._cache is None or self._cache() is not cache or made_from != self._made_from:
             self._stack = DecodeStack.of(model, cache)
-            self._cache = weakref.ref(cache)
+            self._cache, self._made_from = weakref.ref(cache), made_from
         return self._stack

@@ -86,6 +86,39 @@ def test_same_bits_every_time(engines):
     assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("n", [3, 5, 7])
+def test_launched_one_by_one_with_any_number_of_rows(engines, n):
+    """Without graphs no rows fill a step up to a power of two; sums over the keys may be divided otherwise."""
+    _d, eng = engines("group8")
+    lens = [33, 64, 129, 5, 700, 64, 1][:n]
+    _t, ref = played(eng, lens, 2, 31)
+    eng.use_graphs = False
+    try:
+        _t, got = played(eng, lens, 2, 31)
+    finally:
+        eng.use_graphs = True
+    err = float((got.double() - ref.double()).norm() / ref.double().norm())
+    assert err < 0.02, err
+
+
+def test_other_weights_are_seen(engines):
+    """A norm's weight that changes, and a weight that is replaced, reach steps that are launched one by one."""
+    _d, eng = engines("group2")
+    eng.use_graphs = False
+    norm = eng.model.blocks[0].norm2.weight
+    before = norm.clone()
+    try:
+        _t, a = played(eng, [40], 1, 41)
+        norm.mul_(0.5)
+        _t, b = played(eng, [40], 1, 41)
+        norm.copy_(before)
+        _t, c = played(eng, [40], 1, 41)
+    finally:
+        norm.copy_(before)
+        eng.use_graphs = True
+    assert torch.equal(a, c) and not torch.equal(a, b)
+
+
 def test_more_rows_than_the_kernel_takes_go_layer_by_layer(engines):
     from grout_b200.engine.batch import make_context
     _d, eng = engines("group2")
