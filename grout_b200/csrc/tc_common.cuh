@@ -72,8 +72,9 @@ __device__ __forceinline__ unsigned long long now_ns() {
 // or (where a flag is given) another role of the block has already given up.
 // The loop is one copy of the poll (left to itself the compiler unrolls it, a few KB of
 // instructions at each of a kernel's dozen waits, and a role that waits then runs through
-// instructions that are in no cache: one user's request at the 4B sizes, 36 steps, 84.0 ms
-// with the polls written out, 80.5 with one; a prompt of 2,048 tokens 15.9 and 15.5).
+// instructions that are in no cache: one user's request at the 4B sizes, 36 steps kernel by
+// kernel, 84.0 ms with the polls written out, 80.5 with one; a prompt of 2,048 tokens no
+// different beyond what two runs differ by).
 __device__ __forceinline__ bool mbar_wait(void* bar, uint32_t parity, volatile int* abort_flag,
                                           unsigned long long limit_ns = TC_WAIT_LIMIT_NS) {
   if (mbar_try(bar, parity)) return true;

@@ -146,6 +146,8 @@ class StackOf:
         self._cache, self._made_from, self._stack = None, None, None
 
     def get(self, model, cache) -> Optional[DecodeStack]:
+        if model.ctx.dtype != torch.bfloat16 or not model.blocks or type(model.blocks[0]) is not PreNormBlock:
+            return None                  # (nothing to look up in every step of another kind of model)
         made_from = _weights_of(model)
         if self._cache is None or self._cache() is not cache or made_from != self._made_from:
             self._stack = DecodeStack.of(model, cache)
