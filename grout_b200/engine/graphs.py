@@ -94,6 +94,7 @@ class StepGraph:
             self.views.append({name: flat[o:o + cnt] for name, (o, cnt) in self.off.items()})
         self.dev = torch.zeros(total, dtype=torch.int32, device=device)
         self.graph = None
+        self.holds = None
         self.logits = None
         self.kernels_per_replay = 0
 
@@ -113,8 +114,14 @@ class StepGraph:
     def _fill_padding(self) -> None:
         raise NotImplementedError
 
+    def _hold(self) -> None:
+        """Keeps what the captured kernels read and write at every replay and what the model may replace meanwhile.
+        Asked for on the stream that steps run on: memory that is made here is given back in that stream's order."""
+        self.holds = self.model.decode_stack(self.cache) if self.decode else None
+
     def _capture(self) -> None:
         """Warm-up with padding rows only (which store nothing), then capture."""
+        self._hold()
         self._fill_padding()
         meta = dict(n_tokens=self.n_tokens, n_seqs=self.n_seqs, n_want=self.n_want, off=self.off,
                     q_lens=(), starts=(), slot_list=(), decode=self.decode,

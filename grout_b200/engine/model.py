@@ -115,6 +115,11 @@ class Model:
                    for p in _walk(top))
 
     # -- forward -----------------------------------------------------------
+    def decode_stack(self, cache: SequenceCache):
+        """What runs a decode step's layers over this cache as one kernel (None: layer by layer).  A captured step
+        reads its memory at every replay, so whoever keeps the graph keeps this too."""
+        return self._stack.get(self, cache)
+
     def forward(self, step: StepContext, cache: SequenceCache) -> Optional[torch.Tensor]:
         """Runs the step's tokens through every scheduled layer; returns 32-bit
         logits [n_want, vocab] at ``step.want_rows`` (None when nothing is wanted)."""
@@ -135,7 +140,7 @@ class Model:
         res = None
         if self.embedding.starts_stream:      # the embedding is the 32-bit stream already
             res, pending = pending, None
-        stack = self._stack.get(self, cache) if step.decode else None
+        stack = self.decode_stack(cache) if step.decode else None
         entries = self.plan.schedule
         if stack is not None and stack.takes(step):
             res, pending, entries = stack.forward(res, pending, step), None, ()
