@@ -71,13 +71,15 @@ struct StackLayer {
   CUtensorMap k, v;
 };
 // What else a layer has, as 32-bit words in one row: the two norms' weights [hidden], those of q and k [128] (ones where
-// the heads have no norms), the addresses of its pages of keys and of values [2 each].
-__host__ __device__ __forceinline__ int stack_row_words(int hidden) { return 2 * hidden + 256 + 4; }
+// the heads have no norms), the addresses of its pages of keys and of values, the addresses of the four norms' own
+// tensors [2 words each], and of these whether they are bfloat16.  Every launch fills in the weights from there.
+__host__ __device__ __forceinline__ int stack_row_norms(int hidden) { return 2 * hidden + 256 + 4; }
+__host__ __device__ __forceinline__ int stack_row_words(int hidden) { return stack_row_norms(hidden) + 8 + 4; }
 static_assert(sizeof(StackLayer) % 64 == 0, "tensor maps are 64-byte aligned");
 
 struct StackArgs {
   const StackLayer* layers;
-  const float* rows;                         // [n_layers][stack_row_words]
+  float* rows;                               // [n_layers][stack_row_words]
   int n_layers, T, hidden, ff, nq, nkv;      // T: activation rows = sequences, head size 128
   int slot_bytes, n_slots, act_at;           // the ring, where a slot's activations begin
   int kb_qkv, kb_o, kb_down;                 // 64-column blocks of a stage
@@ -756,6 +758,44 @@ struct StackConsumer {
   }
 };
 
+// The norms' weights as they are at this launch, into the layers' rows: the weights of the block's columns, which nobody
+// else reads, and those of q and k of every P-th layer, which others read behind a grid barrier.  (Read where they are
+// used, through their address, each would be two trips in front of a phase; here they are behind the plan of the
+// attention's units, which one thread makes.)
+__device__ __forceinline__ void stack_norms(const StackArgs& a, int warp, int warps, int lane, int c0, int c_rows, int p, int P) {
+  const int words = stack_row_words(a.hidden), at = stack_row_norms(a.hidden);
+  auto weight = [&](const float* row, int which, int i) -> float {
+    const void* src = *reinterpret_cast<const void* const*>(row + at + 2 * which);
+    return reinterpret_cast<const int*>(row + at + 8)[which] ? __bfloat162float(static_cast<const bf16*>(src)[i])
+                                                             : static_cast<const float*>(src)[i];
+  };
+  if (lane < c_rows) {
+    const int n = 2 * a.n_layers;
+#pragma unroll 1
+    for (int i0 = warp; i0 < n; i0 += 6 * warps) {
+      float v[6];
+#pragma unroll
+      for (int j = 0; j < 6; ++j) {                // (loads that do not wait for one another)
+        const int i = min(i0 + j * warps, n - 1);
+        v[j] = weight(a.rows + (size_t)(i >> 1) * words, i & 1, c0 + lane);
+      }
+#pragma unroll
+      for (int j = 0; j < 6; ++j) {
+        const int i = i0 + j * warps;
+        if (i < n) a.rows[(size_t)(i >> 1) * words + (i & 1) * a.hidden + c0 + lane] = v[j];
+      }
+    }
+  }
+  if (a.qk_norm) {
+#pragma unroll 1
+    for (int layer = p; layer < a.n_layers; layer += P)
+      for (int i = warp * 32 + lane; i < 256; i += warps * 32) {
+        float* row = a.rows + (size_t)layer * words;
+        row[2 * a.hidden + i] = weight(row, 2 + (i >> 7), i & 127);
+      }
+  }
+}
+
 #define DS_STAMP(i)                                                                                         \
   do {                                                                                                      \
     if (a.stamps && tid == 0 && layer == a.n_layers - 2) a.stamps[(size_t)blockIdx.x * 16 + (i)] = now_ns(); \
@@ -781,7 +821,13 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
   }
   if (tid < a.T) sh.tiles[tid] = a.slots[tid] < 0 ? 0 : (a.kv_len[tid] + 63) / 64;
   __syncthreads();
+  // rows of the products that are this block's
+  const int q0 = stack_first_row(N, p, P), q_rows = stack_first_row(N, p + 1, P) - q0;
+  const int c0 = stack_first_row(a.hidden, p, P), c_rows = stack_first_row(a.hidden, p + 1, P) - c0;
+  const StackShare share = stack_share(a.ff / 8, p, P);
+  const int gu_rows = share.whole * 16 + (share.half >= 0 ? 8 : 0);
   const int unit_tiles = stack_unit_tiles(sh.tiles, a.T, a.nkv, P);
+  if (warp > 0) stack_norms(a, warp - 1, DS_THREADS / 32 - 1, lane, c0, c_rows, p, P);
   if (tid == 0) {
     int n = 0, first = 0, any = 0;
     for (int t = 0; t < a.T; ++t) {
@@ -819,11 +865,6 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
   }
   __syncthreads();
 
-  // rows of the products that are this block's
-  const int q0 = stack_first_row(N, p, P), q_rows = stack_first_row(N, p + 1, P) - q0;
-  const int c0 = stack_first_row(a.hidden, p, P), c_rows = stack_first_row(a.hidden, p + 1, P) - c0;
-  const StackShare share = stack_share(a.ff / 8, p, P);
-  const int gu_rows = share.whole * 16 + (share.half >= 0 ? 8 : 0);
   // The phases in turn, one copy of the code of each: what all warps run through again and again must stay in the
   // instruction caches (as 300 KB, with products, barriers and polls written out, fetching it took most of the time:
   // 3,240 us a step of one row at the 4B sizes).

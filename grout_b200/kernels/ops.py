@@ -1838,8 +1838,8 @@ def decode_stack_takes(hidden: int, ff: int, nq: int, nkv: int, device) -> bool:
 
 def decode_stack_state(layers, hidden: int, ff: int, nq: int, nkv: int, max_rows: int, device) -> dict:
     """What launches over these layers share: their table on the device and scratch for ``max_rows`` rows.
-    ``layers``: dicts of the weights (bf16: qkv, o, gate_up, down), pages and norm weights of each.  Weights and pages
-    must outlive the state; launches that use it must be ordered on one stream."""
+    ``layers``: dicts of the weights (bf16: qkv, o, gate_up, down), pages and norm weights of each (32-bit or bf16), all
+    of which launches read where they lie: they must outlive the state.  Launches that use it must be ordered on one stream."""
     P = _sm_count(device)
     size = _fn("decode_stack", "gb_decode_stack_layer_bytes", "iiiii")(hidden, ff, nq, nkv, P)
     if size <= 0:
@@ -1848,7 +1848,8 @@ def decode_stack_state(layers, hidden: int, ff: int, nq: int, nkv: int, max_rows
     skip = -host.data_ptr() % 64                 # tensor maps lie on 64 bytes
     encode = _fn("decode_stack", "gb_decode_stack_encode", "piiiiippppppl")
     words = _fn("decode_stack", "gb_decode_stack_row_words", "i")(hidden)
-    rows = torch.ones((len(layers), words), dtype=torch.float32, device=device)   # a layer's norms, and where its pages are
+    # a layer's row: its norms' weights, which launches fill in, and where its pages and its norms are
+    rows = torch.ones((len(layers), words), dtype=torch.float32)
     normed = layers[0]["q_norm"] is not None
     for i, t in enumerate(layers):
         for n, shape in (("qkv", ((nq + 2 * nkv) * 128, hidden)), ("o", (hidden, nq * 128)),
@@ -1860,17 +1861,19 @@ def decode_stack_state(layers, hidden: int, ff: int, nq: int, nkv: int, max_rows
             _need(t[n], n, torch.bfloat16, 4)
             if tuple(t[n].shape[1:]) != (nkv, 64, 128) or t[n].shape != t["k_pages"].shape:
                 raise KernelError(f"{n} are {tuple(t[n].shape)}, expected [*, {nkv}, 64, 128]")
+        where, narrow = [t["k_pages"].data_ptr(), t["v_pages"].data_ptr()], []
         for n, width in (("norm1", hidden), ("norm2", hidden), ("q_norm", 128), ("k_norm", 128)):
             if normed or n in ("norm1", "norm2"):
                 _need(t[n], n, ndim=1)
-                if t[n].shape[0] != width:
-                    raise KernelError(f"{n} has {t[n].shape[0]} elements, expected {width}")
-                at = {"norm1": 0, "norm2": hidden, "q_norm": 2 * hidden, "k_norm": 2 * hidden + 128}[n]
-                rows[i, at:at + width] = t[n].float()
+                if t[n].shape[0] != width or t[n].dtype not in (torch.float32, torch.bfloat16):
+                    raise KernelError(f"{n} is {t[n].dtype} of {t[n].shape[0]} elements, expected {width} in 32-bit or bfloat16")
+                where.append(t[n].data_ptr())
+                narrow.append(int(t[n].dtype == torch.bfloat16))
             elif t[n] is not None:
                 raise KernelError("either all layers have norms of q and k or none has")
-        where = torch.tensor([t["k_pages"].data_ptr(), t["v_pages"].data_ptr()], dtype=torch.int64)
-        rows.view(torch.int32)[i, words - 4:] = where.view(torch.int32).to(device)
+        bits = rows.view(torch.int32)[i, 2 * hidden + 256:]
+        bits[:2 * len(where)] = torch.tensor(where, dtype=torch.int64).view(torch.int32)
+        bits[12:12 + len(narrow)] = torch.tensor(narrow, dtype=torch.int32)
         _check(encode(host.data_ptr() + skip + i * size, hidden, ff, nq, nkv, P, t["qkv"].data_ptr(), t["o"].data_ptr(),
                       t["gate_up"].data_ptr(), t["down"].data_ptr(), t["k_pages"].data_ptr(), t["v_pages"].data_ptr(),
                       t["k_pages"].shape[0]),
@@ -1879,7 +1882,7 @@ def decode_stack_state(layers, hidden: int, ff: int, nq: int, nkv: int, max_rows
     b16 = lambda n: torch.zeros(n, dtype=torch.bfloat16, device=device)
     T, splits = max_rows, 32
     return dict(sizes=(len(layers), hidden, ff, nq, nkv), rows=T, blocks=P,
-                layers=host[skip:skip + size * len(layers)].to(device), table=rows, qk_norm=int(normed),
+                layers=host[skip:skip + size * len(layers)].to(device), table=rows.to(device), qk_norm=int(normed),
                 xb=b16(T * hidden), ab=b16(T * nq * 128), hb=b16(T * ff), ss=f32(T * P), qkv=f32(T * (nq + 2 * nkv) * 128),
                 part_o=f32(T * nq * splits * 128), part_ml=f32(T * nq * splits * 2),
                 sync=torch.zeros(2, dtype=torch.int32, device=device))

@@ -133,3 +133,68 @@ def test_other_layers_go_layer_by_layer(change):
     from grout_b200.engine import Engine
     eng = Engine.random(dict(config(256, 1216, 4, 2), **change), 0, max_tokens=512, max_batch=2, max_seq_len=256)
     assert eng.model._stack.get(eng.model, eng.cache) is None
+
+
+def test_a_replayed_step_sees_norms_that_were_changed_in_place(engines):
+    """As the kernels of each layer do: the norms' weights are read where they lie, by captured steps too, also when a
+    step that was launched by itself came between."""
+    from safetensors import safe_open
+    d, eng = engines("group2")
+    with safe_open(f"{d}/model.safetensors", "pt") as f:
+        w = {k: f.get_tensor(k) for k in f.keys()}
+    block = eng.model.blocks[1]
+    norms = {"model.layers.1.input_layernorm.weight": block.norm1.weight,
+             "model.layers.1.post_attention_layernorm.weight": block.norm2.weight,
+             "model.layers.1.self_attn.q_norm.weight": block.mixer.q_norm_w,
+             "model.layers.1.self_attn.k_norm.weight": block.mixer.k_norm_w}
+    before = {k: t.clone() for k, t in norms.items()}
+
+    def compare(what):
+        toks, got = played(eng, [100], 2, 51)
+        assert_close(got[0], plain.logits(w, MODELS["group2"], toks[0], rows=[100, 101]), "bfloat16", what)
+        return got
+
+    a = compare("captured")
+    try:
+        for k, t in norms.items():          # every second channel: a common factor would be normalised away again
+            t[::2] *= 1.5
+            w[k] = t.cpu()
+        b = compare("replayed")
+        eng.use_graphs = False
+        compare("launched by itself")
+        eng.use_graphs = True
+        c = compare("replayed again")
+    finally:
+        eng.use_graphs = True
+        for k, t in norms.items():
+            t.copy_(before[k])
+    assert torch.equal(b, c) and not torch.equal(a, b) and torch.equal(a, played(eng, [100], 2, 51)[1])
+
+
+def test_norms_in_32_bit(engines):
+    """bfloat16 weights beside norms that are kept in 32-bit give the same bits as the same norms in bfloat16."""
+    _d, eng = engines("group1")
+    parts = [n for b in eng.model.blocks for n in (b.norm1, b.norm2)]
+    mixers = [b.mixer for b in eng.model.blocks]
+    kept = [p.weight for p in parts], [(m.q_norm_w, m.k_norm_w) for m in mixers]
+    out = []
+    eng.use_graphs = False
+    try:
+        for wide in (False, True):
+            slot = eng.open_sequence()
+            eng.step([(slot, list(range(70)))], [[]])
+            if wide:
+                for p in parts:
+                    p.weight = p.weight.float()
+                for m in mixers:
+                    m.q_norm_w, m.k_norm_w = m.q_norm_w.float(), m.k_norm_w.float()
+            out.append(eng.step([(slot, [5])], [[0]]))
+            eng.close_sequence(slot)
+        eng.check()
+    finally:
+        eng.use_graphs = True
+        for p, t in zip(parts, kept[0]):
+            p.weight = t
+        for m, (q, k) in zip(mixers, kept[1]):
+            m.q_norm_w, m.k_norm_w = q, k
+    assert torch.equal(*out)
