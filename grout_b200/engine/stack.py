@@ -125,7 +125,7 @@ class DecodeStack:
 
 
 def _weights_of(model) -> tuple:
-    """What a ``DecodeStack`` was made from: where the weights lie and, of the norms, which it copies, which version."""
+    """What a ``DecodeStack`` was made from: where the weights lie, which the kernel reads there at every launch."""
     out = []
     for b in model.blocks:
         for lin in (getattr(getattr(b, "mixer", None), "qkv", None), getattr(getattr(b, "mixer", None), "o", None),
@@ -134,7 +134,7 @@ def _weights_of(model) -> tuple:
             out.append(lin.weight.data_ptr() if type(lin) is Linear else id(lin))
         for w in (getattr(getattr(b, "norm1", None), "weight", None), getattr(getattr(b, "norm2", None), "weight", None),
                   getattr(getattr(b, "mixer", None), "q_norm_w", None), getattr(getattr(b, "mixer", None), "k_norm_w", None)):
-            out.append((w.data_ptr(), w._version) if isinstance(w, torch.Tensor) else id(w))
+            out.append((w.data_ptr(), w.dtype) if isinstance(w, torch.Tensor) else id(w))
     return tuple(out)
 
 

@@ -61,3 +61,11 @@ def test_a_captured_step_keeps_what_it_was_captured_with(model):
     del g
     gc.collect()
     assert seen() is None
+
+
+def test_weights_made_in_inference_mode(model):
+    """They have no version counter; a model that the kernel does not take is asked about like any other."""
+    with torch.inference_mode():
+        for config in (CONFIG, dict(CONFIG, head_dim=64)):
+            m, cache = load(config), Cache()
+            assert isinstance(m.decode_stack(cache), Made) and m.decode_stack(cache) is m.decode_stack(cache)

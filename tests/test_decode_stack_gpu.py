@@ -198,3 +198,18 @@ def test_norms_in_32_bit(engines):
         for m, (q, k) in zip(mixers, kept[1]):
             m.q_norm_w, m.k_norm_w = q, k
     assert torch.equal(*out)
+
+
+@pytest.mark.parametrize("graphs", [True, False])
+def test_an_engine_made_in_inference_mode(engines, graphs):
+    from grout_b200.engine import Engine
+    d, eng = engines("group2")
+    eng.use_graphs = graphs
+    try:
+        _t, want = played(eng, [70, 3], 2, 71)
+        with torch.inference_mode():
+            own = Engine.load(d, dtype="bfloat16", max_tokens=8192, max_batch=9, max_seq_len=2048, use_graphs=graphs)
+            _t, got = played(own, [70, 3], 2, 71)
+    finally:
+        eng.use_graphs = True
+    assert torch.equal(got, want)
