@@ -70,16 +70,19 @@ struct StackLayer {
   CUtensorMap half;                // half a group of eight gates and their ups: 4 + 4 rows
   CUtensorMap k, v;
 };
-// What else a layer has, as 32-bit words in one row: the two norms' weights [hidden], those of q and k [128] (ones where
-// the heads have no norms), the addresses of its pages of keys and of values, the addresses of the four norms' own
-// tensors [2 words each], and of these whether they are bfloat16.  Every launch fills in the weights from there.
-__host__ __device__ __forceinline__ int stack_row_norms(int hidden) { return 2 * hidden + 256 + 4; }
-__host__ __device__ __forceinline__ int stack_row_words(int hidden) { return stack_row_norms(hidden) + 8 + 4; }
+// What else a layer has: its pages and the weights of its norms (in front of qkv and of gate|up, of q and of k) where
+// they lie, and whether these are bfloat16 or 32-bit.  Both are read from there by every launch.
+struct StackRow {
+  bf16* pages[2];
+  const void* norm[4];
+  int narrow[4];
+};
+static_assert(sizeof(StackRow) == 64, "copied in four pieces");
 static_assert(sizeof(StackLayer) % 64 == 0, "tensor maps are 64-byte aligned");
 
 struct StackArgs {
   const StackLayer* layers;
-  float* rows;                               // [n_layers][stack_row_words]
+  const StackRow* rows;                      // [n_layers]
   int n_layers, T, hidden, ff, nq, nkv;      // T: activation rows = sequences, head size 128
   int slot_bytes, n_slots, act_at;           // the ring, where a slot's activations begin
   int kb_qkv, kb_o, kb_down;                 // 64-column blocks of a stage
@@ -231,9 +234,9 @@ struct StackShared {
   float2 turn[DS_UNITS_MOST][64];        // cosine and sine of a unit's new position
   float rstd[DS_ROWS];
   float ss[DS_ROWS * DS_BLOCKS_MOST];    // the blocks' sums of squares, on their way while a product runs
-  float norm[DS_ROWS * 32];              // the weights of the norm behind o or down, a copy a row
-  float qk_w[256];                       // the layer's norms of q and k ...
-  bf16* kv_pages[2];                     // ... and its pages
+  uint32_t norm[DS_ROWS * 32];           // the weights of the norm behind o or down as they lie in memory, a copy a row
+  uint32_t qk_w[256];                    // those of the layer's norms of q and k, 128 words each
+  StackRow rows[2];                      // of the layers with even and odd numbers
   float red_m[DS_WARPS * 8], red_l[DS_WARPS * 8];
   StackUnit units[DS_UNITS_MOST];
   int n_units, split_any;
@@ -243,7 +246,7 @@ struct StackShared {
 };
 
 static_assert(offsetof(StackShared, turn) % 16 == 0 && offsetof(StackShared, qk_w) % 16 == 0 &&
-                  offsetof(StackShared, kv_pages) % 16 == 0,
+                  offsetof(StackShared, rows) % 16 == 0,
               "copied or read by 16 bytes");
 
 // A place in the order of stages, which is the same for the warps that fill the ring and for
@@ -280,7 +283,7 @@ struct StackConsumer {
   uint8_t* ring;
   float* red;
   StackRing at;                // the first stage of the phase
-  int tid, warp, lane, p, P, c_rows;
+  int tid, warp, lane, p, P, c0, c_rows;
   bool bad;
   int gone;
   unsigned arrived;            // arrivals the grid barrier has had when all have come
@@ -344,24 +347,43 @@ struct StackConsumer {
   // What the phase needs behind its product, asked for in front of it: read where it is used, each cost a trip to
   // L2 or, the weights between one step and the next having been through it, to memory.
   // In front of a product of normalised rows the blocks' sums of squares (a warp a row), of qkv the attention's vectors
-  // too; else `norm`, the weights of the next norm.
-  __device__ __forceinline__ void ask(const float* row, const float* norm, bool normed, bool qkv) {
+  // and where the next layer's lie too; else the weights of the next norm, `which` of `row`.
+  __device__ __forceinline__ void ask(int layer, const StackRow& row, int which, bool normed, bool qkv) {
     if (warp < a.T) {
       if (normed) {
         for (int i = lane; i < P; i += 32)
           asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(sh.ss + warp * DS_BLOCKS_MOST + i)),
                        "l"(a.ss + warp * P + i)
                        : "memory");
-      } else if (lane < c_rows) {
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(sh.norm + warp * 32 + lane)), "l"(norm + lane)
-                     : "memory");
+      } else {
+        // (the words in which the block's columns lie, two columns a word where they are bfloat16)
+        const int narrow = row.narrow[which], word0 = c0 >> narrow, words = ((c0 + c_rows - 1) >> narrow) - word0 + 1;
+        if (lane < words)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(sh.norm + warp * 32 + lane)),
+                       "l"(static_cast<const uint32_t*>(row.norm[which]) + word0 + lane)
+                       : "memory");
       }
     } else if (qkv && warp >= DS_ROWS) {
-      const int i = (warp - DS_ROWS) * 32 + lane;
-      if (i < 65)
-        cp_async16(i < 64 ? (void*)(sh.qk_w + i * 4) : (void*)sh.kv_pages, row + 2 * a.hidden + i * 4, true);
+      const int j = warp - DS_ROWS;                // q's, k's, the next layer's
+      if (j < 2) {
+        if (a.qk_norm && lane < (row.narrow[2 + j] ? 16 : 32))
+          cp_async16(sh.qk_w + j * 128 + lane * 4, static_cast<const uint32_t*>(row.norm[2 + j]) + lane * 4, true);
+      } else if (j == 2 && lane < 4 && layer + 1 < a.n_layers) {
+        cp_async16(reinterpret_cast<uint4*>(&sh.rows[(layer + 1) & 1]) + lane,
+                   reinterpret_cast<const uint4*>(a.rows + layer + 1) + lane, true);
+      }
     }
     cp_async_commit();
+  }
+  // Element i of weights that begin with the word at `w`.
+  __device__ __forceinline__ static float widened(const uint32_t* w, int i, int narrow) {
+    if (!narrow) return __uint_as_float(w[i]);
+    return __uint_as_float((i & 1) ? w[i >> 1] & 0xffff0000u : w[i >> 1] << 16);
+  }
+  // Elements 2 i and 2 i + 1.
+  __device__ __forceinline__ static float2 widened2(const uint32_t* w, int i, int narrow) {
+    if (!narrow) return reinterpret_cast<const float2*>(w)[i];
+    return make_float2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
   }
   // 1 / rms of the rows
   __device__ __forceinline__ void row_factors() {
@@ -491,7 +513,7 @@ struct StackConsumer {
   }
 
   // ---- attention -----------------------------------------------------------------------------
-  __device__ __forceinline__ void attention() {
+  __device__ __forceinline__ void attention(const StackRow& row) {
     const int G = a.nq / a.nkv, N = (a.nq + 2 * a.nkv) * 128;
     const int g = lane >> 2, c = lane & 3;
     bf16* q_s = reinterpret_cast<bf16*>(red);              // [8][DS_QLD]
@@ -513,10 +535,11 @@ struct StackConsumer {
         const float2 hi = __ldcg(reinterpret_cast<const float2*>(src + 64) + lane);
         float x0 = lo.x, x1 = lo.y, y0 = hi.x, y1 = hi.y;
         if (a.qk_norm && !is_v) {
-          const float2* w = reinterpret_cast<const float2*>(sh.qk_w + (warp < G ? 0 : 128));
+          const uint32_t* w = sh.qk_w + (warp < G ? 0 : 128);
+          const int narrow = row.narrow[warp < G ? 2 : 3];
           const float ssq = warp_sum(x0 * x0 + x1 * x1 + y0 * y0 + y1 * y1);
           const float f = rsqrtf(ssq / 128.f + a.qk_eps);
-          const float2 wl = w[lane], wh = w[32 + lane];
+          const float2 wl = widened2(w, lane, narrow), wh = widened2(w, 32 + lane, narrow);
           x0 = x0 * f * wl.x, x1 = x1 * f * wl.y, y0 = y0 * f * wh.x, y1 = y1 * f * wh.y;
         }
         if (a.inv_freq && !is_v) {
@@ -530,7 +553,7 @@ struct StackConsumer {
         reinterpret_cast<uint32_t*>(dst)[lane] = p0;
         reinterpret_cast<uint32_t*>(dst + 64)[lane] = p1;
         if (warp >= G) {
-          bf16* page = sh.kv_pages[is_v] + (((size_t)u.page * a.nkv + u.kvh) * 64 + (pos & 63)) * 128;
+          bf16* page = row.pages[is_v] + (((size_t)u.page * a.nkv + u.kvh) * 64 + (pos & 63)) * 128;
           reinterpret_cast<uint32_t*>(page)[lane] = p0;
           reinterpret_cast<uint32_t*>(page + 64)[lane] = p1;
         }
@@ -758,44 +781,6 @@ struct StackConsumer {
   }
 };
 
-// The norms' weights as they are at this launch, into the layers' rows: the weights of the block's columns, which nobody
-// else reads, and those of q and k of every P-th layer, which others read behind a grid barrier.  (Read where they are
-// used, through their address, each would be two trips in front of a phase; here they are behind the plan of the
-// attention's units, which one thread makes.)
-__device__ __forceinline__ void stack_norms(const StackArgs& a, int warp, int warps, int lane, int c0, int c_rows, int p, int P) {
-  const int words = stack_row_words(a.hidden), at = stack_row_norms(a.hidden);
-  auto weight = [&](const float* row, int which, int i) -> float {
-    const void* src = *reinterpret_cast<const void* const*>(row + at + 2 * which);
-    return reinterpret_cast<const int*>(row + at + 8)[which] ? __bfloat162float(static_cast<const bf16*>(src)[i])
-                                                             : static_cast<const float*>(src)[i];
-  };
-  if (lane < c_rows) {
-    const int n = 2 * a.n_layers;
-#pragma unroll 1
-    for (int i0 = warp; i0 < n; i0 += 6 * warps) {
-      float v[6];
-#pragma unroll
-      for (int j = 0; j < 6; ++j) {                // (loads that do not wait for one another)
-        const int i = min(i0 + j * warps, n - 1);
-        v[j] = weight(a.rows + (size_t)(i >> 1) * words, i & 1, c0 + lane);
-      }
-#pragma unroll
-      for (int j = 0; j < 6; ++j) {
-        const int i = i0 + j * warps;
-        if (i < n) a.rows[(size_t)(i >> 1) * words + (i & 1) * a.hidden + c0 + lane] = v[j];
-      }
-    }
-  }
-  if (a.qk_norm) {
-#pragma unroll 1
-    for (int layer = p; layer < a.n_layers; layer += P)
-      for (int i = warp * 32 + lane; i < 256; i += warps * 32) {
-        float* row = a.rows + (size_t)layer * words;
-        row[2 * a.hidden + i] = weight(row, 2 + (i >> 7), i & 127);
-      }
-  }
-}
-
 #define DS_STAMP(i)                                                                                         \
   do {                                                                                                      \
     if (a.stamps && tid == 0 && layer == a.n_layers - 2) a.stamps[(size_t)blockIdx.x * 16 + (i)] = now_ns(); \
@@ -819,6 +804,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
     sh.issued = sh.go = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (warp == 1 && lane < 4) reinterpret_cast<uint4*>(&sh.rows[0])[lane] = reinterpret_cast<const uint4*>(a.rows)[lane];
   if (tid < a.T) sh.tiles[tid] = a.slots[tid] < 0 ? 0 : (a.kv_len[tid] + 63) / 64;
   __syncthreads();
   // rows of the products that are this block's
@@ -827,7 +813,6 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
   const StackShare share = stack_share(a.ff / 8, p, P);
   const int gu_rows = share.whole * 16 + (share.half >= 0 ? 8 : 0);
   const int unit_tiles = stack_unit_tiles(sh.tiles, a.T, a.nkv, P);
-  if (warp > 0) stack_norms(a, warp - 1, DS_THREADS / 32 - 1, lane, c0, c_rows, p, P);
   if (tid == 0) {
     int n = 0, first = 0, any = 0;
     for (int t = 0; t < a.T; ++t) {
@@ -1027,14 +1012,17 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
     __syncwarp();
   } else {
     // ------------------------------------------------------------------ the work
-    StackConsumer w = {a, sh, ring, red, {0, 0}, tid, warp, lane, p, P, c_rows, false, 0, 0u};
+    StackConsumer w = {a, sh, ring, red, {0, 0}, tid, warp, lane, p, P, c0, c_rows, false, 0, 0u};
     // the block's columns of the stream: a warp a row of the batch, a lane a column
     float x = 0.f;
     if (warp < a.T) {
       if (lane < c_rows) {
         const size_t i = (size_t)warp * a.hidden + c0 + lane;
         x = a.res_in ? a.res_in[i] : __bfloat162float(a.x_in[i]);
-        a.xb[stack_fragment(c0 + lane, warp, a.T)] = __float2bfloat16(x * a.rows[c0 + lane]);
+        const StackRow& row = sh.rows[0];
+        const float weight = row.narrow[0] ? __bfloat162float(static_cast<const bf16*>(row.norm[0])[c0 + lane])
+                                           : static_cast<const float*>(row.norm[0])[c0 + lane];
+        a.xb[stack_fragment(c0 + lane, warp, a.T)] = __float2bfloat16(x * weight);
       }
       w.publish(warp, x * x);
       ds_fence_async();
@@ -1049,7 +1037,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
       if (phase == MERGE && !sh.split_any) ++phase;
       DS_STAMP(phase * 2);
       if (phase == ATTENTION) {
-        w.attention();
+        w.attention(sh.rows[layer & 1]);
         DS_STAMP(phase * 2 + 1);
       } else if (phase == MERGE) {
         w.merge(unit_tiles);
@@ -1058,10 +1046,11 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
         const bool normed = phase == QKV || phase == GATE_UP;
         const int rows = phase == QKV ? q_rows : (phase == GATE_UP ? gu_rows : c_rows);
         const bool last = phase == DOWN && layer + 1 == a.n_layers;
-        const float* row = a.rows + (size_t)layer * stack_row_words(a.hidden);
+        // whose norm comes behind the product (behind the last layer none of the stack's: its weights are read and not used)
+        const int which = phase == O ? 1 : 0;
+        const StackRow& row = sh.rows[(phase == DOWN && !last ? layer + 1 : layer) & 1];
         w.go();
-        // (behind the last layer comes no norm of the stack's: its factors are read and not used)
-        w.ask(row, (phase == O ? row + a.hidden : (last ? row : row + stack_row_words(a.hidden))) + c0, normed, phase == QKV);
+        w.ask(layer, row, which, normed, phase == QKV);
         int pitch;
         const int parts = w.product(normed ? a.hidden : (phase == O ? a.nq * 128 : a.ff), rows,
                                     phase == QKV ? a.kb_qkv : (phase == O ? a.kb_o : (phase == DOWN ? a.kb_down : 1)), pitch);
@@ -1073,7 +1062,8 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
         if (!normed) {
           if (warp < a.T) {
             if (lane < c_rows) {
-              const float weight = sh.norm[warp * 32 + lane];
+              const int narrow = row.narrow[which];
+              const float weight = w.widened(sh.norm + warp * 32, narrow ? lane + (c0 & 1) : lane, narrow);
               x += w.summed(red + warp * pitch + lane, parts, stride);
               a.xb[stack_fragment(c0 + lane, warp, a.T)] = __float2bfloat16(x * weight);
               if (last) a.x_out[(size_t)warp * a.hidden + c0 + lane] = x;
@@ -1202,8 +1192,6 @@ GB_EXPORT int gb_decode_stack_share(int hidden, int ff, int nq, int nkv, int P, 
   return 0;
 }
 GB_EXPORT int gb_decode_stack_fragment(int k, int t, int T) { return stack_fragment(k, t, T); }
-
-GB_EXPORT int gb_decode_stack_row_words(int hidden) { return stack_row_words(hidden); }
 
 // Writes a layer's entry (its tensor maps) to host memory.
 GB_EXPORT int gb_decode_stack_encode(void* entry, int hidden, int ff, int nq, int nkv, int P, const void* w_qkv,

@@ -29,8 +29,14 @@ def _plain_linear(lin, out_features: int, in_features: int) -> bool:
             and lin.weight.data_ptr() % 16 == 0)
 
 
+def _plain_weights(w, width: int) -> bool:
+    """A norm's weights as the kernel reads them: in pieces of 16 bytes, 32-bit or bfloat16."""
+    return (isinstance(w, torch.Tensor) and tuple(w.shape) == (width,) and w.dtype in (torch.float32, torch.bfloat16)
+            and w.is_contiguous() and w.data_ptr() % 16 == 0)
+
+
 def _plain_norm(norm, width: int) -> bool:
-    return type(norm) is RMSNorm and norm.weight is not None and tuple(norm.weight.shape) == (width,)
+    return type(norm) is RMSNorm and _plain_weights(norm.weight, width)
 
 
 def _plain_attention(m) -> bool:
@@ -40,6 +46,7 @@ def _plain_attention(m) -> bool:
             and m.window is None and not m.chunk and not m.keep_first and m.softcap is None and m.sink is None
             and not m.head_gate and not m.beside and not m.shares_kv and not m.values_are_keys
             and not m.conv_path and m.q_temp is None
+            and all(w is None if m.qk_norm_eps is None else _plain_weights(w, HEAD) for w in (m.q_norm_w, m.k_norm_w))
             and _plain_linear(m.qkv, (m.nq + 2 * m.nkv) * HEAD, m.hidden) and _plain_linear(m.o, m.hidden, m.nq * HEAD))
 
 

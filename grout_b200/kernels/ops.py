@@ -1847,9 +1847,7 @@ def decode_stack_state(layers, hidden: int, ff: int, nq: int, nkv: int, max_rows
     host = torch.zeros(size * len(layers) + 64, dtype=torch.uint8)
     skip = -host.data_ptr() % 64                 # tensor maps lie on 64 bytes
     encode = _fn("decode_stack", "gb_decode_stack_encode", "piiiiippppppl")
-    words = _fn("decode_stack", "gb_decode_stack_row_words", "i")(hidden)
-    # a layer's row: its norms' weights, which launches fill in, and where its pages and its norms are
-    rows = torch.ones((len(layers), words), dtype=torch.float32)
+    rows = torch.zeros((len(layers), 16), dtype=torch.int32)       # StackRow: where a layer's pages and norms are
     normed = layers[0]["q_norm"] is not None
     for i, t in enumerate(layers):
         for n, shape in (("qkv", ((nq + 2 * nkv) * 128, hidden)), ("o", (hidden, nq * 128)),
@@ -1867,25 +1865,33 @@ def decode_stack_state(layers, hidden: int, ff: int, nq: int, nkv: int, max_rows
                 _need(t[n], n, ndim=1)
                 if t[n].shape[0] != width or t[n].dtype not in (torch.float32, torch.bfloat16):
                     raise KernelError(f"{n} is {t[n].dtype} of {t[n].shape[0]} elements, expected {width} in 32-bit or bfloat16")
+                if t[n].data_ptr() % 16:
+                    raise KernelError(f"{n} does not lie on 16 bytes")
                 where.append(t[n].data_ptr())
                 narrow.append(int(t[n].dtype == torch.bfloat16))
             elif t[n] is not None:
                 raise KernelError("either all layers have norms of q and k or none has")
-        bits = rows.view(torch.int32)[i, 2 * hidden + 256:]
-        bits[:2 * len(where)] = torch.tensor(where, dtype=torch.int64).view(torch.int32)
-        bits[12:12 + len(narrow)] = torch.tensor(narrow, dtype=torch.int32)
+        rows[i, :2 * len(where)] = torch.tensor(where, dtype=torch.int64).view(torch.int32)
+        rows[i, 12:12 + len(narrow)] = torch.tensor(narrow, dtype=torch.int32)
         _check(encode(host.data_ptr() + skip + i * size, hidden, ff, nq, nkv, P, t["qkv"].data_ptr(), t["o"].data_ptr(),
                       t["gate_up"].data_ptr(), t["down"].data_ptr(), t["k_pages"].data_ptr(), t["v_pages"].data_ptr(),
                       t["k_pages"].shape[0]),
                "decode_stack_encode", 0)
-    f32 = lambda n: torch.zeros(n, dtype=torch.float32, device=device)
-    b16 = lambda n: torch.zeros(n, dtype=torch.bfloat16, device=device)
-    T, splits = max_rows, 32
-    return dict(sizes=(len(layers), hidden, ff, nq, nkv), rows=T, blocks=P,
-                layers=host[skip:skip + size * len(layers)].to(device), table=rows.to(device), qk_norm=int(normed),
-                xb=b16(T * hidden), ab=b16(T * nq * 128), hb=b16(T * ff), ss=f32(T * P), qkv=f32(T * (nq + 2 * nkv) * 128),
-                part_o=f32(T * nq * splits * 128), part_ml=f32(T * nq * splits * 2),
-                sync=torch.zeros(2, dtype=torch.int32, device=device))
+    # All in one piece, what is read most often side by side: laid wherever there was room, a step of one row of the 4B
+    # sizes took 1,819 to 1,834 us from one state to the next.
+    T, splits, f32, b16 = max_rows, 32, torch.float32, torch.bfloat16
+    pieces = dict(sync=(2, torch.int32), table=(rows.numel(), torch.int32), layers=(size * len(layers), torch.uint8),
+                  xb=(T * hidden, b16), ab=(T * nq * 128, b16), hb=(T * ff, b16), ss=(T * P, f32), qkv=(T * (nq + 2 * nkv) * 128, f32),
+                  part_ml=(T * nq * splits * 2, f32), part_o=(T * nq * splits * 128, f32))
+    at, places = 0, {}
+    for name, (n, dtype) in pieces.items():
+        places[name] = at
+        at += -(-n * dtype.itemsize // 1024) * 1024
+    whole = torch.zeros(at, dtype=torch.uint8, device=device)
+    state = {name: whole[places[name]:places[name] + n * dtype.itemsize].view(dtype) for name, (n, dtype) in pieces.items()}
+    state["table"].copy_(rows.view(-1))
+    state["layers"].copy_(host[skip:skip + size * len(layers)])
+    return dict(state, sizes=(len(layers), hidden, ff, nq, nkv), rows=T, blocks=P, qk_norm=int(normed))
 
 
 def _cost_decode_stack(out, state, res, pending, *, kv_len, slots, **kw):
