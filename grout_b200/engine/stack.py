@@ -4,7 +4,8 @@ The kernel runs a plain pre-norm decoder layer: RMS norms, grouped-query attenti
 paged cache with 128-wide heads (with or without the heads' norms, the whole head rotated), a
 gated SiLU feed-forward, bfloat16 weights.  ``stack_layers`` says whether a model is that, layer
 by layer and attribute by attribute; anything else (a window, a cap, a bias, a part of the
-caller's own, 32-bit weights, another product kernel asked for) goes layer by layer as before."""
+caller's own, 32-bit weights, another product kernel or a decode attention asked for) goes layer
+by layer as before."""
 from __future__ import annotations
 
 import weakref
@@ -155,6 +156,8 @@ class StackOf:
     def get(self, model, cache) -> Optional[DecodeStack]:
         if model.ctx.dtype != torch.bfloat16 or not model.blocks or type(model.blocks[0]) is not PreNormBlock:
             return None                  # (nothing to look up in every step of another kind of model)
+        if ops.DECODE_ATTENTION != "auto" or ops.DECODE_SPLITS_OVERRIDE or ops.DECODE_TMA_STAGES:
+            return None                  # (a kernel, or its division of the keys, is asked for)
         made_from = _weights_of(model)
         if self._cache is None or self._cache() is not cache or made_from != self._made_from:
             self._stack = DecodeStack.of(model, cache)

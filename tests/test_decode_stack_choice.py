@@ -10,6 +10,7 @@ from grout_b200.config import resolve_architecture
 from grout_b200.engine import stack
 from grout_b200.engine.graphs import StepGraph
 from grout_b200.engine.model import Model
+from grout_b200.kernels import ops
 from grout_b200.parts.base import BuildContext
 from grout_b200.weights import random_tensor
 
@@ -69,3 +70,12 @@ def test_weights_made_in_inference_mode(model):
         for config in (CONFIG, dict(CONFIG, head_dim=64)):
             m, cache = load(config), Cache()
             assert isinstance(m.decode_stack(cache), Made) and m.decode_stack(cache) is m.decode_stack(cache)
+
+
+@pytest.mark.parametrize("name,value", [("DECODE_ATTENTION", "tma"), ("DECODE_ATTENTION", "mma"),
+                                        ("DECODE_SPLITS_OVERRIDE", 4), ("DECODE_TMA_STAGES", 3)])
+def test_a_decode_attention_that_is_asked_for_is_taken(model, monkeypatch, name, value):
+    cache = Cache()
+    assert model.decode_stack(cache) is not None
+    monkeypatch.setattr(ops, name, value)
+    assert model.decode_stack(cache) is None
