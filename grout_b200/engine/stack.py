@@ -24,8 +24,19 @@ from ..parts.position import RotaryHalfSplit
 HEAD = 128
 
 
+#: What the kernel does in place of these; where one has been replaced (to look at what a layer does, for instance),
+#: in its class or on one object, layers run one by one.
+_DONE = {PreNormBlock: ("forward",), GQAAttention: ("forward", "_attend"), SwiGLU: ("forward",),
+         RMSNorm: ("add_norm", "forward"), RotaryHalfSplit: ("rotary",), Linear: ("__call__", "silu_mul")}
+_METHODS = tuple((cls, name, getattr(cls, name)) for cls, names in _DONE.items() for name in names)
+
+
+def _as_it_is(x) -> bool:
+    return vars(x).keys().isdisjoint(_DONE[type(x)])
+
+
 def _plain_linear(lin, out_features: int, in_features: int) -> bool:
-    return (type(lin) is Linear and lin.weight.dtype == torch.bfloat16 and lin.decode_kernel == "tc"
+    return (type(lin) is Linear and _as_it_is(lin) and lin.weight.dtype == torch.bfloat16 and lin.decode_kernel == "tc"
             and lin.weight.is_contiguous() and tuple(lin.weight.shape) == (out_features, in_features)
             and lin.weight.data_ptr() % 16 == 0)
 
@@ -37,22 +48,29 @@ def _plain_weights(w, width: int) -> bool:
 
 
 def _plain_norm(norm, width: int) -> bool:
-    return type(norm) is RMSNorm and _plain_weights(norm.weight, width)
+    return type(norm) is RMSNorm and _as_it_is(norm) and _plain_weights(norm.weight, width)
+
+
+def _plain_rotation(position) -> bool:
+    if type(position) is not RotaryHalfSplit or not _as_it_is(position):
+        return False
+    rot = position.rotary()
+    return (rot.rot_dim == HEAD and not rot.interleaved and rot.amplitude == 1.0 and rot.inv_freq.is_contiguous()
+            and rot.inv_freq.dtype == torch.float32)
 
 
 def _plain_attention(m) -> bool:
-    rot = m.position.rotary() if type(m) is GQAAttention else None
-    return (type(m) is GQAAttention and m.D == m.Dv == m.Ds == HEAD and type(m.position) is RotaryHalfSplit
-            and rot is not None and rot.rot_dim == HEAD and not rot.interleaved and rot.amplitude == 1.0
+    return (type(m) is GQAAttention and _as_it_is(m) and m.D == m.Dv == m.Ds == HEAD and _plain_rotation(m.position)
             and m.window is None and not m.chunk and not m.keep_first and m.softcap is None and m.sink is None
             and not m.head_gate and not m.beside and not m.shares_kv and not m.values_are_keys
-            and not m.conv_path and m.q_temp is None
+            and not m.conv_path and m.taps == 1 and m.q_temp is None
             and all(w is None if m.qk_norm_eps is None else _plain_weights(w, HEAD) for w in (m.q_norm_w, m.k_norm_w))
             and _plain_linear(m.qkv, (m.nq + 2 * m.nkv) * HEAD, m.hidden) and _plain_linear(m.o, m.hidden, m.nq * HEAD))
 
 
 def _plain_layer(block) -> bool:
-    if type(block) is not PreNormBlock or type(block.feedforward) is not SwiGLU or not _plain_attention(block.mixer):
+    if (type(block) is not PreNormBlock or not _as_it_is(block) or type(block.feedforward) is not SwiGLU
+            or not _as_it_is(block.feedforward) or not _plain_attention(block.mixer)):
         return False
     m, f = block.mixer, block.feedforward
     return (f.interleave == 8 and f.hidden == m.hidden and _plain_linear(f.gate_up, 2 * f.intermediate, f.hidden)
@@ -67,22 +85,31 @@ def _sizes(block):
 
 
 def stack_layers(model) -> Optional[List]:
-    """The model's blocks in the order they run when the kernel can run all of them, else None."""
-    plan = model.plan
-    if model.ctx.dtype != torch.bfloat16 or not plan.schedule:
+    """The model's blocks in the order they run when the kernel can run all of them, else None (as soon as one is found
+    that it cannot: every decode step that is not replayed asks)."""
+    if model.ctx.dtype != torch.bfloat16 or any(getattr(cls, name) is not f for cls, name, f in _METHODS):
         return None
-    if any(e.cache_of is not None or e.add is not None or e.average is not None for e in plan.schedule):
-        return None
-    blocks = [model.blocks[e.layer] for e in plan.schedule]
-    if not all(_plain_layer(b) for b in blocks) or len({_sizes(b) for b in blocks}) != 1:
-        return None
-    first = blocks[0]
-    if first.norm1.eps != first.norm2.eps:
-        return None
-    freq = first.mixer.position.rotary().inv_freq
-    if not all(torch.equal(b.mixer.position.rotary().inv_freq, freq) for b in blocks[1:]):
-        return None
-    return blocks
+    blocks = []
+    for e in model.plan.schedule:
+        block = model.blocks[e.layer]
+        if (e.cache_of is not None or e.add is not None or e.average is not None or not _plain_layer(block)
+                or (blocks and _sizes(block) != _sizes(blocks[0]))):
+            return None
+        blocks.append(block)
+    return blocks if blocks and blocks[0].norm1.eps == blocks[0].norm2.eps else None
+
+
+def _made_from(blocks) -> tuple:
+    """What a ``DecodeStack`` takes from the layers: their sizes and constants, where the weights lie, which the kernel
+    reads there at every launch, and the rotations' tables, of which it reads the first layer's."""
+    out = [_sizes(blocks[0])]
+    for b in blocks:
+        m, f, freq = b.mixer, b.feedforward, b.mixer.position.rotary().inv_freq
+        out.append(tuple(lin.weight.data_ptr() for lin in (m.qkv, m.o, f.gate_up, f.down)))
+        out.append(tuple((w.data_ptr(), w.dtype) for w in (b.norm1.weight, b.norm2.weight, m.q_norm_w, m.k_norm_w)
+                         if w is not None))
+        out.append((freq.data_ptr(), 0 if freq.is_inference() else freq._version))
+    return tuple(out)
 
 
 class DecodeStack:
@@ -103,14 +130,11 @@ class DecodeStack:
         self.block_table = views[0].block_table
         self.state = ops.decode_stack_state(self._layers, hidden, ff, nq, nkv, max_rows, device)
         self.args = dict(eps=eps, qk_eps=qk_eps or 0.0, scale=scale,
-                         inv_freq=blocks[0].mixer.position.rotary().inv_freq.contiguous())
+                         inv_freq=blocks[0].mixer.position.rotary().inv_freq)
 
     @classmethod
-    def of(cls, model, cache) -> Optional["DecodeStack"]:
-        """None when the model is not one that the kernel runs, or its sizes have no plan."""
-        blocks = stack_layers(model)
-        if blocks is None:
-            return None
+    def of(cls, blocks, cache) -> Optional["DecodeStack"]:
+        """None when the cache is not one that the kernel reads, the layers rotate differently or their sizes have no plan."""
         views = [cache.view(i) for i in range(len(blocks))]
         table = views[0].block_table
         for b, v in zip(blocks, views):
@@ -118,6 +142,9 @@ class DecodeStack:
                     or tuple(v.k_pages.shape[1:]) != (b.mixer.nkv, 64, HEAD) or v.v_pages.shape != v.k_pages.shape
                     or v.k_pages.data_ptr() == v.v_pages.data_ptr()):
                 return None
+        freq = blocks[0].mixer.position.rotary().inv_freq
+        if not all(torch.equal(b.mixer.position.rotary().inv_freq, freq) for b in blocks[1:]):
+            return None
         hidden, ff, nq, nkv = _sizes(blocks[0])[:4]
         if not ops.decode_stack_takes(hidden, ff, nq, nkv, table.device):
             return None
@@ -132,34 +159,24 @@ class DecodeStack:
                                 block_table=self.block_table, **self.args)
 
 
-def _weights_of(model) -> tuple:
-    """What a ``DecodeStack`` was made from: where the weights lie, which the kernel reads there at every launch."""
-    out = []
-    for b in model.blocks:
-        for lin in (getattr(getattr(b, "mixer", None), "qkv", None), getattr(getattr(b, "mixer", None), "o", None),
-                    getattr(getattr(b, "feedforward", None), "gate_up", None),
-                    getattr(getattr(b, "feedforward", None), "down", None)):
-            out.append(lin.weight.data_ptr() if type(lin) is Linear else id(lin))
-        for w in (getattr(getattr(b, "norm1", None), "weight", None), getattr(getattr(b, "norm2", None), "weight", None),
-                  getattr(getattr(b, "mixer", None), "q_norm_w", None), getattr(getattr(b, "mixer", None), "k_norm_w", None)):
-            out.append((w.data_ptr(), w.dtype) if isinstance(w, torch.Tensor) else id(w))
-    return tuple(out)
-
-
 class StackOf:
-    """A model's ``DecodeStack``, made for the cache that its steps use, and made anew for another cache or other weights
-    (steps that are replayed from a captured graph do not come here: they read what was there at the capture)."""
+    """A model's ``DecodeStack``, made for the cache that its steps use, and made anew for another cache or when what it
+    takes from the layers has changed (steps that are replayed from a captured graph do not come here: they run what was
+    there at the capture)."""
 
     def __init__(self):
         self._cache, self._made_from, self._stack = None, None, None
 
     def get(self, model, cache) -> Optional[DecodeStack]:
-        if model.ctx.dtype != torch.bfloat16 or not model.blocks or type(model.blocks[0]) is not PreNormBlock:
-            return None                  # (nothing to look up in every step of another kind of model)
         if ops.DECODE_ATTENTION != "auto" or ops.DECODE_SPLITS_OVERRIDE or ops.DECODE_TMA_STAGES:
             return None                  # (a kernel, or its division of the keys, is asked for)
-        made_from = _weights_of(model)
+        blocks = stack_layers(model)
+        if blocks is None:
+            return None
+        made_from = _made_from(blocks)
         if self._cache is None or self._cache() is not cache or made_from != self._made_from:
-            self._stack = DecodeStack.of(model, cache)
+            if torch.cuda.is_available() and torch.cuda.is_current_stream_capturing():
+                return None              # (it takes copies and comparisons that the host waits for)
+            self._stack = DecodeStack.of(blocks, cache)
             self._cache, self._made_from = weakref.ref(cache), made_from
         return self._stack

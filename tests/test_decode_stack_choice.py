@@ -38,7 +38,7 @@ def load(config=CONFIG, dtype=torch.bfloat16):
 
 @pytest.fixture
 def model(monkeypatch):
-    monkeypatch.setattr(stack.DecodeStack, "of", classmethod(lambda cls, model, cache: Made()))
+    monkeypatch.setattr(stack.DecodeStack, "of", classmethod(lambda cls, *args: Made()))
     return load()
 
 
@@ -67,9 +67,9 @@ def test_a_captured_step_keeps_what_it_was_captured_with(model):
 def test_weights_made_in_inference_mode(model):
     """They have no version counter; a model that the kernel does not take is asked about like any other."""
     with torch.inference_mode():
-        for config in (CONFIG, dict(CONFIG, head_dim=64)):
-            m, cache = load(config), Cache()
-            assert isinstance(m.decode_stack(cache), Made) and m.decode_stack(cache) is m.decode_stack(cache)
+        m, cache = load(), Cache()
+        assert isinstance(m.decode_stack(cache), Made) and m.decode_stack(cache) is m.decode_stack(cache)
+        assert load(dict(CONFIG, head_dim=64)).decode_stack(cache) is None
 
 
 @pytest.mark.parametrize("name,value", [("DECODE_ATTENTION", "tma"), ("DECODE_ATTENTION", "mma"),
@@ -78,4 +78,46 @@ def test_a_decode_attention_that_is_asked_for_is_taken(model, monkeypatch, name,
     cache = Cache()
     assert model.decode_stack(cache) is not None
     monkeypatch.setattr(ops, name, value)
+    assert model.decode_stack(cache) is None
+
+
+CHANGES = {
+    "a window": lambda b: setattr(b.mixer, "window", 64),
+    "a softcap": lambda b: setattr(b.mixer, "softcap", 30.0),
+    "a query temperature": lambda b: setattr(b.mixer, "q_temp", (0.1, 64)),
+    "a scale": lambda b: setattr(b.mixer, "scale", 0.5),
+    "an epsilon": lambda b: setattr(b.norm2, "eps", 1e-3),
+    "another product kernel": lambda b: setattr(b.feedforward.down, "decode_kernel", "skinny"),
+    "a weight that is not contiguous": lambda b: setattr(b.mixer.o, "weight", b.mixer.o.weight.t().contiguous().t()),
+    "a norm at an odd place": lambda b: setattr(b.norm1, "weight", torch.ones(257, dtype=torch.bfloat16)[1:]),
+    "a mixer that is looked at": lambda b: setattr(b.mixer, "forward", lambda *a: type(b.mixer).forward(b.mixer, *a)),
+    "a product that is looked at": lambda b: setattr(b.feedforward.gate_up, "silu_mul", lambda *a: None),
+}
+
+
+@pytest.mark.parametrize("change", CHANGES)
+def test_layers_that_change_after_the_first_step_run_one_by_one(model, change):
+    """A step that is not replayed reads what the layers are then, as it does without the kernel."""
+    cache = Cache()
+    assert model.decode_stack(cache) is not None
+    CHANGES[change](model.blocks[1])
+    assert model.decode_stack(cache) is None
+
+
+def test_what_all_layers_share_may_change(model):
+    cache = Cache()
+    a = model.decode_stack(cache)
+    for b in model.blocks:
+        b.mixer.scale = 0.5
+    b = model.decode_stack(cache)
+    assert b is not None and b is not a and model.decode_stack(cache) is b
+    model.blocks[0].mixer.position.rotary().inv_freq.mul_(0.5)       # (what it is is compared when the state is made)
+    assert model.decode_stack(cache) is not b
+
+
+def test_a_class_whose_method_is_replaced(model, monkeypatch):
+    cache, mixer = Cache(), type(model.blocks[0].mixer)
+    assert model.decode_stack(cache) is not None
+    was = mixer.forward
+    monkeypatch.setattr(mixer, "forward", lambda self, *a: was(self, *a))
     assert model.decode_stack(cache) is None
