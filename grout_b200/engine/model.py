@@ -72,6 +72,7 @@ class Model:
 
     def load(self, get: Callable[[str], torch.Tensor]) -> None:
         """``get(name)`` returns the placed tensor; each part takes its own."""
+        self._stack.clear()
         for prefix, part in self._named_parts():
             specs = part.param_specs()
             if specs:

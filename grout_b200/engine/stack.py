@@ -160,12 +160,16 @@ class DecodeStack:
 
 
 class StackOf:
-    """A model's ``DecodeStack``, made for the cache that its steps use, and made anew for another cache or when what it
-    takes from the layers has changed (steps that are replayed from a captured graph do not come here: they run what was
-    there at the capture)."""
+    """A model's ``DecodeStack``s, one for each cache that its steps use, made anew when what they take from the layers has
+    changed (steps that are replayed from a captured graph do not come here: they run what was there at the capture).
+    They hold the caches' pages, so they go with their caches."""
 
     def __init__(self):
-        self._cache, self._made_from, self._stack = None, None, None
+        self._stacks = weakref.WeakKeyDictionary()       # cache -> (what it was made from, stack)
+
+    def clear(self) -> None:
+        """Lets go of the weights and pages that the stacks hold."""
+        self._stacks.clear()
 
     def get(self, model, cache) -> Optional[DecodeStack]:
         if ops.DECODE_ATTENTION != "auto" or ops.DECODE_SPLITS_OVERRIDE or ops.DECODE_TMA_STAGES:
@@ -174,9 +178,11 @@ class StackOf:
         if blocks is None:
             return None
         made_from = _made_from(blocks)
-        if self._cache is None or self._cache() is not cache or made_from != self._made_from:
+        known, stack = self._stacks.get(cache, (None, None))
+        if known != made_from:
             if torch.cuda.is_available() and torch.cuda.is_current_stream_capturing():
                 return None              # (it takes copies and comparisons that the host waits for)
-            self._stack = DecodeStack.of(blocks, cache)
-            self._cache, self._made_from = weakref.ref(cache), made_from
-        return self._stack
+            self._stacks.pop(cache, None)
+            stack = DecodeStack.of(blocks, cache)
+            self._stacks[cache] = (made_from, stack)
+        return stack

@@ -121,3 +121,32 @@ def test_a_class_whose_method_is_replaced(model, monkeypatch):
     was = mixer.forward
     monkeypatch.setattr(mixer, "forward", lambda self, *a: was(self, *a))
     assert model.decode_stack(cache) is None
+
+
+def test_a_stack_goes_with_its_cache(monkeypatch):
+    """It holds the cache's pages; and two engines over one model do not take turns at one stack."""
+    def made(cls, blocks, cache):
+        out = Made()
+        out.pages = cache.pages
+        return out
+    monkeypatch.setattr(stack.DecodeStack, "of", classmethod(made))
+    model, caches = load(), [Cache(), Cache()]
+    for c in caches:
+        c.pages = Made()
+    stacks = [model.decode_stack(c) for c in caches]
+    assert stacks[0] is not stacks[1] and [model.decode_stack(c) for c in caches] == stacks
+    pages = weakref.ref(caches[0].pages)
+    del stacks, c
+    caches.pop(0)
+    gc.collect()
+    assert pages() is None
+
+
+def test_other_tensors_are_loaded(model):
+    """The tensors that were there before are not kept until the next step."""
+    cache = Cache()
+    held = weakref.ref(model.decode_stack(cache))
+    expected = model.expected()
+    model.load(lambda name: random_tensor(name, expected[name], 2, torch.bfloat16, torch.device("cpu")))
+    gc.collect()
+    assert held() is None
