@@ -143,7 +143,7 @@ class Model:
             res, pending = pending, None
         stack = self.decode_stack(cache) if step.decode else None
         entries = self.plan.schedule
-        if stack is not None and stack.takes(step):
+        if stack is not None and stack.takes(step) and stack.reads(res, pending):
             res, pending, entries = stack.forward(res, pending, step), None, ()
         for i, e in enumerate(entries):
             owner = i if e.cache_of is None else e.cache_of

@@ -153,6 +153,14 @@ class DecodeStack:
     def takes(self, step) -> bool:
         return step.decode and 0 < step.n_tokens <= self.max_rows and step.n_seqs == step.n_tokens
 
+    def reads(self, res, pending) -> bool:
+        """Whether the kernel reads what stands in front of the layers: the 32-bit stream or its first contribution in
+        bfloat16, as this library's embeddings leave it (a caller's own may leave something else)."""
+        x = pending if res is None else res
+        return ((res is None or pending is None) and isinstance(x, torch.Tensor) and x.dim() == 2
+                and x.shape[1] == self.hidden and x.is_contiguous()
+                and x.dtype == (torch.bfloat16 if res is None else torch.float32))
+
     def forward(self, res, pending, step) -> torch.Tensor:
         """The 32-bit stream behind the last layer, [T, hidden]."""
         return ops.decode_stack(self.state, res, pending, slots=step.slots, kv_len=step.kv_len,

@@ -150,3 +150,16 @@ def test_other_tensors_are_loaded(model):
     model.load(lambda name: random_tensor(name, expected[name], 2, torch.bfloat16, torch.device("cpu")))
     gc.collect()
     assert held() is None
+
+
+def test_what_stands_in_front_of_the_layers(monkeypatch):
+    """A caller's own embedding may leave partial sums, a wider type or a ``Contribution``; the norms take them all."""
+    from grout_b200.parts.norm import Contribution
+    monkeypatch.setattr(stack.ops, "decode_stack_state", lambda *args: None)
+    view = type("View", (), {"k_pages": None, "v_pages": None, "block_table": None})
+    st = stack.DecodeStack(load().blocks, [view] * 3)
+    narrow, wide = torch.zeros((2, 256), dtype=torch.bfloat16), torch.zeros((2, 256))
+    assert st.reads(None, narrow) and st.reads(wide, None)
+    for res, pending in ((None, wide), (narrow, None), (wide, narrow), (None, None), (None, wide[None].expand(3, 2, 256)),
+                         (None, Contribution(narrow)), (None, narrow.t().contiguous().t())):
+        assert not st.reads(res, pending)
