@@ -34,8 +34,8 @@
 // order.  Sums are 32-bit throughout.
 //
 // Every wait (a stage of the ring, the grid barrier) is bounded by wall-clock time; a block that
-// gives up records a code, lets its copies in flight land and leaves.  The launch is cooperative:
-// all blocks are resident or none.
+// gives up records a code and says so to the others, and each block lets its copies in flight land
+// and leaves.  The launch is cooperative: all blocks are resident or none.
 #include <stddef.h>
 
 #include "tc_common.cuh"
@@ -99,8 +99,9 @@ struct StackArgs {
   float* ss;                                 // [T, P] sums of squares
   float* qkv;                                // [T, (nq + 2 nkv) * 128]
   float *part_o, *part_ml;                   // [T, nq, DS_SPLITS_MOST, 128 | 2]
-  unsigned* sync;                            // [2]: arrivals, blocks that are done; zero between launches
+  unsigned* sync;                            // [3]: arrivals, blocks that are done, whether one gave up; zero between launches
   int* error;
+  unsigned long long wait_ns;                // the bound of a wait
   unsigned long long* stamps;                // optional [blocks][16] %globaltimer stamps of a layer's phases, or null
 };
 
@@ -264,17 +265,23 @@ struct StackRing {
 };
 
 // Waits, as a whole warp, until a counter of the block is beyond a value; false when a wait has given up.
-__device__ __forceinline__ bool stack_until(volatile int* count, int more_than, volatile int* abort_flag) {
+__device__ __forceinline__ bool stack_until(volatile int* count, int more_than, volatile int* abort_flag,
+                                            unsigned long long wait_ns) {
   if (__all_sync(0xffffffffu, *count > more_than)) return true;
   const unsigned long long t0 = now_ns();
 #pragma unroll 1
   for (int i = 1;; ++i) {
     if (__all_sync(0xffffffffu, *count > more_than)) return true;
-    if ((i & 63) == 0 && __any_sync(0xffffffffu, *abort_flag || now_ns() - t0 > TC_WAIT_LIMIT_NS)) return false;
+    if ((i & 63) == 0 && __any_sync(0xffffffffu, *abort_flag || now_ns() - t0 > wait_ns)) return false;
   }
 }
-__device__ __forceinline__ bool stack_issued(StackShared& sh, int stage) {
-  return stack_until(&sh.issued, stage, &sh.abort);
+
+// A wait of this block has given up: the launch's results are void, and the block and the others leave.  (The error flag
+// is the host's; another kernel's error, which it may hold from before, is no reason to leave.)
+__device__ __forceinline__ void stack_give_up(const StackArgs& a, StackShared& sh, int code) {
+  if (!*(volatile int*)&sh.abort) atomicCAS(a.error, 0, code);
+  *(volatile int*)&sh.abort = 1;
+  *(volatile unsigned*)(a.sync + 2) = 1;
 }
 
 struct StackConsumer {
@@ -289,20 +296,21 @@ struct StackConsumer {
   unsigned arrived;            // arrivals the grid barrier has had when all have come
 
   __device__ __forceinline__ void give_up(int code) {
-    if (lane == 0 && !*(volatile int*)&sh.abort) atomicCAS(a.error, 0, code);
-    *(volatile int*)&sh.abort = 1;
+    if (lane == 0) stack_give_up(a, sh, code);
     bad = true;
   }
   // (A slot's stage may be another four's than the one before it, which may not have landed yet: before a barrier is
   // asked about a stage, the stage has to be on its way, or the answer may be about the stage before the last.)
   __device__ __forceinline__ void wait_full(const StackRing& r) {
     if (bad) return;
-    if (!stack_issued(sh, (int)r.round * a.n_slots + r.slot) || !mbar_wait_warp(&sh.full[r.slot], r.round & 1, &sh.abort))
+    if (!stack_until(&sh.issued, (int)r.round * a.n_slots + r.slot, &sh.abort, a.wait_ns) ||
+        !mbar_wait_warp(&sh.full[r.slot], r.round & 1, &sh.abort, a.wait_ns))
       give_up(GB_ERR_STACK_STAGE);
   }
+  // (Not behind a wait that has given up: the stage may be on its way, and another must not be copied over it.)
   __device__ __forceinline__ void release(const StackRing& r) {
     __syncwarp();
-    if (lane == 0) mbar_arrive(&sh.empty[r.slot]);
+    if (lane == 0 && !bad) mbar_arrive(&sh.empty[r.slot]);
   }
   __device__ __forceinline__ void pass(int stages) {
     const int to = at.slot + stages, rounds = to / a.n_slots;
@@ -322,9 +330,8 @@ struct StackConsumer {
       const unsigned long long t0 = now_ns();
 #pragma unroll 1
       for (int i = 1; ds_load_acquire(a.sync) < arrived; ++i) {
-        if ((i & 255) == 0 && (now_ns() - t0 > TC_WAIT_LIMIT_NS || *(volatile int*)a.error)) {
-          atomicCAS(a.error, 0, GB_ERR_STACK_BARRIER);
-          *(volatile int*)&sh.abort = 1;
+        if ((i & 255) == 0 && (now_ns() - t0 > a.wait_ns || *(volatile unsigned*)(a.sync + 2))) {
+          stack_give_up(a, sh, GB_ERR_STACK_BARRIER);
           bad = true;
           break;
         }
@@ -864,9 +871,8 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
       bool ok = true;
       // the next stage's place, once it is free; its barrier expects `bytes`
       auto next_stage = [&](uint32_t bytes) -> uint8_t* {
-        if (at.round > 0 && !mbar_wait(&sh.empty[at.slot], (at.round & 1) ^ 1, &sh.abort)) {
-          if (!*(volatile int*)&sh.abort) atomicCAS(a.error, 0, GB_ERR_STACK_RING);
-          *(volatile int*)&sh.abort = 1;
+        if (at.round > 0 && !mbar_wait(&sh.empty[at.slot], (at.round & 1) ^ 1, &sh.abort, a.wait_ns)) {
+          stack_give_up(a, sh, GB_ERR_STACK_RING);
           ok = false;
           return nullptr;
         }
@@ -943,14 +949,6 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
           }
         }
       }
-      if (!ok) {
-        // let the copies that were issued land before the block leaves: each slot's last stage (bounded: where the
-        // activations never came, its barrier never completes)
-        for (int i = 0; i < a.n_slots; ++i) {
-          const int rounds = (int)at.round + (i < at.slot);
-          if (rounds > 0) mbar_wait(&sh.full[i], (rounds - 1) & 1, nullptr, 10000000ull);
-        }
-      }
     }
     __syncwarp();
   } else if (warp == DS_WARPS + 1) {
@@ -969,7 +967,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
         const unsigned long long t0 = now_ns();
 #pragma unroll 1
         for (int i = 1; (n = *count) <= more_than; ++i)
-          if ((i & 63) == 0 && (*(volatile int*)&sh.abort || now_ns() - t0 > TC_WAIT_LIMIT_NS)) {
+          if ((i & 63) == 0 && (*(volatile int*)&sh.abort || now_ns() - t0 > a.wait_ns)) {
             ok = false;
             break;
           }
@@ -1101,12 +1099,21 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_kernel(const __gri
     if (!ok) *(volatile int*)&sh.abort = 1;
   }
   __syncthreads();
-  // the last block to leave sets the counters back: nobody polls them any more
   if (tid == 0) {
+    if (sh.abort) {
+      // No warp asks for copies any more: let those that were asked for land before the block leaves, each slot's last
+      // stage (10 ms: where its activations were never asked for, its barrier does not complete).
+      const int rounds = sh.issued / a.n_slots, more = sh.issued - rounds * a.n_slots;
+#pragma unroll 1
+      for (int i = 0; i < a.n_slots; ++i) {
+        const int n = rounds + (i < more);
+        if (n > 0) mbar_wait(&sh.full[i], (n - 1) & 1, nullptr, 10000000ull);
+      }
+    }
+    // the last block to leave sets the counters back: nobody polls them any more
     __threadfence();
     if (atomicAdd(a.sync + 1, 1u) == (unsigned)P - 1) {
-      a.sync[0] = 0;
-      a.sync[1] = 0;
+      a.sync[0] = a.sync[1] = a.sync[2] = 0;
       __threadfence();
     }
   }
@@ -1237,6 +1244,7 @@ GB_EXPORT int gb_decode_stack(StackArgs* a, int P, cudaStream_t s) {
       !a->kv_len || !a->block_table || !a->xb || !a->ab || !a->hb || !a->ss || !a->qkv || !a->part_o || !a->part_ml ||
       !a->sync || !a->error)
     return GB_ERR_BAD_ARG;
+  if (!a->wait_ns) a->wait_ns = TC_WAIT_LIMIT_NS;
   a->slot_bytes = plan.slot_bytes, a->n_slots = plan.n_slots;
   a->act_at = plan.act_at, a->kb_qkv = plan.kb_qkv, a->kb_o = a->kb_down = plan.kb_o[a->T > DS_FEW];
   const size_t smem = 1024 + (size_t)plan.n_slots * plan.slot_bytes + DS_RED_BYTES + sizeof(StackShared);

@@ -1824,10 +1824,11 @@ class _StackArgs(ctypes.Structure):
                 ("qk_norm", _I), ("eps", _F), ("qk_eps", _F), ("scale_log2", _F), ("x_in", _P), ("res_in", _P), ("x_out", _P),
                 ("inv_freq", _P), ("slots", _P), ("kv_len", _P), ("block_table", _P), ("max_pages", _I),
                 ("xb", _P), ("ab", _P), ("hb", _P), ("ss", _P), ("qkv", _P), ("part_o", _P), ("part_ml", _P),
-                ("sync", _P), ("error", _P), ("stamps", _P)]
+                ("sync", _P), ("error", _P), ("wait_ns", ctypes.c_ulonglong), ("stamps", _P)]
 
 
 DECODE_STACK_ROWS = 8          # DS_ROWS
+DECODE_STACK_WAIT_NS = 0       # the bound of the kernel's waits (0: 2 s)
 DECODE_STACK_STAMPS = None     # int64 [blocks, 16]: times of the phases of a layer (tuning)
 
 
@@ -1880,7 +1881,7 @@ def decode_stack_state(layers, hidden: int, ff: int, nq: int, nkv: int, max_rows
     # All in one piece, what is read most often side by side: laid wherever there was room, a step of one row of the 4B
     # sizes took 1,819 to 1,834 us from one state to the next.
     T, splits, f32, b16 = max_rows, 32, torch.float32, torch.bfloat16
-    pieces = dict(sync=(2, torch.int32), table=(rows.numel(), torch.int32), layers=(size * len(layers), torch.uint8),
+    pieces = dict(sync=(3, torch.int32), table=(rows.numel(), torch.int32), layers=(size * len(layers), torch.uint8),
                   xb=(T * hidden, b16), ab=(T * nq * 128, b16), hb=(T * ff, b16), ss=(T * P, f32), qkv=(T * (nq + 2 * nkv) * 128, f32),
                   part_ml=(T * nq * splits * 2, f32), part_o=(T * nq * splits * 128, f32))
     at, places = 0, {}
@@ -1935,6 +1936,7 @@ def decode_stack(state: dict, res: Optional[torch.Tensor], pending: Optional[tor
     for name in ("xb", "ab", "hb", "ss", "qkv", "part_o", "part_ml", "sync"):
         setattr(a, name, state[name].data_ptr())
     a.error, a.stamps = _tc_error_flag(src.device).data_ptr(), _ptr(DECODE_STACK_STAMPS)
+    a.wait_ns = DECODE_STACK_WAIT_NS
     with torch.cuda.device(src.device):
         _check(_fn("decode_stack", "gb_decode_stack", "pip")(
             ctypes.addressof(a), state["blocks"], _stream()), "decode_stack")

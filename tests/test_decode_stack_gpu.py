@@ -213,3 +213,44 @@ def test_an_engine_made_in_inference_mode(engines, graphs):
     finally:
         eng.use_graphs = True
     assert torch.equal(got, want)
+
+
+def one_step(eng, n=300):
+    slot = eng.open_sequence()
+    eng.step([(slot, list(range(n)))], [[]])
+    out = eng.step([(slot, [7])], [[0]])
+    eng.close_sequence(slot)
+    return out
+
+
+def test_another_kernels_error_does_not_end_a_step(engines):
+    from grout_b200.kernels import ops
+    _d, eng = engines("group1")
+    want = one_step(eng)
+    flag = ops._tc_error_flag(torch.device("cuda:0"))
+    flag.fill_(101)
+    got = one_step(eng)
+    with pytest.raises(ops.KernelError):
+        eng.check()
+    assert torch.equal(got, want)
+
+
+def test_a_wait_that_runs_out_voids_the_step_and_not_the_next(engines, monkeypatch):
+    """With next to no time to wait, blocks give up on stages, on room in the ring and on one another: they leave, the
+    host is told, and the counters are as they were."""
+    from grout_b200.kernels import ops
+    _d, eng = engines("group1")
+    want = one_step(eng)
+    st = eng.model.decode_stack(eng.cache)
+    monkeypatch.setattr(ops, "DECODE_STACK_WAIT_NS", 1)
+    eng.use_graphs = False
+    try:
+        one_step(eng)
+    finally:
+        eng.use_graphs = True
+    with pytest.raises(ops.KernelError, match="layers' kernel"):
+        eng.check()
+    assert st.state["sync"].tolist() == [0, 0, 0]
+    monkeypatch.setattr(ops, "DECODE_STACK_WAIT_NS", 0)
+    assert torch.equal(one_step(eng), want)
+    eng.check()
