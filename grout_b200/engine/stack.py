@@ -23,6 +23,21 @@ from ..parts.position import RotaryHalfSplit
 
 HEAD = 128
 
+# Up to how many keys a step of so many (sequence, kv head) pairs goes to the kernel; (the most pairs, the most keys).
+# The kernel divides a pair's keys into units that are a block's whole work, one block an SM, so with many pairs a long
+# sequence among short ones is cut into few units and most blocks wait for its: with 16 kv heads one of 32,768 keys
+# beside seven of 100 is two units a head.  Measured on 148 SMs, captured steps, us a step by this kernel / layer by
+# layer, the worst of all ways to mix long sequences with short ones, at the sizes (hidden, kv heads, feed-forward,
+# layers) where layer by layer does best:
+#   up to 32 pairs    4 sequences of 39,000 keys (4096, 8, 12288, 12) 2,052 / 2,324; 1 of 4,000 (4096, 20, 12288, 8) 742 / 783
+#   up to 64 pairs    5 of 4,000 and 2 of 100 (4096, 9, 12288, 8) 833 / 832, 8 of 2,000 (4096, 8, 12288, 12) 1,140 / 1,175;
+#                     but 6 of 12,000 and 2 of 100 (the same) 1,588 / 1,572, 6 of 32,000 and 2 of 100 2,581 / 2,411
+#   up to 128 pairs   3 of 1,010 and 5 of 100 (4096, 12, 12288, 8) 751 / 753; but 2 of 2,000 and 6 of 100
+#                     (4096, 16, 12288, 8) 818 / 797, 2 of 32,000 and 6 of 100 2,923 / 2,019
+#   more              2 of 500 and 6 of 100 (4096, 20, 12288, 8) 770 / 773; but 1 of 1,010 and 7 of 100 807 / 802, 1 of
+#                     32,000 and 7 of 100 (3072, 24, 8192, 8) 2,767 / 1,087
+KEYS_MOST = ((32, None), (64, 4096), (128, 1024), (None, 512))
+
 
 #: What the kernel does in place of these; where one has been replaced (to look at what a layer does, for instance),
 #: in its class or on one object, layers run one by one.
@@ -120,7 +135,7 @@ class DecodeStack:
     def __init__(self, blocks, views, max_rows: int = ops.DECODE_STACK_ROWS):
         hidden, ff, nq, nkv, scale, qk_eps, eps, _eps = _sizes(blocks[0])
         device = blocks[0].mixer.qkv.weight.device
-        self.hidden, self.max_rows = hidden, max_rows
+        self.hidden, self.nkv, self.max_rows = hidden, nkv, max_rows
         self._layers = []                 # (the tensors that the device's table points at)
         for b, view in zip(blocks, views):
             m, f = b.mixer, b.feedforward
@@ -151,7 +166,11 @@ class DecodeStack:
         return cls(blocks, views)
 
     def takes(self, step) -> bool:
-        return step.decode and 0 < step.n_tokens <= self.max_rows and step.n_seqs == step.n_tokens
+        """Whether the step is one that the kernel runs, and runs faster: decided by what a captured step is bounded by."""
+        if not step.decode or not 0 < step.n_tokens <= self.max_rows or step.n_seqs != step.n_tokens:
+            return False
+        keys = next(keys for pairs, keys in KEYS_MOST if pairs is None or step.n_tokens * self.nkv <= pairs)
+        return keys is None or step.max_kv_len <= keys
 
     def reads(self, res, pending) -> bool:
         """Whether the kernel reads what stands in front of the layers: the 32-bit stream or its first contribution in

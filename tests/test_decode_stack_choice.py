@@ -152,14 +152,30 @@ def test_other_tensors_are_loaded(model):
     assert held() is None
 
 
+def bare_stack(monkeypatch, nkv=1):
+    monkeypatch.setattr(ops, "decode_stack_state", lambda *args: None)
+    view = type("View", (), {"k_pages": None, "v_pages": None, "block_table": None})
+    return stack.DecodeStack(load(dict(CONFIG, num_attention_heads=nkv, num_key_value_heads=nkv)).blocks, [view] * 3)
+
+
 def test_what_stands_in_front_of_the_layers(monkeypatch):
     """A caller's own embedding may leave partial sums, a wider type or a ``Contribution``; the norms take them all."""
     from grout_b200.parts.norm import Contribution
-    monkeypatch.setattr(stack.ops, "decode_stack_state", lambda *args: None)
-    view = type("View", (), {"k_pages": None, "v_pages": None, "block_table": None})
-    st = stack.DecodeStack(load().blocks, [view] * 3)
+    st = bare_stack(monkeypatch)
     narrow, wide = torch.zeros((2, 256), dtype=torch.bfloat16), torch.zeros((2, 256))
     assert st.reads(None, narrow) and st.reads(wide, None)
     for res, pending in ((None, wide), (narrow, None), (wide, narrow), (None, None), (None, wide[None].expand(3, 2, 256)),
                          (None, Contribution(narrow)), (None, narrow.t().contiguous().t())):
         assert not st.reads(res, pending)
+
+
+@pytest.mark.parametrize("nkv,rows,most", [(8, 1, 1 << 20), (8, 4, 1 << 20), (32, 1, 1 << 20), (8, 5, 4096), (8, 8, 4096),
+                                           (16, 4, 4096), (16, 5, 1024), (16, 8, 1024), (17, 8, 512), (32, 8, 512)])
+def test_as_many_keys_as_the_kernel_is_faster_with(monkeypatch, nkv, rows, most):
+    st = bare_stack(monkeypatch, nkv)
+    step = type("Step", (), dict(decode=True, n_tokens=rows, n_seqs=rows, max_kv_len=most))
+    assert st.takes(step)
+    step.max_kv_len = most + 1
+    assert st.takes(step) is (rows * nkv <= 32)
+    step.max_kv_len, step.decode = 1, False
+    assert not st.takes(step)
