@@ -254,3 +254,106 @@ def test_a_wait_that_runs_out_voids_the_step_and_not_the_next(engines, monkeypat
     monkeypatch.setattr(ops, "DECODE_STACK_WAIT_NS", 0)
     assert torch.equal(one_step(eng), want)
     eng.check()
+
+
+@pytest.fixture
+def launches(monkeypatch):
+    """The rows of every launch of the kernel (replays do not come here)."""
+    from grout_b200.kernels import ops
+    rows, run = [], ops.decode_stack
+
+    def counted(state, res, pending, **kw):
+        out = run(state, res, pending, **kw)
+        rows.append(out.shape[0])
+        return out
+    monkeypatch.setattr(ops, "decode_stack", counted)
+    return rows
+
+
+def test_the_kernel_is_what_runs(engines, launches):
+    _d, eng = engines("group4")
+    eng.graphs.decode_graphs.clear()
+    played(eng, [100, 900, 3], 2, 5)
+    assert launches == [4, 4]              # the warm-up and the capture of one bucket, whose second step is a replay
+    eng.use_graphs = False
+    try:
+        played(eng, [100, 900, 3], 2, 5)
+        assert launches == [4, 4, 3, 3]
+        played(eng, [9] * 9, 1, 5)
+        assert launches == [4, 4, 3, 3]    # nine rows go layer by layer
+    finally:
+        eng.use_graphs = True
+
+
+def test_a_replaced_weight_is_seen(engines, launches):
+    from safetensors import safe_open
+    d, eng = engines("group2")
+    with safe_open(f"{d}/model.safetensors", "pt") as f:
+        w = {k: f.get_tensor(k) for k in f.keys()}
+    lin = eng.model.blocks[0].mixer.o
+    before = lin.weight
+    eng.use_graphs = False
+    try:
+        lin.weight = before.flip(0).contiguous()
+        w["model.layers.0.self_attn.o_proj.weight"] = lin.weight.cpu()
+        toks, got = played(eng, [100], 2, 81)
+    finally:
+        lin.weight = before
+        eng.use_graphs = True
+    assert launches == [1, 1]
+    assert_close(got[0], plain.logits(w, MODELS["group2"], toks[0], rows=[100, 101]), "bfloat16", "another o projection")
+
+
+MODELS["many_kv"] = config(256, 1216, 32, 32)
+
+
+@pytest.mark.parametrize("lens", [[5, 500, 64, 127, 300], [1, 62, 190, 191, 192, 333, 508, 64]], ids=str)
+def test_two_units_of_attention_in_a_block(engines, launches, lens):
+    """More (sequence, kv head) pairs than blocks."""
+    from safetensors import safe_open
+    d, eng = engines("many_kv")
+    with safe_open(f"{d}/model.safetensors", "pt") as f:
+        w = {k: f.get_tensor(k) for k in f.keys()}
+    eng.use_graphs = False
+    try:
+        toks, got = played(eng, lens, 3, 13)
+    finally:
+        eng.use_graphs = True
+    assert launches[-3:] == [len(lens)] * 3          # (a prompt of one token is a decode step of its own)
+    for i, n in enumerate(lens):
+        want = plain.logits(w, MODELS["many_kv"], toks[i], rows=list(range(n, n + 3)))
+        assert_close(got[i], want, "bfloat16", f"{lens} sequence {i}")
+
+
+@pytest.mark.parametrize("nq,nkv,lens", [(8, 1, [6100]), (32, 32, [35000]), (16, 8, [33000, 20000, 34000, 200])], ids=str)
+def test_long_sequences(launches, nq, nkv, lens):
+    """The most splits of a head's keys (96 tiles in 32), more tiles in a block (137) than it keeps the pages of, and long
+    sequences beside a short one; keys and values are random.  Against the kernels of each layer, as above."""
+    from grout_b200.engine import Engine, stack
+    eng = Engine.random(dict(config(256, 1216, nq, nkv), max_position_embeddings=40960), 4, max_batch=4, max_seq_len=40960,
+                        max_tokens=sum(lens) + 64 * 8, use_graphs=False)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    for i in range(2):
+        view = eng.cache.view(i)
+        view.k_pages.normal_(generator=g)
+        view.v_pages.normal_(generator=g)
+    slots = [eng.open_sequence() for _ in lens]
+    for s, n in zip(slots, lens):
+        eng.cache.reserve(s, n + 1)
+        eng.cache.length[s] = n
+
+    def step():
+        out = eng.step([(s, [7 + s]) for s in slots], [[0]] * len(slots))
+        for s, n in zip(slots, lens):
+            eng.cache.length[s] = n
+        return out.double()
+
+    got = step()
+    assert launches == [len(lens)]
+    with pytest.MonkeyPatch.context() as m:
+        m.setattr(stack.DecodeStack, "takes", lambda self, step: False)
+        want = step()
+    eng.check()
+    assert launches == [len(lens)]
+    err = float((got - want).norm() / want.norm())
+    assert err < 0.02, err
